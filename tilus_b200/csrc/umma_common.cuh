@@ -11,6 +11,15 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// One elected lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: inside
+// a branch on elect.sync the compiler keeps them there, while inside `if (lane == 0)` it moves every
+// operand over for each instruction - measured 116 cycles per MMA whatever its shape, against 128 / 64 /
+// 32 / 16 / 9 cycles for 256 / 128 / 64 / 32 / 16 columns with the elected lane.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 // bounded wait (about a quarter of a second); also gives up as soon as another thread raised the abort flag
 __device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   uint64_t t0 = 0;

@@ -118,7 +118,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
 
   // tile t -> (split, n_tile, m_tile).  Inside a split the row tiles are taken in groups of MG: all
   // column tiles of one group (row tile fastest) before the next group, so that the CTAs running
@@ -451,7 +451,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
     }
   } else {
     // ================= MMA issuer =================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc<ACT>(TM);
       bool good = true;
       int ai = 0, tile_it = 0;

@@ -128,7 +128,7 @@ wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap tmap_a) {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = bars->tmem_base;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem_base, 0);
 
   // work item w -> (split, n_tile, m_tile), m fastest
 #define ITEM_COORDS(w)                                         \
@@ -417,7 +417,7 @@ wide_kernel(const WideParams p, const __grid_constant__ CUtensorMap tmap_a) {
     }
   } else {
     // ================= MMA issuer =================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = (umma_idesc<ACT>(256) & ~(31u << 24)) | ((uint32_t)(UM >> 4) << 24);  // M = UM, N = 256
       bool good = true;
       int bi = 0, it = 0;
