@@ -118,6 +118,31 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_native = None
+
+
+def native():
+    """The _native extension (csrc/native.cpp), bound to the library load() opened; raises if either has
+    not been built."""
+    global _native
+    if _native is None:
+        lib = load()
+        try:
+            from . import _native as ext
+        except ImportError as exc:
+            raise ImportError("tilus_b200/_native.so is missing or does not fit the installed torch: build it with "
+                              f"`python -m tilus_b200.build` ({exc})") from exc
+
+        def unsupported(M, N, K):
+            raise B200QError(ST_UNSUPPORTED, f"no kernel for M={M} N={N} K={K}")
+
+        addresses = [ctypes.cast(getattr(lib, "b200q_" + name), ctypes.c_void_p).value
+                     for name in ("gemm", "gemm_host", "gemm_swiglu_cast", "workspace_bytes")]
+        ext.bind(*addresses, check, unsupported)
+        _native = ext
+    return _native
+
+
 def check(status: int) -> None:
     if status != ST_OK:
         lib = load()

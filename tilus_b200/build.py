@@ -1,20 +1,23 @@
-"""Ahead-of-time build of libb200q.so (sm_100a only) with nvcc.
+"""Ahead-of-time build of libb200q.so (sm_100a only, nvcc) and of the _native extension (g++).
 
 The kernels are compiled here, in the source tree, not JIT-compiled at first use:
 `python -m tilus_b200.build` (or `__graft_entry__.build()`) leaves
-tilus_b200/libb200q.so next to the package.  nvcc cross-compiles without a GPU.
+tilus_b200/libb200q.so and tilus_b200/_native.so next to the package.  nvcc cross-compiles
+without a GPU.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_build")
 LIB = os.path.join(HERE, "libb200q.so")
+NATIVE = os.path.join(HERE, "_native.so")
 NPARTS = 8
 
 # Extra -D definitions for experiments (e.g. B200Q_EXTRA_DEFS="-DB200Q_GPW=2") and an
@@ -52,6 +55,26 @@ def _jobs():
     return jobs
 
 
+def build_native(force: bool = False) -> str:
+    """The host path of QuantizedLinear (csrc/native.cpp) as a CPython extension against the installed torch."""
+    src = os.path.join(CSRC, "native.cpp")
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= os.path.getmtime(src):
+        return NATIVE
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"), src, "-o", NATIVE,
+           "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for native.cpp:\n{r.stdout}\n{r.stderr}")
+    return NATIVE
+
+
 def _sources_mtime() -> float:
     paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
     paths.append(os.path.join(os.path.dirname(HERE), "include", "b200q.h"))
@@ -60,6 +83,7 @@ def _sources_mtime() -> float:
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
+    build_native(force)
     os.makedirs(OBJ, exist_ok=True)
     newest = _sources_mtime()
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= newest:

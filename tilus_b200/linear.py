@@ -19,6 +19,7 @@ import torch
 from torch import nn
 
 from . import ops, packing, quantize
+from ._lib import native
 from .dtypes import KIND_UINT, act_dtype, weight_dtype
 
 _TORCH_ACT = {"float16": torch.float16, "bfloat16": torch.bfloat16}
@@ -58,8 +59,8 @@ class QuantizedLinear(nn.Module):
             torch.empty(in_features // group_size, out_features, dtype=self.act_torch_dtype), requires_grad=False
         )
         self.register_buffer("layout_version", torch.tensor(packing.LAYOUT_VERSION, dtype=torch.int32))
-        self._ws_need = {}  # workspace bytes per batch size M (filled on first use)
-        self._host_calls = {}  # prepared b200q_gemm_host calls per (buffers, stream), see ops.linear_forward_host
+        # what every call of this layer has in common, in the order csrc/native.cpp takes it
+        self._call = (w_dtype.code, self.zero_point, group_size, in_features, out_features)
 
     # -- loading ---------------------------------------------------------------------
     def load_and_quantize(self, weight: torch.Tensor):
@@ -139,13 +140,11 @@ class QuantizedLinear(nn.Module):
                               self.zero_point)
 
     # -- compute ---------------------------------------------------------------------
+    # The checks, output and workspace tensors, stream lookup and library call of the three methods below
+    # are one native function each (csrc/native.cpp): a decode call takes the GPU 5..15 us.
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        x2 = x if x.dim() == 2 else x.reshape(-1, self.in_features)
-        if x2.shape[1] != self.in_features:
-            raise ValueError(f"expected {self.in_features} input features, got {x2.shape[1]}")
-        out = ops.linear_forward(x2, self.quantized_weight.data, self.scales.data, self.w_dtype.code, self.zero_point,
-                                 self.group_size, self.in_features, self.out_features, self._ws_need)
-        return out if x.dim() == 2 else out.reshape(*x.shape[:-1], self.out_features)
+        p = self._parameters
+        return native().linear(x, p["quantized_weight"], p["scales"], self._call)
 
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor | None = None) -> torch.Tensor:
         """forward() for activations kept in host memory: ``x_host`` [M, in_features] fp16 (pinned
@@ -154,36 +153,17 @@ class QuantizedLinear(nn.Module):
         library call (b200q_gemm_host); synchronise the stream before reading the result."""
         if out_host is None:
             out_host = torch.empty(x_host.shape[0], self.out_features, dtype=self.act_torch_dtype).pin_memory()
-        return ops.linear_forward_host(x_host, out_host, self.quantized_weight.data, self.scales.data,
-                                       self.w_dtype.code, self.zero_point, self.group_size, self.in_features,
-                                       self.out_features, self._ws_need, self._host_calls)
+        p = self._parameters
+        return native().linear_host(x_host, out_host, p["quantized_weight"], p["scales"], self._call)
 
     def forward_swiglu_cast(self, x: torch.Tensor, num_per_channels: int = 128, swiglu_clamp_value=None):
         """For a gate_up projection (out_features = 2 * hidden, gate columns first): this layer's GEMM
         followed by SwiGLU and the per-token FP8 cast, queued by one library call
         (b200q_gemm_swiglu_cast).  Returns (out float8_e4m3fn [M, hidden], out_sf float32
         [M, hidden / num_per_channels], gate_up [M, out_features])."""
-        from . import _lib
-
-        x2 = x if x.dim() == 2 else x.reshape(-1, self.in_features)
-        if not x2.is_cuda or x2.dtype != self.act_torch_dtype or x2.stride(1) != 1:
-            raise ValueError(f"activations must be CUDA {self.act_torch_dtype} with unit inner stride")
-        M, N, K = x2.shape[0], self.out_features, self.in_features
-        H = N // 2
-        dev = x2.device
-        gate_up = torch.empty(M, N, dtype=x2.dtype, device=dev)
-        out = torch.empty(M, H, dtype=torch.float8_e4m3fn, device=dev)
-        sf = torch.empty(M, H // num_per_channels, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            ws = ops.get_workspace(dev, ops.workspace_bytes(M, N, K, self.w_dtype, self.zero_point, self.group_size))
-            st = _lib.load().b200q_gemm_swiglu_cast(
-                x2.data_ptr(), x2.stride(0), self.quantized_weight.data_ptr(), self.scales.data_ptr(),
-                gate_up.data_ptr(), N, out.data_ptr(), H, sf.data_ptr(), M, N, K, self.w_dtype.code, self.zero_point,
-                self.group_size, ops.act_code(x2.dtype), num_per_channels, 0 if swiglu_clamp_value is None else 1,
-                0.0 if swiglu_clamp_value is None else float(swiglu_clamp_value), ws.data_ptr(), ws.numel(),
-                torch.cuda.current_stream(dev).cuda_stream)
-        _lib.check(st)
-        return out, sf, gate_up
+        p = self._parameters
+        return native().gate_up_cast(x, p["quantized_weight"], p["scales"], self._call, num_per_channels,
+                                     swiglu_clamp_value)
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, x_dtype={self.x_dtype.name}, "

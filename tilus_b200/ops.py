@@ -16,9 +16,6 @@ from . import _lib
 from .dtypes import weight_dtype
 from .packing import BLOCK_K, BLOCK_N
 
-_workspaces = {}
-
-
 def act_code(dtype: torch.dtype) -> int:
     """Activation dtype tag of the C ABI (B200Q_F16 / B200Q_BF16)."""
     if dtype == torch.float16:
@@ -41,14 +38,10 @@ def workspace_bytes(M: int, N: int, K: int, w_dtype, zero_point: int = 0, group_
 
 
 def get_workspace(device, nbytes: int) -> torch.Tensor:
-    """Per (device, stream) zero-initialised workspace, grown on demand.  The kernels
-    leave it zeroed, so it is cleared only when (re)allocated."""
-    key = (torch.device(device).index, _stream_ptr(device))
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    """Zero-initialised workspace of the device's current stream, grown on demand and shared with the
+    layers' own calls.  The kernels leave it zeroed, so it is cleared only when (re)allocated."""
+    index = torch.device(device).index
+    return _lib.native().workspace(torch.cuda.current_device() if index is None else index, nbytes)
 
 
 def plan(M: int, N: int, K: int, w_dtype, zero_point: int = 0, group_size: int = 128) -> dict:
@@ -98,121 +91,6 @@ def quantized_matmul(a: torch.Tensor, bq: torch.Tensor, scales: torch.Tensor, w_
             st = lib.b200q_gemm_planned(*args, ctypes.byref(pl))
     _lib.check(st)
     return out
-
-
-def linear_forward(x2: torch.Tensor, bq: torch.Tensor, scales: torch.Tensor, code: int, zero_point: int,
-                   group_size: int, K: int, N: int, ws_need: dict) -> torch.Tensor:
-    """The call QuantizedLinear.forward makes: same kernel launch as quantized_matmul, with the
-    layer's constants already validated at construction and the workspace size cached per M
-    (``ws_need``), so that a decode step spends its host time in the launch, not in checks."""
-    if not x2.is_cuda:
-        raise ValueError("QuantizedLinear needs CUDA tensors (there is no CPU path)")
-    if x2.dtype != scales.dtype or x2.stride(1) != 1:
-        raise TypeError(f"activations must be {scales.dtype} with unit inner stride")
-    act = act_code(x2.dtype)
-    lib = _lib.load()
-    M = x2.shape[0]
-    out = torch.empty(M, N, dtype=x2.dtype, device=x2.device)
-    if M == 0:
-        return out
-    dev = x2.device
-    need = ws_need.get(M)
-    if need is None:
-        need = lib.b200q_workspace_bytes(M, N, K, code, zero_point, group_size)
-        if need == 0:
-            raise _lib.B200QError(_lib.ST_UNSUPPORTED, f"no kernel for M={M} N={N} K={K}")
-        ws_need[M] = need
-    switch = torch.cuda.current_device() != dev.index
-    if switch:
-        prev = torch.cuda.current_device()
-        torch.cuda.set_device(dev)
-    try:
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        key = (dev.index, stream)
-        ws = _workspaces.get(key)
-        if ws is None or ws.numel() < need:
-            ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-            _workspaces[key] = ws
-        st = lib.b200q_gemm(x2.data_ptr(), x2.stride(0), bq.data_ptr(), scales.data_ptr(), out.data_ptr(), N, M, N, K,
-                            code, zero_point, group_size, act, ws.data_ptr(), ws.numel(), stream)
-    finally:
-        if switch:
-            torch.cuda.set_device(prev)
-    if st != 0:
-        _lib.check(st)
-    return out
-
-
-_host_staging: dict = {}
-
-
-def linear_forward_host(x_host: torch.Tensor, out_host: torch.Tensor, bq: torch.Tensor, scales: torch.Tensor,
-                        code: int, zero_point: int, group_size: int, K: int, N: int, ws_need: dict,
-                        prepared: dict) -> torch.Tensor:
-    """QuantizedLinear.forward_host: activations and result live in host memory (pinned, so that the
-    copies are asynchronous).  One library call queues copy-in, GEMM and copy-out on the current
-    stream of the layer's device; the caller synchronises that stream before reading ``out_host``."""
-    # A serving loop calls this with the same pinned buffers over and over: everything the checks
-    # below depend on is in the key, and a hit goes straight to the library call with the
-    # arguments prepared the first time (the checks and conversions cost more than the call).
-    dev = bq.device
-    stream = torch._C._cuda_getCurrentRawStream(dev.index)
-    key = (x_host.data_ptr(), out_host.data_ptr(), x_host.shape, x_host.stride(), out_host.stride(), x_host.dtype,
-           out_host.dtype, stream, bq.data_ptr(), scales.data_ptr())
-    hit = prepared.get(key)
-    if hit is not None:
-        if torch._C._cuda_getDevice() == dev.index:
-            st = hit[0](*hit[1])
-        else:
-            with torch.cuda.device(dev):
-                st = hit[0](*hit[1])
-        if st != 0:
-            _lib.check(st)
-        return out_host
-    if x_host.is_cuda or out_host.is_cuda:
-        raise ValueError("forward_host takes host tensors (use forward for device tensors)")
-    if x_host.dtype != scales.dtype or out_host.dtype != scales.dtype:
-        raise TypeError(f"activations and result must be {scales.dtype}")
-    act = act_code(x_host.dtype)
-    if x_host.dim() != 2 or x_host.stride(1) != 1 or x_host.shape[1] != K:
-        raise ValueError(f"x_host must be [M, {K}] with unit inner stride")
-    M = x_host.shape[0]
-    if out_host.dim() != 2 or out_host.stride(1) != 1 or tuple(out_host.shape) != (M, N):
-        raise ValueError(f"out_host must be [{M}, {N}] with unit inner stride")
-    if M == 0:
-        return out_host
-    lib = _lib.load()
-    need = ws_need.get(M)
-    if need is None:
-        need = lib.b200q_workspace_bytes(M, N, K, code, zero_point, group_size)
-        if need == 0:
-            raise _lib.B200QError(_lib.ST_UNSUPPORTED, f"no kernel for M={M} N={N} K={K}")
-        ws_need[M] = need
-    with torch.cuda.device(dev):
-        wkey = (dev.index, stream)
-        ws = _workspaces.get(wkey)
-        if ws is None or ws.numel() < need:
-            ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=dev)
-            _workspaces[wkey] = ws
-        # Decode batches (the kernel's own CTAs fetch the activations and consecutive calls overlap) keep
-        # staging buffers of their own, so that a call for a larger batch in between does not make the
-        # next decode call wait for it (the library only lets a call start early behind a call of its kind).
-        skey = wkey + (M <= 16,)
-        stage = _host_staging.get(skey)
-        if stage is None or stage[0].numel() < M * K or stage[1].numel() < M * N:
-            stage = (torch.empty(M * K, dtype=torch.int16, device=dev), torch.empty(M * N, dtype=torch.int16, device=dev))
-            _host_staging[skey] = stage
-        args = (x_host.data_ptr(), x_host.stride(0), bq.data_ptr(), scales.data_ptr(), out_host.data_ptr(),
-                out_host.stride(0), M, N, K, code, zero_point, group_size, act, stage[0].data_ptr(),
-                stage[1].data_ptr(), ws.data_ptr(), ws.numel(), stream)
-        st = lib.b200q_gemm_host(*args)
-    if st != 0:
-        _lib.check(st)
-    if len(prepared) > 256:  # a caller that keeps changing buffers: start over rather than grow
-        prepared.clear()
-    # the entry keeps the device buffers it names alive (a later, larger request replaces them in the pools)
-    prepared[key] = (lib.b200q_gemm_host, args, ws, stage)
-    return out_host
 
 
 def dequantize(bq: torch.Tensor, scales: torch.Tensor, w_dtype, group_size: int, zero_point: int = 0) -> torch.Tensor:
