@@ -70,10 +70,9 @@ class QuantizedLinear(nn.Module):
             raise ValueError("load_and_quantize is symmetric: use a signed or float weight type "
                              "(unsigned codes come in through load_codes / load_packed)")
         dev = self.quantized_weight.device
-        if dev.type == "cuda":  # one fused pass on the GPU: scales, codes, packing
-            packed, scales = quantize.quantize_and_pack(weight.to(dev), self.w_dtype, self.group_size,
-                                                        self.act_torch_dtype)
-            self.load_packed(packed, scales, layout="b200")
+        if dev.type == "cuda":  # on the GPU: scales, codes and packing, straight into the parameters
+            quantize.quantize_and_pack(weight.to(dev), self.w_dtype, self.group_size, self.act_torch_dtype,
+                                       out=(self.quantized_weight.data, self.scales.data))
             return
         codes, scales = quantize.quantize_weight(weight.to(dev), self.w_dtype, self.group_size, self.act_torch_dtype)
         self.load_codes(codes, scales)

@@ -67,10 +67,11 @@ def quantize_weight(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: tor
     return codes.view(in_f, out_f), scales.view(in_f // group_size, out_f)
 
 
-def quantize_and_pack(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: torch.dtype = torch.float16):
+def quantize_and_pack(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: torch.dtype = torch.float16,
+                      out: tuple | None = None):
     """weight[out, in] on a CUDA device (fp16, bf16 or fp32) -> (packed b200 bytes uint8[K*N*b/8],
-    scales x_dtype[K/group, N]) in one library call (two kernels): the same arithmetic as
-    quantize_weight followed by packing.interleave, bit for bit."""
+    scales x_dtype[K/group, N]) in one library call: the same arithmetic as quantize_weight followed
+    by packing.interleave, bit for bit.  ``out``: the two (contiguous) tensors to write."""
     from . import _lib
     from .ops import act_code
 
@@ -82,8 +83,11 @@ def quantize_and_pack(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: t
     wcode = {torch.float16: 0, torch.float32: 1, torch.bfloat16: 2}[weight.dtype]
     weight = weight.contiguous()
     out_f, in_f = weight.shape
-    bq = torch.empty(in_f * out_f * dt.nbits // 8, dtype=torch.uint8, device=weight.device)
-    scales = torch.empty(in_f // group_size, out_f, dtype=x_dtype, device=weight.device)
+    if out is None:
+        bq = torch.empty(in_f * out_f * dt.nbits // 8, dtype=torch.uint8, device=weight.device)
+        scales = torch.empty(in_f // group_size, out_f, dtype=x_dtype, device=weight.device)
+    else:
+        bq, scales = out
     with torch.cuda.device(weight.device):
         st = _lib.load().b200q_quantize(weight.data_ptr(), wcode, in_f,
                                         bq.data_ptr(), scales.data_ptr(), out_f, in_f, dt.code, group_size,
