@@ -315,3 +315,18 @@ def test_errors_are_loud():
     small_ws = torch.zeros(256, dtype=torch.uint8, device=dev)
     with pytest.raises(Exception):
         ops.quantized_matmul(prob["a"].to(dev), bq, prob["scales"].to(dev), D.uint4b, 128, 8, workspace=small_ws)
+
+
+@pytest.mark.parametrize("M", [17, 64, 65, 100, 128])
+@pytest.mark.parametrize("dt,zp,group", [(D.int8, 0, 64), (D.uint8, 128, 32), (D.float8_e5m2, 0, 64), (D.int7b, 0, 32),
+                                         (D.uint2b, 2, 128), (D.int5b, 0, 128)], ids=lambda x: getattr(x, "name", str(x)))
+def test_small_batch_kernel_ring_depths(M, dt, zp, group):
+    """The small-batch kernel where its packed-weight ring is shallowest (8-bit weights with several scale
+    rows per 128-row group next to many activation rows) and for swizzled and dense stages; a ragged last
+    column tile, runs that start and end inside tiles."""
+    prob = synth.make_problem(M, 1424, 1408, dt, group, seed=M)
+    prob["zero_point"] = zp
+    assert ops.plan(M, 1424, 1408, dt, zp, group)["kernel"] == 3
+    c, _, _ = _run(prob)
+    ref = qo.quantized_matmul(prob["a"].numpy(), prob["codes"].numpy(), prob["scales"].numpy(), dt, group, zp)
+    assert _rel_err(c, ref) <= REL_TOL

@@ -34,13 +34,12 @@ cudaError_t quantize_launch(const void* w, int w_dtype, int ldw, void* bq, void*
   cudaError_t umma_launch_part##i(int, const UmmaParams&, const void*, int, cudaStream_t);
 B200Q_DECL_UPART(0) B200Q_DECL_UPART(1) B200Q_DECL_UPART(2) B200Q_DECL_UPART(3)
 B200Q_DECL_UPART(4) B200Q_DECL_UPART(5) B200Q_DECL_UPART(6) B200Q_DECL_UPART(7)
-#define B200Q_DECL_WPART(i) \
-  cudaError_t wide_launch_part##i(int, const WideParams&, const void*, int, cudaStream_t);
-B200Q_DECL_WPART(0) B200Q_DECL_WPART(1) B200Q_DECL_WPART(2) B200Q_DECL_WPART(3)
-B200Q_DECL_WPART(4) B200Q_DECL_WPART(5) B200Q_DECL_WPART(6) B200Q_DECL_WPART(7)
-int wide_smem_bytes(int bits, int wg_stages, int a_rows, int rpg);
-int wide_wg_stages(int bits, int max_smem, int a_rows, int rpg);
-int wide_a_rows(int M);
+#define B200Q_DECL_BPART(i) \
+  cudaError_t batch_launch_part##i(int, const BatchParams&, const void*, int, cudaStream_t);
+B200Q_DECL_BPART(0) B200Q_DECL_BPART(1) B200Q_DECL_BPART(2) B200Q_DECL_BPART(3)
+B200Q_DECL_BPART(4) B200Q_DECL_BPART(5) B200Q_DECL_BPART(6) B200Q_DECL_BPART(7)
+int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg);
+void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages);
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg);
 int umma_a_stages(int tm, int bits, int max_smem, int rpg);
 
@@ -59,16 +58,16 @@ static cudaError_t stream_launch(int var, const StreamParams& p, int mt, int sme
   }
 }
 
-static cudaError_t wide_launch(int var, const WideParams& p, const void* tmap, int smem, cudaStream_t s) {
+static cudaError_t batch_launch(int var, const BatchParams& p, const void* tmap, int smem, cudaStream_t s) {
   switch (var % B200Q_NPARTS) {
-    case 0: return wide_launch_part0(var, p, tmap, smem, s);
-    case 1: return wide_launch_part1(var, p, tmap, smem, s);
-    case 2: return wide_launch_part2(var, p, tmap, smem, s);
-    case 3: return wide_launch_part3(var, p, tmap, smem, s);
-    case 4: return wide_launch_part4(var, p, tmap, smem, s);
-    case 5: return wide_launch_part5(var, p, tmap, smem, s);
-    case 6: return wide_launch_part6(var, p, tmap, smem, s);
-    default: return wide_launch_part7(var, p, tmap, smem, s);
+    case 0: return batch_launch_part0(var, p, tmap, smem, s);
+    case 1: return batch_launch_part1(var, p, tmap, smem, s);
+    case 2: return batch_launch_part2(var, p, tmap, smem, s);
+    case 3: return batch_launch_part3(var, p, tmap, smem, s);
+    case 4: return batch_launch_part4(var, p, tmap, smem, s);
+    case 5: return batch_launch_part5(var, p, tmap, smem, s);
+    case 6: return batch_launch_part6(var, p, tmap, smem, s);
+    default: return batch_launch_part7(var, p, tmap, smem, s);
   }
 }
 
@@ -284,23 +283,29 @@ static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo
   pl->pdl = 0;
 }
 
-// wide tcgen05 kernel (kernel 3): 128-row x 256-column tiles, split-K while the tiles do not fill the SMs
-static const int kWideMaxRows = 128;
-static void plan_wide(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
-  const int m_tiles = (M + 127) / 128, n_tiles = (N + 255) / 256;
-  const int tiles = m_tiles * n_tiles, G = K / 128;
-  int splits = 1;
-  for (int s = 2; s <= 32; ++s)
-    if (G % s == 0 && G / s >= 2 && tiles * s <= di.sm_count + di.sm_count / 8) splits = s;
+// small-batch tcgen05 kernel (kernel 3): equal runs of (128-column tile, 128-row group) pairs, one CTA per SM
+static const int kBatchMaxRows = 128;
+static int batch_rows(int M) { return (M + 15) / 16 * 16; }
+// arrival counts and fp32 sums of the column tiles
+static size_t batch_count_bytes(int N) { return ((size_t)((N + 127) / 128) * 32 * sizeof(int) + 255) / 256 * 256; }
+static size_t batch_scratch_bytes(int M, int N) {
+  return batch_count_bytes(N) + (size_t)((N + 127) / 128) * batch_rows(M) * 128 * sizeof(float);
+}
+static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
+  const int n_tiles = (N + 127) / 128, G = K / 128;
+  const long long groups = (long long)n_tiles * G;
+  long long grid = (groups + 1) / 2;  // at least two groups per CTA
+  if (grid > di.sm_count) grid = di.sm_count;
   pl->kernel = 3;
-  pl->m_tiles = m_tiles;
-  pl->splits = splits;
+  pl->m_tiles = 1;
+  pl->splits = 1;
   pl->cluster = 1;
-  pl->ctas_per_split = tiles;
-  pl->stages = wide_wg_stages(bits, di.max_smem, wide_a_rows(M), rpg_of(group));
-  pl->smem_bytes = wide_smem_bytes(bits, pl->stages, wide_a_rows(M), rpg_of(group));
-  pl->tile_m = 128;
-  pl->warps = 23;
+  pl->ctas_per_split = (int)grid;
+  int a_stages;
+  batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
+  pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group));
+  pl->tile_m = batch_rows(M);
+  pl->warps = 16;
   pl->passes = 1;
   pl->pdl = 1;  // always launched as a programmatic dependent
 }
@@ -337,9 +342,11 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
       return ST_OK;
     }
   }
-  // a few dozen rows: weights on the wide side of the MMA; beyond, the transposed prefill kernel
-  if (M <= kWideMaxRows) {
-    plan_wide(M, N, K, bits, group, di, pl);
+  // up to 128 rows the small-batch kernel (weights streamed once); beyond, the prefill kernel
+  if (M <= kBatchMaxRows) {
+    plan_batch(M, N, K, bits, group, di, pl);
+    pl->workspace_bytes = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M, N);
+    return ST_OK;
   } else {
     // A last row tile of at most 16 rows (M = 4097: one row) would cost a whole 256-row tile per
     // column tile; those rows go to the decode kernel in a second launch instead (passes = 2).
@@ -353,15 +360,13 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
       plan_umma(M, N, K, bits, group, di, pl);
     }
   }
-  size_t part = pl->splits > 1 ? (size_t)M * N * sizeof(float) : 0;
-  if (pl->kernel == 1) {  // fp32 slabs per tile slot: every tile of a split-K launch, or the cut tiles of the last round
-    const int Mu = pl->passes == 2 ? M - M % 256 : M;
-    const int tiles = ((Mu + pl->tile_m - 1) / pl->tile_m) * ((N + 127) / 128);
-    const int grid = tiles * pl->splits < di.sm_count ? tiles * pl->splits : di.sm_count;
-    int tail_splits;
-    const int tail = umma_tail(tiles, grid, K / 64, pl->splits, N, &tail_splits);
-    part = umma_partial_bytes(pl->splits > 1 ? tiles : tail, pl->tile_m);
-  }
+  // fp32 slabs per tile slot: every tile of a split-K launch, or the cut tiles of the last round
+  const int Mu = pl->passes == 2 ? M - M % 256 : M;
+  const int tiles = ((Mu + pl->tile_m - 1) / pl->tile_m) * ((N + 127) / 128);
+  const int grid = tiles * pl->splits < di.sm_count ? tiles * pl->splits : di.sm_count;
+  int tail_splits;
+  const int tail = umma_tail(tiles, grid, K / 64, pl->splits, N, &tail_splits);
+  const size_t part = umma_partial_bytes(pl->splits > 1 ? tiles : tail, pl->tile_m);
   size_t need = WS_HEADER_BYTES + ws_counter_bytes(N) + part;
   if (pl->passes == 2 && need < stream_workspace_bytes(N)) need = stream_workspace_bytes(N);
   pl->workspace_bytes = need;
@@ -461,47 +466,75 @@ static int run_umma(const void* a, int lda, const void* bq, const void* scales, 
   return ST_OK;
 }
 
-static int run_wide(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
-                    int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream,
-                    const b200q_plan_t& pl) {
+// Packed weights as a 3-D tensor of 8-byte elements for one tiled copy per 128-row group of `pieces` 16-column
+// pieces: {a group's 256 * bits bytes, groups, pieces}, or for the swizzled widths {128-byte line, lines of
+// all groups, pieces} with the 16-byte chunks of a line swizzled by line.
+static int encode_weights(EncodeTiledFn enc, CUtensorMap* tmap, const void* bq, int N, int G, int bits, int pieces) {
+  const bool swizzled = bits == 2 || bits == 4 || bits == 8;
+  const cuuint64_t inner = swizzled ? 16 : 32 * bits, mid = swizzled ? (cuuint64_t)G * 2 * bits : (cuuint64_t)G;
+  const cuuint64_t gdim[3] = {inner, mid, (cuuint64_t)(N / BLOCK_N)};
+  const cuuint64_t gstride[2] = {inner * 8, inner * 8 * mid};
+  const cuuint32_t box[3] = {(cuuint32_t)inner, swizzled ? 2u * bits : 1u, (cuuint32_t)pieces};
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  const CUresult r = enc(tmap, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, const_cast<void*>(bq), gdim, gstride, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { g_last_cuda_error = (int)r; return ST_CUDA; }
+  return ST_OK;
+}
+
+static int run_batch(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
+                     int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream,
+                     const b200q_plan_t& pl) {
   const int bits = var_bits(var);
-  const int m_tiles = (M + 127) / 128, n_tiles = (N + 255) / 256, G = K / 128;
-  if (pl.splits < 1 || G % pl.splits != 0) return ST_INVALID_ARG;  // whole 128-row groups per split
-  if ((ldc % 8) != 0 || (((uintptr_t)scales) & 15)) return ST_INVALID_ARG;  // 16-byte stores, bulk-copied scale rows
-  const size_t need = WS_HEADER_BYTES + ws_counter_bytes(N) + (pl.splits > 1 ? (size_t)M * N * sizeof(float) : 0);
-  if (!workspace || ws_bytes < need || ((uintptr_t)workspace & 255)) return ST_WORKSPACE;
+  if (M > kBatchMaxRows || pl.splits < 1 || pl.ctas_per_split < 1) return ST_INVALID_ARG;
+  if ((ldc % 8) != 0 || (((uintptr_t)scales) & 15)) return ST_INVALID_ARG;  // 8-byte stores, bulk-copied scale rows
+  const int rows = batch_rows(M), n_tiles = (N + 127) / 128, G = K / 128;
+  const size_t fixed = WS_HEADER_BYTES + ws_counter_bytes(N);
+  if (!workspace || ws_bytes < fixed || ((uintptr_t)workspace & 255)) return ST_WORKSPACE;
+  BatchParams p;
+  p.work = n_tiles * G;
+  p.unit = 1;
+  long long grid = (long long)pl.splits * pl.ctas_per_split;
+  if (grid > device_info().sm_count) grid = device_info().sm_count;
+  if (grid > p.work) grid = p.work;
+  if (ws_bytes < fixed + batch_scratch_bytes(M, N)) {  // a caller with a smaller workspace: whole tiles need none
+    p.work = n_tiles;
+    p.unit = G;
+    grid = n_tiles < device_info().sm_count ? n_tiles : device_info().sm_count;
+  }
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return ST_CUDA;
-  CUtensorMap tmap;
-  const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
-  const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
-  const int a_rows = wide_a_rows(M);
-  const cuuint32_t box[2] = {64u, (cuuint32_t)a_rows};
-  const cuuint32_t estr[2] = {1u, 1u};
-  CUresult r = enc(&tmap, act == B200Q_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(a), gdim, gstride, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { g_last_cuda_error = (int)r; return ST_CUDA; }
-  WideParams p;
-  p.bq = bq;
+  CUtensorMap tmaps[2];  // activations; packed weights
+  {
+    const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
+    const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
+    const cuuint32_t box[2] = {64u, (cuuint32_t)rows};
+    const cuuint32_t estr[2] = {1u, 1u};
+    const CUresult r = enc(&tmaps[0], act == B200Q_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                           const_cast<void*>(a), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { g_last_cuda_error = (int)r; return ST_CUDA; }
+  }
+  {
+    const int r = encode_weights(enc, &tmaps[1], bq, N, G, bits, 8);
+    if (r != ST_OK) return r;
+  }
   p.scales = reinterpret_cast<const __half*>(scales);
   p.c = reinterpret_cast<__half*>(c);
   p.status = reinterpret_cast<int*>(workspace);
-  p.counters = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + WS_HEADER_BYTES);
-  p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + WS_HEADER_BYTES + ws_counter_bytes(N));
-  p.M = M; p.N = N; p.K = K; p.G = K / 128; p.ldc = ldc;
+  p.chunk_counters = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + fixed);
+  p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + fixed + batch_count_bytes(N));
+  p.M = M; p.N = N; p.K = K; p.G = G; p.ldc = ldc;
   p.group = group;
   p.rpg = rpg_of(group);
-  p.m_tiles = m_tiles; p.n_tiles = n_tiles;
-  p.splits = pl.splits; p.kblocks_per_split = 2 * G / pl.splits;
-  p.a_rows = a_rows;
+  p.rows = rows;
+  batch_stages(bits, device_info().max_smem, rows, p.rpg, &p.stages, &p.a_stages);
+  p.grid = (int)grid;
   p.act = act;
-  p.wg_stages = wide_wg_stages(bits, device_info().max_smem, a_rows, rpg_of(group));
-  const int items = pl.splits * m_tiles * n_tiles;
-  p.grid = items < device_info().sm_count ? items : device_info().sm_count;
-  const int smem = wide_smem_bytes(bits, p.wg_stages, a_rows, rpg_of(group));
+  const int smem = batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
-  cudaError_t e = wide_launch(var, p, &tmap, smem, stream);
+  cudaError_t e = batch_launch(var, p, tmaps, smem, stream);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
   return ST_OK;
 }
@@ -638,7 +671,7 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   if (pl.kernel == 2)
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 3)
-    return run_wide(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+    return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   return ST_UNSUPPORTED;
 }
 
@@ -935,10 +968,11 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
   st = make_plan(M, N, K, var, group, &pl);
   if (st != ST_OK) return st;
   if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES) {
-    // beyond the built-in scratch - unless all that asks for the room is the optional K split of the
-    // prefill kernel's last round, which the kernel does without when the scratch is too small
-    const uint64_t without_tail = pl.passes == 2 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
-    if (!(pl.kernel == 1 && pl.splits == 1 && without_tail <= (uint64_t)B200Q_STATIC_WS_BYTES)) return ST_WORKSPACE;
+    // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
+    // without when the scratch is too small (small batches; the prefill kernel's last round)
+    const uint64_t least = pl.passes == 2 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
+    const bool optional = pl.kernel == 3 || (pl.kernel == 1 && pl.splits == 1);
+    if (!(optional && least <= (uint64_t)B200Q_STATIC_WS_BYTES)) return ST_WORKSPACE;
   }
   void* ws = nullptr;
   st = static_ws_pointer(&ws);

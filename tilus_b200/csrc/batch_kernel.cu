@@ -1,0 +1,575 @@
+// Batches of up to 128 rows: C[M, N] = A[M, K] x dequant(Bq[K, N]) on tcgen05, weights streamed once.
+//
+// The product is computed transposed, D[n, m] = sum_k W[k, n] * A[m, k], like the prefill kernel
+// (umma_kernel.cu): the dequantized weights are the tensor-memory operand (128 lanes = 128 columns), the
+// activations the shared-memory operand with as many rows as the batch has, rounded up to 16.  An MMA of
+// 128 x NR x 16 then costs NR / 2 tensor cycles (9 for 16 rows), so that the tensor pipe stays below the HBM
+// time of the weights up to about 80 rows of 4-bit weights, and nothing the weights pass through is
+// wider than their packed form: global -> (tiled copy) -> shared -> registers -> tensor memory.
+//
+// Roles of the 16 warps of a CTA:
+//   * warps 0-7 dequantize, in two sets of four (a set covers the 128 lanes; lane L is column L of the
+//     tile).  Set s takes the 128-row groups s, s + 2, ... of the CTA: a lane reads its column's four
+//     units, decodes and scales them (decode.cuh, unit_decode_scaled: the weights the reference
+//     multiplies by, examples/quantization/matmul_a16wx.py:316-320) and writes 64 tensor-memory columns.
+//     Each set has operand slots and ring stages of its own, so that every barrier has one kind of waiter
+//     and phases cannot be mistaken for one another (a third set measured slower: 12.9 -> 12.3 us at
+//     16 x 4096 x 14336 without it);
+//   * warps 8-11 are the epilogue; the dequantize warps take a share of the run's last segment;
+//   * warp 12 brings the activations, two 2-D tiled TMA copies (128-byte swizzle) per group;
+//   * warp 13 brings packed weights, a 128-row group of the 128 columns at a time: one 3-D tiled
+//     TMA copy for the eight 16-column pieces.  For 2, 4 and 8 bits it swizzles 16-byte chunks by
+//     128-byte line, which spreads eight neighbouring columns over all shared-memory banks (columns are
+//     16 * b bytes apart: unswizzled, 4-bit loads would collide four ways); other widths are left dense
+//     (two-way);
+//   * warp 14 owns tensor memory and issues eight tcgen05.mma per group;
+//   * warp 15 brings the scales.
+// The four single-thread roles run under elect.sync: copies and MMAs take their operands from uniform
+// registers.  (Eight lanes issuing one 1 KB bulk copy each took 1100 cycles per group; the copies of a
+// group may take 360 at the HBM rate of 4-bit weights.)
+//
+// Work split.  The (column tile, 128-row group) pairs are numbered tile by tile and cut into equal
+// contiguous runs, one per CTA, whatever the shape.  A run covers at most one tile's end, whole
+// tiles, and one tile's start.  Whole tiles are written to C; a partial tile's sums are added into an
+// fp32 scratch tile (red.global.add.v4) and counted in, and whoever completes the count converts them,
+// writes C and puts the scratch back to zero (batch_epilogue).
+//
+// Measured (4-bit, group 128, a chain of launches; the kernel before it wrote dequantized weights to
+// 256-column shared-memory operands): 64 x 28672 x 4096 44.1 -> 23.4 us, 64 x 8192 x 8192 27.6 -> 16.4,
+// 128 x 8192 x 8192 34.0 -> 22.7.  What is left at 64 rows is the dequantize warps' instructions and
+// the additions of the partial tiles in L2.
+//
+// Every mbarrier wait is bounded in time; a wait that runs out raises a CTA-wide abort flag, all loops
+// leave, the producers give their copies in flight a bounded chance to land, tensor memory is freed and
+// the status word of the workspace reports it.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "umma_common.cuh"
+
+#ifndef B200Q_PART
+#define B200Q_PART 0
+#endif
+#ifndef B200Q_NPARTS
+#define B200Q_NPARTS 1
+#endif
+
+namespace b200q {
+
+constexpr int BATCH_SETS = 2;                      // dequantize sets of four warps
+constexpr int BATCH_THREADS = BATCH_SETS * 128 + 256;  // + four epilogue warps, three producers, MMA warp
+constexpr int BATCH_SLOTS_MAX = 3 * BATCH_SETS;    // 128-row operand slots
+constexpr int BATCH_STAGES_MAX = 16;               // 128-row groups in the packed ring, a multiple of BATCH_SETS
+constexpr int BATCH_A_MAX = 6;                     // 128-row activation groups in shared memory, at most the slots
+
+struct BatchBarriers {
+  uint64_t slot_full[BATCH_SLOTS_MAX];
+  uint64_t done[BATCH_SLOTS_MAX];  // [i]: the MMAs of a group in slot i have completed
+  uint64_t a_full[BATCH_A_MAX];
+  uint64_t g_full[BATCH_STAGES_MAX], g_empty[BATCH_STAGES_MAX];
+  uint64_t d_full[2], d_empty[2];
+  uint32_t tmem_base;
+  volatile int abort_flag;
+};
+
+// a ring stage: 128 columns x 128 rows of packed weights, and (in a region of their own) rpg rows of 128 scales
+__host__ __device__ constexpr int batch_stage_bytes(int bits, int rpg) { return 2048 * bits + 256 * rpg; }
+// widths whose stages are swizzled by 128-byte line (see above)
+__host__ __device__ constexpr bool batch_swizzled(int bits) { return bits == 2 || bits == 4 || bits == 8; }
+// tensor memory (all 512 columns): two D accumulators of nr columns, then as many operand slots as fit
+__host__ __device__ constexpr int batch_d_stride(int nr) { return nr <= 64 ? 64 : 128; }
+__host__ __device__ constexpr int batch_slots_per_set(int nr) { return nr <= 64 ? 3 : 2; }
+
+// 16 registers -> 16 consecutive tensor-memory columns of this thread's lane
+__device__ __forceinline__ void tmem_st_16(uint32_t taddr, const uint32_t (&o)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+      "%14, %15, %16};" ::"r"(taddr),
+      "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]),
+      "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
+      : "memory");
+}
+
+// Four rows (m .. m + 3) of one column per lane -> each lane stores four consecutive columns of one row.
+template <int ACT>
+__device__ __forceinline__ void batch_store4(const BatchParams& p, int n, int lane, int m, const float4& v) {
+  const bool b0 = lane & 1, b1 = lane & 2;
+  // two 16-bit rows per register, then two exchange rounds
+  const uint32_t r01 = pack2<ACT>(v.x, v.y), r23 = pack2<ACT>(v.z, v.w);
+  // round 1 (columns n and n ^ 1): even lane keeps rows 0 and 2, odd lane rows 1 and 3
+  const uint32_t o01 = __shfl_xor_sync(0xffffffffu, r01, 1), o23 = __shfl_xor_sync(0xffffffffu, r23, 1);
+  const uint32_t x0 = b0 ? __byte_perm(o01, r01, 0x7632) : __byte_perm(r01, o01, 0x5410);  // row 0 + b0
+  const uint32_t x2 = b0 ? __byte_perm(o23, r23, 0x7632) : __byte_perm(r23, o23, 0x5410);  // row 2 + b0
+  // round 2 (column pairs): lanes with b1 = 0 take row b0, those with b1 = 1 row 2 + b0
+  const uint32_t got = __shfl_xor_sync(0xffffffffu, b1 ? x0 : x2, 2);
+  const uint2 o = b1 ? make_uint2(got, x2) : make_uint2(x0, got);
+  const int row = m + (b1 ? 2 : 0) + (b0 ? 1 : 0);
+  if (row < p.M && n < p.N)
+    *reinterpret_cast<uint2*>(reinterpret_cast<unsigned short*>(p.c) + (size_t)row * p.ldc + (n & ~3)) = o;
+}
+
+// The 2 * B words of units 2h and 2h + 1 of column `nl` from a ring stage.
+template <int B>
+__device__ __forceinline__ void batch_load_units(uint32_t stage, int nl, int h, uint32_t (&w)[2 * B]) {
+  const uint32_t off = (uint32_t)((nl >> 4) * (256 * B) + (nl & 15) * (16 * B) + h * (8 * B));
+  if constexpr (batch_swizzled(B)) {
+    const uint32_t line = off >> 7;
+#pragma unroll
+    for (int q = 0; q < B / 2; ++q) {
+      const uint32_t chunk = ((off >> 4) + (uint32_t)q) & 7u;  // a block's chunks lie in one line
+      const uint4 v = lds_u4(stage + (line << 7) + ((chunk ^ (line & 7u)) << 4));
+      w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+    }
+  } else {
+    lds_two_units<B>(stage + off, w);
+  }
+}
+
+// first group of CTA c's run
+__device__ __forceinline__ int batch_run_start(const BatchParams& p, int c) {
+  return (int)((long long)p.work * c / p.grid) * p.unit;
+}
+
+// Lane i's count says whether this warp's i-th 16-row chunk (chunk part + i * parts) of the tile's sums is
+// complete; the complete ones are converted, written to C and put back to zero.
+template <int ACT>
+__device__ __forceinline__ void batch_finish(const BatchParams& p, int tile, int len, int wq, int lane, int part, int parts) {
+  const int nl = wq * 32 + lane, n = tile * 128 + nl;
+  float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;  // [rows / 4][128] quads
+  int complete = 0;
+  const int chunk = part + lane * parts;
+  __syncwarp();
+  if (chunk * 16 < p.M) {
+    int* counter = p.chunk_counters + tile * 32 + wq * 8 + chunk;
+    __threadfence();  // cumulative over the warp's additions (ordered by the barrier above)
+    complete = atomicAdd(counter, len) + len == p.G ? 1 : 0;
+    if (complete) {
+      *counter = 0;
+      __threadfence();
+    }
+  }
+  unsigned mask = __ballot_sync(0xffffffffu, complete);
+  while (mask) {
+    const int mc0 = (part + (__ffs(mask) - 1) * parts) * 4;
+    mask &= mask - 1;
+    float4 x[4];  // independent loads
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if ((mc0 + u) * 4 < p.M) x[u] = __ldcg(sums + (mc0 + u) * 128);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if ((mc0 + u) * 4 < p.M) {
+        __stcg(sums + (mc0 + u) * 128, make_float4(0.f, 0.f, 0.f, 0.f));
+        batch_store4<ACT>(p, n, lane, (mc0 + u) * 4, x[u]);
+      }
+  }
+}
+
+// The epilogue of one segment, shared out over `parts` groups of four warps (this warp belongs to group
+// `part`): rows in chunks of 16 from tensor memory, to C (a whole tile) or added into the tile's scratch.
+// Each (lane quadrant, chunk) of a tile is counted by itself, in 128-row groups: the warp that completes
+// the count converts its sums, writes C and puts sums and count back to zero.  Nothing waits for the rest of
+// the CTA.  (Slabs per CTA with plain stores, added up by the last to arrive, measured slower: its loads of
+// lines other SMs have just written cost 2 - 8 us more than these additions.)
+template <int ACT>
+__device__ __forceinline__ void batch_epilogue(const BatchParams& p, uint32_t d_t, uint32_t d_empty, int tile, int len,
+                                               int wq, int lane, int part, int parts) {
+  const int nl = wq * 32 + lane, n = tile * 128 + nl;
+  const bool whole = len == p.G;
+  float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;
+  for (int c0 = part * 16; c0 < p.M; c0 += 16 * parts) {
+    uint32_t v[16];
+    tmem_ld_16(d_t + (uint32_t)c0, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int m = c0 + q * 4;
+      if (m >= p.M) continue;
+      const float4 f = make_float4(__uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]), __uint_as_float(v[4 * q + 2]),
+                                   __uint_as_float(v[4 * q + 3]));
+      if (whole)
+        batch_store4<ACT>(p, n, lane, m, f);
+      else
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(sums + (m >> 2) * 128), "f"(f.x), "f"(f.y),
+                     "f"(f.z), "f"(f.w)
+                     : "memory");
+    }
+  }
+  // the accumulator has been read: the MMAs of the segment after next may overwrite it
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if (d_empty != 0 && lane == 0) mbar_arrive(d_empty);
+  if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, part, parts);
+}
+
+template <int VAR, int ACT>
+__global__ void __launch_bounds__(BATCH_THREADS, 1)
+batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
+  constexpr int B = var_bits(VAR);
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t smem_unaligned = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  const uint32_t smem_base = (smem_unaligned + 1023u) & ~1023u;
+  unsigned char* smem_al = smem_raw + (smem_base - smem_unaligned);
+  const int NR = p.rows, WS = p.stages, AS = p.a_stages;
+  constexpr uint32_t WSTAGE = 2048u * B;
+  const uint32_t ASTAGE = (uint32_t)NR * 256u, SSTAGE = 256u * (uint32_t)p.rpg;
+  const uint32_t ring_off = (uint32_t)AS * ASTAGE, scales_off = ring_off + (uint32_t)WS * WSTAGE;
+  const uint32_t ring_s = smem_base + ring_off, scales_s = smem_base + scales_off;
+  const uint32_t bars_off = scales_off + (uint32_t)WS * SSTAGE;
+  BatchBarriers* bars = reinterpret_cast<BatchBarriers*>(smem_al + bars_off);
+  const uint32_t bars_s = smem_base + bars_off;
+#define BAR_ADDR(field, i) (bars_s + (uint32_t)offsetof(BatchBarriers, field) + (uint32_t)(i) * 8u)
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  volatile int* abort_flag = &bars->abort_flag;
+  // this CTA's run of groups, counted tile by tile over the whole matrix
+  const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
+
+  if (tid == 0) {
+    for (int i = 0; i < BATCH_SLOTS_MAX; ++i) { mbar_init(BAR_ADDR(slot_full, i), 4); mbar_init(BAR_ADDR(done, i), 1); }
+    for (int i = 0; i < AS; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
+    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(d_full, i), 1); mbar_init(BAR_ADDR(d_empty, i), 4); }
+    bars->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  __syncthreads();
+  // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
+  // this SM may still hold it)
+  constexpr int TM_THREADS = BATCH_SETS * 128 + 160;
+  constexpr int W_EPI = BATCH_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
+                W_SCALES = W_EPI + 7;
+  if (warp == W_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp < W_ACT || warp == W_MMA) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(TM_THREADS) : "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  const uint32_t tmem = (warp < W_ACT || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
+  const int sps = batch_slots_per_set(NR);
+  const uint32_t slots_t = tmem + (uint32_t)(batch_d_stride(NR) * 2);
+
+  // one segment of the run: pos -> tile, groups
+#define SEGMENT(pos)                                     \
+  const int tile = (pos) / p.G, g0 = (pos) - tile * p.G; \
+  const int len = min(p.G - g0, run1 - (pos));           \
+  const bool last_seg = (pos) + len == run1;             \
+  (void)last_seg;
+
+  if (warp < W_EPI) {
+    // ================= dequantize (and a share of the last segment's epilogue) =================
+    const int set = warp >> 2, wq = warp & 3;
+    const int nl = wq * 32 + lane;  // lane of tensor memory = column inside the tile
+    const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
+    bool good = true;
+    int stage = set, slot = set;    // stages of a set: set, set + BATCH_SETS, ...; slots likewise
+    uint32_t ring_phase = 0, slot_phase = 1;
+    for (int g_own = set; g_own < run1 - run0; g_own += BATCH_SETS) {
+      if (!mbar_wait_abortable(BAR_ADDR(g_full, stage), ring_phase, abort_flag)) { good = false; break; }
+      const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
+      const uint32_t sc = scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u;
+      uint32_t w[2][2 * B], s2[4];
+      unsigned short sb;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc));
+      s2[0] = s2[1] = s2[2] = s2[3] = (uint32_t)sb * 0x00010001u;  // the 16-bit scale in both halves
+      if (p.rpg > 1) {
+#pragma unroll
+        for (int u = 1; u < 4; ++u) {
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc + (uint32_t)((u * p.rpg) >> 2) * 256u));
+          s2[u] = (uint32_t)sb * 0x00010001u;
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        batch_load_units<B>(st, nl, h, w[h]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          uint32_t out[16];
+          unit_decode_scaled<VAR, ACT>(w[h] + u * B, s2[2 * h + u], out);
+          if (h == 0 && u == 0) {  // the MMAs have read what the set stored here before
+            if (!mbar_wait_abortable(BAR_ADDR(done, slot), slot_phase, abort_flag)) { good = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+          if (h == 1 && u == 0) {  // the stage has been read (its values fed the arithmetic above)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR_ADDR(g_empty, stage));
+          }
+          tmem_st_16(slots_t + lane_t + (uint32_t)(slot * 64 + h * 32 + u * 16), out);
+        }
+        if (!good) break;
+      }
+      if (!good) break;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_ADDR(slot_full, slot));
+      slot += BATCH_SETS;
+      if (slot >= BATCH_SETS * sps) { slot = set; slot_phase ^= 1u; }
+      stage += BATCH_SETS;
+      if (stage >= WS) { stage = set; ring_phase ^= 1u; }
+    }
+    if (good) {
+      int pos = run0, seg = 0;  // the last segment
+      while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
+      SEGMENT(pos)
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
+      if (mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), 0u, tile, len, wq, lane, set,
+                            BATCH_SETS + 1);
+      }
+    }
+  } else if (warp < W_ACT) {
+    // ================= epilogue =================
+    const int wq = warp & 3;
+    const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
+    int seg = 0;
+    for (int pos = run0; pos < run1; ++seg) {
+      SEGMENT(pos)
+      if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
+                          len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
+      pos += len;
+    }
+  } else if (warp == W_ACT) {
+    // ================= TMA producer: activations =================
+    if (elect_one()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      // The ring's stage of group i held group i - AS, whose MMAs report on its slot's barrier: one commit per
+      // group frees slot and activations (a second commit right behind the first costs the issuing thread
+      // 600 cycles).
+      int stage = 0, n_issued = 0, slot = 0;
+      uint32_t phase = 0;
+      bool good = true;
+      int g = run0 % p.G;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (n_issued >= AS) {
+          if (!mbar_wait_abortable(BAR_ADDR(done, slot), phase, abort_flag)) { good = false; break; }
+          if (++slot == BATCH_SETS * sps) { slot = 0; phase ^= 1u; }
+        }
+        const uint32_t bar = BAR_ADDR(a_full, stage);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(ASTAGE) : "memory");
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile(
+              "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+              ::"r"(smem_base + (uint32_t)stage * ASTAGE + (uint32_t)h * (ASTAGE / 2)), "l"(&tmap_a), "r"(bar),
+              "r"(g * 128 + h * 64), "r"(0)
+              : "memory");
+        ++n_issued;
+        if (++stage == AS) stage = 0;
+        if (++g == p.G) g = 0;
+      }
+      if (!good) {  // a copy in flight must not outlive the CTA: a bounded wait for the groups issued last
+        for (int i = max(0, n_issued - AS); i < n_issued; ++i)
+          mbar_wait_bounded(BAR_ADDR(a_full, i % AS), (uint32_t)(i / AS) & 1u);
+      }
+    }
+  } else if (warp == W_WEIGHTS) {
+    // ================= TMA producer: packed weights =================
+    if (elect_one()) {
+      int stage = 0, n_issued = 0;
+      uint32_t phase = 1;
+      bool good = true;
+      int tile = run0 / p.G, g = run0 - tile * p.G;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = BAR_ADDR(g_full, stage);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(WSTAGE) : "memory");
+        // (pieces past the last column are filled with zeros and count as bytes all the same)
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+            ::"r"(ring_s + (uint32_t)stage * WSTAGE), "l"(&tmap_w), "r"(bar), "r"(0),
+            "r"(batch_swizzled(B) ? g * (2 * B) : g), "r"(tile * 8)
+            : "memory");
+        ++n_issued;
+        if (++g == p.G) { g = 0; ++tile; }
+        if (++stage == WS) { stage = 0; phase ^= 1u; }
+      }
+      if (!good) {
+        for (int i = max(0, n_issued - WS); i < n_issued; ++i)
+          mbar_wait_bounded(BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
+      }
+    }
+  } else if (warp == W_SCALES) {
+    // ================= bulk-copy producer: scales (a thread of its own: issuing takes 100 cycles a copy) =================
+    if (elect_one()) {
+      int stage = 0, n_issued = 0;
+      uint32_t phase = 1;
+      bool good = true;
+      int tile = run0 / p.G, g = run0 - tile * p.G;
+      // scale row(s) of the group: p.rpg rows per group, or one row for p.group / 128 groups
+      const int groups_per_row = p.rpg == 1 ? p.group / 128 : 1;
+      int in_row = g % groups_per_row;
+      const __half* sc = p.scales + (size_t)(p.rpg == 1 ? g / groups_per_row : g * p.rpg) * p.N + tile * 128;
+      uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = BAR_ADDR(g_full, stage);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(sc_bytes * (uint32_t)p.rpg)
+                     : "memory");
+        for (int i = 0; i < p.rpg; ++i)
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  scales_s + (uint32_t)stage * SSTAGE + (uint32_t)i * 256u),
+              "l"(sc + (size_t)i * p.N), "r"(sc_bytes), "r"(bar)
+              : "memory");
+        ++n_issued;
+        if (++in_row == groups_per_row) { in_row = 0; sc += (size_t)p.rpg * p.N; }
+        if (++g == p.G) {
+          g = 0; in_row = 0; ++tile;
+          sc = p.scales + tile * 128;
+          sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
+        }
+        if (++stage == WS) { stage = 0; phase ^= 1u; }
+      }
+      if (!good) {
+        for (int i = max(0, n_issued - WS); i < n_issued; ++i)
+          mbar_wait_bounded(BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
+      }
+    }
+  } else {
+    // ================= MMA issuer =================
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc<ACT>(NR);
+      bool good = true;
+      int slot = 0, stage = 0, seg = 0;
+      const int nslots = BATCH_SETS * sps;
+      uint32_t slot_phase = 0, a_phase = 0;
+      // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
+      // the look (twice 100 cycles) lies under them; only a group that was not ready then is waited for
+      bool ready = false;
+      for (int pos = run0; pos < run1 && good; ++seg) {
+        SEGMENT(pos)
+        if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d_t = tmem + (uint32_t)((seg & 1) * batch_d_stride(NR));
+        for (int i = 0; i < len && good; ++i) {
+          if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), slot_phase, abort_flag) ||
+                         !mbar_wait_abortable(BAR_ADDR(a_full, stage), a_phase, abort_flag))) { good = false; break; }
+          const int slot1 = slot + 1 == nslots ? 0 : slot + 1, stage1 = stage + 1 == AS ? 0 : stage + 1;
+          const uint32_t slot_phase1 = slot_phase ^ (slot1 == 0 ? 1u : 0u), a_phase1 = a_phase ^ (stage1 == 0 ? 1u : 0u);
+          const bool next0 = mbar_test(BAR_ADDR(slot_full, slot1), slot_phase1);
+          const bool next1 = mbar_test(BAR_ADDR(a_full, stage1), a_phase1);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)stage * ASTAGE);
+          const uint32_t a_t = slots_t + (uint32_t)(slot * 64), half = ASTAGE >> 5;  // second block, in 16-byte units
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {
+            const uint32_t accumulate = (i > 0 || ks > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                ::"r"(d_t), "r"(a_t + (uint32_t)(ks * 8)), "l"(bdesc + (uint64_t)((ks & 3) * 2) + (ks < 4 ? 0u : half)),
+                "r"(idesc), "r"(accumulate)
+                : "memory");
+          }
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           BAR_ADDR(done, slot))
+                       : "memory");
+          ready = next0 && next1;
+          slot = slot1; slot_phase = slot_phase1; stage = stage1; a_phase = a_phase1;
+        }
+        if (good)
+          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                           BAR_ADDR(d_full, seg & 1))
+                       : "memory");
+        pos += len;
+      }
+    }
+  }
+
+  // ================= teardown =================
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*abort_flag && tid == 0) {
+    atomicExch(p.status, ST_DEVICE_TIMEOUT);
+    p.status[1] = 6;  // where: small-batch tcgen05 kernel pipeline
+    p.status[2] = blockIdx.x;
+    p.status[3] = 0;
+  }
+  if (warp == W_MMA) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+#undef BAR_ADDR
+#undef SEGMENT
+}
+
+template <int VAR, int ACT>
+static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
+  auto kern = batch_kernel<VAR, ACT>;
+  static int configured_smem[16] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
+  cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, p, tmaps[0], tmaps[1]);
+}
+
+template <int VAR>
+static cudaError_t batch_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
+                                    cudaStream_t stream) {
+  if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
+    if (var == VAR)
+      return p.act == 0 ? batch_launch_one<VAR, 0>(p, tmaps, smem_bytes, stream)
+                        : batch_launch_one<VAR, 1>(p, tmaps, smem_bytes, stream);
+  }
+  if constexpr (VAR + 1 < VAR_COUNT) return batch_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
+  else return cudaErrorInvalidValue;
+}
+
+#define B200Q_CAT2(a, b) a##b
+#define B200Q_CAT(a, b) B200Q_CAT2(a, b)
+
+// One of these per compiled part; api.cu picks the part as var % B200Q_NPARTS.
+cudaError_t B200Q_CAT(batch_launch_part, B200Q_PART)(int var, const BatchParams& p, const void* tmaps, int smem_bytes,
+                                                     cudaStream_t stream) {
+  return batch_launch_var<0>(var, p, reinterpret_cast<const CUtensorMap*>(tmaps), smem_bytes, stream);
+}
+
+#if B200Q_PART == 0
+// dynamic shared memory: alignment slack + activation groups + packed ring + scales + barriers
+int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
+  return 1024 + a_stages * rows * 256 + stages * batch_stage_bytes(bits, rpg) + (int)sizeof(BatchBarriers);
+}
+// Activation groups (at most as many as there are operand slots) and ring stages (a multiple of the dequantize
+// sets) in the rest.  Batches of up to 64 rows stay within half an SM's shared memory, so that the next
+// launch of the stream becomes resident beside this one and fills its ring while this one ends
+// (4096 x 4096, 16 rows: 8.2 -> 6.4 us against twice the stages without a neighbour).
+void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {
+  const int cap = rows <= 64 ? 113 * 1024 : max_smem;
+  *a_stages = rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
+  int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
+  while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg) > cap) st -= BATCH_SETS;
+  *stages = st;
+}
+#endif
+
+}  // namespace b200q

@@ -133,24 +133,22 @@ struct UmmaParams {
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
 };
 
-// ---- wide tcgen05 kernel (a few dozen rows): weights on the 256-column side of the MMA ---------
-struct WideParams {
-  const void* bq;        // b200 layout
+// ---- small-batch tcgen05 kernel (up to 128 rows): weights streamed once -------------------------
+struct BatchParams {
   const __half* scales;  // [K/group, N]
   __half* c;             // [M, N], leading dimension ldc (multiple of 8)
-  float* partial;        // [M, N] fp32 split-K scratch, zero on entry and on exit
-  int* counters;         // [n_tiles * m_tiles], zero on entry and on exit
+  float* partial;        // fp32 scratch [column tile][rows / 4][128][4], zero on entry and on exit
+  int* chunk_counters;   // arrived 128-row groups per tile, lane quadrant and 16-row chunk [tile][4][8], zero on entry and on exit
   int* status;           // workspace status header
   int M, N, K, G;        // G = K / 128
   int ldc;
   int group;             // rows per scale: 32, 64 or a multiple of 128
   int rpg;               // scale rows per 128-row group: 128 / group for group < 128, else 1
-  int m_tiles, n_tiles;  // ceil(M / 128), ceil(N / 256)
-  int splits;            // split-K factor
-  int kblocks_per_split; // 64-row k blocks per work item (even)
-  int wg_stages;         // packed 128-row weight groups in the shared-memory ring
-  int a_rows;            // rows per activation copy: 32, 64 or 128
-  int grid;              // persistent CTAs: min(work items, SMs)
+  int rows;              // M rounded up to 16: the N extent of the MMA
+  int work, unit;        // work units of the launch and 128-row groups per unit (1, or G: whole column tiles)
+  int stages;            // packed 128-row groups in the shared-memory ring
+  int a_stages;          // 128-row activation groups in shared memory
+  int grid;              // CTAs: each takes an equal contiguous run of work units
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
 };
 
@@ -222,23 +220,44 @@ __device__ __forceinline__ void red_add_v2(float* addr, float x, float y) {
 
 // ---- shared-memory and mbarrier helpers of the mma.sync kernels ----------------------------------
 // Waits on an mbarrier phase for at most about a quarter of a second; false when that ran out.
+constexpr long long WAIT_LIMIT_CLOCKS = 450000000ll;  // 0.23 s at 1.965 GHz
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
-  uint64_t t0 = 0;
+  long long t0 = 0;
   for (int it = 0;; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 0x100000;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
-    uint64_t now;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    const long long now = clock64();
     if (it == 0) t0 = now;
-    else if (now - t0 > 250000000ull) return false;
+    else if (now - t0 > WAIT_LIMIT_CLOCKS) return false;
   }
+}
+// One elected lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: inside
+// a branch on elect.sync the compiler keeps them there, while inside `if (lane == 0)` it moves every
+// operand over for each instruction - measured 116 cycles per MMA whatever its shape, against 128 / 64 /
+// 32 / 16 / 9 cycles for 256 / 128 / 64 / 32 / 16 columns with the elected lane.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// one non-blocking look at an mbarrier phase
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 
 __device__ __forceinline__ uint4 lds_u4(uint32_t addr) {

@@ -133,19 +133,6 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
   return bits_from_h2(__floats2half2_rn(lo, hi));
 }
 
-// one non-blocking look at an mbarrier phase
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
 // Shared-memory layout (byte offsets from the dynamic smem base):
 //   [0, HDR)     mbarriers [warp][stage]   (up to 8 stages of 8 bytes per warp, HDR a multiple of 1 KB)
 //   [HDR, ...)   rings [warp][stage][ITEM_BYTES] of packed weights

@@ -11,33 +11,25 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One elected lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: inside
-// a branch on elect.sync the compiler keeps them there, while inside `if (lane == 0)` it moves every
-// operand over for each instruction - measured 116 cycles per MMA whatever its shape, against 128 / 64 /
-// 32 / 16 / 9 cycles for 256 / 128 / 64 / 32 / 16 columns with the elected lane.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-// bounded wait (about a quarter of a second); also gives up as soon as another thread raised the abort flag
+// Bounded wait (about a quarter of a second); also gives up as soon as another thread raised the abort flag.
+// The bound is counted in SM clocks: %globaltimer, read between two looks at a barrier, costs far more than
+// the look itself.
 __device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  uint64_t t0 = 0;
+  long long t0 = 0;
   for (int it = 0;; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 0x10000;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 0x989680;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
         : "memory");
     if (ok) return true;
     if (*abort_flag) return false;
-    uint64_t now;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    const long long now = clock64();
     if (it == 0) t0 = now;
-    else if (now - t0 > 250000000ull) { *abort_flag = 1; return false; }
+    else if (now - t0 > WAIT_LIMIT_CLOCKS) { *abort_flag = 1; return false; }
   }
 }
 
