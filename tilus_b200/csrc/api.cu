@@ -532,6 +532,7 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   batch_stages(bits, device_info().max_smem, rows, p.rpg, &p.stages, &p.a_stages);
   p.grid = (int)grid;
   p.act = act;
+  p.exact = rows == 16 && p.rpg == 1 ? 1 : 0;
   const int smem = batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
   cudaError_t e = batch_launch(var, p, tmaps, smem, stream);

@@ -68,6 +68,8 @@ struct BatchBarriers {
   uint64_t a_full[BATCH_A_MAX];
   uint64_t g_full[BATCH_STAGES_MAX], g_empty[BATCH_STAGES_MAX];
   uint64_t d_full[2], d_empty[2];
+  uint64_t s_full[BATCH_STAGES_MAX], s_empty[BATCH_STAGES_MAX];  // EXACT: the scales' own ring
+  uint64_t x_empty[BATCH_SLOTS_MAX];                             // EXACT: [i]: the sums of slot i have been read
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -201,8 +203,14 @@ __device__ __forceinline__ void batch_epilogue(const BatchParams& p, uint32_t d_
   if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, part, parts);
 }
 
-template <int VAR, int ACT>
-__global__ void __launch_bounds__(BATCH_THREADS, 1)
+#ifndef EXACT_SPS
+#define EXACT_SPS 3
+#endif
+#ifndef EXACT_CTAS
+#define EXACT_CTAS 2
+#endif
+template <int VAR, int ACT, bool EXACT>
+__global__ void __launch_bounds__(BATCH_THREADS, EXACT ? EXACT_CTAS : 1)
 batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
   constexpr int B = var_bits(VAR);
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -228,7 +236,11 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   if (tid == 0) {
     for (int i = 0; i < BATCH_SLOTS_MAX; ++i) { mbar_init(BAR_ADDR(slot_full, i), 4); mbar_init(BAR_ADDR(done, i), 1); }
     for (int i = 0; i < AS; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
-    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
+    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), EXACT ? 1 : 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
+    if (EXACT) {
+      for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(s_full, i), 1); mbar_init(BAR_ADDR(s_empty, i), 4); }
+      for (int i = 0; i < BATCH_SLOTS_MAX; ++i) mbar_init(BAR_ADDR(x_empty, i), 4);
+    }
     for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(d_full, i), 1); mbar_init(BAR_ADDR(d_empty, i), 4); }
     bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -241,11 +253,13 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
   constexpr int TM_THREADS = BATCH_SETS * 128 + 160;
+  constexpr int TM_COLS = EXACT && EXACT_SPS == 1 ? 256 : 512;
   constexpr int W_EPI = BATCH_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
                 W_SCALES = W_EPI + 7;
   if (warp == W_MMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
-                     bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base))
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base)),
+                 "r"(TM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -255,8 +269,9 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
   const uint32_t tmem = (warp < W_ACT || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
-  const int sps = batch_slots_per_set(NR);
-  const uint32_t slots_t = tmem + (uint32_t)(batch_d_stride(NR) * 2);
+  const int sps = EXACT ? EXACT_SPS : batch_slots_per_set(NR);
+  // EXACT: a 16-column accumulator per operand slot, then the slots
+  const uint32_t slots_t = tmem + (uint32_t)(EXACT ? 16 * BATCH_SLOTS_MAX : batch_d_stride(NR) * 2);
 
   // one segment of the run: pos -> tile, groups
 #define SEGMENT(pos)                                     \
@@ -278,14 +293,16 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
       const uint32_t sc = scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u;
       uint32_t w[2][2 * B], s2[4];
-      unsigned short sb;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc));
-      s2[0] = s2[1] = s2[2] = s2[3] = (uint32_t)sb * 0x00010001u;  // the 16-bit scale in both halves
-      if (p.rpg > 1) {
+      if constexpr (!EXACT) {
+        unsigned short sb;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc));
+        s2[0] = s2[1] = s2[2] = s2[3] = (uint32_t)sb * 0x00010001u;  // the 16-bit scale in both halves
+        if (p.rpg > 1) {
 #pragma unroll
-        for (int u = 1; u < 4; ++u) {
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc + (uint32_t)((u * p.rpg) >> 2) * 256u));
-          s2[u] = (uint32_t)sb * 0x00010001u;
+          for (int u = 1; u < 4; ++u) {
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc + (uint32_t)((u * p.rpg) >> 2) * 256u));
+            s2[u] = (uint32_t)sb * 0x00010001u;
+          }
         }
       }
 #pragma unroll
@@ -294,7 +311,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           uint32_t out[16];
-          unit_decode_scaled<VAR, ACT>(w[h] + u * B, s2[2 * h + u], out);
+          if constexpr (EXACT) unit_decode_exact<VAR, ACT>(w[h] + u * B, out);
+          else unit_decode_scaled<VAR, ACT>(w[h] + u * B, s2[2 * h + u], out);
           if (h == 0 && u == 0) {  // the MMAs have read what the set stored here before
             if (!mbar_wait_abortable(BAR_ADDR(done, slot), slot_phase, abort_flag)) { good = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -317,7 +335,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       stage += BATCH_SETS;
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
-    if (good) {
+    if (!EXACT && good) {
       int pos = run0, seg = 0;  // the last segment
       while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
@@ -332,15 +350,67 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     // ================= epilogue =================
     const int wq = warp & 3;
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
-    int seg = 0;
-    for (int pos = run0; pos < run1; ++seg) {
-      SEGMENT(pos)
-      if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
-                          len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
-      pos += len;
+    if constexpr (EXACT) {
+      // Each group's sums, times the group's scale in fp32, onto the segment's sums in registers.
+      const int nl = wq * 32 + lane;
+      int slot = 0, stage = 0;
+      uint32_t slot_phase = 0, s_phase = 0;
+      bool good = true, waited = false;
+      for (int pos = run0; pos < run1 && good;) {
+        SEGMENT(pos)
+        float acc[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+        for (int g = 0; g < len; ++g) {
+          if (!mbar_wait_abortable(BAR_ADDR(s_full, stage), s_phase, abort_flag)) { good = false; break; }
+          unsigned short sb;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u));
+          if (!mbar_wait_abortable(BAR_ADDR(done, slot), slot_phase, abort_flag)) { good = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          uint32_t v[16];
+          tmem_ld_16(tmem + lane_t + (uint32_t)(slot * 16), v);
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          const float sf = ACT == 0 ? __half2float(__ushort_as_half(sb)) : __uint_as_float((uint32_t)sb << 16);
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(BAR_ADDR(x_empty, slot));
+            mbar_arrive(BAR_ADDR(s_empty, stage));
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) acc[i] = fmaf(sf, __uint_as_float(v[i]), acc[i]);
+          if (++slot == BATCH_SETS * sps) { slot = 0; slot_phase ^= 1u; }
+          if (++stage == WS) { stage = 0; s_phase ^= 1u; }
+        }
+        if (!good) break;
+        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use
+        waited = true;
+        const bool whole = len == p.G;
+        float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (q * 4 >= p.M) continue;
+          const float4 f = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+          if (whole)
+            batch_store4<ACT>(p, tile * 128 + nl, lane, q * 4, f);
+          else
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(sums + q * 128), "f"(f.x), "f"(f.y),
+                         "f"(f.z), "f"(f.w)
+                         : "memory");
+        }
+        if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, 0, 1);
+        pos += len;
+      }
+    } else {
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
+      int seg = 0;
+      for (int pos = run0; pos < run1; ++seg) {
+        SEGMENT(pos)
+        if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
+                            len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
+        pos += len;
+      }
     }
   } else if (warp == W_ACT) {
     // ================= TMA producer: activations =================
@@ -415,8 +485,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const __half* sc = p.scales + (size_t)(p.rpg == 1 ? g / groups_per_row : g * p.rpg) * p.N + tile * 128;
       uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
       for (int pos = run0; pos < run1; ++pos) {
-        if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
-        const uint32_t bar = BAR_ADDR(g_full, stage);
+        if (!mbar_wait_abortable(EXACT ? BAR_ADDR(s_empty, stage) : BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = EXACT ? BAR_ADDR(s_full, stage) : BAR_ADDR(g_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(sc_bytes * (uint32_t)p.rpg)
                      : "memory");
         for (int i = 0; i < p.rpg; ++i)
@@ -436,7 +506,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       }
       if (!good) {
         for (int i = max(0, n_issued - WS); i < n_issued; ++i)
-          mbar_wait_bounded(BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
+          mbar_wait_bounded(EXACT ? BAR_ADDR(s_full, i % WS) : BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
       }
     }
   } else {
@@ -448,26 +518,28 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const int nslots = BATCH_SETS * sps;
       uint32_t slot_phase = 0, a_phase = 0;
       // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
-      // the look (twice 100 cycles) lies under them; only a group that was not ready then is waited for
+      // the looks (100 cycles each) lies under them; only a group that was not ready then is waited for
       bool ready = false;
       for (int pos = run0; pos < run1 && good; ++seg) {
         SEGMENT(pos)
-        if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        if (!EXACT && !mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d_t = tmem + (uint32_t)((seg & 1) * batch_d_stride(NR));
         for (int i = 0; i < len && good; ++i) {
           if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), slot_phase, abort_flag) ||
+                         (EXACT && !mbar_wait_abortable(BAR_ADDR(x_empty, slot), slot_phase ^ 1u, abort_flag)) ||
                          !mbar_wait_abortable(BAR_ADDR(a_full, stage), a_phase, abort_flag))) { good = false; break; }
           const int slot1 = slot + 1 == nslots ? 0 : slot + 1, stage1 = stage + 1 == AS ? 0 : stage + 1;
           const uint32_t slot_phase1 = slot_phase ^ (slot1 == 0 ? 1u : 0u), a_phase1 = a_phase ^ (stage1 == 0 ? 1u : 0u);
           const bool next0 = mbar_test(BAR_ADDR(slot_full, slot1), slot_phase1);
           const bool next1 = mbar_test(BAR_ADDR(a_full, stage1), a_phase1);
+          const bool next2 = !EXACT || mbar_test(BAR_ADDR(x_empty, slot1), slot_phase1 ^ 1u);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)stage * ASTAGE);
           const uint32_t a_t = slots_t + (uint32_t)(slot * 64), half = ASTAGE >> 5;  // second block, in 16-byte units
+          const uint32_t d_t = tmem + (uint32_t)(EXACT ? slot * 16 : (seg & 1) * batch_d_stride(NR));
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t accumulate = (i > 0 || ks > 0) ? 1u : 0u;
+            const uint32_t accumulate = ((!EXACT && i > 0) || ks > 0) ? 1u : 0u;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, %4, 0;\n\t"
@@ -479,10 +551,10 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(done, slot))
                        : "memory");
-          ready = next0 && next1;
+          ready = next0 && next1 && next2;
           slot = slot1; slot_phase = slot_phase1; stage = stage1; a_phase = a_phase1;
         }
-        if (good)
+        if (!EXACT && good)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(d_full, seg & 1))
                        : "memory");
@@ -503,15 +575,15 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   }
   if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
   }
 #undef BAR_ADDR
 #undef SEGMENT
 }
 
-template <int VAR, int ACT>
+template <int VAR, int ACT, bool EXACT>
 static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
-  auto kern = batch_kernel<VAR, ACT>;
+  auto kern = batch_kernel<VAR, ACT, EXACT>;
   static int configured_smem[16] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -537,9 +609,13 @@ template <int VAR>
 static cudaError_t batch_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
                                     cudaStream_t stream) {
   if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
-    if (var == VAR)
-      return p.act == 0 ? batch_launch_one<VAR, 0>(p, tmaps, smem_bytes, stream)
-                        : batch_launch_one<VAR, 1>(p, tmaps, smem_bytes, stream);
+    if (var == VAR) {
+      if (p.exact)
+        return p.act == 0 ? batch_launch_one<VAR, 0, true>(p, tmaps, smem_bytes, stream)
+                          : batch_launch_one<VAR, 1, true>(p, tmaps, smem_bytes, stream);
+      return p.act == 0 ? batch_launch_one<VAR, 0, false>(p, tmaps, smem_bytes, stream)
+                        : batch_launch_one<VAR, 1, false>(p, tmaps, smem_bytes, stream);
+    }
   }
   if constexpr (VAR + 1 < VAR_COUNT) return batch_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
   else return cudaErrorInvalidValue;
@@ -565,7 +641,7 @@ int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
 // (4096 x 4096, 16 rows: 8.2 -> 6.4 us against twice the stages without a neighbour).
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {
   const int cap = rows <= 64 ? 113 * 1024 : max_smem;
-  *a_stages = rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
+  *a_stages = rows <= 16 ? BATCH_SETS * EXACT_SPS : rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
   int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
   while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg) > cap) st -= BATCH_SETS;
   *stages = st;

@@ -150,6 +150,7 @@ struct BatchParams {
   int a_stages;          // 128-row activation groups in shared memory
   int grid;              // CTAs: each takes an equal contiguous run of work units
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
+  int exact;             // up to 16 rows, one scale row per 128-row group at most: scales applied to the sums in fp32
 };
 
 // ---- dequantize kernel -----------------------------------------------------------------------

@@ -96,6 +96,16 @@ B200Q_HD constexpr int int_target(int b, int h) {
   return 10 - b;
 }
 
+// The same for a bf16 pattern, whose mantissa has 7 bits (b <= 7).
+B200Q_HD constexpr int int_target_bf16(int b, int h) {
+  const int p0 = plane_width(b, 0);
+  const int t0 = (h % (16 / p0)) * p0 - plane_lo(b, 0);
+  if (t0 >= 0 && t0 + b <= 7) return t0;
+  if (t0 - 8 >= 0 && t0 - 8 + b <= 7) return t0 - 8;
+  if (t0 < 0) return 0;
+  return 7 - b;
+}
+
 template <int B, int H, int T, int I>
 struct GatherPlanes {
   static B200Q_HD uint32_t run(const uint32_t* w, uint32_t acc) {
@@ -214,22 +224,54 @@ __device__ __forceinline__ __half2 pair_value(const uint32_t* w) {
   }
 }
 
-// pair H times the scale, in the arithmetic of the activation dtype.  ACT 0: one fp16 multiply,
-// fp16_rn(value * s).  ACT 1: the value (at most 8 significant bits, so exact in bf16) is
-// converted fp16 -> fp32 -> bf16 without rounding and multiplied once in bf16, bf16_rn(value * s):
-// the reference's cast to the activation dtype followed by its elementwise multiply
+__device__ __forceinline__ __nv_bfloat162 bf2_from_bits(uint32_t x) { return *reinterpret_cast<__nv_bfloat162*>(&x); }
+__device__ __forceinline__ uint32_t bits_from_bf2(__nv_bfloat162 x) { return *reinterpret_cast<uint32_t*>(&x); }
+
+// bf16 pattern of a non-negative integer of at most 8 significant bits
+B200Q_HD constexpr uint32_t bf16_bits_of_uint(uint32_t v) {
+  if (v == 0) return 0;
+  int e = 0;
+  while ((2u << e) <= v) ++e;
+  return ((uint32_t)(127 + e) << 7) | (e <= 7 ? (v - (1u << e)) << (7 - e) : (v - (1u << e)) >> (e - 7));
+}
+
+// Exact value of pair H as bf16x2 (every type's values have at most 8 significant bits).  The fp16 recipe with
+// bf16's fields: integers of up to 7 bits are OR-ed into the mantissa of 128 (ulp 1) and rebased by one fma,
+// floats are placed over exponent and mantissa and rebased by one exact multiply.  8-bit integers do not
+// fit the mantissa and 5 exponent bits are fp16's own (with its Inf / NaN): these convert from fp16.
+template <int VAR, int H>
+__device__ __forceinline__ __nv_bfloat162 pair_value_bf16(const uint32_t* w) {
+  constexpr int B = var_bits(VAR);
+  if constexpr (!var_is_float(VAR) && B <= 7) {
+    constexpr int T = int_target_bf16(B, H);
+    constexpr uint32_t mul = dup16((uint32_t)(127 - T) << 7);                                           // 2^-T
+    constexpr uint32_t add = dup16(0x8000u | bf16_bits_of_uint((1u << (7 - T)) + var_bias(VAR)));  // -(2^(7-T) + bias)
+    return __hfma2(bf2_from_bits(gather_pair<B, H, T>(w, 0x43004300u)), bf2_from_bits(mul), bf2_from_bits(add));
+  } else if constexpr (var_is_float(VAR) && var_float_ebits(VAR) < 5) {
+    constexpr int E = var_float_ebits(VAR), M = B - 1 - E, T = 7 - M;
+    constexpr uint32_t mag = (((1u << (B - 1)) - 1u) << T) * 0x00010001u;
+    constexpr uint32_t mul = dup16((uint32_t)(254 - ((1 << (E - 1)) - 1)) << 7);  // 2^(127 - bias)
+    const uint32_t r = gather_pair<B, H, T>(w, 0u);
+    return __hmul2(bf2_from_bits((r & mag) | ((r << (15 - (T + B - 1))) & 0x80008000u)), bf2_from_bits(mul));
+  } else {
+    const float2 f = __half22float2(pair_value<VAR, H>(w));
+    return __floats2bfloat162_rn(f.x, f.y);
+  }
+}
+// exact value of pair H in the activation dtype (0 fp16, 1 bf16)
+template <int VAR, int H, int ACT>
+__device__ __forceinline__ uint32_t pair_exact(const uint32_t* w) {
+  if constexpr (ACT == 0) return bits_from_h2(pair_value<VAR, H>(w));
+  else return bits_from_bf2(pair_value_bf16<VAR, H>(w));
+}
+
+// pair H times the scale, one rounding in the activation dtype (ACT 0: fp16_rn(value * s), ACT 1:
+// bf16_rn(value * s)): the reference's cast to the activation dtype followed by its elementwise multiply
 // (examples/quantization/matmul_a16wx.py:316-320).  `scale2` holds the 16-bit scale in both halves.
 template <int VAR, int H, int ACT>
 __device__ __forceinline__ uint32_t pair_scaled(const uint32_t* w, uint32_t scale2) {
-  const __half2 v = pair_value<VAR, H>(w);
-  if constexpr (ACT == 0) {
-    return bits_from_h2(__hmul2(v, h2_from_bits(scale2)));
-  } else {
-    const float2 f = __half22float2(v);
-    const __nv_bfloat162 b = __floats2bfloat162_rn(f.x, f.y);
-    const __nv_bfloat162 r = __hmul2(b, *reinterpret_cast<const __nv_bfloat162*>(&scale2));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
+  if constexpr (ACT == 0) return bits_from_h2(__hmul2(pair_value<VAR, H>(w), h2_from_bits(scale2)));
+  else return bits_from_bf2(__hmul2(pair_value_bf16<VAR, H>(w), bf2_from_bits(scale2)));
 }
 
 template <int VAR, int H, int ACT>
@@ -239,6 +281,19 @@ struct UnitLoop {
     if constexpr (H + 1 < 16) UnitLoop<VAR, H + 1, ACT>::run(w, scale2, out);
   }
 };
+
+template <int VAR, int H, int ACT>
+struct UnitExactLoop {
+  static __device__ __forceinline__ void run(const uint32_t* w, uint32_t* out) {
+    out[H] = pair_exact<VAR, H, ACT>(w);
+    if constexpr (H + 1 < 16) UnitExactLoop<VAR, H + 1, ACT>::run(w, out);
+  }
+};
+// out[h] = exact values of pair h in the activation dtype, without the scale
+template <int VAR, int ACT>
+__device__ __forceinline__ void unit_decode_exact(const uint32_t* w, uint32_t* out) {
+  UnitExactLoop<VAR, 0, ACT>::run(w, out);
+}
 
 template <int VAR, int H>
 struct UnitLinLoop {
