@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
   // accumulator fragment of the first MMA of a group: [group][MT][j = 0..3] x {row 2j, row 2j+1, row 2j, row 2j+1}
   float* sNb = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(sA) + (size_t)p.M * p.pitch * 2 + 64);
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int r = lane >> 2, j = lane & 3;
   const int chunk = blockIdx.x % p.S, ci = blockIdx.x / p.S;
   const int kb_base = chunk * p.KBc;
@@ -233,12 +233,15 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
              (size_t)q * ITEM_BYTES;
   };
   if (cA > 0) cursor_set(tileA, qA); else cursor_set(tileB, qB);
-  auto issue_next = [&](uint32_t bar, uint32_t dst) {  // lane 0
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(ITEM_BYTES) : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(pc_src), "r"(ITEM_BYTES), "r"(bar)
-        : "memory");
+  // (the whole warp moves the cursor; the copy takes its operands from uniform registers, see elect_one)
+  auto issue_next = [&](uint32_t bar, uint32_t dst) {
+    if (elect_one()) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(ITEM_BYTES) : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+          "l"(pc_src), "r"(ITEM_BYTES), "r"(bar)
+          : "memory");
+    }
     if (++issued == cA) {
       cursor_set(tileB, qB);
     } else {
@@ -273,8 +276,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
-  if (lane == 0)
-    for (int s = 0; s < NST && issued < n_items; ++s) issue_next(bar0 + s * 8, ring_s + s * SLOT_BYTES);
+  for (int s = 0; s < NST && issued < n_items; ++s) issue_next(bar0 + s * 8, ring_s + s * SLOT_BYTES);
   // the first fill of the scale cache: requested now, stored after the activations have been
   // requested as well (a CTA that starts after its predecessor has finished then waits for the
   // two round trips at the same time, not one after the other)
@@ -582,9 +584,9 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
           unit_decode_linear<VAR>(w1, W1);
           if (gi == GI - 1) {
             // every lane has turned its copy of the item's last group into operands (the loads have
-            // returned: their values were used), so lane 0 may ask for the next item into this slot
+            // returned: their values were used), so the warp may ask for the next item into this slot
             __syncwarp();
-            if (lane == 0 && issued < n_items) issue_next(bar, ring_s + slot_off);
+            if (issued < n_items) issue_next(bar, ring_s + slot_off);
           }
           const uint32_t koff = (uint32_t)((g0 + gi) * 320);  // bytes: 128 columns + 4 x 8 of padding per group
           // two accumulation chains per 8-row tile; the first starts from the zero-point term of the group
