@@ -45,6 +45,8 @@ def _jobs():
     for part in range(NPARTS):
         jobs.append(("batch_kernel.cu", f"batch_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
     for part in range(NPARTS):
+        jobs.append(("exact_kernel.cu", f"exact_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
+    for part in range(NPARTS):
         jobs.append(("umma_kernel.cu", f"umma_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
     jobs.append(("dequant_kernel.cu", "dequant.o", []))
     jobs.append(("quantize_kernel.cu", "quantize.o", []))

@@ -38,6 +38,12 @@ B200Q_DECL_UPART(4) B200Q_DECL_UPART(5) B200Q_DECL_UPART(6) B200Q_DECL_UPART(7)
   cudaError_t batch_launch_part##i(int, const BatchParams&, const void*, int, cudaStream_t);
 B200Q_DECL_BPART(0) B200Q_DECL_BPART(1) B200Q_DECL_BPART(2) B200Q_DECL_BPART(3)
 B200Q_DECL_BPART(4) B200Q_DECL_BPART(5) B200Q_DECL_BPART(6) B200Q_DECL_BPART(7)
+#define B200Q_DECL_EPART(i) \
+  cudaError_t exact_launch_part##i(int, const BatchParams&, const void*, int, cudaStream_t);
+B200Q_DECL_EPART(0) B200Q_DECL_EPART(1) B200Q_DECL_EPART(2) B200Q_DECL_EPART(3)
+B200Q_DECL_EPART(4) B200Q_DECL_EPART(5) B200Q_DECL_EPART(6) B200Q_DECL_EPART(7)
+int exact_smem_bytes(int bits, int stages);
+int exact_stages(int bits);
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg);
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages);
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg);
@@ -68,6 +74,19 @@ static cudaError_t batch_launch(int var, const BatchParams& p, const void* tmap,
     case 5: return batch_launch_part5(var, p, tmap, smem, s);
     case 6: return batch_launch_part6(var, p, tmap, smem, s);
     default: return batch_launch_part7(var, p, tmap, smem, s);
+  }
+}
+
+static cudaError_t exact_launch(int var, const BatchParams& p, const void* tmap, int smem, cudaStream_t s) {
+  switch (var % B200Q_NPARTS) {
+    case 0: return exact_launch_part0(var, p, tmap, smem, s);
+    case 1: return exact_launch_part1(var, p, tmap, smem, s);
+    case 2: return exact_launch_part2(var, p, tmap, smem, s);
+    case 3: return exact_launch_part3(var, p, tmap, smem, s);
+    case 4: return exact_launch_part4(var, p, tmap, smem, s);
+    case 5: return exact_launch_part5(var, p, tmap, smem, s);
+    case 6: return exact_launch_part6(var, p, tmap, smem, s);
+    default: return exact_launch_part7(var, p, tmap, smem, s);
   }
 }
 
@@ -193,7 +212,8 @@ static int stream_ctas_per_chunk(int NT, int s, int per_sm, const DeviceInfo& di
     if (NT % c == 0) return c;
   return full > NT ? NT : full;
 }
-static const int kStreamMaxRows = 16;
+static const int kStreamMaxRows = 16;  // what the kernel takes
+static const int kStreamPlanRows = 8;  // what the plan gives it (gather launches and row tails: all of the above)
 static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counter_bytes(N) + (size_t)16 * N * sizeof(float); }
 // K is cut into S chunks (a divisor of K/512, at most one per SM) so that the activation chunk
 // [M, K/S] fits next to the rings; the grid is S * CPC.  Measured preferences, in this order: all of
@@ -291,19 +311,27 @@ static size_t batch_count_bytes(int N) { return ((size_t)((N + 127) / 128) * 32 
 static size_t batch_scratch_bytes(int M, int N) {
   return batch_count_bytes(N) + (size_t)((N + 127) / 128) * batch_rows(M) * 128 * sizeof(float);
 }
+// up to 16 rows with one scale per 128-row group at most: weights stay exact, scales go to the sums (exact_kernel.cu)
+static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; }
 static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
   const int n_tiles = (N + 127) / 128, G = K / 128;
   const long long groups = (long long)n_tiles * G;
   long long grid = (groups + 1) / 2;  // at least two groups per CTA
   if (grid > di.sm_count) grid = di.sm_count;
   pl->kernel = 3;
+  const bool exact = batch_exact(M, group);
   pl->m_tiles = 1;
   pl->splits = 1;
   pl->cluster = 1;
   pl->ctas_per_split = (int)grid;
-  int a_stages;
-  batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
-  pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group));
+  if (exact) {
+    pl->stages = exact_stages(bits);
+    pl->smem_bytes = exact_smem_bytes(bits, pl->stages);
+  } else {
+    int a_stages;
+    batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
+    pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group));
+  }
   pl->tile_m = batch_rows(M);
   pl->warps = 16;
   pl->passes = 1;
@@ -333,19 +361,24 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
   const DeviceInfo di = device_info();
   std::memset(pl, 0, sizeof(*pl));
   const int bits = var_bits(var);
-  // up to 16 rows: the mma.sync stream kernel (one weight decode per 16 x 128 tile feeds one or two
-  // 8-row activation tiles); above, the tcgen05 kernels
-  if (M <= kStreamMaxRows && stream_takes(K, group)) {
+  // Up to 8 rows the mma.sync stream kernel, whose second 8-row tile would double its staging and MMAs; above,
+  // the tcgen05 kernels (at 8 rows the two are within 5 % of each other, at 9 rows the second is 1.2 - 1.8 x faster).
+  if (M <= kStreamPlanRows && stream_takes(K, group)) {
     if (plan_stream(M, N, K, bits, di, pl) == ST_OK) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
       return ST_OK;
     }
   }
-  // up to 128 rows the small-batch kernel (weights streamed once); beyond, the prefill kernel
+  // up to 128 rows the small-batch kernels (weights streamed once); beyond, the prefill kernel
   if (M <= kBatchMaxRows) {
     plan_batch(M, N, K, bits, group, di, pl);
     pl->workspace_bytes = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M, N);
+    if (M <= kStreamMaxRows && stream_takes(K, group)) {  // the decode path's other form, see b200q_plan_t
+      pl->kernel = 2;
+      pl->m_tiles = 2;
+      if (pl->workspace_bytes < stream_workspace_bytes(N)) pl->workspace_bytes = stream_workspace_bytes(N);
+    }
     return ST_OK;
   } else {
     // A last row tile of at most 16 rows (M = 4097: one row) would cost a whole 256-row tile per
@@ -368,7 +401,11 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
   const int tail = umma_tail(tiles, grid, K / 64, pl->splits, N, &tail_splits);
   const size_t part = umma_partial_bytes(pl->splits > 1 ? tiles : tail, pl->tile_m);
   size_t need = WS_HEADER_BYTES + ws_counter_bytes(N) + part;
-  if (pl->passes == 2 && need < stream_workspace_bytes(N)) need = stream_workspace_bytes(N);
+  if (pl->passes == 2) {
+    const size_t rows = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M % 256, N);
+    if (need < stream_workspace_bytes(N)) need = stream_workspace_bytes(N);
+    if (need < rows) need = rows;
+  }
   pl->workspace_bytes = need;
   return ST_OK;
 }
@@ -529,13 +566,14 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   p.group = group;
   p.rpg = rpg_of(group);
   p.rows = rows;
+  const bool exact = batch_exact(M, group);
   batch_stages(bits, device_info().max_smem, rows, p.rpg, &p.stages, &p.a_stages);
+  if (exact) p.stages = exact_stages(bits);
   p.grid = (int)grid;
   p.act = act;
-  p.exact = rows == 16 && p.rpg == 1 ? 1 : 0;
-  const int smem = batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
+  const int smem = exact ? exact_smem_bytes(bits, p.stages) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
-  cudaError_t e = batch_launch(var, p, tmaps, smem, stream);
+  cudaError_t e = exact ? exact_launch(var, p, tmaps, smem, stream) : batch_launch(var, p, tmaps, smem, stream);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
   return ST_OK;
 }
@@ -644,6 +682,9 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
   return ST_OK;
 }
 
+// the form of the decode path (kernel 2) that exact_kernel.cu runs
+static bool plan_is_exact(const b200q_plan_t& pl) { return pl.tile_m == 16 && pl.splits == 1; }
+
 static int run_gemm(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
                     int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream,
                     const b200q_plan_t& pl) {
@@ -656,19 +697,21 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     const int tail = M % 256;
     if (M <= 256 || tail < 1 || tail > kStreamMaxRows) return ST_INVALID_ARG;
     b200q_plan_t tail_plan;
-    std::memset(&tail_plan, 0, sizeof(tail_plan));
-    if (plan_stream(tail, N, K, var_bits(var), device_info(), &tail_plan) != ST_OK) return ST_UNSUPPORTED;
+    int st = make_plan(tail, N, K, var, group, &tail_plan);
+    if (st != ST_OK) return st;
     b200q_plan_t head = pl;
     head.passes = 1;
-    const int st = run_umma(a, lda, bq, scales, c, ldc, M - tail, N, K, var, group, act, workspace, ws_bytes, stream, head);
+    st = run_umma(a, lda, bq, scales, c, ldc, M - tail, N, K, var, group, act, workspace, ws_bytes, stream, head);
     if (st != ST_OK) return st;
     const size_t row0 = (size_t)(M - tail);
-    return run_stream(reinterpret_cast<const unsigned short*>(a) + row0 * lda, lda, bq, scales,
-                      reinterpret_cast<unsigned short*>(c) + row0 * ldc, ldc, tail, N, K, var, group, act, workspace,
-                      ws_bytes, stream, tail_plan);
+    return run_gemm(reinterpret_cast<const unsigned short*>(a) + row0 * lda, lda, bq, scales,
+                    reinterpret_cast<unsigned short*>(c) + row0 * ldc, ldc, tail, N, K, var, group, act, workspace,
+                    ws_bytes, stream, tail_plan);
   }
   if (pl.kernel == 1)
     return run_umma(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+  if (pl.kernel == 2 && plan_is_exact(pl))
+    return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2)
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 3)
@@ -740,10 +783,8 @@ int b200q_gemm_gather(const void* a, int lda, const void* bq, const void* scales
   int var;
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
-  b200q_plan_t pl;
-  st = make_plan(M, N, K, var, group, &pl);  // the fused gather lives in the stream kernel only
-  if (st != ST_OK) return st;
-  if (pl.kernel != 2) return ST_UNSUPPORTED;
+  b200q_plan_t pl;  // the fused gather lives in the stream kernel only
+  if (!stream_takes(K, group) || plan_stream(M, N, K, var_bits(var), device_info(), &pl) != ST_OK) return ST_UNSUPPORTED;
   return run_stream(a, lda, bq, scales, nullptr, gather->ldc, M, N, K, var, group, act_dtype, workspace,
                     workspace_bytes, reinterpret_cast<cudaStream_t>(stream), pl, gather);
 }
@@ -880,8 +921,7 @@ int b200q_gemm_host(const void* a_host, int lda, const void* bq, const void* sca
     b200q_plan_t pl;
     cudaPointerAttributes cattr;
     if (check_problem(M, N, K, wtype, zero_point, group, true, &var) == ST_OK &&
-        make_plan(M, N, K, var, group, &pl) == ST_OK && pl.kernel == 2 && pl.passes == 1 &&
-        M <= stream_rows_per_pass(M) && pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M)) {
+        M <= kStreamMaxRows && stream_takes(K, group) && plan_stream(M, N, K, var_bits(var), device_info(), &pl) == ST_OK && pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M)) {
       if (cudaPointerGetAttributes(&cattr, c_host) == cudaSuccess && cattr.type == cudaMemoryTypeHost &&
           cattr.devicePointer && (((uintptr_t)cattr.devicePointer) & 15) == 0) {
         if (!bq || !scales) return ST_INVALID_ARG;
@@ -972,7 +1012,7 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
     // without when the scratch is too small (small batches; the prefill kernel's last round)
     const uint64_t least = pl.passes == 2 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
-    const bool optional = pl.kernel == 3 || (pl.kernel == 1 && pl.splits == 1);
+    const bool optional = pl.kernel == 3 || (pl.kernel == 2 && plan_is_exact(pl)) || (pl.kernel == 1 && pl.splits == 1);
     if (!(optional && least <= (uint64_t)B200Q_STATIC_WS_BYTES)) return ST_WORKSPACE;
   }
   void* ws = nullptr;

@@ -45,7 +45,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
-#include "umma_common.cuh"
+#include "batch_common.cuh"
 
 #ifndef B200Q_PART
 #define B200Q_PART 0
@@ -68,104 +68,13 @@ struct BatchBarriers {
   uint64_t a_full[BATCH_A_MAX];
   uint64_t g_full[BATCH_STAGES_MAX], g_empty[BATCH_STAGES_MAX];
   uint64_t d_full[2], d_empty[2];
-  uint64_t s_full[BATCH_STAGES_MAX], s_empty[BATCH_STAGES_MAX];  // EXACT: the scales' own ring
-  uint64_t x_empty[BATCH_SLOTS_MAX];                             // EXACT: [i]: the sums of slot i have been read
   uint32_t tmem_base;
   volatile int abort_flag;
 };
 
-// a ring stage: 128 columns x 128 rows of packed weights, and (in a region of their own) rpg rows of 128 scales
-__host__ __device__ constexpr int batch_stage_bytes(int bits, int rpg) { return 2048 * bits + 256 * rpg; }
-// widths whose stages are swizzled by 128-byte line (see above)
-__host__ __device__ constexpr bool batch_swizzled(int bits) { return bits == 2 || bits == 4 || bits == 8; }
 // tensor memory (all 512 columns): two D accumulators of nr columns, then as many operand slots as fit
 __host__ __device__ constexpr int batch_d_stride(int nr) { return nr <= 64 ? 64 : 128; }
 __host__ __device__ constexpr int batch_slots_per_set(int nr) { return nr <= 64 ? 3 : 2; }
-
-// 16 registers -> 16 consecutive tensor-memory columns of this thread's lane
-__device__ __forceinline__ void tmem_st_16(uint32_t taddr, const uint32_t (&o)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15, %16};" ::"r"(taddr),
-      "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(o[8]), "r"(o[9]),
-      "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15])
-      : "memory");
-}
-
-// Four rows (m .. m + 3) of one column per lane -> each lane stores four consecutive columns of one row.
-template <int ACT>
-__device__ __forceinline__ void batch_store4(const BatchParams& p, int n, int lane, int m, const float4& v) {
-  const bool b0 = lane & 1, b1 = lane & 2;
-  // two 16-bit rows per register, then two exchange rounds
-  const uint32_t r01 = pack2<ACT>(v.x, v.y), r23 = pack2<ACT>(v.z, v.w);
-  // round 1 (columns n and n ^ 1): even lane keeps rows 0 and 2, odd lane rows 1 and 3
-  const uint32_t o01 = __shfl_xor_sync(0xffffffffu, r01, 1), o23 = __shfl_xor_sync(0xffffffffu, r23, 1);
-  const uint32_t x0 = b0 ? __byte_perm(o01, r01, 0x7632) : __byte_perm(r01, o01, 0x5410);  // row 0 + b0
-  const uint32_t x2 = b0 ? __byte_perm(o23, r23, 0x7632) : __byte_perm(r23, o23, 0x5410);  // row 2 + b0
-  // round 2 (column pairs): lanes with b1 = 0 take row b0, those with b1 = 1 row 2 + b0
-  const uint32_t got = __shfl_xor_sync(0xffffffffu, b1 ? x0 : x2, 2);
-  const uint2 o = b1 ? make_uint2(got, x2) : make_uint2(x0, got);
-  const int row = m + (b1 ? 2 : 0) + (b0 ? 1 : 0);
-  if (row < p.M && n < p.N)
-    *reinterpret_cast<uint2*>(reinterpret_cast<unsigned short*>(p.c) + (size_t)row * p.ldc + (n & ~3)) = o;
-}
-
-// The 2 * B words of units 2h and 2h + 1 of column `nl` from a ring stage.
-template <int B>
-__device__ __forceinline__ void batch_load_units(uint32_t stage, int nl, int h, uint32_t (&w)[2 * B]) {
-  const uint32_t off = (uint32_t)((nl >> 4) * (256 * B) + (nl & 15) * (16 * B) + h * (8 * B));
-  if constexpr (batch_swizzled(B)) {
-    const uint32_t line = off >> 7;
-#pragma unroll
-    for (int q = 0; q < B / 2; ++q) {
-      const uint32_t chunk = ((off >> 4) + (uint32_t)q) & 7u;  // a block's chunks lie in one line
-      const uint4 v = lds_u4(stage + (line << 7) + ((chunk ^ (line & 7u)) << 4));
-      w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
-    }
-  } else {
-    lds_two_units<B>(stage + off, w);
-  }
-}
-
-// first group of CTA c's run
-__device__ __forceinline__ int batch_run_start(const BatchParams& p, int c) {
-  return (int)((long long)p.work * c / p.grid) * p.unit;
-}
-
-// Lane i's count says whether this warp's i-th 16-row chunk (chunk part + i * parts) of the tile's sums is
-// complete; the complete ones are converted, written to C and put back to zero.
-template <int ACT>
-__device__ __forceinline__ void batch_finish(const BatchParams& p, int tile, int len, int wq, int lane, int part, int parts) {
-  const int nl = wq * 32 + lane, n = tile * 128 + nl;
-  float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;  // [rows / 4][128] quads
-  int complete = 0;
-  const int chunk = part + lane * parts;
-  __syncwarp();
-  if (chunk * 16 < p.M) {
-    int* counter = p.chunk_counters + tile * 32 + wq * 8 + chunk;
-    __threadfence();  // cumulative over the warp's additions (ordered by the barrier above)
-    complete = atomicAdd(counter, len) + len == p.G ? 1 : 0;
-    if (complete) {
-      *counter = 0;
-      __threadfence();
-    }
-  }
-  unsigned mask = __ballot_sync(0xffffffffu, complete);
-  while (mask) {
-    const int mc0 = (part + (__ffs(mask) - 1) * parts) * 4;
-    mask &= mask - 1;
-    float4 x[4];  // independent loads
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if ((mc0 + u) * 4 < p.M) x[u] = __ldcg(sums + (mc0 + u) * 128);
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if ((mc0 + u) * 4 < p.M) {
-        __stcg(sums + (mc0 + u) * 128, make_float4(0.f, 0.f, 0.f, 0.f));
-        batch_store4<ACT>(p, n, lane, (mc0 + u) * 4, x[u]);
-      }
-  }
-}
 
 // The epilogue of one segment, shared out over `parts` groups of four warps (this warp belongs to group
 // `part`): rows in chunks of 16 from tensor memory, to C (a whole tile) or added into the tile's scratch.
@@ -203,14 +112,8 @@ __device__ __forceinline__ void batch_epilogue(const BatchParams& p, uint32_t d_
   if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, part, parts);
 }
 
-#ifndef EXACT_SPS
-#define EXACT_SPS 3
-#endif
-#ifndef EXACT_CTAS
-#define EXACT_CTAS 2
-#endif
-template <int VAR, int ACT, bool EXACT>
-__global__ void __launch_bounds__(BATCH_THREADS, EXACT ? EXACT_CTAS : 1)
+template <int VAR, int ACT>
+__global__ void __launch_bounds__(BATCH_THREADS, 1)
 batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
   constexpr int B = var_bits(VAR);
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -236,11 +139,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   if (tid == 0) {
     for (int i = 0; i < BATCH_SLOTS_MAX; ++i) { mbar_init(BAR_ADDR(slot_full, i), 4); mbar_init(BAR_ADDR(done, i), 1); }
     for (int i = 0; i < AS; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
-    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), EXACT ? 1 : 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
-    if (EXACT) {
-      for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(s_full, i), 1); mbar_init(BAR_ADDR(s_empty, i), 4); }
-      for (int i = 0; i < BATCH_SLOTS_MAX; ++i) mbar_init(BAR_ADDR(x_empty, i), 4);
-    }
+    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
     for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(d_full, i), 1); mbar_init(BAR_ADDR(d_empty, i), 4); }
     bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -253,13 +152,11 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
   constexpr int TM_THREADS = BATCH_SETS * 128 + 160;
-  constexpr int TM_COLS = EXACT && EXACT_SPS == 1 ? 256 : 512;
   constexpr int W_EPI = BATCH_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
                 W_SCALES = W_EPI + 7;
   if (warp == W_MMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base)),
-                 "r"(TM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -269,9 +166,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
   const uint32_t tmem = (warp < W_ACT || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
-  const int sps = EXACT ? EXACT_SPS : batch_slots_per_set(NR);
-  // EXACT: a 16-column accumulator per operand slot, then the slots
-  const uint32_t slots_t = tmem + (uint32_t)(EXACT ? 16 * BATCH_SLOTS_MAX : batch_d_stride(NR) * 2);
+  const int sps = batch_slots_per_set(NR);
+  const uint32_t slots_t = tmem + (uint32_t)(batch_d_stride(NR) * 2);
 
   // one segment of the run: pos -> tile, groups
 #define SEGMENT(pos)                                     \
@@ -293,16 +189,14 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
       const uint32_t sc = scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u;
       uint32_t w[2][2 * B], s2[4];
-      if constexpr (!EXACT) {
-        unsigned short sb;
-        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc));
-        s2[0] = s2[1] = s2[2] = s2[3] = (uint32_t)sb * 0x00010001u;  // the 16-bit scale in both halves
-        if (p.rpg > 1) {
+      unsigned short sb;
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc));
+      s2[0] = s2[1] = s2[2] = s2[3] = (uint32_t)sb * 0x00010001u;  // the 16-bit scale in both halves
+      if (p.rpg > 1) {
 #pragma unroll
-          for (int u = 1; u < 4; ++u) {
-            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc + (uint32_t)((u * p.rpg) >> 2) * 256u));
-            s2[u] = (uint32_t)sb * 0x00010001u;
-          }
+        for (int u = 1; u < 4; ++u) {
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(sc + (uint32_t)((u * p.rpg) >> 2) * 256u));
+          s2[u] = (uint32_t)sb * 0x00010001u;
         }
       }
 #pragma unroll
@@ -311,8 +205,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           uint32_t out[16];
-          if constexpr (EXACT) unit_decode_exact<VAR, ACT>(w[h] + u * B, out);
-          else unit_decode_scaled<VAR, ACT>(w[h] + u * B, s2[2 * h + u], out);
+          unit_decode_scaled<VAR, ACT>(w[h] + u * B, s2[2 * h + u], out);
           if (h == 0 && u == 0) {  // the MMAs have read what the set stored here before
             if (!mbar_wait_abortable(BAR_ADDR(done, slot), slot_phase, abort_flag)) { good = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -335,7 +228,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       stage += BATCH_SETS;
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
-    if (!EXACT && good) {
+    if (good) {
       int pos = run0, seg = 0;  // the last segment
       while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
@@ -350,67 +243,15 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     // ================= epilogue =================
     const int wq = warp & 3;
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
-    if constexpr (EXACT) {
-      // Each group's sums, times the group's scale in fp32, onto the segment's sums in registers.
-      const int nl = wq * 32 + lane;
-      int slot = 0, stage = 0;
-      uint32_t slot_phase = 0, s_phase = 0;
-      bool good = true, waited = false;
-      for (int pos = run0; pos < run1 && good;) {
-        SEGMENT(pos)
-        float acc[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-        for (int g = 0; g < len; ++g) {
-          if (!mbar_wait_abortable(BAR_ADDR(s_full, stage), s_phase, abort_flag)) { good = false; break; }
-          unsigned short sb;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u));
-          if (!mbar_wait_abortable(BAR_ADDR(done, slot), slot_phase, abort_flag)) { good = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          uint32_t v[16];
-          tmem_ld_16(tmem + lane_t + (uint32_t)(slot * 16), v);
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          const float sf = ACT == 0 ? __half2float(__ushort_as_half(sb)) : __uint_as_float((uint32_t)sb << 16);
-          __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(BAR_ADDR(x_empty, slot));
-            mbar_arrive(BAR_ADDR(s_empty, stage));
-          }
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[i] = fmaf(sf, __uint_as_float(v[i]), acc[i]);
-          if (++slot == BATCH_SETS * sps) { slot = 0; slot_phase ^= 1u; }
-          if (++stage == WS) { stage = 0; s_phase ^= 1u; }
-        }
-        if (!good) break;
-        if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use
-        waited = true;
-        const bool whole = len == p.G;
-        float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q * 4 >= p.M) continue;
-          const float4 f = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-          if (whole)
-            batch_store4<ACT>(p, tile * 128 + nl, lane, q * 4, f);
-          else
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(sums + q * 128), "f"(f.x), "f"(f.y),
-                         "f"(f.z), "f"(f.w)
-                         : "memory");
-        }
-        if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, 0, 1);
-        pos += len;
-      }
-    } else {
-      asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
-      int seg = 0;
-      for (int pos = run0; pos < run1; ++seg) {
-        SEGMENT(pos)
-        if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
-                            len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
-        pos += len;
-      }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
+    int seg = 0;
+    for (int pos = run0; pos < run1; ++seg) {
+      SEGMENT(pos)
+      if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
+                          len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
+      pos += len;
     }
   } else if (warp == W_ACT) {
     // ================= TMA producer: activations =================
@@ -485,8 +326,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const __half* sc = p.scales + (size_t)(p.rpg == 1 ? g / groups_per_row : g * p.rpg) * p.N + tile * 128;
       uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
       for (int pos = run0; pos < run1; ++pos) {
-        if (!mbar_wait_abortable(EXACT ? BAR_ADDR(s_empty, stage) : BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
-        const uint32_t bar = EXACT ? BAR_ADDR(s_full, stage) : BAR_ADDR(g_full, stage);
+        if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = BAR_ADDR(g_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(sc_bytes * (uint32_t)p.rpg)
                      : "memory");
         for (int i = 0; i < p.rpg; ++i)
@@ -506,7 +347,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       }
       if (!good) {
         for (int i = max(0, n_issued - WS); i < n_issued; ++i)
-          mbar_wait_bounded(EXACT ? BAR_ADDR(s_full, i % WS) : BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
+          mbar_wait_bounded(BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
       }
     }
   } else {
@@ -518,28 +359,26 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       const int nslots = BATCH_SETS * sps;
       uint32_t slot_phase = 0, a_phase = 0;
       // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
-      // the looks (100 cycles each) lies under them; only a group that was not ready then is waited for
+      // the look (twice 100 cycles) lies under them; only a group that was not ready then is waited for
       bool ready = false;
       for (int pos = run0; pos < run1 && good; ++seg) {
         SEGMENT(pos)
-        if (!EXACT && !mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t d_t = tmem + (uint32_t)((seg & 1) * batch_d_stride(NR));
         for (int i = 0; i < len && good; ++i) {
           if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), slot_phase, abort_flag) ||
-                         (EXACT && !mbar_wait_abortable(BAR_ADDR(x_empty, slot), slot_phase ^ 1u, abort_flag)) ||
                          !mbar_wait_abortable(BAR_ADDR(a_full, stage), a_phase, abort_flag))) { good = false; break; }
           const int slot1 = slot + 1 == nslots ? 0 : slot + 1, stage1 = stage + 1 == AS ? 0 : stage + 1;
           const uint32_t slot_phase1 = slot_phase ^ (slot1 == 0 ? 1u : 0u), a_phase1 = a_phase ^ (stage1 == 0 ? 1u : 0u);
           const bool next0 = mbar_test(BAR_ADDR(slot_full, slot1), slot_phase1);
           const bool next1 = mbar_test(BAR_ADDR(a_full, stage1), a_phase1);
-          const bool next2 = !EXACT || mbar_test(BAR_ADDR(x_empty, slot1), slot_phase1 ^ 1u);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)stage * ASTAGE);
           const uint32_t a_t = slots_t + (uint32_t)(slot * 64), half = ASTAGE >> 5;  // second block, in 16-byte units
-          const uint32_t d_t = tmem + (uint32_t)(EXACT ? slot * 16 : (seg & 1) * batch_d_stride(NR));
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t accumulate = ((!EXACT && i > 0) || ks > 0) ? 1u : 0u;
+            const uint32_t accumulate = (i > 0 || ks > 0) ? 1u : 0u;
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, %4, 0;\n\t"
@@ -551,10 +390,10 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(done, slot))
                        : "memory");
-          ready = next0 && next1 && next2;
+          ready = next0 && next1;
           slot = slot1; slot_phase = slot_phase1; stage = stage1; a_phase = a_phase1;
         }
-        if (!EXACT && good)
+        if (good)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(d_full, seg & 1))
                        : "memory");
@@ -575,15 +414,15 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   }
   if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
 #undef BAR_ADDR
 #undef SEGMENT
 }
 
-template <int VAR, int ACT, bool EXACT>
+template <int VAR, int ACT>
 static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
-  auto kern = batch_kernel<VAR, ACT, EXACT>;
+  auto kern = batch_kernel<VAR, ACT>;
   static int configured_smem[16] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -609,13 +448,9 @@ template <int VAR>
 static cudaError_t batch_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
                                     cudaStream_t stream) {
   if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
-    if (var == VAR) {
-      if (p.exact)
-        return p.act == 0 ? batch_launch_one<VAR, 0, true>(p, tmaps, smem_bytes, stream)
-                          : batch_launch_one<VAR, 1, true>(p, tmaps, smem_bytes, stream);
-      return p.act == 0 ? batch_launch_one<VAR, 0, false>(p, tmaps, smem_bytes, stream)
-                        : batch_launch_one<VAR, 1, false>(p, tmaps, smem_bytes, stream);
-    }
+    if (var == VAR)
+      return p.act == 0 ? batch_launch_one<VAR, 0>(p, tmaps, smem_bytes, stream)
+                        : batch_launch_one<VAR, 1>(p, tmaps, smem_bytes, stream);
   }
   if constexpr (VAR + 1 < VAR_COUNT) return batch_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
   else return cudaErrorInvalidValue;
@@ -641,7 +476,7 @@ int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
 // (4096 x 4096, 16 rows: 8.2 -> 6.4 us against twice the stages without a neighbour).
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {
   const int cap = rows <= 64 ? 113 * 1024 : max_smem;
-  *a_stages = rows <= 16 ? BATCH_SETS * EXACT_SPS : rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
+  *a_stages = rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
   int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
   while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg) > cap) st -= BATCH_SETS;
   *stages = st;

@@ -133,7 +133,7 @@ struct UmmaParams {
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
 };
 
-// ---- small-batch tcgen05 kernel (up to 128 rows): weights streamed once -------------------------
+// ---- small-batch tcgen05 kernels (up to 128 rows, batch_kernel.cu and exact_kernel.cu) ---------------
 struct BatchParams {
   const __half* scales;  // [K/group, N]
   __half* c;             // [M, N], leading dimension ldc (multiple of 8)
@@ -150,7 +150,6 @@ struct BatchParams {
   int a_stages;          // 128-row activation groups in shared memory
   int grid;              // CTAs: each takes an equal contiguous run of work units
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
-  int exact;             // up to 16 rows, one scale row per 128-row group at most: scales applied to the sums in fp32
 };
 
 // ---- dequantize kernel -----------------------------------------------------------------------

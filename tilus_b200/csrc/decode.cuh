@@ -295,6 +295,26 @@ __device__ __forceinline__ void unit_decode_exact(const uint32_t* w, uint32_t* o
   UnitExactLoop<VAR, 0, ACT>::run(w, out);
 }
 
+// The linear pattern of pair H with every code at the same place: an integer code at mantissa bit 0 of an fp16
+// subnormal (value code * 2^-24), a float code in its own fields (value * 2^-(15 - bias)).  No factor depends
+// on the pair, so the activations are taken as they are.
+template <int VAR, int H>
+__device__ __forceinline__ uint32_t pair_lin_uniform(const uint32_t* w) {
+  if constexpr (!var_is_float(VAR)) return gather_pair<var_bits(VAR), H, 0>(w, 0u);
+  else return pair_raw<VAR, H>(w);
+}
+template <int VAR, int H>
+struct UnitLinUniformLoop {
+  static __device__ __forceinline__ void run(const uint32_t* w, uint32_t* out) {
+    out[H] = pair_lin_uniform<VAR, H>(w);
+    if constexpr (H + 1 < 16) UnitLinUniformLoop<VAR, H + 1>::run(w, out);
+  }
+};
+template <int VAR>
+__device__ __forceinline__ void unit_decode_linear_uniform(const uint32_t* w, uint32_t* out) {
+  UnitLinUniformLoop<VAR, 0>::run(w, out);
+}
+
 template <int VAR, int H>
 struct UnitLinLoop {
   static __device__ __forceinline__ void run(const uint32_t* w, uint32_t* out) {

@@ -1,0 +1,454 @@
+// Batches of up to 16 rows on tcgen05: C[M, N] = A[M, K] x dequant(Bq[K, N]) with exact weights.
+//
+// Same product and work split as batch_kernel.cu (weights of 128 columns in tensor memory, equal runs of 128-row
+// groups per CTA), but the scale is not applied to the weights.  Every group's product is a sum of its own,
+// multiplied by the group's scale in fp32 when it is added to the column's sum - no weight is rounded, as in
+// stream_kernel.cu - and the decode shrinks to bit extraction:
+//   * fp16 activations: an integer code sits at bit 0 of an fp16 subnormal (value code * 2^-24), a float code
+//     in its own fields (decode.cuh, pair_lin_uniform).  The tensor core multiplies these exactly.  The zero
+//     point is subtracted by a second set of MMAs whose weight operand is the constant -zero_point * 2^-24;
+//   * bf16 activations: exact bf16 values (pair_exact; bf16 has no room for the subnormal trick).
+// That is what decides this kernel's speed: integer, shift and half instructions issue every second cycle
+// per SM quadrant on this GPU (measured: LOP3, SHF, PRMT, HFMA2 2.0 cycles, LOP3 + HFMA2 3.7 together, FFMA 1.0),
+// and a 128 x 128 group of 4-bit weights costs 112 of them per thread here against 208 with scaled weights.
+// The HBM time of such a group is 355 cycles per SM.
+//
+// Roles of the 16 warps of a CTA:
+//   * warps 0-7 decode, in two sets of four (lane L of a set's four warps is column L of the tile); set s takes
+//     the groups s, s + 2, ... of the CTA's run, three operand slots each.  Before a set stores into a slot
+//     it reads the sums of the group that was there (16 columns of tensor memory) and adds them, times their
+//     scale, to its fp32 sums of the column: one wait serves the slot and the sums;
+//   * warps 8-11 finish column tiles: the sets hand over their sums through shared memory, so that the
+//     decoding goes on while a tile's last contributions are counted and written;
+//   * warp 12 brings the activations, warp 13 the packed weights, warp 15 the scales (one elected thread each);
+//   * warp 14 owns tensor memory and issues the MMAs: 8 (or 16 with a zero point) per group, one commit.
+//
+// Measured (4-bit, group 128, 16 rows, a chain of launches; stream_kernel.cu before): 28672 x 4096 37.2 -> 20.6 us,
+// 8192 x 8192 19.0 -> 14.2, 4096 x 4096 10.1 -> 7.9.  Without the decode the first takes 17.4 us, without
+// decode and sums 15.6, against 9.4 us of HBM time: what is left is the start and the end of a launch
+// (about 5 us) and the decode's instructions.
+//
+// Every mbarrier wait is bounded in time; a wait that runs out raises a CTA-wide abort flag, all loops
+// leave, the producers give their copies in flight a bounded chance to land, tensor memory is freed and
+// the status word of the workspace reports it.
+#include <cuda.h>
+
+#include "batch_common.cuh"
+
+#ifndef B200Q_PART
+#define B200Q_PART 0
+#endif
+#ifndef B200Q_NPARTS
+#define B200Q_NPARTS 1
+#endif
+
+namespace b200q {
+
+constexpr int EXACT_THREADS = 512;
+constexpr int EXACT_SPS = 3;                 // operand slots per set
+constexpr int EXACT_SLOTS = 2 * EXACT_SPS;   // also: activation groups in shared memory
+constexpr int EXACT_STAGES_MAX = 16;         // 128-row groups in the packed ring (even)
+constexpr uint32_t EXACT_ASTAGE = 16 * 256;  // 16 rows x 128 columns, two swizzled 64-column blocks
+constexpr uint32_t EXACT_HAND = 16 * 128 * 4;  // a set's sums of one tile
+
+struct ExactBarriers {
+  uint64_t slot_full[EXACT_SLOTS];
+  uint64_t done[EXACT_SLOTS];  // [i]: the MMAs of a group in slot i have completed
+  uint64_t a_full[EXACT_SLOTS];
+  uint64_t g_full[EXACT_STAGES_MAX], g_empty[EXACT_STAGES_MAX];
+  uint64_t hand_full[2], hand_empty[2];  // a set's sums of a segment are in shared memory / have been taken
+  uint32_t tmem_base;
+  volatile int abort_flag;
+};
+
+template <int VAR, int ACT>
+__global__ void __launch_bounds__(EXACT_THREADS, 1)
+exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
+  constexpr int B = var_bits(VAR);
+  constexpr int BIAS = ACT == 0 ? var_bias(VAR) : 0;  // what the constant operand subtracts
+  constexpr float F = ACT == 0 ? (float)(1u << lin_factor_log2(VAR)) : 1.0f;
+  constexpr uint32_t WSTAGE = 2048u * B, SSTAGE = 256u;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t smem_unaligned = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  const uint32_t smem_base = (smem_unaligned + 1023u) & ~1023u;
+  unsigned char* smem_al = smem_raw + (smem_base - smem_unaligned);
+  const int WS = p.stages;
+  const uint32_t ring_s = smem_base + EXACT_SLOTS * EXACT_ASTAGE;
+  const uint32_t scales_s = ring_s + (uint32_t)WS * WSTAGE;
+  const uint32_t hand_off = EXACT_SLOTS * EXACT_ASTAGE + (uint32_t)WS * (WSTAGE + SSTAGE);
+  const uint32_t bars_off = hand_off + 2 * EXACT_HAND;
+  ExactBarriers* bars = reinterpret_cast<ExactBarriers*>(smem_al + bars_off);
+  const uint32_t bars_s = smem_base + bars_off;
+#define BAR_ADDR(field, i) (bars_s + (uint32_t)offsetof(ExactBarriers, field) + (uint32_t)(i) * 8u)
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  volatile int* abort_flag = &bars->abort_flag;
+  // this CTA's run of groups, counted tile by tile over the whole matrix
+  const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
+
+  if (tid == 0) {
+    for (int i = 0; i < EXACT_SLOTS; ++i) {
+      mbar_init(BAR_ADDR(slot_full, i), 4);
+      mbar_init(BAR_ADDR(done, i), 1);
+      mbar_init(BAR_ADDR(a_full, i), 1);
+    }
+    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(hand_full, i), 4); mbar_init(BAR_ADDR(hand_empty, i), 4); }
+    bars->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  __syncthreads();
+  // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
+  // this SM may still hold it)
+  constexpr int W_EPI = 8, W_ACT = 12, W_WEIGHTS = 13, W_MMA = 14;
+  if (warp == W_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     bars_s + (uint32_t)offsetof(ExactBarriers, tmem_base))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp < W_EPI || warp == W_MMA) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.sync 1, 288;" ::: "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
+  const uint32_t tmem = (warp < W_EPI || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
+  // tensor memory: 16 columns of sums per slot, 64 columns of weights per slot, 8 columns of the constant operand
+  const uint32_t slots_t = tmem + 16 * EXACT_SLOTS, const_t = slots_t + 64 * EXACT_SLOTS;
+
+  if (warp < W_EPI) {
+    // ================= decode =================
+    const int set = warp >> 2, wq = warp & 3;
+    const int nl = wq * 32 + lane;  // lane of tensor memory = column inside the tile
+    const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
+    if (BIAS != 0 && set == 0) {  // the constant operand: seen by the MMAs behind the first slot_full of set 0
+      const uint32_t v = dup16(0x8000u | (uint32_t)BIAS);  // -zero_point * 2^-24
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(const_t + lane_t),
+                   "r"(v)
+                   : "memory");
+    }
+    float acc[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+    float sq[EXACT_SPS];  // scales of the groups in the set's slots
+    int stage = set;      // the set's stages: set, set + 2, ...
+    uint32_t ring_phase = 0, hand_phase = 1;
+    const int n_own = (run1 - run0 - set + 1) / 2;
+    const bool more = p.M > 4, most = p.M > 8;
+    int seg_end = min((run0 / p.G + 1) * p.G, run1);  // of the segment the sums belong to
+    int pos = run0 + set;                             // group whose sums are added next
+    while (pos >= seg_end && seg_end < run1) seg_end = min(seg_end + p.G, run1);  // (a first segment of one group)
+    bool good = true;
+    for (int i0 = 0; i0 < n_own + EXACT_SPS && good; i0 += EXACT_SPS) {
+#pragma unroll
+      for (int j = 0; j < EXACT_SPS; ++j) {
+        const int i = i0 + j, slot = set + 2 * j;
+        const bool have = i < n_own;
+        if (i >= EXACT_SPS && i - EXACT_SPS < n_own) {
+          // the group this slot held: its sums, times its scale
+          if (!mbar_wait_abortable(BAR_ADDR(done, slot), (uint32_t)(i / EXACT_SPS - 1) & 1u, abort_flag)) { good = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t d_t = tmem + lane_t + (uint32_t)(slot * 16);
+          uint32_t v[16];
+          tmem_ld_4_async(d_t, v);
+          if (more) tmem_ld_4_async(d_t + 4, v + 4);
+          if (most) tmem_ld_8_async(d_t + 8, v + 8);
+          tmem_ld_wait(v);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[q] = fmaf(sq[j], __uint_as_float(v[q]), acc[q]);
+          if (more) {
+#pragma unroll
+            for (int q = 4; q < 8; ++q) acc[q] = fmaf(sq[j], __uint_as_float(v[q]), acc[q]);
+          }
+          if (most) {
+#pragma unroll
+            for (int q = 8; q < 16; ++q) acc[q] = fmaf(sq[j], __uint_as_float(v[q]), acc[q]);
+          }
+          if (pos + 2 >= seg_end) {  // the set's last group of the column tile: hand the sums over
+            if (!mbar_wait_abortable(BAR_ADDR(hand_empty, set), hand_phase, abort_flag)) { good = false; break; }
+            hand_phase ^= 1u;
+            float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)set * EXACT_HAND) + nl;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              if (q * 4 < p.M) hand[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+              acc[4 * q] = acc[4 * q + 1] = acc[4 * q + 2] = acc[4 * q + 3] = 0.f;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR_ADDR(hand_full, set));
+            // (a segment of one group that the other set holds has nothing of this set: passed over)
+            do seg_end = min(seg_end + p.G, run1); while (pos + 2 >= seg_end && seg_end < run1);
+          }
+          pos += 2;
+        }
+        if (have) {
+          if (!mbar_wait_abortable(BAR_ADDR(g_full, stage), ring_phase, abort_flag)) { good = false; break; }
+          const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
+          unsigned short sb;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sb) : "r"(scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u));
+          uint32_t w[2][2 * B];
+          batch_load_units<B>(st, nl, 0, w[0]);
+          if (B <= 4) batch_load_units<B>(st, nl, 1, w[1]);
+          sq[j] = (ACT == 0 ? __half2float(__ushort_as_half(sb)) : __uint_as_float((uint32_t)sb << 16)) * F;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (B > 4 && u == 2) batch_load_units<B>(st, nl, 1, w[1]);
+            uint32_t out[16];
+            if constexpr (ACT == 0) unit_decode_linear_uniform<VAR>(w[u >> 1] + (u & 1) * B, out);
+            else unit_decode_exact<VAR, ACT>(w[u >> 1] + (u & 1) * B, out);
+            if (u == 3) {  // the stage has been read (its values fed the arithmetic above)
+              __syncwarp();
+              if (lane == 0) mbar_arrive(BAR_ADDR(g_empty, stage));
+            }
+            tmem_st_16(slots_t + lane_t + (uint32_t)(slot * 64 + u * 16), out);
+          }
+          stage += 2;
+          if (stage >= WS) { stage = set; ring_phase ^= 1u; }
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(BAR_ADDR(slot_full, slot));
+        }
+      }
+    }
+  } else if (warp < W_ACT) {
+    // ================= column tiles: sums of both sets, to C or to the tile's scratch =================
+    const int wq = warp & 3, nl = wq * 32 + lane;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
+    uint32_t phase[2] = {0u, 0u};
+    bool good = true;
+    for (int pos = run0; pos < run1 && good;) {
+      const int tile = pos / p.G, len = min((tile + 1) * p.G, run1) - pos;
+      float4 f[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) f[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int set = 0; set < 2; ++set) {
+        if (len == 1 && ((pos - run0) & 1) != set) continue;
+        if (!mbar_wait_abortable(BAR_ADDR(hand_full, set), phase[set], abort_flag)) { good = false; break; }
+        phase[set] ^= 1u;
+        const float4* hand = reinterpret_cast<const float4*>(smem_al + hand_off + (uint32_t)set * EXACT_HAND) + nl;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (q * 4 < p.M) {
+            const float4 x = hand[q * 128];
+            f[q].x += x.x; f[q].y += x.y; f[q].z += x.z; f[q].w += x.w;
+          }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(BAR_ADDR(hand_empty, set));
+      }
+      if (!good) break;
+      const bool whole = len == p.G;
+      float4* sums = reinterpret_cast<float4*>(p.partial) + (size_t)tile * (p.rows * 32) + nl;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q * 4 >= p.M) continue;
+        if (whole)
+          batch_store4<ACT>(p, tile * 128 + nl, lane, q * 4, f[q]);
+        else
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(sums + q * 128), "f"(f[q].x), "f"(f[q].y),
+                       "f"(f[q].z), "f"(f[q].w)
+                       : "memory");
+      }
+      if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, 0, 1);
+      pos += len;
+    }
+  } else if (warp == W_ACT) {
+    // ================= TMA producer: activations =================
+    if (elect_one()) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      int stage = 0, n_issued = 0;
+      uint32_t phase = 1;  // of the group that held the stage, whose MMAs report on its slot's barrier
+      bool good = true;
+      int g = run0 % p.G;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (n_issued >= EXACT_SLOTS && !mbar_wait_abortable(BAR_ADDR(done, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = BAR_ADDR(a_full, stage);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(EXACT_ASTAGE) : "memory");
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile(
+              "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+              ::"r"(smem_base + (uint32_t)stage * EXACT_ASTAGE + (uint32_t)h * (EXACT_ASTAGE / 2)), "l"(&tmap_a), "r"(bar),
+              "r"(g * 128 + h * 64), "r"(0)
+              : "memory");
+        ++n_issued;
+        if (++stage == EXACT_SLOTS) { stage = 0; phase ^= 1u; }
+        if (++g == p.G) g = 0;
+      }
+      if (!good) {  // a copy in flight must not outlive the CTA: a bounded wait for the groups issued last
+        for (int i = max(0, n_issued - EXACT_SLOTS); i < n_issued; ++i)
+          mbar_wait_bounded(BAR_ADDR(a_full, i % EXACT_SLOTS), (uint32_t)(i / EXACT_SLOTS) & 1u);
+      }
+    }
+  } else if (warp != W_MMA) {
+    // ================= TMA producers: packed weights (warp 13), scales (warp 15) =================
+    if (elect_one()) {
+      const bool weights = warp == W_WEIGHTS;
+      int stage = 0, n_issued = 0;
+      uint32_t phase = 1;
+      bool good = true;
+      int tile = run0 / p.G, g = run0 - tile * p.G;
+      const int groups_per_row = p.group / 128;  // 128-row groups per scale row
+      int in_row = g % groups_per_row;
+      const __half* sc = p.scales + (size_t)(g / groups_per_row) * p.N + tile * 128;
+      uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
+        const uint32_t bar = BAR_ADDR(g_full, stage);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(weights ? WSTAGE : sc_bytes)
+                     : "memory");
+        if (weights)  // (pieces past the last column are filled with zeros and count as bytes all the same)
+          asm volatile(
+              "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+              ::"r"(ring_s + (uint32_t)stage * WSTAGE), "l"(&tmap_w), "r"(bar), "r"(0),
+              "r"(batch_swizzled(B) ? g * (2 * B) : g), "r"(tile * 8)
+              : "memory");
+        else
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                  scales_s + (uint32_t)stage * SSTAGE),
+              "l"(sc), "r"(sc_bytes), "r"(bar)
+              : "memory");
+        ++n_issued;
+        if (++in_row == groups_per_row) { in_row = 0; sc += p.N; }
+        if (++g == p.G) {
+          g = 0; in_row = 0; ++tile;
+          sc = p.scales + tile * 128;
+          sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
+        }
+        if (++stage == WS) { stage = 0; phase ^= 1u; }
+      }
+      if (!good) {
+        for (int i = max(0, n_issued - WS); i < n_issued; ++i)
+          mbar_wait_bounded(BAR_ADDR(g_full, i % WS), (uint32_t)(i / WS) & 1u);
+      }
+    }
+  } else {
+    // ================= MMA issuer =================
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc<ACT>(16);
+      int slot = 0;
+      uint32_t phase = 0;
+      // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
+      // the looks lies under them; only a group that was not ready then is waited for
+      bool ready = false;
+      for (int pos = run0; pos < run1; ++pos) {
+        if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), phase, abort_flag) ||
+                       !mbar_wait_abortable(BAR_ADDR(a_full, slot), phase, abort_flag))) break;
+        const int slot1 = slot + 1 == EXACT_SLOTS ? 0 : slot + 1;
+        const uint32_t phase1 = phase ^ (slot1 == 0 ? 1u : 0u);
+        const bool next0 = mbar_test(BAR_ADDR(slot_full, slot1), phase1);
+        const bool next1 = mbar_test(BAR_ADDR(a_full, slot1), phase1);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)slot * EXACT_ASTAGE);
+        const uint32_t a_t = slots_t + (uint32_t)(slot * 64), d_t = tmem + (uint32_t)(slot * 16);
+#pragma unroll
+        for (int ks = 0; ks < (BIAS != 0 ? 16 : 8); ++ks) {
+          const uint64_t bd = bdesc + (uint64_t)((ks & 3) * 2) + ((ks & 4) ? EXACT_ASTAGE >> 5 : 0u);
+          if (ks == 0)
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, 0, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                ::"r"(d_t), "r"(a_t), "l"(bd), "r"(idesc)
+                : "memory");
+          else
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.eq.b32 p, 0, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                ::"r"(d_t), "r"(ks < 8 ? a_t + (uint32_t)(ks * 8) : const_t), "l"(bd), "r"(idesc)
+                : "memory");
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         BAR_ADDR(done, slot))
+                     : "memory");
+        ready = next0 && next1;
+        slot = slot1; phase = phase1;
+      }
+    }
+  }
+
+  // ================= teardown =================
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*abort_flag && tid == 0) {
+    atomicExch(p.status, ST_DEVICE_TIMEOUT);
+    p.status[1] = 10;  // where: exact small-batch kernel pipeline
+    p.status[2] = blockIdx.x;
+    p.status[3] = 0;
+  }
+  if (warp == W_MMA) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+#undef BAR_ADDR
+}
+
+template <int VAR, int ACT>
+static cudaError_t exact_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
+  auto kern = exact_kernel<VAR, ACT>;
+  static int configured_smem[16] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
+  cfg.blockDim = dim3(EXACT_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, p, tmaps[0], tmaps[1]);
+}
+
+template <int VAR>
+static cudaError_t exact_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
+                                    cudaStream_t stream) {
+  if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
+    if (var == VAR)
+      return p.act == 0 ? exact_launch_one<VAR, 0>(p, tmaps, smem_bytes, stream)
+                        : exact_launch_one<VAR, 1>(p, tmaps, smem_bytes, stream);
+  }
+  if constexpr (VAR + 1 < VAR_COUNT) return exact_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
+  else return cudaErrorInvalidValue;
+}
+
+#define B200Q_CAT2(a, b) a##b
+#define B200Q_CAT(a, b) B200Q_CAT2(a, b)
+
+// One of these per compiled part; api.cu picks the part as var % B200Q_NPARTS.
+cudaError_t B200Q_CAT(exact_launch_part, B200Q_PART)(int var, const BatchParams& p, const void* tmaps, int smem_bytes,
+                                                     cudaStream_t stream) {
+  return exact_launch_var<0>(var, p, reinterpret_cast<const CUtensorMap*>(tmaps), smem_bytes, stream);
+}
+
+#if B200Q_PART == 0
+// dynamic shared memory: alignment slack + activation groups + packed ring with scales + handed sums + barriers
+int exact_smem_bytes(int bits, int stages) {
+  return 1024 + EXACT_SLOTS * (int)EXACT_ASTAGE + stages * batch_stage_bytes(bits, 1) + 2 * (int)EXACT_HAND +
+         (int)sizeof(ExactBarriers);
+}
+// Ring stages (even) within half an SM's shared memory: the next launch of the stream becomes resident beside
+// this one and fills its ring while this one ends.
+int exact_stages(int bits) {
+  int st = EXACT_STAGES_MAX;
+  while (st > 2 && exact_smem_bytes(bits, st) > 113 * 1024) st -= 2;
+  return st;
+}
+#endif
+
+}  // namespace b200q
