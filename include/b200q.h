@@ -57,7 +57,8 @@ typedef struct b200q_plan {
                             once (M <= 128), 1 = tcgen05 kernel for larger M */
   int32_t m_tiles;       /* kernel 2: 8-row activation tiles per pass (1 or 2); kernels 1, 3: tiles along M */
   int32_t splits;        /* k chunks (kernel 2) / split-K factor (kernel 1); kernel 3: 1 */
-  int32_t cluster;       /* 1 (no kernel launches clusters) */
+  int32_t cluster;       /* kernel 3 and the tcgen05 form of kernel 2: CTAs that share a column tile's K and add up
+                            in distributed shared memory (ctas_per_split = column tiles * cluster); else 1 */
   int32_t ctas_per_split;/* kernel 2: CTAs per k chunk, grid = splits * ctas_per_split; kernel 3: CTAs;
                             kernel 1: output tiles */
   int32_t smem_bytes;    /* dynamic shared memory per CTA */

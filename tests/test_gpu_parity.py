@@ -330,3 +330,15 @@ def test_small_batch_kernel_ring_depths(M, dt, zp, group):
     c, _, _ = _run(prob)
     ref = qo.quantized_matmul(prob["a"].numpy(), prob["codes"].numpy(), prob["scales"].numpy(), dt, group, zp)
     assert _rel_err(c, ref) <= REL_TOL
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 64, 128])
+@pytest.mark.parametrize("N,K,cluster", [(4096, 4096, 4), (8192, 2048, 2), (400, 2176, 8), (5760, 1152, 3), (272, 640, 2)])
+def test_small_batch_kernels_cluster_form(M, N, K, cluster):
+    """Column tiles shared by the CTAs of a cluster: K ranges of unequal length, ragged last column tiles, row
+    quads that do not divide among the CTAs - against the oracle, twice, and against equal runs."""
+    dt = D.int4b
+    tiles = (N + 127) // 128
+    assert K // 128 >= 2 * cluster
+    _forced(M, N, K, dt, 0, dict(splits=1, cluster=cluster, ctas_per_split=tiles * cluster), seed=M + N)
+    _forced(M, N, K, dt, 0, dict(splits=1, cluster=1, ctas_per_split=min(148, tiles * (K // 128))), seed=M + N)

@@ -44,6 +44,7 @@ B200Q_DECL_EPART(0) B200Q_DECL_EPART(1) B200Q_DECL_EPART(2) B200Q_DECL_EPART(3)
 B200Q_DECL_EPART(4) B200Q_DECL_EPART(5) B200Q_DECL_EPART(6) B200Q_DECL_EPART(7)
 int exact_smem_bytes(int bits, int stages);
 int exact_stages(int bits);
+int batch_max_clusters(int c);
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg);
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages);
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg);
@@ -305,6 +306,7 @@ static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo
 
 // small-batch tcgen05 kernel (kernel 3): equal runs of (128-column tile, 128-row group) pairs, one CTA per SM
 static const int kBatchMaxRows = 128;
+static const int kOneCtaSmem = 116 * 1024;  // more than half an SM
 static int batch_rows(int M) { return (M + 15) / 16 * 16; }
 // arrival counts and fp32 sums of the column tiles
 static size_t batch_count_bytes(int N) { return ((size_t)((N + 127) / 128) * 32 * sizeof(int) + 255) / 256 * 256; }
@@ -313,17 +315,52 @@ static size_t batch_scratch_bytes(int M, int N) {
 }
 // up to 16 rows with one scale per 128-row group at most: weights stay exact, scales go to the sums (exact_kernel.cu)
 static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; }
-static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
-  const int n_tiles = (N + 127) / 128, G = K / 128;
-  const long long groups = (long long)n_tiles * G;
-  long long grid = (groups + 1) / 2;  // at least two groups per CTA
+// How the column tiles are shared out, as (CTAs, CTAs per cluster):
+//  - equal runs of 128-row groups, one per SM: no SM idles, but the tiles' sums meet in L2;
+//  - a cluster of c CTAs per tile: sums meet in distributed shared memory (at most as many tiles as clusters fit);
+//  - one CTA per tile.
+// The times are fits to chains of launches on B200 (4-bit weights, us; 2048^2 .. 4096 x 14336, 16 .. 128 rows, each
+// form forced; within 15 %).  Fewer CTAs start and end cheaper because the next launch finds SMs free.
+static int max_clusters(int c) {
+  static int cache[16][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { (void)cudaGetLastError(); dev = -1; }
+  if (dev >= 0 && dev < 16 && cache[dev][c] > 0) return cache[dev][c] - 1;
+  static const int typical[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  const int n = dev >= 0 ? batch_max_clusters(c) : 0;
+  if (n <= 0) return typical[c];
+  if (dev < 16) cache[dev][c] = n + 1;
+  return n;
+}
+static void batch_split(int M, int group, int n_tiles, int G, const DeviceInfo& di, int* ctas, int* cluster) {
+  long long grid = ((long long)n_tiles * G + 1) / 2;  // at least two groups per CTA
   if (grid > di.sm_count) grid = di.sm_count;
+  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * ((double)n_tiles * G / grid);
+  *ctas = (int)grid;
+  *cluster = 1;
+  // (kernels whose CTAs share SMs stay with equal runs: CTAs of such launches must not meet two to an SM while
+  // others idle; the exact kernel's registers allow one CTA per SM)
+  const bool one_per_sm = batch_exact(M, group) || !batch_shares_sm(batch_rows(M));
+  for (int c = 1; c <= 8 && one_per_sm; ++c) {
+    if ((c > 1 && G < 2 * c) || n_tiles * c > di.sm_count || (c > 1 && n_tiles > max_clusters(c))) continue;
+    const double start = 0.05 * (n_tiles * c) - 1.1;
+    const double t = (start > 2.3 ? start : 2.3) + 0.033 * M + 0.29 * ((G + c - 1) / c);
+    if (t < best) {
+      best = t;
+      *ctas = n_tiles * c;
+      *cluster = c;
+    }
+  }
+}
+static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
+  int ctas, cluster;
+  batch_split(M, group, (N + 127) / 128, K / 128, di, &ctas, &cluster);
   pl->kernel = 3;
   const bool exact = batch_exact(M, group);
   pl->m_tiles = 1;
   pl->splits = 1;
-  pl->cluster = 1;
-  pl->ctas_per_split = (int)grid;
+  pl->cluster = cluster;
+  pl->ctas_per_split = ctas;
   if (exact) {
     pl->stages = exact_stages(bits);
     pl->smem_bytes = exact_smem_bytes(bits, pl->stages);
@@ -332,6 +369,7 @@ static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInf
     batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
     pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group));
   }
+  if (!exact && !batch_shares_sm(batch_rows(M)) && pl->smem_bytes < kOneCtaSmem) pl->smem_bytes = kOneCtaSmem;
   pl->tile_m = batch_rows(M);
   pl->warps = 16;
   pl->passes = 1;
@@ -535,7 +573,11 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   long long grid = (long long)pl.splits * pl.ctas_per_split;
   if (grid > device_info().sm_count) grid = device_info().sm_count;
   if (grid > p.work) grid = p.work;
-  if (ws_bytes < fixed + batch_scratch_bytes(M, N)) {  // a caller with a smaller workspace: whole tiles need none
+  // the plan's clusters, unless the caller has asked for another number of CTAs
+  p.cluster = pl.cluster > 1 && pl.cluster <= 8 && grid == (long long)n_tiles * pl.cluster && G >= 2 * pl.cluster ? pl.cluster : 1;
+  if (p.cluster > 1) {
+    // (distributed shared memory needs no scratch)
+  } else if (ws_bytes < fixed + batch_scratch_bytes(M, N)) {  // a caller with a smaller workspace: whole tiles need none
     p.work = n_tiles;
     p.unit = G;
     grid = n_tiles < device_info().sm_count ? n_tiles : device_info().sm_count;
@@ -571,7 +613,8 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   if (exact) p.stages = exact_stages(bits);
   p.grid = (int)grid;
   p.act = act;
-  const int smem = exact ? exact_smem_bytes(bits, p.stages) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
+  int smem = exact ? exact_smem_bytes(bits, p.stages) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
+  if (!exact && (p.cluster > 1 || !batch_shares_sm(rows)) && smem < kOneCtaSmem) smem = kOneCtaSmem;
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
   cudaError_t e = exact ? exact_launch(var, p, tmaps, smem, stream) : batch_launch(var, p, tmaps, smem, stream);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }

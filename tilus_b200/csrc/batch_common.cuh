@@ -59,7 +59,58 @@ __device__ __forceinline__ void batch_load_units(uint32_t stage, int nl, int h, 
 
 // first group of CTA c's run
 __device__ __forceinline__ int batch_run_start(const BatchParams& p, int c) {
+  if (p.cluster > 1) return (c / p.cluster) * p.G + (c % p.cluster) * p.G / p.cluster;
   return (int)((long long)p.work * c / p.grid) * p.unit;
+}
+
+// ---- column tiles shared by the CTAs of a cluster ------------------------------------------------
+// Cluster form of a launch (p.cluster > 1): a cluster owns one column tile, its CTAs equal ranges of K.  Every CTA
+// leaves its sums in its own shared memory, [quad of four rows][128 columns] float4, and gives its tensor
+// memory back BEFORE it waits for the others (another CTA of the cluster may share the SM and wait for that
+// memory).  The rows are cut into quads of four; CTA o adds up the quads [Q * o / c, Q * (o + 1) / c) of all
+// CTAs in rank order and writes C.
+__device__ __forceinline__ void cluster_arrive() {  // orders shared memory accesses before it
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 cluster_load4(uint32_t smem_addr, int rank) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_addr), "r"(rank));
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+// This CTA's quads, dealt over `parts` groups of four warps.  The sums of CTA r lie at sums_s (the same address
+// in every CTA), `sets` of them set_bytes apart.
+template <int ACT>
+__device__ __forceinline__ void cluster_finish(const BatchParams& p, uint32_t sums_s, int sets, uint32_t set_bytes, int rank,
+                                               int tile, int nl, int lane, int part, int parts) {
+  const int quads = (p.M + 3) / 4;
+  const int first = quads * rank / p.cluster, last = quads * (rank + 1) / p.cluster;
+  for (int q = first + part; q < last; q += parts) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < p.cluster; r += 2) {  // two CTAs' loads in flight
+      float4 x[2][2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (r + u < p.cluster && t < sets)
+            x[u][t] = cluster_load4(sums_s + (uint32_t)t * set_bytes + (uint32_t)(q * 2048 + nl * 16), r + u);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+          if (r + u < p.cluster && t < sets) {
+            sum.x += x[u][t].x; sum.y += x[u][t].y; sum.z += x[u][t].z; sum.w += x[u][t].w;
+          }
+    }
+    batch_store4<ACT>(p, tile * 128 + nl, lane, q * 4, sum);
+  }
 }
 
 // Lane i's count says whether this warp's i-th 16-row chunk (chunk part + i * parts) of the tile's sums is

@@ -32,7 +32,10 @@
 // contiguous runs, one per CTA, whatever the shape.  A run covers at most one tile's end, whole
 // tiles, and one tile's start.  Whole tiles are written to C; a partial tile's sums are added into an
 // fp32 scratch tile (red.global.add.v4) and counted in, and whoever completes the count converts them,
-// writes C and puts the scratch back to zero (batch_epilogue).
+// writes C and puts the scratch back to zero (batch_epilogue).  These additions are the price of the form:
+// 4.8 MB of them at 64 rows keep L2 busy for 6 us.  Where the column tiles are few enough that every one can have
+// a cluster of CTAs to itself, the launch takes the cluster form instead (batch_common.cuh; the rule is in
+// api.cu).
 //
 // Measured (4-bit, group 128, a chain of launches; the kernel before it wrote dequantized weights to
 // 256-column shared-memory operands): 64 x 28672 x 4096 44.1 -> 23.4 us, 64 x 8192 x 8192 27.6 -> 16.4,
@@ -147,7 +150,6 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
   }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncthreads();
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
@@ -159,6 +161,10 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
                      bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    // Only now may the next launch start: a CTA of it that got this SM's tensor memory first would wait for this
+    // launch to complete, and this launch for the tensor memory.  (With this order a launch whose CTAs wait for
+    // their predecessor never holds tensor memory that the predecessor still has to get, on whatever streams.)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
   if (warp < W_ACT || warp == W_MMA) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -228,7 +234,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       stage += BATCH_SETS;
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
-    if (good) {
+    if (good && p.cluster <= 1) {
       int pos = run0, seg = 0;  // the last segment
       while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
@@ -245,7 +251,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
     int seg = 0;
-    for (int pos = run0; pos < run1; ++seg) {
+    for (int pos = run0; pos < run1 && p.cluster <= 1; ++seg) {
       SEGMENT(pos)
       if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -402,6 +408,25 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     }
   }
 
+  if (p.cluster > 1 && warp < W_ACT) {
+    // the tile's sums to shared memory, over activations and ring (all MMAs have completed: nobody reads them)
+    __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
+    if (mbar_wait_abortable(BAR_ADDR(d_full, 0), 0, abort_flag)) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float4* sums = reinterpret_cast<float4*>(smem_al) + (warp & 3) * 32 + lane;
+      for (int c0 = (warp >> 2) * 16; c0 < p.M; c0 += 48) {
+        uint32_t v[16];
+        tmem_ld_16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c0 + 4 * i < p.M)
+            sums[(c0 / 4 + i) * 128] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                   __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
+      }
+    }
+  }
+
   // ================= teardown =================
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -415,6 +440,15 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+  if (p.cluster > 1) {
+    cluster_arrive();
+    cluster_wait();
+    if (warp < W_ACT && !*abort_flag)
+      cluster_finish<ACT>(p, smem_base, 1, 0u, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
+                          warp >> 2, 3);
+    cluster_arrive();  // nobody leaves while its sums are being read
+    cluster_wait();
   }
 #undef BAR_ADDR
 #undef SEGMENT
@@ -436,11 +470,15 @@ static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tma
   cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, p, tmaps[0], tmaps[1]);
 }
 
@@ -466,17 +504,39 @@ cudaError_t B200Q_CAT(batch_launch_part, B200Q_PART)(int var, const BatchParams&
 }
 
 #if B200Q_PART == 0
+// clusters of c CTAs that the current device holds at a time with one CTA per SM; 0 without a device
+int batch_max_clusters(int c) {
+  auto kern = batch_kernel<0, 0>;
+  const int smem = 200 * 1024;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)c, 1, 1);
+  cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)c;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  return n;
+}
 // dynamic shared memory: alignment slack + activation groups + packed ring + scales + barriers
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
   return 1024 + a_stages * rows * 256 + stages * batch_stage_bytes(bits, rpg) + (int)sizeof(BatchBarriers);
 }
 // Activation groups (at most as many as there are operand slots) and ring stages (a multiple of the dequantize
-// sets) in the rest.  Batches of up to 64 rows stay within half an SM's shared memory, so that the next
-// launch of the stream becomes resident beside this one and fills its ring while this one ends
-// (4096 x 4096, 16 rows: 8.2 -> 6.4 us against twice the stages without a neighbour).
+// sets) in the rest.  Up to 32 rows a CTA stays within half an SM's shared memory, so that the next launch of the
+// stream becomes resident beside this one and fills its ring while this one ends (a Llama-3-8B block of
+// linears at 32 rows: 51 us, 56 with one CTA per SM).  Above, a CTA takes more than half: the activations leave
+// too little for the ring, and launches that leave SMs free (clusters, one CTA per column tile) would meet others
+// two to an SM, where one waits for the other's tensor memory (64 rows: 81 us with the two kinds mixed, 62).
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {
-  const int cap = rows <= 64 ? 113 * 1024 : max_smem;
-  *a_stages = rows <= 32 ? 6 : (rows <= 64 ? 3 : 4);
+  const int cap = batch_shares_sm(rows) ? 113 * 1024 : max_smem;
+  *a_stages = rows <= 64 ? 6 : 4;
   int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
   while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg) > cap) st -= BATCH_SETS;
   *stages = st;

@@ -149,8 +149,12 @@ struct BatchParams {
   int stages;            // packed 128-row groups in the shared-memory ring
   int a_stages;          // 128-row activation groups in shared memory
   int grid;              // CTAs: each takes an equal contiguous run of work units
+  int cluster;           // > 1: CTAs per column tile, which share its K and add up in distributed shared memory
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
 };
+
+// batch_kernel.cu: whether two CTAs share an SM (see batch_stages)
+inline bool batch_shares_sm(int rows) { return rows <= 32; }
 
 // ---- dequantize kernel -----------------------------------------------------------------------
 struct DequantParams {

@@ -101,7 +101,6 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
   }
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __syncthreads();
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
@@ -111,6 +110,10 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
                      bars_s + (uint32_t)offsetof(ExactBarriers, tmem_base))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    // Only now may the next launch start: a CTA of it that got this SM's tensor memory first would wait for this
+    // launch to complete, and this launch for the tensor memory.  (With this order a launch whose CTAs wait for
+    // their predecessor never holds tensor memory that the predecessor still has to get, on whatever streams.)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
   if (warp < W_EPI || warp == W_MMA) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -121,25 +124,26 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   // tensor memory: 16 columns of sums per slot, 64 columns of weights per slot, 8 columns of the constant operand
   const uint32_t slots_t = tmem + 16 * EXACT_SLOTS, const_t = slots_t + 64 * EXACT_SLOTS;
 
+  float acc[16];  // decode warps: this column's sums
   if (warp < W_EPI) {
     // ================= decode =================
     const int set = warp >> 2, wq = warp & 3;
     const int nl = wq * 32 + lane;  // lane of tensor memory = column inside the tile
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
     if (BIAS != 0 && set == 0) {  // the constant operand: seen by the MMAs behind the first slot_full of set 0
       const uint32_t v = dup16(0x8000u | (uint32_t)BIAS);  // -zero_point * 2^-24
       asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(const_t + lane_t),
                    "r"(v)
                    : "memory");
     }
-    float acc[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
     float sq[EXACT_SPS];  // scales of the groups in the set's slots
     int stage = set;      // the set's stages: set, set + 2, ...
     uint32_t ring_phase = 0, hand_phase = 1;
     const int n_own = (run1 - run0 - set + 1) / 2;
     const bool more = p.M > 4, most = p.M > 8;
+    const bool alone = p.cluster <= 1;
     int seg_end = min((run0 / p.G + 1) * p.G, run1);  // of the segment the sums belong to
     int pos = run0 + set;                             // group whose sums are added next
     while (pos >= seg_end && seg_end < run1) seg_end = min(seg_end + p.G, run1);  // (a first segment of one group)
@@ -169,7 +173,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 #pragma unroll
             for (int q = 8; q < 16; ++q) acc[q] = fmaf(sq[j], __uint_as_float(v[q]), acc[q]);
           }
-          if (pos + 2 >= seg_end) {  // the set's last group of the column tile: hand the sums over
+          if (alone && pos + 2 >= seg_end) {  // the set's last group of the column tile: hand the sums over
             if (!mbar_wait_abortable(BAR_ADDR(hand_empty, set), hand_phase, abort_flag)) { good = false; break; }
             hand_phase ^= 1u;
             float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)set * EXACT_HAND) + nl;
@@ -221,7 +225,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
     uint32_t phase[2] = {0u, 0u};
     bool good = true;
-    for (int pos = run0; pos < run1 && good;) {
+    for (int pos = run0; pos < run1 && good && p.cluster <= 1;) {
       const int tile = pos / p.G, len = min((tile + 1) * p.G, run1) - pos;
       float4 f[4];
 #pragma unroll
@@ -374,6 +378,16 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     }
   }
 
+  if (p.cluster > 1 && warp < W_EPI) {
+    // the tile's sums to the set's hand-over buffer
+    __syncwarp();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
+    float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)(warp >> 2) * EXACT_HAND) + (warp & 3) * 32 + lane;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (q * 4 < p.M) hand[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+  }
+
   // ================= teardown =================
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -387,6 +401,15 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+  if (p.cluster > 1) {
+    cluster_arrive();
+    cluster_wait();
+    if (warp < W_EPI && !*abort_flag)
+      cluster_finish<ACT>(p, smem_base + hand_off, 2, EXACT_HAND, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
+                          warp >> 2, 2);
+    cluster_arrive();  // nobody leaves while its sums are being read
+    cluster_wait();
   }
 #undef BAR_ADDR
 }
@@ -407,11 +430,15 @@ static cudaError_t exact_launch_one(const BatchParams& p, const CUtensorMap* tma
   cfg.blockDim = dim3(EXACT_THREADS, 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, p, tmaps[0], tmaps[1]);
 }
 
