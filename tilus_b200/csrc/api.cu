@@ -42,8 +42,8 @@ B200Q_DECL_BPART(4) B200Q_DECL_BPART(5) B200Q_DECL_BPART(6) B200Q_DECL_BPART(7)
   cudaError_t exact_launch_part##i(int, const BatchParams&, const void*, int, cudaStream_t);
 B200Q_DECL_EPART(0) B200Q_DECL_EPART(1) B200Q_DECL_EPART(2) B200Q_DECL_EPART(3)
 B200Q_DECL_EPART(4) B200Q_DECL_EPART(5) B200Q_DECL_EPART(6) B200Q_DECL_EPART(7)
-int exact_smem_bytes(int bits, int stages);
-int exact_stages(int bits);
+int exact_smem_bytes(int bits, int stages, int M);
+int exact_stages(int bits, int max_smem, int M);
 int batch_max_clusters(int c);
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg);
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages);
@@ -214,7 +214,7 @@ static int stream_ctas_per_chunk(int NT, int s, int per_sm, const DeviceInfo& di
   return full > NT ? NT : full;
 }
 static const int kStreamMaxRows = 16;  // what the kernel takes
-static const int kStreamPlanRows = 8;  // what the plan gives it (gather launches and row tails: all of the above)
+static const int kStreamPlanRows = 4;  // what the plan gives it (gather launches and row tails: all of the above)
 static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counter_bytes(N) + (size_t)16 * N * sizeof(float); }
 // K is cut into S chunks (a divisor of K/512, at most one per SM) so that the activation chunk
 // [M, K/S] fits next to the rings; the grid is S * CPC.  Measured preferences, in this order: all of
@@ -362,8 +362,8 @@ static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInf
   pl->cluster = cluster;
   pl->ctas_per_split = ctas;
   if (exact) {
-    pl->stages = exact_stages(bits);
-    pl->smem_bytes = exact_smem_bytes(bits, pl->stages);
+    pl->stages = exact_stages(bits, di.max_smem, M);
+    pl->smem_bytes = exact_smem_bytes(bits, pl->stages, M);
   } else {
     int a_stages;
     batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
@@ -371,7 +371,7 @@ static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInf
   }
   if (!exact && !batch_shares_sm(batch_rows(M)) && pl->smem_bytes < kOneCtaSmem) pl->smem_bytes = kOneCtaSmem;
   pl->tile_m = batch_rows(M);
-  pl->warps = 16;
+  pl->warps = exact ? 20 : 16;
   pl->passes = 1;
   pl->pdl = 1;  // always launched as a programmatic dependent
 }
@@ -399,8 +399,10 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
   const DeviceInfo di = device_info();
   std::memset(pl, 0, sizeof(*pl));
   const int bits = var_bits(var);
-  // Up to 8 rows the mma.sync stream kernel, whose second 8-row tile would double its staging and MMAs; above,
-  // the tcgen05 kernels (at 8 rows the two are within 5 % of each other, at 9 rows the second is 1.2 - 1.8 x faster).
+  // Up to 4 rows the mma.sync stream kernel; above, the tcgen05 kernels, whose cost hardly depends on the rows.  A
+  // Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 / 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8
+  // rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's second 8-row tile doubles
+  // its staging and MMAs.
   if (M <= kStreamPlanRows && stream_takes(K, group)) {
     if (plan_stream(M, N, K, bits, di, pl) == ST_OK) {
       pl->passes = 1;
@@ -414,7 +416,7 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
     pl->workspace_bytes = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M, N);
     if (M <= kStreamMaxRows && stream_takes(K, group)) {  // the decode path's other form, see b200q_plan_t
       pl->kernel = 2;
-      pl->m_tiles = 2;
+      pl->m_tiles = stream_mt(M);
       if (pl->workspace_bytes < stream_workspace_bytes(N)) pl->workspace_bytes = stream_workspace_bytes(N);
     }
     return ST_OK;
@@ -610,10 +612,10 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   p.rows = rows;
   const bool exact = batch_exact(M, group);
   batch_stages(bits, device_info().max_smem, rows, p.rpg, &p.stages, &p.a_stages);
-  if (exact) p.stages = exact_stages(bits);
+  if (exact) p.stages = exact_stages(bits, device_info().max_smem, M);
   p.grid = (int)grid;
   p.act = act;
-  int smem = exact ? exact_smem_bytes(bits, p.stages) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
+  int smem = exact ? exact_smem_bytes(bits, p.stages, M) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
   if (!exact && (p.cluster > 1 || !batch_shares_sm(rows)) && smem < kOneCtaSmem) smem = kOneCtaSmem;
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
   cudaError_t e = exact ? exact_launch(var, p, tmaps, smem, stream) : batch_launch(var, p, tmaps, smem, stream);
@@ -753,6 +755,13 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   }
   if (pl.kernel == 1)
     return run_umma(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+  if (pl.kernel == 2 && plan_is_exact(pl) && act == B200Q_BF16 && M <= 8) {
+    // bf16 costs the exact kernel one more half instruction per pair of weights and the stream kernel only a
+    // conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit)
+    b200q_plan_t rows;
+    if (plan_stream(M, N, K, var_bits(var), device_info(), &rows) == ST_OK && ws_bytes >= stream_workspace_bytes(N))
+      return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, rows);
+  }
   if (pl.kernel == 2 && plan_is_exact(pl))
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2)
@@ -1055,7 +1064,7 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
     // without when the scratch is too small (small batches; the prefill kernel's last round)
     const uint64_t least = pl.passes == 2 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
-    const bool optional = pl.kernel == 3 || (pl.kernel == 2 && plan_is_exact(pl)) || (pl.kernel == 1 && pl.splits == 1);
+    const bool optional = pl.kernel == 3 || (pl.kernel == 1 && pl.splits == 1);
     if (!(optional && least <= (uint64_t)B200Q_STATIC_WS_BYTES)) return ST_WORKSPACE;
   }
   void* ws = nullptr;

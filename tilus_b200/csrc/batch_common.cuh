@@ -85,27 +85,27 @@ __device__ __forceinline__ float4 cluster_load4(uint32_t smem_addr, int rank) {
   return v;
 }
 // This CTA's quads, dealt over `parts` groups of four warps.  The sums of CTA r lie at sums_s (the same address
-// in every CTA), `sets` of them set_bytes apart.
-template <int ACT>
-__device__ __forceinline__ void cluster_finish(const BatchParams& p, uint32_t sums_s, int sets, uint32_t set_bytes, int rank,
+// in every CTA), SETS of them set_bytes apart.
+template <int ACT, int SETS>
+__device__ __forceinline__ void cluster_finish(const BatchParams& p, uint32_t sums_s, uint32_t set_bytes, int rank,
                                                int tile, int nl, int lane, int part, int parts) {
   const int quads = (p.M + 3) / 4;
   const int first = quads * rank / p.cluster, last = quads * (rank + 1) / p.cluster;
   for (int q = first + part; q < last; q += parts) {
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int r = 0; r < p.cluster; r += 2) {  // two CTAs' loads in flight
-      float4 x[2][2];
+      float4 x[2][SETS];
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-          if (r + u < p.cluster && t < sets)
+        for (int t = 0; t < SETS; ++t)
+          if (r + u < p.cluster)
             x[u][t] = cluster_load4(sums_s + (uint32_t)t * set_bytes + (uint32_t)(q * 2048 + nl * 16), r + u);
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-          if (r + u < p.cluster && t < sets) {
+        for (int t = 0; t < SETS; ++t)
+          if (r + u < p.cluster) {
             sum.x += x[u][t].x; sum.y += x[u][t].y; sum.z += x[u][t].z; sum.w += x[u][t].w;
           }
     }

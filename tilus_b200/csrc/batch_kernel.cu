@@ -445,7 +445,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     cluster_arrive();
     cluster_wait();
     if (warp < W_ACT && !*abort_flag)
-      cluster_finish<ACT>(p, smem_base, 1, 0u, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
+      cluster_finish<ACT, 1>(p, smem_base, 0u, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
                           warp >> 2, 3);
     cluster_arrive();  // nobody leaves while its sums are being read
     cluster_wait();

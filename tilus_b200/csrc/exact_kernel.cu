@@ -13,15 +13,17 @@
 // and a 128 x 128 group of 4-bit weights costs 112 of them per thread here against 208 with scaled weights.
 // The HBM time of such a group is 355 cycles per SM.
 //
-// Roles of the 16 warps of a CTA:
-//   * warps 0-7 decode, in two sets of four (lane L of a set's four warps is column L of the tile); set s takes
-//     the groups s, s + 2, ... of the CTA's run, three operand slots each.  Before a set stores into a slot
+// Roles of the warps of a CTA (20 of them; one CTA per SM):
+//   * warps 0-11 decode, in three sets of four (lane L of a set's four warps is column L of the tile); set s takes
+//     the groups s, s + 3, ... of the CTA's run, two operand slots each.  Before a set stores into a slot
 //     it reads the sums of the group that was there (16 columns of tensor memory) and adds them, times their
-//     scale, to its fp32 sums of the column: one wait serves the slot and the sums;
-//   * warps 8-11 finish column tiles: the sets hand over their sums through shared memory, so that the
+//     scale, to its fp32 sums of the column: one wait serves the slot and the sums.  A set needs about 1200
+//     cycles per group, most of them latencies of its barriers and of tensor memory, so their number sets the
+//     rate of narrow weights (two sets with three slots each: 13.8 us for 8192 x 8192 of 1 .. 4 bits);
+//   * four warps finish column tiles: the sets hand over their sums through shared memory, so that the
 //     decoding goes on while a tile's last contributions are counted and written;
-//   * warp 12 brings the activations, warp 13 the packed weights, warp 15 the scales (one elected thread each);
-//   * warp 14 owns tensor memory and issues the MMAs: 8 (or 16 with a zero point) per group, one commit.
+//   * one warp each (one elected thread) brings the activations, the packed weights, the scales;
+//   * one warp owns tensor memory and issues the MMAs: 8 (or 16 with a zero point) per group, one commit.
 //
 // Measured (4-bit, group 128, 16 rows, a chain of launches; stream_kernel.cu before): 28672 x 4096 37.2 -> 20.6 us,
 // 8192 x 8192 19.0 -> 14.2, 4096 x 4096 10.1 -> 7.9.  Without the decode the first takes 17.4 us, without
@@ -44,19 +46,21 @@
 
 namespace b200q {
 
-constexpr int EXACT_THREADS = 512;
-constexpr int EXACT_SPS = 3;                 // operand slots per set
-constexpr int EXACT_SLOTS = 2 * EXACT_SPS;   // also: activation groups in shared memory
-constexpr int EXACT_STAGES_MAX = 16;         // 128-row groups in the packed ring (even)
+constexpr int EXACT_SETS = 3;                // decode sets of four warps
+constexpr int EXACT_SPS = 2;                 // operand slots per set
+constexpr int EXACT_SLOTS = EXACT_SETS * EXACT_SPS;  // also: activation groups in shared memory
+constexpr int EXACT_THREADS = EXACT_SETS * 128 + 256;
+constexpr int EXACT_STAGES_MAX = 18;         // 128-row groups in the packed ring (a multiple of the sets)
 constexpr uint32_t EXACT_ASTAGE = 16 * 256;  // 16 rows x 128 columns, two swizzled 64-column blocks
-constexpr uint32_t EXACT_HAND = 16 * 128 * 4;  // a set's sums of one tile
+// a set's sums of one tile: quads of four rows x 128 columns
+__host__ __device__ constexpr uint32_t exact_hand_bytes(int M) { return (uint32_t)((M + 3) / 4) * 2048u; }
 
 struct ExactBarriers {
   uint64_t slot_full[EXACT_SLOTS];
   uint64_t done[EXACT_SLOTS];  // [i]: the MMAs of a group in slot i have completed
   uint64_t a_full[EXACT_SLOTS];
   uint64_t g_full[EXACT_STAGES_MAX], g_empty[EXACT_STAGES_MAX];
-  uint64_t hand_full[2], hand_empty[2];  // a set's sums of a segment are in shared memory / have been taken
+  uint64_t hand_full[EXACT_SETS], hand_empty[EXACT_SETS];  // a set's sums of a segment are in shared memory / have been taken
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -73,10 +77,11 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   const uint32_t smem_base = (smem_unaligned + 1023u) & ~1023u;
   unsigned char* smem_al = smem_raw + (smem_base - smem_unaligned);
   const int WS = p.stages;
+  const uint32_t HAND = exact_hand_bytes(p.M);
   const uint32_t ring_s = smem_base + EXACT_SLOTS * EXACT_ASTAGE;
   const uint32_t scales_s = ring_s + (uint32_t)WS * WSTAGE;
   const uint32_t hand_off = EXACT_SLOTS * EXACT_ASTAGE + (uint32_t)WS * (WSTAGE + SSTAGE);
-  const uint32_t bars_off = hand_off + 2 * EXACT_HAND;
+  const uint32_t bars_off = hand_off + EXACT_SETS * HAND;
   ExactBarriers* bars = reinterpret_cast<ExactBarriers*>(smem_al + bars_off);
   const uint32_t bars_s = smem_base + bars_off;
 #define BAR_ADDR(field, i) (bars_s + (uint32_t)offsetof(ExactBarriers, field) + (uint32_t)(i) * 8u)
@@ -94,7 +99,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       mbar_init(BAR_ADDR(a_full, i), 1);
     }
     for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
-    for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(hand_full, i), 4); mbar_init(BAR_ADDR(hand_empty, i), 4); }
+    for (int i = 0; i < EXACT_SETS; ++i) { mbar_init(BAR_ADDR(hand_full, i), 4); mbar_init(BAR_ADDR(hand_empty, i), 4); }
     bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -104,7 +109,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   __syncthreads();
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
-  constexpr int W_EPI = 8, W_ACT = 12, W_WEIGHTS = 13, W_MMA = 14;
+  constexpr int W_EPI = EXACT_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6;
   if (warp == W_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      bars_s + (uint32_t)offsetof(ExactBarriers, tmem_base))
@@ -117,7 +122,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   }
   if (warp < W_EPI || warp == W_MMA) {
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    asm volatile("bar.sync 1, 288;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(EXACT_SETS * 128 + 32) : "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
   const uint32_t tmem = (warp < W_EPI || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
@@ -139,19 +144,19 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
                    : "memory");
     }
     float sq[EXACT_SPS];  // scales of the groups in the set's slots
-    int stage = set;      // the set's stages: set, set + 2, ...
+    int stage = set;      // the set's stages: set, set + EXACT_SETS, ...
     uint32_t ring_phase = 0, hand_phase = 1;
-    const int n_own = (run1 - run0 - set + 1) / 2;
+    const int n_own = (run1 - run0 - set + EXACT_SETS - 1) / EXACT_SETS;
     const bool more = p.M > 4, most = p.M > 8;
     const bool alone = p.cluster <= 1;
     int seg_end = min((run0 / p.G + 1) * p.G, run1);  // of the segment the sums belong to
     int pos = run0 + set;                             // group whose sums are added next
-    while (pos >= seg_end && seg_end < run1) seg_end = min(seg_end + p.G, run1);  // (a first segment of one group)
+    while (pos >= seg_end && seg_end < run1) seg_end = min(seg_end + p.G, run1);  // (first segments without a group of this set)
     bool good = true;
     for (int i0 = 0; i0 < n_own + EXACT_SPS && good; i0 += EXACT_SPS) {
 #pragma unroll
       for (int j = 0; j < EXACT_SPS; ++j) {
-        const int i = i0 + j, slot = set + 2 * j;
+        const int i = i0 + j, slot = set + EXACT_SETS * j;
         const bool have = i < n_own;
         if (i >= EXACT_SPS && i - EXACT_SPS < n_own) {
           // the group this slot held: its sums, times its scale
@@ -173,10 +178,10 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 #pragma unroll
             for (int q = 8; q < 16; ++q) acc[q] = fmaf(sq[j], __uint_as_float(v[q]), acc[q]);
           }
-          if (alone && pos + 2 >= seg_end) {  // the set's last group of the column tile: hand the sums over
+          if (alone && pos + EXACT_SETS >= seg_end) {  // the set's last group of the column tile: hand the sums over
             if (!mbar_wait_abortable(BAR_ADDR(hand_empty, set), hand_phase, abort_flag)) { good = false; break; }
             hand_phase ^= 1u;
-            float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)set * EXACT_HAND) + nl;
+            float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)set * HAND) + nl;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               if (q * 4 < p.M) hand[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
@@ -184,10 +189,10 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR_ADDR(hand_full, set));
-            // (a segment of one group that the other set holds has nothing of this set: passed over)
-            do seg_end = min(seg_end + p.G, run1); while (pos + 2 >= seg_end && seg_end < run1);
+            // (segments without a group of this set are passed over)
+            do seg_end = min(seg_end + p.G, run1); while (pos + EXACT_SETS >= seg_end && seg_end < run1);
           }
-          pos += 2;
+          pos += EXACT_SETS;
         }
         if (have) {
           if (!mbar_wait_abortable(BAR_ADDR(g_full, stage), ring_phase, abort_flag)) { good = false; break; }
@@ -210,7 +215,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
             }
             tmem_st_16(slots_t + lane_t + (uint32_t)(slot * 64 + u * 16), out);
           }
-          stage += 2;
+          stage += EXACT_SETS;
           if (stage >= WS) { stage = set; ring_phase ^= 1u; }
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -220,10 +225,10 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       }
     }
   } else if (warp < W_ACT) {
-    // ================= column tiles: sums of both sets, to C or to the tile's scratch =================
+    // ================= column tiles: sums of all sets, to C or to the tile's scratch =================
     const int wq = warp & 3, nl = wq * 32 + lane;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
-    uint32_t phase[2] = {0u, 0u};
+    uint32_t phase = 0u;  // bit s: of set s
     bool good = true;
     for (int pos = run0; pos < run1 && good && p.cluster <= 1;) {
       const int tile = pos / p.G, len = min((tile + 1) * p.G, run1) - pos;
@@ -231,11 +236,11 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 #pragma unroll
       for (int q = 0; q < 4; ++q) f[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int set = 0; set < 2; ++set) {
-        if (len == 1 && ((pos - run0) & 1) != set) continue;
-        if (!mbar_wait_abortable(BAR_ADDR(hand_full, set), phase[set], abort_flag)) { good = false; break; }
-        phase[set] ^= 1u;
-        const float4* hand = reinterpret_cast<const float4*>(smem_al + hand_off + (uint32_t)set * EXACT_HAND) + nl;
+      for (int set = 0; set < EXACT_SETS; ++set) {
+        if ((set + EXACT_SETS - (pos - run0) % EXACT_SETS) % EXACT_SETS >= len) continue;  // no group of this set
+        if (!mbar_wait_abortable(BAR_ADDR(hand_full, set), (phase >> set) & 1u, abort_flag)) { good = false; break; }
+        phase ^= 1u << set;
+        const float4* hand = reinterpret_cast<const float4*>(smem_al + hand_off + (uint32_t)set * HAND) + nl;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           if (q * 4 < p.M) {
@@ -290,7 +295,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       }
     }
   } else if (warp != W_MMA) {
-    // ================= TMA producers: packed weights (warp 13), scales (warp 15) =================
+    // ================= TMA producers: packed weights, scales =================
     if (elect_one()) {
       const bool weights = warp == W_WEIGHTS;
       int stage = 0, n_issued = 0;
@@ -382,7 +387,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     // the tile's sums to the set's hand-over buffer
     __syncwarp();
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
-    float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)(warp >> 2) * EXACT_HAND) + (warp & 3) * 32 + lane;
+    float4* hand = reinterpret_cast<float4*>(smem_al + hand_off + (uint32_t)(warp >> 2) * HAND) + (warp & 3) * 32 + lane;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (q * 4 < p.M) hand[q * 128] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
@@ -406,8 +411,8 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     cluster_arrive();
     cluster_wait();
     if (warp < W_EPI && !*abort_flag)
-      cluster_finish<ACT>(p, smem_base + hand_off, 2, EXACT_HAND, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
-                          warp >> 2, 2);
+      cluster_finish<ACT, EXACT_SETS>(p, smem_base + hand_off, HAND, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
+                          warp >> 2, EXACT_SETS);
     cluster_arrive();  // nobody leaves while its sums are being read
     cluster_wait();
   }
@@ -465,15 +470,16 @@ cudaError_t B200Q_CAT(exact_launch_part, B200Q_PART)(int var, const BatchParams&
 
 #if B200Q_PART == 0
 // dynamic shared memory: alignment slack + activation groups + packed ring with scales + handed sums + barriers
-int exact_smem_bytes(int bits, int stages) {
-  return 1024 + EXACT_SLOTS * (int)EXACT_ASTAGE + stages * batch_stage_bytes(bits, 1) + 2 * (int)EXACT_HAND +
+int exact_smem_bytes(int bits, int stages, int M) {
+  return 1024 + EXACT_SLOTS * (int)EXACT_ASTAGE + stages * batch_stage_bytes(bits, 1) + EXACT_SETS * (int)exact_hand_bytes(M) +
          (int)sizeof(ExactBarriers);
 }
-// Ring stages (even) within half an SM's shared memory: the next launch of the stream becomes resident beside
-// this one and fills its ring while this one ends.
-int exact_stages(int bits) {
+// Ring stages (a multiple of the sets).  Up to 8 rows within half an SM's shared memory, like stream_kernel.cu, whose
+// launches may follow: nine stages of 4-bit weights cover the latency of HBM.
+int exact_stages(int bits, int max_smem, int M) {
+  const int cap = M <= 8 ? 113 * 1024 : max_smem;
   int st = EXACT_STAGES_MAX;
-  while (st > 2 && exact_smem_bytes(bits, st) > 113 * 1024) st -= 2;
+  while (st > EXACT_SETS && exact_smem_bytes(bits, st, M) > cap) st -= EXACT_SETS;
   return st;
 }
 #endif
