@@ -282,7 +282,10 @@ static int gshift_of(int group) {  // log2(group / 128) when that is a power of 
 static int rpg_of(int group) { return group < 128 ? 128 / group : 1; }
 
 static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
-  const int tm = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  int tm = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+#ifndef UMMA_NO384
+  if (M > 512 && ((M + 383) / 384) * ((N + 127) / 128) >= 2 * di.sm_count) tm = 384;
+#endif
   const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
   const int ctas = m_tiles * n_tiles;
   const int kblocks = K / 64;
@@ -488,7 +491,7 @@ static int run_umma(const void* a, int lda, const void* bq, const void* scales, 
                     int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream,
                     const b200q_plan_t& pl) {
   const int tm = pl.tile_m;
-  if (tm != 32 && tm != 64 && tm != 128 && tm != 256) return ST_INVALID_ARG;
+  if (tm != 32 && tm != 64 && tm != 128 && tm != 256 && tm != 384) return ST_INVALID_ARG;
   const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
   const int kblocks = K / 64;
   if (pl.splits < 1 || kblocks % (2 * pl.splits) != 0) return ST_INVALID_ARG;  // whole 128-row groups per split
@@ -512,7 +515,7 @@ static int run_umma(const void* a, int lda, const void* bq, const void* scales, 
   CUtensorMap tmap;
   const cuuint64_t gdim[2] = {(cuuint64_t)K, (cuuint64_t)M};
   const cuuint64_t gstride[1] = {(cuuint64_t)lda * 2};
-  const cuuint32_t box[2] = {64u, (cuuint32_t)tm};
+  const cuuint32_t box[2] = {64u, (cuuint32_t)(tm > 256 ? tm / 2 : tm)};
   const cuuint32_t estr[2] = {1u, 1u};
   CUresult r = enc(&tmap, act == B200Q_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(a), gdim, gstride, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,

@@ -120,7 +120,7 @@ struct UmmaParams {
   int ldc;
   int group;             // rows per scale: 32, 64 or a multiple of 128
   int rpg;               // scale rows per 128-row group: 128 / group for group < 128, else 1
-  int tm;                // activation rows per CTA tile = N extent of the MMA (32, 64, 128 or 256)
+  int tm;                // activation rows per CTA tile: N extent of the MMA (32, 64, 128 or 256) or two of 192 (384)
   int m_tiles, n_tiles;  // ceil(M / tm), ceil(N / 128)
   int splits;            // split-K factor
   int kblocks_per_split; // 64-row k blocks per tile (even)

@@ -3,11 +3,12 @@
 // The product is computed transposed, D[n, m] = sum_k W[k, n] * A[m, k], so that the
 // dequantized weights are the operand that lives in tensor memory and the activations are
 // the operand that TMA brings to shared memory.  A CTA is persistent: it walks over output
-// tiles of 128 weight columns x TM activation rows (TM = 32 .. 256, the N extent of the MMA),
+// tiles of 128 weight columns x TM activation rows (TM = 32 .. 256, the N extent of the MMA, or 384 in two MMAs
+// of 192: a weight stage is dequantized once for all of them),
 // each over all of K (or one of S splits of it), with the pipelines running across tile
 // boundaries.  Warp roles:
 //
-//   * warp 17, weight producer: per 128-row group it brings the packed weights of the tile's
+//   * weight producer (one warp): per 128-row group it brings the packed weights of the tile's
 //     128 columns (eight 16-column pieces of 256*b contiguous bytes, cp.async.bulk) and their
 //     128 fp16 scales into a 4-deep shared-memory ring;
 //   * warps 0-7 dequantize.  Thread t of warp w is lane n = 32 * (w % 4) + t of tensor
@@ -17,14 +18,14 @@
 //     multiplies by, examples/quantization/matmul_a16wx.py:316-320) and writes the 32 half2
 //     results to 32 columns of tensor memory with one tcgen05.st.  Warps 0-3 take the even
 //     64-blocks, warps 4-7 the odd ones;
-//   * warp 16, activation producer: one 2-D tiled TMA copy (128-byte swizzle) per 64-block
+//   * activation producer (one warp): one 2-D tiled TMA copy (128-byte swizzle) per 64-block
 //     brings A[m0 : m0+TM, k : k+64] into a shared-memory ring; rows past M read as zero;
-//   * warp 18 owns tensor memory (alloc / dealloc) and issues the MMAs: per 64-block four
+//   * one warp owns tensor memory (alloc / dealloc) and issues the MMAs: per 64-block four
 //     tcgen05.mma.cta_group::1.kind::f16 (K = 16 each) with the weight operand in tensor
 //     memory, the activation operand through a shared-memory descriptor and the fp32
 //     accumulator D (128 lanes x TM columns) in tensor memory; tcgen05.commit releases the
 //     activation stage and the weight stage when the MMAs have read them;
-//   * warps 8-15, epilogue (two per lane quadrant, alternate 32-column chunks): when a tile's last
+//   * warps 8-19, epilogue (three per lane quadrant, every third 32-column chunk): when a tile's last
 //     MMA has completed they read D with
 //     tcgen05.ld, convert to fp16 and store C[m, n] (or add into the fp32 split-K scratch),
 //     then hand D back.  Meanwhile the producers and the dequantizers are already working on
@@ -47,16 +48,20 @@
 
 namespace b200q {
 
-constexpr int UMMA_THREADS = 608;   // 8 dequant warps, 8 epilogue warps, 2 producers, MMA warp
+constexpr int UMMA_EPI = 3;         // epilogue warps per lane quadrant
+constexpr int UMMA_EPI_THREADS = UMMA_EPI * 128;
+constexpr int UMMA_THREADS = 256 + UMMA_EPI_THREADS + 96;  // 8 dequant warps, epilogue, 2 producers, MMA warp
 constexpr int UMMA_SA_MAX = 6;      // activation stages (most)
-constexpr int UMMA_SW = 8;          // weight stages in tensor memory (32 columns each)
+constexpr int UMMA_SW_MAX = 8;      // weight stages in tensor memory (32 columns each), most
 constexpr int UMMA_WG = 4;          // 128-row weight groups in the shared-memory ring
-constexpr int UMMA_WCOL0 = 256;     // first tensor-memory column of the weight stages
+// tensor memory: tm columns of D, then the weight stages
+__host__ __device__ constexpr int umma_wcol0(int tm) { return tm > 256 ? 384 : 256; }
+__host__ __device__ constexpr int umma_sw(int tm) { return tm > 256 ? 4 : 8; }
 constexpr int UMMA_TMEM_COLS = 512;
 
 struct UmmaBarriers {
-  uint64_t a_full[UMMA_SA_MAX], a_empty[UMMA_SA_MAX];
-  uint64_t w_full[UMMA_SW], w_empty[UMMA_SW];
+  uint64_t a_full[UMMA_SA_MAX];
+  uint64_t w_full[UMMA_SW_MAX], w_empty[UMMA_SW_MAX];
   uint64_t g_full[UMMA_WG], g_empty[UMMA_WG];
   uint64_t d_full, d_empty;
   uint32_t tmem_base;
@@ -79,7 +84,8 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   const uint32_t smem_base = (smem_unaligned + 1023u) & ~1023u;
   unsigned char* smem_al = smem_raw + (smem_base - smem_unaligned);
   const int TM = p.tm;
-  const int SA = p.a_stages;
+  const int SA = p.a_stages, SW = umma_sw(TM), WCOL0 = umma_wcol0(TM);
+  const int BOX = TM > 256 ? TM / 2 : TM;  // rows of an activation copy and of an MMA
   const uint32_t stage_bytes = (uint32_t)TM * 128u;
   const uint32_t wring_s = smem_base + (uint32_t)SA * stage_bytes;
   const uint32_t bars_off = (uint32_t)SA * stage_bytes + UMMA_WG * WSTAGE;
@@ -98,17 +104,18 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   volatile int* abort_flag = &bars->abort_flag;
 
   if (tid == 0) {
-    for (int i = 0; i < UMMA_SA_MAX; ++i) { mbar_init(BAR_ADDR(a_full, i), 1); mbar_init(BAR_ADDR(a_empty, i), 1); }
-    for (int i = 0; i < UMMA_SW; ++i) { mbar_init(BAR_ADDR(w_full, i), 4); mbar_init(BAR_ADDR(w_empty, i), 1); }
+    for (int i = 0; i < UMMA_SA_MAX; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
+    for (int i = 0; i < UMMA_SW_MAX; ++i) { mbar_init(BAR_ADDR(w_full, i), 4); mbar_init(BAR_ADDR(w_empty, i), 1); }
     for (int i = 0; i < UMMA_WG; ++i) { mbar_init(BAR_ADDR(g_full, i), 1); mbar_init(BAR_ADDR(g_empty, i), 8); }
     mbar_init(BAR_ADDR(d_full, 0), 1);
-    mbar_init(BAR_ADDR(d_empty, 0), 8);
+    mbar_init(BAR_ADDR(d_empty, 0), 4 * UMMA_EPI);
     bars->abort_flag = 0;
     bars->last_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 18) {
+  constexpr int W_ACT = 8 + 4 * UMMA_EPI, W_WEIGHTS = W_ACT + 1, W_MMA = W_ACT + 2;
+  if (warp == W_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      bars_s + (uint32_t)offsetof(UmmaBarriers, tmem_base)),
                  "r"(UMMA_TMEM_COLS)
@@ -153,7 +160,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
     const int nl = (warp & 3) * 32 + lane;  // lane of tensor memory = column inside the tile
     // this column inside a ring stage: 16-column piece nl / 16, then unit (half*32 + r*4 + j)
     const uint32_t lane_off = (uint32_t)((nl >> 4) * (256 * B) + (((nl >> 3) & 1) * 32 + (nl & 7) * 4 + grp * 2) * (B * 4));
-    const uint32_t taddr_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + UMMA_WCOL0;
+    const uint32_t taddr_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)WCOL0;
     int g_run = 0;  // groups consumed so far (all tiles)
     bool good = true;
     for (int t = blockIdx.x; t < total_tiles && good; t += gridDim.x) {
@@ -182,8 +189,8 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR_ADDR(g_empty, gs));
         const int wi = 2 * g_run + grp;  // running 64-block index
-        const int sw = wi % UMMA_SW;
-        if (!mbar_wait_abortable(BAR_ADDR(w_empty, sw), ((uint32_t)(wi / UMMA_SW) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        const int sw = wi % SW;
+        if (!mbar_wait_abortable(BAR_ADDR(w_empty, sw), ((uint32_t)(wi / SW) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t taddr = taddr_lane + (uint32_t)(sw * 32);
         asm volatile(
@@ -202,11 +209,11 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         if (lane == 0) mbar_arrive(BAR_ADDR(w_full, sw));
       }
     }
-  } else if (warp < 16) {
+  } else if (warp < W_ACT) {
     // ================= epilogue: read D, write C (or add into the split-K scratch) =================
-    // two warps per lane quadrant of tensor memory; they take alternate 32-column chunks of D
+    // UMMA_EPI warps per lane quadrant of tensor memory; they share its 32-column chunks of D
     const int ew = warp & 3;            // lane quadrant this warp may read
-    const int chunk0 = (warp - 8) >> 2; // first chunk of this warp
+    const int chunk0 = (warp - 8) >> 2; // first chunk of this warp, then every UMMA_EPI-th
     const int nl = ew * 32 + lane;
     const uint32_t daddr = tmem + ((uint32_t)(ew * 32) << 16);
     int tile_it = 0;
@@ -228,7 +235,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         uint32_t hb[4][16];  // chunk ci, rows (2i, 2i+1) of column n
 #pragma unroll
         for (int ci = 0; ci < 4; ++ci) {
-          const int c0 = chunk0 * 32 + ci * 64;
+          const int c0 = chunk0 * 32 + ci * (32 * UMMA_EPI);
           if (c0 < TM) {
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {  // 16 columns at a time: few registers live next to hb
@@ -249,7 +256,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         const int n8 = n_tile * 128 + (nl & ~7);
 #pragma unroll
         for (int ci = 0; ci < 4; ++ci) {
-          const int c0 = chunk0 * 32 + ci * 64;
+          const int c0 = chunk0 * 32 + ci * (32 * UMMA_EPI);
           if (c0 < TM && m0 + c0 < p.M) {
             uint32_t h[16];  // exchange 1: columns (n & ~1, +1), row 2 i + b0
 #pragma unroll
@@ -282,15 +289,15 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
           }
         }
       } else {
-        if (chunk0 * 32 >= TM) {  // nothing of this tile is this warp's (TM = 32): hand D back at once
+        if (chunk0 * 32 >= TM) {  // nothing of this tile is this warp's (TM = 32, 64): hand D back at once
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(BAR_ADDR(d_empty, 0));
         }
-        for (int c0 = chunk0 * 32; c0 < TM; c0 += 64) {
+        for (int c0 = chunk0 * 32; c0 < TM; c0 += 32 * UMMA_EPI) {
           uint32_t v[32];
           tmem_ld_32(daddr + (uint32_t)c0, v);
-          if (c0 + 64 >= TM) {
+          if (c0 + 32 * UMMA_EPI >= TM) {
             // this warp's last chunk of D is in registers: the next tile's MMAs may overwrite it
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -350,7 +357,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         // the last K range to arrive converts the tile's fp32 sums (kept per tile slot: [slot][row][128
         // columns]) and restores the zeros
         const int nsplit = in_tail ? p.tail_splits : p.splits;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(UMMA_EPI_THREADS) : "memory");
         if (warp == 8 && lane == 0) {
           __threadfence();
           const int old = atomicAdd(p.counters + slot, 1);
@@ -358,22 +365,22 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
           if (last) __threadfence();
           bars->last_flag = last;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(UMMA_EPI_THREADS) : "memory");
         if (bars->last_flag) {
           // eight independent loads per thread in flight: one L2 round trip per batch, not per load
           float* tile_sums = p.partial + (size_t)slot * TM * 128;
-          for (int base = tid - 256; base < 64 * TM; base += 8 * 256) {
+          for (int base = tid - 256; base < 64 * TM; base += 8 * UMMA_EPI_THREADS) {
             float2 x[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const int idx = base + u * 256;
+              const int idx = base + u * UMMA_EPI_THREADS;
               const int nn = n_tile * 128 + (idx & 63) * 2, m = m0 + (idx >> 6);
               if (idx < 64 * TM && nn < p.N && m < p.M)
                 x[u] = __ldcg(reinterpret_cast<const float2*>(tile_sums + (size_t)idx * 2));
             }
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const int idx = base + u * 256;
+              const int idx = base + u * UMMA_EPI_THREADS;
               const int nn = n_tile * 128 + (idx & 63) * 2, m = m0 + (idx >> 6);
               if (idx < 64 * TM && nn < p.N && m < p.M) {
                 *reinterpret_cast<uint32_t*>(p.c + (size_t)m * p.ldc + nn) = pack2<ACT>(x[u].x, x[u].y);
@@ -383,31 +390,34 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
           }
           if (warp == 8 && lane == 0) p.counters[slot] = 0;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // last_flag may be rewritten by the next item
+        asm volatile("bar.sync 1, %0;" ::"n"(UMMA_EPI_THREADS) : "memory");  // last_flag may be rewritten by the next item
       }
     }
-  } else if (warp == 16) {
+  } else if (warp == W_ACT) {
     // ================= TMA producer: activations =================
-    if (lane == 0) {
+    if (elect_one()) {
       int ai = 0;
       bool good = true;
       for (int t = blockIdx.x; t < total_tiles && good; t += gridDim.x) {
         TILE_COORDS(t)
         for (int i = 0; i < nkk; ++i, ++ai) {
           const int sa = ai % SA;
-          if (!mbar_wait_abortable(BAR_ADDR(a_empty, sa), ((uint32_t)(ai / SA) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+          // the stage held block ai - SA, whose MMAs report on its weight stage's barrier (SA <= SW)
+          const int prev = ai - SA;
+          if (prev >= 0 && !mbar_wait_abortable(BAR_ADDR(w_empty, prev % SW), (uint32_t)(prev / SW) & 1u, abort_flag)) { good = false; break; }
           const uint32_t bar = BAR_ADDR(a_full, sa);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes)
                        : "memory");
           const int kx = (kk0 + i) * 64;
-          asm volatile(
-              "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-              ::"r"(smem_base + (uint32_t)sa * stage_bytes), "l"(&tmap_a), "r"(bar), "r"(kx), "r"(m0)
-              : "memory");
+          for (int b = 0; b < TM; b += BOX)  // one or two boxes of rows
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                ::"r"(smem_base + (uint32_t)sa * stage_bytes + (uint32_t)b * 128u), "l"(&tmap_a), "r"(bar), "r"(kx), "r"(m0 + b)
+                : "memory");
         }
       }
     }
-  } else if (warp == 17) {
+  } else if (warp == W_WEIGHTS) {
     // ================= bulk-copy producer: packed weights and scales =================
     int g_run = 0;
     bool good = true;
@@ -452,22 +462,26 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   } else {
     // ================= MMA issuer =================
     if (elect_one()) {
-      const uint32_t idesc = umma_idesc<ACT>(TM);
       bool good = true;
       int ai = 0, tile_it = 0;
       for (int t = blockIdx.x; t < total_tiles && good; t += gridDim.x, ++tile_it) {
         TILE_COORDS(t)
+        // rows of the tile that exist, rounded up to 16, in the one or two MMAs of a K step: a short last row
+        // tile costs what its rows cost
+        const int rows = min(TM, (p.M - m0 + 15) & ~15);
+        const int n1 = rows > BOX ? rows - BOX : 0;
+        const uint32_t idesc0 = umma_idesc<ACT>(min(rows, BOX)), idesc1 = umma_idesc<ACT>(n1 > 0 ? n1 : 16);
         // D must have been read out by the epilogue of the previous tile
         if (!mbar_wait_abortable(BAR_ADDR(d_empty, 0), ((uint32_t)tile_it & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int i = 0; i < nkk; ++i, ++ai) {
-          const int sa = ai % SA, sw = ai % UMMA_SW;
+          const int sa = ai % SA, sw = ai % SW;
           good = mbar_wait_abortable(BAR_ADDR(a_full, sa), (uint32_t)(ai / SA) & 1u, abort_flag) &&
-                 mbar_wait_abortable(BAR_ADDR(w_full, sw), (uint32_t)(ai / UMMA_SW) & 1u, abort_flag);
+                 mbar_wait_abortable(BAR_ADDR(w_full, sw), (uint32_t)(ai / SW) & 1u, abort_flag);
           if (!good) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)sa * stage_bytes);
-          const uint32_t a_tmem = tmem + UMMA_WCOL0 + (uint32_t)(sw * 32);
+          const uint32_t a_tmem = tmem + (uint32_t)WCOL0 + (uint32_t)(sw * 32);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks) {
             const uint32_t accumulate = (i > 0 || ks > 0) ? 1u : 0u;
@@ -475,14 +489,20 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, %4, 0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                ::"r"(tmem), "r"(a_tmem + (uint32_t)(ks * 8)), "l"(bdesc + (uint64_t)(ks * 2)), "r"(idesc),
+                ::"r"(tmem), "r"(a_tmem + (uint32_t)(ks * 8)), "l"(bdesc + (uint64_t)(ks * 2)), "r"(idesc0),
                 "r"(accumulate)
                 : "memory");
+            if (n1 > 0)
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\t"
+                  "setp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                  ::"r"(tmem + (uint32_t)BOX), "r"(a_tmem + (uint32_t)(ks * 8)),
+                  "l"(bdesc + (uint64_t)(BOX * 8 + ks * 2)), "r"(idesc1), "r"(accumulate)
+                  : "memory");
           }
-          // the stages may be overwritten once these MMAs have read them
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           BAR_ADDR(a_empty, sa))
-                       : "memory");
+          // both stages may be overwritten once these MMAs have read them: one commit (a second one right behind
+          // the first would cost the issuing thread 600 cycles, more than the MMAs of the block)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(w_empty, sw))
                        : "memory");
@@ -505,7 +525,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
     p.status[2] = blockIdx.x;
     p.status[3] = 0;
   }
-  if (warp == 18) {
+  if (warp == W_MMA) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(UMMA_TMEM_COLS) : "memory");
   }
@@ -555,9 +575,9 @@ cudaError_t B200Q_CAT(umma_launch_part, B200Q_PART)(int var, const UmmaParams& p
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg) {
   return 1024 + a_stages * tm * 128 + UMMA_WG * umma_wstage_bytes(bits, rpg) + (int)sizeof(UmmaBarriers) + 64;
 }
-// most activation stages (<= UMMA_SA_MAX) that fit next to the weight ring
+// most activation stages (<= UMMA_SA_MAX, and at most as many as weight stages) that fit next to the weight ring
 int umma_a_stages(int tm, int bits, int max_smem, int rpg) {
-  int sa = UMMA_SA_MAX;
+  int sa = UMMA_SA_MAX < umma_sw(tm) ? UMMA_SA_MAX : umma_sw(tm);
   while (sa > 2 && umma_smem_bytes(tm, bits, sa, rpg) > max_smem) --sa;
   return sa;
 }
