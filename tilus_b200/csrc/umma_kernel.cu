@@ -56,7 +56,7 @@ constexpr int UMMA_SW_MAX = 8;      // weight stages in tensor memory (32 column
 constexpr int UMMA_WG = 4;          // 128-row weight groups in the shared-memory ring
 // tensor memory: tm columns of D, then the weight stages
 __host__ __device__ constexpr int umma_wcol0(int tm) { return tm > 256 ? 384 : 256; }
-__host__ __device__ constexpr int umma_sw(int tm) { return tm > 256 ? 4 : 8; }
+__host__ __device__ constexpr int umma_sw_log2(int tm) { return tm > 256 ? 2 : 3; }
 constexpr int UMMA_TMEM_COLS = 512;
 
 struct UmmaBarriers {
@@ -84,7 +84,9 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   const uint32_t smem_base = (smem_unaligned + 1023u) & ~1023u;
   unsigned char* smem_al = smem_raw + (smem_base - smem_unaligned);
   const int TM = p.tm;
-  const int SA = p.a_stages, SW = umma_sw(TM), WCOL0 = umma_wcol0(TM);
+  // (ring positions are counted or masked: a division by a run-time ring depth is a chain of some 100 cycles)
+  const int SA = p.a_stages, SWL = umma_sw_log2(TM), WCOL0 = umma_wcol0(TM);
+  const int SW_MASK = (1 << SWL) - 1;
   const int BOX = TM > 256 ? TM / 2 : TM;  // rows of an activation copy and of an MMA
   const uint32_t stage_bytes = (uint32_t)TM * 128u;
   const uint32_t wring_s = smem_base + (uint32_t)SA * stage_bytes;
@@ -189,8 +191,8 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         __syncwarp();
         if (lane == 0) mbar_arrive(BAR_ADDR(g_empty, gs));
         const int wi = 2 * g_run + grp;  // running 64-block index
-        const int sw = wi % SW;
-        if (!mbar_wait_abortable(BAR_ADDR(w_empty, sw), ((uint32_t)(wi / SW) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        const int sw = wi & SW_MASK;
+        if (!mbar_wait_abortable(BAR_ADDR(w_empty, sw), ((uint32_t)(wi >> SWL) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t taddr = taddr_lane + (uint32_t)(sw * 32);
         asm volatile(
@@ -396,15 +398,14 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
   } else if (warp == W_ACT) {
     // ================= TMA producer: activations =================
     if (elect_one()) {
-      int ai = 0;
+      int ai = 0, sa = 0;
       bool good = true;
       for (int t = blockIdx.x; t < total_tiles && good; t += gridDim.x) {
         TILE_COORDS(t)
         for (int i = 0; i < nkk; ++i, ++ai) {
-          const int sa = ai % SA;
           // the stage held block ai - SA, whose MMAs report on its weight stage's barrier (SA <= SW)
           const int prev = ai - SA;
-          if (prev >= 0 && !mbar_wait_abortable(BAR_ADDR(w_empty, prev % SW), (uint32_t)(prev / SW) & 1u, abort_flag)) { good = false; break; }
+          if (prev >= 0 && !mbar_wait_abortable(BAR_ADDR(w_empty, prev & SW_MASK), (uint32_t)(prev >> SWL) & 1u, abort_flag)) { good = false; break; }
           const uint32_t bar = BAR_ADDR(a_full, sa);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(stage_bytes)
                        : "memory");
@@ -414,6 +415,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
                 "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                 ::"r"(smem_base + (uint32_t)sa * stage_bytes + (uint32_t)b * 128u), "l"(&tmap_a), "r"(bar), "r"(kx), "r"(m0 + b)
                 : "memory");
+          if (++sa == SA) sa = 0;
         }
       }
     }
@@ -463,7 +465,8 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
     // ================= MMA issuer =================
     if (elect_one()) {
       bool good = true;
-      int ai = 0, tile_it = 0;
+      int ai = 0, tile_it = 0, sa = 0;
+      uint32_t sa_phase = 0;
       for (int t = blockIdx.x; t < total_tiles && good; t += gridDim.x, ++tile_it) {
         TILE_COORDS(t)
         // rows of the tile that exist, rounded up to 16, in the one or two MMAs of a K step: a short last row
@@ -475,9 +478,9 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
         if (!mbar_wait_abortable(BAR_ADDR(d_empty, 0), ((uint32_t)tile_it & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int i = 0; i < nkk; ++i, ++ai) {
-          const int sa = ai % SA, sw = ai % SW;
-          good = mbar_wait_abortable(BAR_ADDR(a_full, sa), (uint32_t)(ai / SA) & 1u, abort_flag) &&
-                 mbar_wait_abortable(BAR_ADDR(w_full, sw), (uint32_t)(ai / SW) & 1u, abort_flag);
+          const int sw = ai & SW_MASK;
+          good = mbar_wait_abortable(BAR_ADDR(a_full, sa), sa_phase, abort_flag) &&
+                 mbar_wait_abortable(BAR_ADDR(w_full, sw), (uint32_t)(ai >> SWL) & 1u, abort_flag);
           if (!good) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)sa * stage_bytes);
@@ -506,6 +509,7 @@ umma_kernel(const UmmaParams p, const __grid_constant__ CUtensorMap tmap_a) {
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            BAR_ADDR(w_empty, sw))
                        : "memory");
+          if (++sa == SA) { sa = 0; sa_phase ^= 1u; }
         }
         if (good)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -577,7 +581,7 @@ int umma_smem_bytes(int tm, int bits, int a_stages, int rpg) {
 }
 // most activation stages (<= UMMA_SA_MAX, and at most as many as weight stages) that fit next to the weight ring
 int umma_a_stages(int tm, int bits, int max_smem, int rpg) {
-  int sa = UMMA_SA_MAX < umma_sw(tm) ? UMMA_SA_MAX : umma_sw(tm);
+  int sa = min(UMMA_SA_MAX, 1 << umma_sw_log2(tm));
   while (sa > 2 && umma_smem_bytes(tm, bits, sa, rpg) > max_smem) --sa;
   return sa;
 }
