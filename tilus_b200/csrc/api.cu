@@ -281,19 +281,43 @@ static int gshift_of(int group) {  // log2(group / 128) when that is a power of 
 // tcgen05 kernel: tile rows, tiles and split-K so that the grid fills the SMs
 static int rpg_of(int group) { return group < 128 ? 128 / group : 1; }
 
-static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
-  int tm = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
-#ifndef UMMA_NO384
-  if (M > 512 && ((M + 383) / 384) * ((N + 127) / 128) >= 2 * di.sm_count) tm = 384;
-#endif
-  const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
-  const int ctas = m_tiles * n_tiles;
+static int umma_tail(int tiles, int grid, int kblocks, int uniform_splits, int N, int* splits);
+// uniform split-K of a launch whose tiles leave half of the SMs idle
+static int umma_splits(int ctas, int N, int K, const DeviceInfo& di) {
   const int kblocks = K / 64;
   int splits = 1;
   if (ctas * 2 <= di.sm_count && ctas <= N / BLOCK_N) {
     for (int s = 2; s <= 16; ++s)
       if (kblocks % (2 * s) == 0 && kblocks / s >= 8 && ctas * s <= di.sm_count + di.sm_count / 8) splits = s;
   }
+  return splits;
+}
+// Cost of a launch with tiles of tm rows, in rows: rounds of the persistent CTAs (a round cut along K takes its
+// fraction and 0.3 of a tile for the sums that meet in L2) times the rows of a tile (the last row tile costs its own
+// rows only; a single round lasts as long as its largest tile) and 160 rows' worth for dequantizing the tile's weights.
+// Fitted to 256 against 384 rows at 27 shapes, 300 .. 4096 rows, 1264 .. 28672 columns: it picks the faster one at
+// 24 of them and loses at most 10 % at the others.  4-bit weights, 256 / 384 rows, us: 300 x 28672 x 4096 131 / 84,
+// 640 x 8192 x 4096 55 / 39, 1024 x 4096 x 4096 33 / 39, 2048 x 4096 x 4096 64 / 69, 4096 x 12288 x 4096 361 / 301.
+static double umma_cost(int M, int N, int K, int tm, const DeviceInfo& di) {
+  const int m_tiles = (M + tm - 1) / tm, tiles = m_tiles * ((N + 127) / 128);
+  const int splits = umma_splits(tiles, N, K, di);
+  double rounds;
+  if (splits > 1 || tiles <= di.sm_count) {
+    rounds = splits > 1 ? 1.0 / splits + 0.3 : 1.0;
+  } else {
+    int tail_splits;
+    const int tail = umma_tail(tiles, di.sm_count, K / 64, 1, N, &tail_splits);
+    rounds = tail > 0 ? tiles / di.sm_count + 1.0 / tail_splits + 0.3 : (tiles + di.sm_count - 1) / di.sm_count;
+  }
+  const double rows = rounds <= 1.0 ? (M < tm ? M : tm) : (double)M / m_tiles;
+  return rounds * (rows + 160.0);
+}
+static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
+  int tm = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  if (M > 256 && umma_cost(M, N, K, 384, di) < umma_cost(M, N, K, 256, di)) tm = 384;
+  const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
+  const int ctas = m_tiles * n_tiles;
+  const int splits = umma_splits(ctas, N, K, di);
   pl->kernel = 1;
   pl->m_tiles = m_tiles;
   pl->splits = splits;
@@ -424,15 +448,17 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
     }
     return ST_OK;
   } else {
-    // A last row tile of at most 16 rows (M = 4097: one row) would cost a whole 256-row tile per
-    // column tile; those rows go to the decode kernel in a second launch instead (passes = 2).
+    // A last row tile of at most 16 rows would cost each column tile the dequantization of its weights once more;
+    // those rows go to the decode kernel in a second launch instead (passes = 2).  Not where the row tiles of the
+    // others have room for them (M = 4097 with tiles of 384 rows: 10 and 257 rows more).
     const int tail = M % 256;
     b200q_plan_t tail_plan;
     if (M > 256 && tail >= 1 && tail <= kStreamMaxRows && stream_takes(K, group) &&
         plan_stream(tail, N, K, bits, di, &tail_plan) == ST_OK) {
       plan_umma(M - tail, N, K, bits, group, di, pl);
       pl->passes = 2;
-    } else {
+    }
+    if (pl->passes != 2 || pl->tile_m * pl->m_tiles >= M) {
       plan_umma(M, N, K, bits, group, di, pl);
     }
   }
