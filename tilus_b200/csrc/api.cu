@@ -326,7 +326,7 @@ static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo
   pl->stages = umma_a_stages(tm, bits, di.max_smem, rpg_of(group));
   pl->smem_bytes = umma_smem_bytes(tm, bits, pl->stages, rpg_of(group));
   pl->tile_m = tm;
-  pl->warps = 19;
+  pl->warps = 23;
   pl->passes = 1;
   pl->pdl = 0;
 }

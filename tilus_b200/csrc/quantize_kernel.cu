@@ -1,5 +1,5 @@
 // load_and_quantize on the GPU: dense weight[out, in] -> per-group scales + packed weights in
-// the b200 layout, in two passes over the dense weight.
+// the b200 layout.
 //
 // The arithmetic is QuantizedLinear.load_and_quantize of the reference
 // (examples/quantization/matmul_a16wx.py:470-528), operation for operation so that the codes
@@ -22,7 +22,7 @@
 // from one multiplication by the reciprocal of the scale, and only a unit with a value within the
 // multiplication's error of a rounding boundary is computed again with the division: the codes are
 // those of the division in every case.  fp16 [28672, 4096] -> int4 g128: 544 us for two scalar passes plus
-// the copy into the layer, see quantize_launch for the present figure.
+// the copy into the layer, 94 us in this form (45 us at the copy rate of HBM).
 #include "common.cuh"
 
 namespace b200q {

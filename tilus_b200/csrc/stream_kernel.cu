@@ -3,7 +3,7 @@
 // Data movement.  The (column tile, k block) items of the weight matrix - GI consecutive
 // 128-row groups of a 16-column x 512-row block, 1..2 KB contiguous - are cut into equal
 // contiguous runs, one per warp, and every CTA gets the same number of items whatever the
-// shape.  Lane 0 of a warp keeps the warp's own shared-memory ring full with TMA bulk copies
+// shape.  One elected lane of a warp keeps the warp's own shared-memory ring full with TMA bulk copies
 // (cp.async.bulk, completion on an mbarrier per slot).  Weights and scales are constants, so
 // the ring is filled and the warp's scales are cached in shared memory before the kernel
 // waits for its predecessor in the stream (programmatic dependent launch): the memory

@@ -10,7 +10,8 @@
 //
 //   * weight producer (one warp): per 128-row group it brings the packed weights of the tile's
 //     128 columns (eight 16-column pieces of 256*b contiguous bytes, cp.async.bulk) and their
-//     128 fp16 scales into a 4-deep shared-memory ring;
+//     128 fp16 scales into a 4-deep shared-memory ring (one tiled TMA copy of the group instead, as in
+//     batch_kernel.cu, ran 7 % slower at 4096 rows);
 //   * warps 0-7 dequantize.  Thread t of warp w is lane n = 32 * (w % 4) + t of tensor
 //     memory.  For a block of 64 k it reads its column's 2 units (64 codes, 16*b contiguous
 //     bytes) from the ring, decodes and scales them in registers with the unit decoder
@@ -30,6 +31,13 @@
 //     tcgen05.ld, convert to fp16 and store C[m, n] (or add into the fp32 split-K scratch),
 //     then hand D back.  Meanwhile the producers and the dequantizers are already working on
 //     the next tile, so the tensor pipe restarts as soon as D is free.
+//
+// What bounds it: at thousands of rows the board's power - 4096 x 12288 x 4096 (4 bits) runs at 1370 TFLOP/s, a
+// long cuBLAS bf16 loop at 1400 - so what pays is less work per multiplication.  Tiles of 384 rows dequantize a
+// weight stage once for 1.5 times the rows of 256 (416 -> 321 us there), one commit per 64-block instead of two
+// and counted ring positions keep the MMA thread ahead (its four divisions per block cost 1000 cycles, the MMAs
+// 128 .. 768: 321 -> 301 us; 256 x 8192 x 8192 51 -> 41).  A third set of dequantizing warps, looking at the next
+// block's barriers ahead, and one commit per 128 rows changed nothing or lost up to 4 % at full power.
 //
 // Every mbarrier wait is bounded in time; a wait that runs out raises a CTA-wide abort flag,
 // all loops leave, tensor memory is still freed and the status word of the workspace reports
