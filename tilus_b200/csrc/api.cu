@@ -313,7 +313,7 @@ static double umma_cost(int M, int N, int K, int tm, const DeviceInfo& di) {
   return rounds * (rows + 160.0);
 }
 static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
-  int tm = M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+  int tm = 256;  // (plans start here at 129 rows; smaller tiles only through an edited plan)
   if (M > 256 && umma_cost(M, N, K, 384, di) < umma_cost(M, N, K, 256, di)) tm = 384;
   const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
   const int ctas = m_tiles * n_tiles;
