@@ -35,3 +35,11 @@ def test_prefill_384_row_tiles_are_planned_and_walked():
 @pytest.mark.parametrize("w,zp", [("uint4b", 8), ("int8", 0), ("float6_e3m2", 0), ("uint1b", 0)])
 def test_exact_small_batch_kernel(M, N, K, group, w, zp):
     _forced(M, N, K, weight_dtype(w), zp, dict(), seed=M + N, group=group)
+
+
+@pytest.mark.parametrize("M", [2, 4])
+def test_few_rows_whose_stream_plan_cuts_k(M):
+    """448 column tiles have no divisor near two CTAs per SM: the exact kernel takes them from two rows on."""
+    dt = weight_dtype("uint4b")
+    assert ops.plan(1, 7168, 2048, dt, 8, 128)["tile_m"] == 0 and ops.plan(M, 7168, 2048, dt, 8, 128)["tile_m"] == 16
+    _forced(M, 7168, 2048, dt, 8, dict(), seed=M)

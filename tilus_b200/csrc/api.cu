@@ -424,6 +424,15 @@ static int umma_tail(int tiles, int grid, int kblocks, int uniform_splits, int N
 // fp32 scratch of the transposed tcgen05 kernel: one [tm][128] slab per tile slot
 static size_t umma_partial_bytes(int slots, int tm) { return (size_t)slots * tm * 128 * sizeof(float); }
 
+// A stream plan that cuts K and still has one CTA per SM at most (no divisor of the column tiles near two per SM): its
+// chunks meet in the scratch like the exact kernel's, at half the warps.  The exact kernel is then faster from two
+// rows on, and for one row from three chunks on; stream / exact, us, chains of cold launches, 4 bits: 7168 x 2048 (2
+// chunks) 9.5 / 8.7, 2448 x 11776 (23) 13.8 / 11.8, 3504 x 9728 (19) 14.9 / 12.3, 5120 x 5120 (2) 11.3 .. 11.8 / 11.6 and 10.9 at
+// one row; 3504 x 9728 in 8 bits 18.9 / 15.3.
+static bool stream_outrun(int M, const b200q_plan_t& pl, const DeviceInfo& di) {
+  return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas_per_split <= di.sm_count;
+}
+
 static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_plan_t* pl) {
   const DeviceInfo di = device_info();
   std::memset(pl, 0, sizeof(*pl));
@@ -433,11 +442,12 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
   // rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's second 8-row tile doubles
   // its staging and MMAs.
   if (M <= kStreamPlanRows && stream_takes(K, group)) {
-    if (plan_stream(M, N, K, bits, di, pl) == ST_OK) {
+    if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di)) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
       return ST_OK;
     }
+    std::memset(pl, 0, sizeof(*pl));
   }
   // up to 128 rows the small-batch kernels (weights streamed once); beyond, the prefill kernel
   if (M <= kBatchMaxRows) {
@@ -788,9 +798,12 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     return run_umma(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2 && plan_is_exact(pl) && act == B200Q_BF16 && M <= 8) {
     // bf16 costs the exact kernel one more half instruction per pair of weights and the stream kernel only a
-    // conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit)
+    // conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit),
+    // unless its plan is one that the exact kernel outruns
     b200q_plan_t rows;
-    if (plan_stream(M, N, K, var_bits(var), device_info(), &rows) == ST_OK && ws_bytes >= stream_workspace_bytes(N))
+    const DeviceInfo di = device_info();
+    if (plan_stream(M, N, K, var_bits(var), di, &rows) == ST_OK && !stream_outrun(M, rows, di) &&
+        ws_bytes >= stream_workspace_bytes(N))
       return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, rows);
   }
   if (pl.kernel == 2 && plan_is_exact(pl))

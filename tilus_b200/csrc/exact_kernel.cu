@@ -475,9 +475,11 @@ int exact_smem_bytes(int bits, int stages, int M) {
          (int)sizeof(ExactBarriers);
 }
 // Ring stages (a multiple of the sets).  Up to 8 rows within half an SM's shared memory, like stream_kernel.cu, whose
-// launches may follow: nine stages of 4-bit weights cover the latency of HBM.
+// launches may follow, where that holds two stages per set (nine of 4-bit weights); 7 and 8 bits get one there, whose
+// copy and decoding cannot overlap (8 x 8192 x 8192, 8 bits: 22.3 us with 3 stages, 20.4 with 9).
 int exact_stages(int bits, int max_smem, int M) {
-  const int cap = M <= 8 ? 113 * 1024 : max_smem;
+  const int half = 113 * 1024;
+  const int cap = M <= 8 && exact_smem_bytes(bits, 2 * EXACT_SETS, M) <= half ? half : max_smem;
   int st = EXACT_STAGES_MAX;
   while (st > EXACT_SETS && exact_smem_bytes(bits, st, M) > cap) st -= EXACT_SETS;
   return st;
