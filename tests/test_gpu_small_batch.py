@@ -1,0 +1,37 @@
+"""The small-batch kernel where a CTA's run covers several short column tiles, in launches queued back to back."""
+import pytest
+import torch
+
+from tilus_b200 import dtypes as D
+from tilus_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [20, 64, 100, 128])
+@pytest.mark.parametrize("N,K", [(28672, 512), (32000, 256), (128256, 256), (18944, 768), (20480, 128)])
+def test_runs_of_many_short_tiles_without_synchronisation(M, N, K):
+    """Few 128-row groups per column tile: the warps that decode weights reach the end of their CTA's run while
+    the MMAs of its first tiles still wait for the launch before.  Twelve launches in a row without a
+    synchronisation, four weights, every output compared in full with an fp32 product of the dequantized weights
+    (bit-exact with the oracle, test_gpu_parity.py).  One rounding of the output is 2^-11 of its size, sums
+    of up to 768 fp32 products stay far below it: 2e-3 of the largest output."""
+    dev = torch.device("cuda:0")
+    dt, group = D.int4b, 128
+    gen = torch.Generator(device=dev).manual_seed(N + K + M)
+    layers = []
+    for _ in range(4):
+        bq = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device=dev, generator=gen)
+        scales = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
+        layers.append((bq, scales))
+    xs = [torch.randn(M, K, device=dev, generator=gen).half() for _ in range(3)]
+    pl = ops.plan(M, N, K, dt, 0, group)
+    assert pl["kernel"] == 3
+    torch.cuda.synchronize()
+    outs = [ops.quantized_matmul(xs[i % 3], *layers[i % 4], dt, group) for i in range(12)]
+    torch.cuda.synchronize()
+    for i, got in enumerate(outs):
+        w = ops.dequantize(*layers[i % 4], dt, group).float()
+        ref = xs[i % 3].float() @ w
+        assert float((got.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max()), i
+    assert ops.device_status(ops.get_workspace(dev, 1 << 20)) == [0, 0, 0, 0]

@@ -12,10 +12,12 @@
 //     tile).  Set s takes the 128-row groups s, s + 2, ... of the CTA: a lane reads its column's four
 //     units, decodes and scales them (decode.cuh, unit_decode_scaled: the weights the reference
 //     multiplies by, examples/quantization/matmul_a16wx.py:316-320) and writes 64 tensor-memory columns.
-//     Each set has operand slots and ring stages of its own, so that every barrier has one kind of waiter
-//     and phases cannot be mistaken for one another (a third set measured slower: 12.9 -> 12.3 us at
-//     16 x 4096 x 14336 without it);
-//   * warps 8-11 are the epilogue; the dequantize warps take a share of the run's last segment;
+//     Each set has operand slots and ring stages of its own, so that every waiter of a ring barrier sees each
+//     of its phases in turn (a third set measured slower: 12.9 -> 12.3 us at 16 x 4096 x 14336 without it);
+//   * warps 8-11 are the epilogue; the dequantize warps take a share of the run's last segment.  They
+//     do not follow the accumulators' barriers (d_full) from segment to segment - with few groups per tile they are
+//     several segments ahead of the MMAs, and a phase of two segments ago would pass for the last one's -
+//     but wait for a barrier of one phase, run_done, that the last MMA of the run completes;
 //   * warp 12 brings the activations, two 2-D tiled TMA copies (128-byte swizzle) per group;
 //   * warp 13 brings packed weights, a 128-row group of the 128 columns at a time: one 3-D tiled
 //     TMA copy for the eight 16-column pieces.  For 2, 4 and 8 bits it swizzles 16-byte chunks by
@@ -71,6 +73,7 @@ struct BatchBarriers {
   uint64_t a_full[BATCH_A_MAX];
   uint64_t g_full[BATCH_STAGES_MAX], g_empty[BATCH_STAGES_MAX];
   uint64_t d_full[2], d_empty[2];
+  uint64_t run_done;  // the MMAs of the whole run have completed
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -144,6 +147,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     for (int i = 0; i < AS; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
     for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
     for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(d_full, i), 1); mbar_init(BAR_ADDR(d_empty, i), 4); }
+    mbar_init(BAR_ADDR(run_done, 0), 1);
     bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -239,7 +243,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
       asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
-      if (mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) {
+      if (mbar_wait_abortable(BAR_ADDR(run_done, 0), 0u, abort_flag)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), 0u, tile, len, wq, lane, set,
                             BATCH_SETS + 1);
@@ -405,6 +409,10 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
                        : "memory");
         pos += len;
       }
+      if (good)
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         BAR_ADDR(run_done, 0))
+                     : "memory");
     }
   }
 
@@ -412,7 +420,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     // the tile's sums to shared memory, over activations and ring (all MMAs have completed: nobody reads them)
     __syncwarp();
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
-    if (mbar_wait_abortable(BAR_ADDR(d_full, 0), 0, abort_flag)) {
+    if (mbar_wait_abortable(BAR_ADDR(run_done, 0), 0u, abort_flag)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float4* sums = reinterpret_cast<float4*>(smem_al) + (warp & 3) * 32 + lane;
       for (int c0 = (warp >> 2) * 16; c0 < p.M; c0 += 48) {
