@@ -43,3 +43,27 @@ def test_few_rows_whose_stream_plan_cuts_k(M):
     dt = weight_dtype("uint4b")
     assert ops.plan(1, 7168, 2048, dt, 8, 128)["tile_m"] == 0 and ops.plan(M, 7168, 2048, dt, 8, 128)["tile_m"] == 16
     _forced(M, 7168, 2048, dt, 8, dict(), seed=M)
+
+
+@pytest.mark.parametrize("w,zp", [("uint8", 128), ("int8", 0), ("int6b", 0), ("uint4b", 8), ("uint1b", 1)])
+def test_exact_small_batch_kernel_keeps_the_bits_of_its_sums(w, zp):
+    """Activations away from zero: the zero point is subtracted while the products are summed, so the fp32 sums
+    stay near their results.  An MMA loses at most 2^-23 of the running sum; 512 of them (16 per 128 rows, 32 groups), as
+    a random walk, 22.6 * 2^-23 of it.  With the running sum no larger than the result, a result within
+    that distance of the middle between two fp16 values (2^-11 apart) may go to the other one: 2 * 22.6 * 2^-23 / 2^-11 =
+    1.1 % of the outputs.  (Zero points subtracted at the end of a group: 6.3 % for 8 bits.)"""
+    import torch
+    from oracle import quant_oracle as qo
+    from tilus_b200 import packing
+
+    m, n, k, group, dt = 8, 1024, 4096, 128, weight_dtype(w)
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(1)
+    codes = torch.randint(0, 1 << dt.nbits, (k, n), device=dev, generator=gen, dtype=torch.int32).to(torch.uint8)
+    a = (torch.randn(m, k, device=dev, generator=gen) + 3.0).half()
+    sc = (torch.rand(k // group, n, device=dev, generator=gen) * 0.01 + 0.002).half()
+    plan = dict(kernel=2, tile_m=16, splits=1, cluster=1, ctas_per_split=128)
+    got = ops.quantized_matmul(a, packing.interleave(codes, dt).to(dev), sc, dt, group, zp, plan_override=plan)
+    value = torch.from_numpy(qo.decode_table(dt)).to(dev)[codes.long()] - zp
+    ref = a.double() @ (value * sc.double().repeat_interleave(group, 0))
+    assert float((got != ref.half()).float().mean()) <= 0.011

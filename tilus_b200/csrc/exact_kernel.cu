@@ -6,7 +6,11 @@
 // stream_kernel.cu - and the decode shrinks to bit extraction:
 //   * fp16 activations: an integer code sits at bit 0 of an fp16 subnormal (value code * 2^-24), a float code
 //     in its own fields (decode.cuh, pair_lin_uniform).  The tensor core multiplies these exactly.  The zero
-//     point is subtracted by a second set of MMAs whose weight operand is the constant -zero_point * 2^-24;
+//     point is subtracted by a second set of MMAs whose weight operand is the constant -zero_point * 2^-24,
+//     each right behind the 16 rows it belongs to.  With all of them behind the group's products the sums ran up to
+//     (code) before they came back to (code - zero point), and the fp32 accumulator lost bits to it: 8 x 4096 x 4096,
+//     uint8, activations around 3, 6.3 % of the outputs were not the nearest fp16 value (stream_kernel.cu 3.3 %;
+//     now 0.3 %).  Single bits need none of this: (code - 1) is a sign and an inverted bit;
 //   * bf16 activations: exact bf16 values (pair_exact; bf16 has no room for the subnormal trick).
 // That is what decides this kernel's speed: integer, shift and half instructions issue every second cycle
 // per SM quadrant on this GPU (measured: LOP3, SHF, PRMT, HFMA2 2.0 cycles, LOP3 + HFMA2 3.7 together, FFMA 1.0),
@@ -69,7 +73,7 @@ template <int VAR, int ACT>
 __global__ void __launch_bounds__(EXACT_THREADS, 1)
 exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
   constexpr int B = var_bits(VAR);
-  constexpr int BIAS = ACT == 0 ? var_bias(VAR) : 0;  // what the constant operand subtracts
+  constexpr int BIAS = ACT == 0 ? lin_uniform_bias(VAR) : 0;  // what the constant operand subtracts
   constexpr float F = ACT == 0 ? (float)(1u << lin_factor_log2(VAR)) : 1.0f;
   constexpr uint32_t WSTAGE = 2048u * B, SSTAGE = 256u;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -356,22 +360,25 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t bdesc = umma_smem_desc(smem_base + (uint32_t)slot * EXACT_ASTAGE);
         const uint32_t a_t = slots_t + (uint32_t)(slot * 64), d_t = tmem + (uint32_t)(slot * 16);
+        // the zero point of every 16 rows right behind their products: the running sum stays a sum of (code - zero point)
 #pragma unroll
-        for (int ks = 0; ks < (BIAS != 0 ? 16 : 8); ++ks) {
+        for (int i = 0; i < (BIAS != 0 ? 16 : 8); ++i) {
+          const int ks = BIAS != 0 ? i >> 1 : i;
+          const uint32_t op_t = BIAS != 0 && (i & 1) ? const_t : a_t + (uint32_t)(ks * 8);
           const uint64_t bd = bdesc + (uint64_t)((ks & 3) * 2) + ((ks & 4) ? EXACT_ASTAGE >> 5 : 0u);
-          if (ks == 0)
+          if (i == 0)
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.ne.b32 p, 0, 0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                ::"r"(d_t), "r"(a_t), "l"(bd), "r"(idesc)
+                ::"r"(d_t), "r"(op_t), "l"(bd), "r"(idesc)
                 : "memory");
           else
             asm volatile(
                 "{\n\t.reg .pred p;\n\t"
                 "setp.eq.b32 p, 0, 0;\n\t"
                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                ::"r"(d_t), "r"(ks < 8 ? a_t + (uint32_t)(ks * 8) : const_t), "l"(bd), "r"(idesc)
+                ::"r"(d_t), "r"(op_t), "l"(bd), "r"(idesc)
                 : "memory");
         }
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
