@@ -298,11 +298,13 @@ __device__ __forceinline__ void unit_decode_exact(const uint32_t* w, uint32_t* o
 // The linear pattern of pair H with every code at the same place: an integer code at mantissa bit 0 of an fp16
 // subnormal (value code * 2^-24), a float code in its own fields (value * 2^-(15 - bias)).  No factor depends
 // on the pair, so the activations are taken as they are.
-// Single bits with zero point 1 carry it themselves, -(1 - code): sign bit and inverted code.
-B200Q_HD constexpr int lin_uniform_bias(int v) { return var_bits(v) == 1 ? 0 : var_bias(v); }
+// Single bits with zero point 1 need no zero point: code - 1 = -(1 - code), the inverted bit (the same LOP3 as the
+// bit itself) and a negative factor.
+B200Q_HD constexpr bool lin_uniform_inverted(int v) { return !var_is_float(v) && var_bits(v) == 1 && var_bias(v) == 1; }
+B200Q_HD constexpr int lin_uniform_bias(int v) { return lin_uniform_inverted(v) ? 0 : var_bias(v); }
 template <int VAR, int H>
 B200Q_HD uint32_t pair_lin_uniform(const uint32_t* w) {
-  if constexpr (!var_is_float(VAR) && var_bias(VAR) == 1) return gather_pair<1, H, 0>(w, 0u) ^ 0x80018001u;
+  if constexpr (lin_uniform_inverted(VAR)) return gather_pair<1, H, 0>(w, 0u) ^ 0x00010001u;
   else if constexpr (!var_is_float(VAR)) return gather_pair<var_bits(VAR), H, 0>(w, 0u);
   else return pair_raw<VAR, H>(w);
 }

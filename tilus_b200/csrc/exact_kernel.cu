@@ -10,7 +10,7 @@
 //     each right behind the 16 rows it belongs to.  With all of them behind the group's products the sums ran up to
 //     (code) before they came back to (code - zero point), and the fp32 accumulator lost bits to it: 8 x 4096 x 4096,
 //     uint8, activations around 3, 6.3 % of the outputs were not the nearest fp16 value (stream_kernel.cu 3.3 %;
-//     now 0.3 %).  Single bits need none of this: (code - 1) is a sign and an inverted bit;
+//     now 0.3 %).  Single bits need none of this: (code - 1) is the inverted bit, negated;
 //   * bf16 activations: exact bf16 values (pair_exact; bf16 has no room for the subnormal trick).
 // That is what decides this kernel's speed: integer, shift and half instructions issue every second cycle
 // per SM quadrant on this GPU (measured: LOP3, SHF, PRMT, HFMA2 2.0 cycles, LOP3 + HFMA2 3.7 together, FFMA 1.0),
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(EXACT_THREADS, 1)
 exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
   constexpr int B = var_bits(VAR);
   constexpr int BIAS = ACT == 0 ? lin_uniform_bias(VAR) : 0;  // what the constant operand subtracts
-  constexpr float F = ACT == 0 ? (float)(1u << lin_factor_log2(VAR)) : 1.0f;
+  constexpr float F = ACT == 0 ? (lin_uniform_inverted(VAR) ? -1.0f : 1.0f) * (float)(1u << lin_factor_log2(VAR)) : 1.0f;
   constexpr uint32_t WSTAGE = 2048u * B, SSTAGE = 256u;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_unaligned = (uint32_t)__cvta_generic_to_shared(smem_raw);
