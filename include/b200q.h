@@ -85,6 +85,9 @@ int b200q_last_cuda_error(void);
 /* Static shape -> tile table for the current device.  Replaces the reference's per-shape
  * autotuning and dispatch table (python/tilus/lang/instantiated_script.py:327-358, :700-801). */
 int b200q_plan(int M, int N, int K, int wtype, int zero_point, int group, b200q_plan_t* plan);
+/* The same for activations of act_dtype (b200q_plan: fp16), which decides between the two forms of kernel 2: what
+ * b200q_gemm and the other unplanned calls launch for that type.  b200q_workspace_bytes covers both types. */
+int b200q_plan_for(int M, int N, int K, int wtype, int zero_point, int group, int act_dtype, b200q_plan_t* plan);
 
 /* Bytes of workspace b200q_gemm needs for this problem.  The workspace must be zeroed
  * once by the caller; every call leaves it zeroed again (as the reference's
@@ -122,7 +125,8 @@ int b200q_gemm_host(const void* a_host, int lda, const void* bq, const void* sca
                     int N, int K, int wtype, int zero_point, int group, int act_dtype, void* a_staging,
                     void* c_staging, void* workspace, size_t workspace_bytes, void* stream);
 
-/* Same as b200q_gemm, with the kernel selection supplied by the caller. */
+/* Same as b200q_gemm, with the kernel selection supplied by the caller: it runs what the plan says, for either
+ * activation type. */
 int b200q_gemm_planned(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N,
                        int K, int wtype, int zero_point, int group, int act_dtype, void* workspace,
                        size_t workspace_bytes, void* stream, const b200q_plan_t* plan);

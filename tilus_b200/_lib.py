@@ -71,6 +71,7 @@ SYMBOLS = {
     "b200q_status_string": (ctypes.c_char_p, [_i]),
     "b200q_last_cuda_error": (_i, []),
     "b200q_plan": (_i, [_i, _i, _i, _i, _i, _i, ctypes.POINTER(Plan)]),
+    "b200q_plan_for": (_i, [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(Plan)]),
     "b200q_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _i]),
     "b200q_gemm": (_i, [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "b200q_gemm_planned": (_i, [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _sz, _vp,

@@ -433,15 +433,25 @@ static bool stream_outrun(int M, const b200q_plan_t& pl, const DeviceInfo& di) {
   return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas_per_split <= di.sm_count;
 }
 
-static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_plan_t* pl) {
+static const int kStreamForm = -1;  // in place of an activation type: the stream kernel's plan for any M that it takes
+
+static int make_plan_uncached(int M, int N, int K, int var, int group, int act, b200q_plan_t* pl) {
   const DeviceInfo di = device_info();
   std::memset(pl, 0, sizeof(*pl));
   const int bits = var_bits(var);
+  if (act == kStreamForm) {
+    if (M > kStreamMaxRows || !stream_takes(K, group)) return ST_UNSUPPORTED;
+    const int st = plan_stream(M, N, K, bits, di, pl);
+    pl->passes = 1;
+    pl->workspace_bytes = stream_workspace_bytes(N);
+    return st;
+  }
   // Up to 4 rows the mma.sync stream kernel; above, the tcgen05 kernels, whose cost hardly depends on the rows.  A
   // Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 / 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8
   // rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's second 8-row tile doubles
-  // its staging and MMAs.
-  if (M <= kStreamPlanRows && stream_takes(K, group)) {
+  // its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
+  // kernel only a conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit).
+  if (M <= (act == B200Q_BF16 ? 8 : kStreamPlanRows) && stream_takes(K, group)) {
     if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di)) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
@@ -494,22 +504,22 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, b200q_pla
 // The table is a pure function of the shape (and of the device's SM count and shared memory, which
 // device_info caches for the current device), and a serving loop asks for the same few shapes over
 // and over: the latest results are kept per thread.
-static int make_plan(int M, int N, int K, int var, int group, b200q_plan_t* pl) {
-  struct Entry { int dev, M, N, K, var, group, status; b200q_plan_t plan; };
+static int make_plan(int M, int N, int K, int var, int group, int act, b200q_plan_t* pl) {
+  struct Entry { int dev, M, N, K, var, group, act, status; b200q_plan_t plan; };
   static thread_local Entry cache[16];
   static thread_local int used = 0, next = 0;
   int dev = 0;
   cudaGetDevice(&dev);
   for (int i = 0; i < used; ++i) {
     const Entry& e = cache[i];
-    if (e.M == M && e.N == N && e.K == K && e.var == var && e.group == group && e.dev == dev) {
+    if (e.M == M && e.N == N && e.K == K && e.var == var && e.group == group && e.act == act && e.dev == dev) {
       *pl = e.plan;
       return e.status;
     }
   }
-  const int status = make_plan_uncached(M, N, K, var, group, pl);
+  const int status = make_plan_uncached(M, N, K, var, group, act, pl);
   Entry& e = cache[next];
-  e.dev = dev; e.M = M; e.N = N; e.K = K; e.var = var; e.group = group; e.status = status; e.plan = *pl;
+  e.dev = dev; e.M = M; e.N = N; e.K = K; e.var = var; e.group = group; e.act = act; e.status = status; e.plan = *pl;
   next = (next + 1) % 16;
   if (used < 16) ++used;
   return status;
@@ -783,7 +793,7 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     const int tail = M % 256;
     if (M <= 256 || tail < 1 || tail > kStreamMaxRows) return ST_INVALID_ARG;
     b200q_plan_t tail_plan;
-    int st = make_plan(tail, N, K, var, group, &tail_plan);
+    int st = make_plan(tail, N, K, var, group, act, &tail_plan);
     if (st != ST_OK) return st;
     b200q_plan_t head = pl;
     head.passes = 1;
@@ -796,16 +806,6 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   }
   if (pl.kernel == 1)
     return run_umma(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
-  if (pl.kernel == 2 && plan_is_exact(pl) && act == B200Q_BF16 && M <= 8) {
-    // bf16 costs the exact kernel one more half instruction per pair of weights and the stream kernel only a
-    // conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit),
-    // unless its plan is one that the exact kernel outruns
-    b200q_plan_t rows;
-    const DeviceInfo di = device_info();
-    if (plan_stream(M, N, K, var_bits(var), di, &rows) == ST_OK && !stream_outrun(M, rows, di) &&
-        ws_bytes >= stream_workspace_bytes(N))
-      return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, rows);
-  }
   if (pl.kernel == 2 && plan_is_exact(pl))
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2)
@@ -841,11 +841,16 @@ const char* b200q_status_string(int status) {
 int b200q_last_cuda_error(void) { return g_last_cuda_error; }
 
 int b200q_plan(int M, int N, int K, int wtype, int zero_point, int group, b200q_plan_t* plan) {
+  return b200q_plan_for(M, N, K, wtype, zero_point, group, B200Q_F16, plan);
+}
+
+int b200q_plan_for(int M, int N, int K, int wtype, int zero_point, int group, int act_dtype, b200q_plan_t* plan) {
   if (!plan) return ST_INVALID_ARG;
+  if (!act_ok(act_dtype)) return ST_UNSUPPORTED;
   int var;
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
-  return make_plan(M, N, K, var, group, plan);
+  return make_plan(M, N, K, var, group, act_dtype, plan);
 }
 
 size_t b200q_workspace_bytes(int M, int N, int K, int wtype, int zero_point, int group) {
@@ -880,7 +885,7 @@ int b200q_gemm_gather(const void* a, int lda, const void* bq, const void* scales
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
   b200q_plan_t pl;  // the fused gather lives in the stream kernel only
-  if (!stream_takes(K, group) || plan_stream(M, N, K, var_bits(var), device_info(), &pl) != ST_OK) return ST_UNSUPPORTED;
+  if (make_plan(M, N, K, var, group, kStreamForm, &pl) != ST_OK) return ST_UNSUPPORTED;
   return run_stream(a, lda, bq, scales, nullptr, gather->ldc, M, N, K, var, group, act_dtype, workspace,
                     workspace_bytes, reinterpret_cast<cudaStream_t>(stream), pl, gather);
 }
@@ -960,7 +965,7 @@ int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void*
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
   b200q_plan_t pl;
-  st = make_plan(M, N, K, var, group, &pl);
+  st = make_plan(M, N, K, var, group, act_dtype, &pl);
   if (st != ST_OK) return st;
   return run_gemm(a, lda, bq, scales, c, ldc, M, N, K, var, group, act_dtype, workspace, workspace_bytes,
                   reinterpret_cast<cudaStream_t>(stream), pl);
@@ -1017,7 +1022,8 @@ int b200q_gemm_host(const void* a_host, int lda, const void* bq, const void* sca
     b200q_plan_t pl;
     cudaPointerAttributes cattr;
     if (check_problem(M, N, K, wtype, zero_point, group, true, &var) == ST_OK &&
-        M <= kStreamMaxRows && stream_takes(K, group) && plan_stream(M, N, K, var_bits(var), device_info(), &pl) == ST_OK && pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M)) {
+        make_plan(M, N, K, var, group, kStreamForm, &pl) == ST_OK &&
+        pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M)) {
       if (cudaPointerGetAttributes(&cattr, c_host) == cudaSuccess && cattr.type == cudaMemoryTypeHost &&
           cattr.devicePointer && (((uintptr_t)cattr.devicePointer) & 15) == 0) {
         if (!bq || !scales) return ST_INVALID_ARG;
@@ -1102,7 +1108,7 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
   b200q_plan_t pl;
-  st = make_plan(M, N, K, var, group, &pl);
+  st = make_plan(M, N, K, var, group, act_dtype, &pl);
   if (st != ST_OK) return st;
   if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES) {
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does

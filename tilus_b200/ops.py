@@ -44,10 +44,11 @@ def get_workspace(device, nbytes: int) -> torch.Tensor:
     return _lib.native().workspace(torch.cuda.current_device() if index is None else index, nbytes)
 
 
-def plan(M: int, N: int, K: int, w_dtype, zero_point: int = 0, group_size: int = 128) -> dict:
+def plan(M: int, N: int, K: int, w_dtype, zero_point: int = 0, group_size: int = 128,
+         act_dtype: torch.dtype = torch.float16) -> dict:
     dt = weight_dtype(w_dtype)
     pl = _lib.Plan()
-    _lib.check(_lib.load().b200q_plan(M, N, K, dt.code, zero_point, group_size, ctypes.byref(pl)))
+    _lib.check(_lib.load().b200q_plan_for(M, N, K, dt.code, zero_point, group_size, act_code(act_dtype), ctypes.byref(pl)))
     return pl.as_dict()
 
 
@@ -85,7 +86,7 @@ def quantized_matmul(a: torch.Tensor, bq: torch.Tensor, scales: torch.Tensor, w_
             st = lib.b200q_gemm(*args)
         else:
             pl = _lib.Plan()
-            _lib.check(lib.b200q_plan(M, N, K, dt.code, zero_point, group_size, ctypes.byref(pl)))
+            _lib.check(lib.b200q_plan_for(M, N, K, dt.code, zero_point, group_size, act, ctypes.byref(pl)))
             for k, v in plan_override.items():
                 setattr(pl, k, v)
             st = lib.b200q_gemm_planned(*args, ctypes.byref(pl))
