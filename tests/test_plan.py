@@ -16,7 +16,7 @@ def lib():
 def test_plans_are_reported_per_activation_type():
     """Up to 8 rows bfloat16 takes the stream kernel where fp16 takes the exact one; the plan says so, and asking for one
     type in between does not change what is reported for the other."""
-    shape = (8, 5120, 4096, "uint4b", 8, 128)
+    shape = (8, 6144, 4096, "uint4b", 8, 128)
     for _ in range(2):
         assert ops.plan(*shape)["tile_m"] == 16
         assert ops.plan(*shape, act_dtype=torch.bfloat16)["tile_m"] == 0
@@ -26,3 +26,16 @@ def test_plans_are_reported_per_activation_type():
         assert ops.workspace_bytes(m, *shape[1:]) >= max(both)
     with pytest.raises(_lib.B200QError):
         ops.plan(8, 5120, 4100, "uint4b", 8, 128, act_dtype=torch.bfloat16)
+
+
+@pytest.mark.parametrize("m,n,k,w,stream", [
+    (4, 4096, 2048, "uint4b", True), (5, 4096, 4096, "uint4b", True), (8, 4096, 4096, "uint4b", True),
+    (5, 28672, 4096, "uint4b", True), (8, 28672, 4096, "uint4b", False), (8, 32768, 2048, "uint4b", True),
+    (8, 8192, 2048, "uint4b", False), (5, 4096, 2048, "uint4b", False), (8, 2048, 4096, "uint4b", False),
+    (8, 2048, 8192, "uint4b", True), (5, 6144, 4096, "uint4b", False), (5, 1024, 4096, "float8_e5m2", True),
+    (5, 2048, 2048, "int7b", False), (6, 8192, 2048, "int8", False), (5, 8192, 4096, "int8", True),
+    (8, 4096, 4096, "int8", False), (9, 4096, 4096, "uint4b", False)])
+def test_five_to_eight_rows_take_the_kernel_measured_faster(m, n, k, w, stream):
+    """Both sides of every line of the rule, at shapes that were timed (fp16, one scale per 128 rows)."""
+    zp = 8 if w == "uint4b" else 0
+    assert (ops.plan(m, n, k, w, zp, 128)["tile_m"] == 0) is stream

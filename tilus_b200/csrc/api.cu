@@ -433,6 +433,33 @@ static bool stream_outrun(int M, const b200q_plan_t& pl, const DeviceInfo& di) {
   return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas_per_split <= di.sm_count;
 }
 
+// fp16, 5..8 rows: the shapes where the stream kernel is still the faster one.  What the exact kernel pays is a start and
+// an end of 5-6 us and, where equal runs share column tiles, sums in L2; what the stream kernel pays is the staging of the
+// activations, once per CTA, and a second pass through the scratch where it cuts K.  Measured, stream / exact, us, cold
+// chains, 11 types x 17 shapes x 5..8 rows:
+//  - two CTAs per SM without cutting K, layers of more than 12 M weights, up to 6 rows (4096 x 4096 at 5 rows: 4 bits 7.2 /
+//    7.9, float6 7.3 / 9.2), from 32 M weights up to 8 rows (32768 x 2048 at 8 rows: 4 bits 12.1 / 14.0); at 7 and 8 rows below
+//    that the exact kernel (8192 x 2048 at 8 rows, 4 bits 7.2 / 6.2), and between 4 M and 12 M, where its clusters have
+//    short ranges, at all (4096 x 2048 at 5 rows, 8 bits 5.8 / 5.1);
+//  - two CTAs per SM with K cut in four or more, small layers (4096 x 4096 at 8 rows, 4 bits 7.3 / 7.9; 2048 x 8192 7.2 / 8.4),
+//    again not between 4 M and 12 M (2048 x 4096 6.3 / 5.5);
+//  - up to 4 M float weights and 6 rows (1024 x 4096 at 5 rows, float8 4.8 / 6.2).
+// 8-bit integers, whose bytes the exact kernel takes with the fewest instructions, only from 32 M weights on (8192 x 2048 at 6
+// rows 7.7 / 6.5, 8192 x 4096 at 5 rows 10.9 / 11.8).  The choice costs 0.2 % against the better of the two over all
+// of them and is never more than 11 % behind the stream kernel (4096 x 8192 at 5 rows, 2 bits 8.6 / 9.5).
+static bool stream_ahead(int M, int N, int K, int var, const b200q_plan_t& pl, const DeviceInfo& di) {
+  const long long million = 1ll << 20, weights = (long long)N * K;
+  if (M <= kStreamPlanRows) return true;
+  if (M > 8) return false;
+  if (pl.splits * pl.ctas_per_split > di.sm_count) {
+    const bool bytes = var_bits(var) == 8 && !var_is_float(var);
+    if (pl.splits == 1) return weights >= 32 * million || (weights > 12 * million && M <= 6 && !bytes);
+    if (pl.splits >= 4) return (weights <= 4 * million || (weights > 12 * million && weights <= 20 * million)) && !bytes;
+    return false;
+  }
+  return var_is_float(var) && M <= 6 && weights <= 4 * million;
+}
+
 static const int kStreamForm = -1;  // in place of an activation type: the stream kernel's plan for any M that it takes
 
 static int make_plan_uncached(int M, int N, int K, int var, int group, int act, b200q_plan_t* pl) {
@@ -446,13 +473,14 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
     pl->workspace_bytes = stream_workspace_bytes(N);
     return st;
   }
-  // Up to 4 rows the mma.sync stream kernel; above, the tcgen05 kernels, whose cost hardly depends on the rows.  A
-  // Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 / 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8
+  // Up to 4 rows the mma.sync stream kernel (to 8 rows where stream_ahead says so); above, the tcgen05 kernels, whose
+  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 / 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8
   // rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's second 8-row tile doubles
   // its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
   // kernel only a conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit).
-  if (M <= (act == B200Q_BF16 ? 8 : kStreamPlanRows) && stream_takes(K, group)) {
-    if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di)) {
+  if (M <= 8 && stream_takes(K, group)) {
+    if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di) &&
+        (act == B200Q_BF16 || stream_ahead(M, N, K, var, *pl, di))) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
       return ST_OK;
