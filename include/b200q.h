@@ -140,7 +140,9 @@ int b200q_gemm_planned(const void* a, int lda, const void* bq, const void* scale
  *
  * Same arguments and results as b200q_gemm without `workspace`: the split-K scratch is a
  * fixed array inside the library, b200q_static_workspace_limit() bytes (8 MiB) per GPU.  Problems
- * whose b200q_workspace_bytes exceeds that limit return B200Q_ERR_WORKSPACE and launch nothing.
+ * whose b200q_workspace_bytes exceeds that limit run without the K split that asks for the room (batches
+ * of 5 rows and more, the prefill kernel's last round); where that leaves the least scratch the kernel
+ * needs above the limit too, the call returns B200Q_ERR_WORKSPACE and launches nothing.
  * The function allocates nothing and frees nothing.  The array belongs to the library's device
  * code: the CUDA runtime reserves its 8 MiB on a GPU when it loads that code there, which with
  * lazy module loading (the default) is the first call of b200q_static_ws_init or of this

@@ -39,3 +39,21 @@ def test_five_to_eight_rows_take_the_kernel_measured_faster(m, n, k, w, stream):
     """Both sides of every line of the rule, at shapes that were timed (fp16, one scale per 128 rows)."""
     zp = 8 if w == "uint4b" else 0
     assert (ops.plan(m, n, k, w, zp, 128)["tile_m"] == 0) is stream
+
+
+def _static_ws_refused(lib, m, n, k, wtype, zero_point=0, group=128, act=0):
+    """Whether b200q_gemm_static_ws turns the problem down for its scratch.  (Null operands: a problem that passes
+    this check is refused for them, or for want of a GPU, right behind it.)"""
+    return lib.b200q_gemm_static_ws(None, k, None, None, None, n, m, n, k, wtype, zero_point, group, act, None) \
+        == _lib.ST_WORKSPACE
+
+
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("m", [1, 4, 5, 8, 16])
+def test_static_workspace_takes_the_decode_path_up_to_one_width(lib, m, act):
+    """16 fp32 sums and a count per column fit the built-in scratch up to 130,544 columns, whichever kernel the rows
+    take; beyond, the problem stays refused."""
+    int4 = (1 << 16) | (4 << 8)
+    for n in (129280, 130544):
+        assert not _static_ws_refused(lib, m, n, 7168, int4, act=act)
+    assert _static_ws_refused(lib, m, 130560, 7168, int4, act=act)

@@ -1140,9 +1140,11 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
   if (st != ST_OK) return st;
   if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES) {
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
-    // without when the scratch is too small (small batches; the prefill kernel's last round)
-    const uint64_t least = pl.passes == 2 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
-    const bool optional = pl.kernel == 3 || (pl.kernel == 1 && pl.splits == 1);
+    // without when the scratch is too small (small batches; the prefill kernel's last round).  The decode path takes
+    // the same problems whichever of its kernels runs: those whose stream scratch fits.
+    const bool exact = pl.kernel == 2 && plan_is_exact(pl);
+    const uint64_t least = pl.passes == 2 || exact ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
+    const bool optional = pl.kernel == 3 || exact || (pl.kernel == 1 && pl.splits == 1);
     if (!(optional && least <= (uint64_t)B200Q_STATIC_WS_BYTES)) return ST_WORKSPACE;
   }
   void* ws = nullptr;
