@@ -33,3 +33,24 @@ def test_bf16_runs_the_form_its_plan_names(M):
     assert close(force(exact_plan), exact)
     assert close(force(stream_plan), saturated)
     assert close(ops.quantized_matmul(a, bq, sc, dt, group), saturated)
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 129280, 512), (16, 129280, 512), (300, 9472, 1024), (326, 6000, 2048)])
+def test_static_workspace_where_the_plan_asks_for_more(M, N, K):
+    """Problems whose plan wants more than the built-in scratch and that run without it: whole column tiles in the
+    exact kernel, tiles of 256 rows instead of 384 in the prefill kernel.  Twice, on the scratch the first one left."""
+    dev = torch.device("cuda:0")
+    lib, dt, group = _lib.load(), D.int4b, 128
+    gen = torch.Generator(device=dev).manual_seed(M)
+    bq = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device=dev, generator=gen)
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
+    a = torch.randn(M, K, device=dev, generator=gen).half()
+    assert lib.b200q_workspace_bytes(M, N, K, dt.code, 0, group) > lib.b200q_static_workspace_limit()
+    outs = [torch.full((M, N), float("nan"), dtype=torch.float16, device=dev) for _ in range(2)]
+    for c in outs:
+        _lib.check(lib.b200q_gemm_static_ws(a.data_ptr(), K, bq.data_ptr(), sc.data_ptr(), c.data_ptr(), N, M, N, K,
+                                            dt.code, 0, group, _lib.ACT_F16, torch.cuda.current_stream().cuda_stream))
+    ref = a.float() @ ops.dequantize(bq, sc, dt, group).float()
+    for c in outs:  # one rounding of the output (2^-11) and of each weight (2^-11, exact kernel: none), see also test_gpu_small_batch.py
+        assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert ops.device_status(None, dev) == [0, 0, 0, 0]

@@ -57,3 +57,11 @@ def test_static_workspace_takes_the_decode_path_up_to_one_width(lib, m, act):
     for n in (129280, 130544):
         assert not _static_ws_refused(lib, m, n, 7168, int4, act=act)
     assert _static_ws_refused(lib, m, 130560, 7168, int4, act=act)
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 9472, 4096), (329, 9280, 6656), (326, 6000, 2048), (1399, 1488, 1920), (272, 8592, 7936)])
+def test_static_workspace_takes_prefill_batches_that_256_row_tiles_fit(lib, m, n, k):
+    """Tiles of 384 rows come with a K split or larger slabs than the built-in scratch holds; tiles of 256 do without."""
+    uint4 = 4 << 8
+    assert ops.plan(m, n, k, "uint4b", 8, 128)["workspace_bytes"] > lib.b200q_static_workspace_limit()
+    assert not _static_ws_refused(lib, m, n, k, uint4, 8)

@@ -314,9 +314,9 @@ static double umma_cost(int M, int N, int K, int tm, const DeviceInfo& di) {
   const double rows = rounds <= 1.0 ? (M < tm ? M : tm) : (double)M / m_tiles;
   return rounds * (rows + 160.0);
 }
-static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
+static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo& di, int max_tm, b200q_plan_t* pl) {
   int tm = 256;  // (plans start here at 129 rows; smaller tiles only through an edited plan)
-  if (M > 256 && umma_cost(M, N, K, 384, di) < umma_cost(M, N, K, 256, di)) tm = 384;
+  if (M > 256 && max_tm >= 384 && umma_cost(M, N, K, 384, di) < umma_cost(M, N, K, 256, di)) tm = 384;
   const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
   const int ctas = m_tiles * n_tiles;
   const int splits = umma_splits(ctas, N, K, di);
@@ -424,6 +424,37 @@ static int umma_tail(int tiles, int grid, int kblocks, int uniform_splits, int N
 // fp32 scratch of the transposed tcgen05 kernel: one [tm][128] slab per tile slot
 static size_t umma_partial_bytes(int slots, int tm) { return (size_t)slots * tm * 128 * sizeof(float); }
 
+// The prefill kernel's plan with row tiles of at most max_tm rows.
+static void plan_prefill(int M, int N, int K, int var, int group, int max_tm, const DeviceInfo& di, b200q_plan_t* pl) {
+  const int bits = var_bits(var);
+  // A last row tile of at most 16 rows would cost each column tile the dequantization of its weights once more;
+  // those rows go to the decode path in a second launch instead (passes = 2).  Not where the row tiles of the
+  // others have room for them (M = 4097 with tiles of 384 rows: 10 and 257 rows more).
+  const int tail_rows = M % 256;
+  b200q_plan_t tail_plan;
+  pl->passes = 0;
+  if (M > 256 && tail_rows >= 1 && tail_rows <= kStreamMaxRows && stream_takes(K, group) &&
+      plan_stream(tail_rows, N, K, bits, di, &tail_plan) == ST_OK) {
+    plan_umma(M - tail_rows, N, K, bits, group, di, max_tm, pl);
+    pl->passes = 2;
+  }
+  if (pl->passes != 2 || pl->tile_m * pl->m_tiles >= M) plan_umma(M, N, K, bits, group, di, max_tm, pl);
+  // fp32 slabs per tile slot: every tile of a split-K launch, or the cut tiles of the last round
+  const int Mu = pl->passes == 2 ? M - M % 256 : M;
+  const int tiles = ((Mu + pl->tile_m - 1) / pl->tile_m) * ((N + 127) / 128);
+  const int grid = tiles * pl->splits < di.sm_count ? tiles * pl->splits : di.sm_count;
+  int tail_splits;
+  const int tail = umma_tail(tiles, grid, K / 64, pl->splits, N, &tail_splits);
+  const size_t part = umma_partial_bytes(pl->splits > 1 ? tiles : tail, pl->tile_m);
+  size_t need = WS_HEADER_BYTES + ws_counter_bytes(N) + part;
+  if (pl->passes == 2) {
+    const size_t rows = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M % 256, N);
+    if (need < stream_workspace_bytes(N)) need = stream_workspace_bytes(N);
+    if (need < rows) need = rows;
+  }
+  pl->workspace_bytes = need;
+}
+
 // A stream plan that cuts K and still has one CTA per SM at most (no divisor of the column tiles near two per SM): its
 // chunks meet in the scratch like the exact kernel's, at half the warps.  The exact kernel is then faster from two
 // rows on, and for one row from three chunks on; stream / exact, us, chains of cold launches, 4 bits: 7168 x 2048 (2
@@ -497,35 +528,8 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
       if (pl->workspace_bytes < stream_workspace_bytes(N)) pl->workspace_bytes = stream_workspace_bytes(N);
     }
     return ST_OK;
-  } else {
-    // A last row tile of at most 16 rows would cost each column tile the dequantization of its weights once more;
-    // those rows go to the decode kernel in a second launch instead (passes = 2).  Not where the row tiles of the
-    // others have room for them (M = 4097 with tiles of 384 rows: 10 and 257 rows more).
-    const int tail = M % 256;
-    b200q_plan_t tail_plan;
-    if (M > 256 && tail >= 1 && tail <= kStreamMaxRows && stream_takes(K, group) &&
-        plan_stream(tail, N, K, bits, di, &tail_plan) == ST_OK) {
-      plan_umma(M - tail, N, K, bits, group, di, pl);
-      pl->passes = 2;
-    }
-    if (pl->passes != 2 || pl->tile_m * pl->m_tiles >= M) {
-      plan_umma(M, N, K, bits, group, di, pl);
-    }
   }
-  // fp32 slabs per tile slot: every tile of a split-K launch, or the cut tiles of the last round
-  const int Mu = pl->passes == 2 ? M - M % 256 : M;
-  const int tiles = ((Mu + pl->tile_m - 1) / pl->tile_m) * ((N + 127) / 128);
-  const int grid = tiles * pl->splits < di.sm_count ? tiles * pl->splits : di.sm_count;
-  int tail_splits;
-  const int tail = umma_tail(tiles, grid, K / 64, pl->splits, N, &tail_splits);
-  const size_t part = umma_partial_bytes(pl->splits > 1 ? tiles : tail, pl->tile_m);
-  size_t need = WS_HEADER_BYTES + ws_counter_bytes(N) + part;
-  if (pl->passes == 2) {
-    const size_t rows = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M % 256, N);
-    if (need < stream_workspace_bytes(N)) need = stream_workspace_bytes(N);
-    if (need < rows) need = rows;
-  }
-  pl->workspace_bytes = need;
+  plan_prefill(M, N, K, var, group, 384, di, pl);
   return ST_OK;
 }
 
@@ -1138,6 +1142,10 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
   b200q_plan_t pl;
   st = make_plan(M, N, K, var, group, act_dtype, &pl);
   if (st != ST_OK) return st;
+  if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES && pl.kernel == 1 && pl.splits > 1 && pl.tile_m > 256) {
+    // row tiles of 384 are chosen with a K split that 256 rows may do without, or with smaller slabs (300 x 9472 x 4096)
+    plan_prefill(M, N, K, var, group, 256, device_info(), &pl);
+  }
   if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES) {
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
     // without when the scratch is too small (small batches; the prefill kernel's last round).  The decode path takes
