@@ -54,3 +54,21 @@ def test_static_workspace_where_the_plan_asks_for_more(M, N, K):
     for c in outs:  # one rounding of the output (2^-11) and of each weight (2^-11, exact kernel: none), see also test_gpu_small_batch.py
         assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert ops.device_status(None, dev) == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M", [1, 3, 5, 9, 16])
+@pytest.mark.parametrize("N,K", [(272, 1024), (4112, 2048)])
+@pytest.mark.parametrize("gap", [1, 4, 6])
+def test_decode_batches_write_rows_at_any_distance(M, N, K, gap):
+    """Outputs that are columns of a wider tensor whose rows are not a multiple of 16 bytes apart; the columns
+    beside them stay untouched."""
+    dev = torch.device("cuda:0")
+    dt, group = D.uint4b, 128
+    prob = synth.make_problem(M, N, K, dt, group, seed=M)
+    wide = torch.full((M, N + gap), 7.0, dtype=torch.float16, device=dev)
+    bq = packing.interleave(prob["codes"], dt).to(dev)
+    a, sc = prob["a"].to(dev), prob["scales"].to(dev)
+    ops.quantized_matmul(a, bq, sc, dt, group, 8, out=wide[:, :N])
+    ref = a.float() @ ops.dequantize(bq, sc, dt, group, 8).float()
+    assert float((wide[:, :N].float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert bool((wide[:, N:] == 7.0).all())

@@ -838,6 +838,13 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   }
   if (pl.kernel == 1)
     return run_umma(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+  if (pl.kernel == 2 && plan_is_exact(pl) && (ldc % 8) != 0) {
+    // rows of C at any distance: the exact kernel stores four columns at a time, the stream kernel single values
+    b200q_plan_t rows;
+    const int st = make_plan(M, N, K, var, group, kStreamForm, &rows);
+    if (st != ST_OK) return st;
+    return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, rows);
+  }
   if (pl.kernel == 2 && plan_is_exact(pl))
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2)
