@@ -72,3 +72,11 @@ def test_decode_batches_write_rows_at_any_distance(M, N, K, gap):
     ref = a.float() @ ops.dequantize(bq, sc, dt, group, 8).float()
     assert float((wide[:, :N].float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert bool((wide[:, N:] == 7.0).all())
+
+
+@pytest.mark.parametrize("M", [129, 200, 385])
+def test_small_batch_kernel_forced_beyond_its_rows(M):
+    """A plan edited to kernel 3 for more rows than one launch takes runs in pieces."""
+    from .test_gpu_parity import _forced
+
+    _forced(M, 272, 1024, D.int4b, 0, dict(kernel=3, splits=2, ctas_per_split=2), seed=M)

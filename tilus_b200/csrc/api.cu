@@ -849,8 +849,16 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 2)
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
-  if (pl.kernel == 3)
-    return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+  if (pl.kernel == 3) {
+    for (int m0 = 0; m0 < M; m0 += kBatchMaxRows) {  // (more rows only by an edited plan)
+      const int st = run_batch(reinterpret_cast<const unsigned short*>(a) + (size_t)m0 * lda, lda, bq, scales,
+                               reinterpret_cast<unsigned short*>(c) + (size_t)m0 * ldc, ldc,
+                               M - m0 < kBatchMaxRows ? M - m0 : kBatchMaxRows, N, K, var, group, act, workspace, ws_bytes,
+                               stream, pl);
+      if (st != ST_OK) return st;
+    }
+    return ST_OK;
+  }
   return ST_UNSUPPORTED;
 }
 
