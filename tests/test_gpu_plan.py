@@ -80,3 +80,14 @@ def test_small_batch_kernel_forced_beyond_its_rows(M):
     from .test_gpu_parity import _forced
 
     _forced(M, 272, 1024, D.int4b, 0, dict(kernel=3, splits=2, ctas_per_split=2), seed=M)
+
+
+@pytest.mark.parametrize("M", [7, 9, 16])
+@pytest.mark.parametrize("N,K,splits", [(272, 1024, 2), (6144, 2048, 4), (6144, 4096, 2)])
+@pytest.mark.parametrize("dt", [D.int4b, D.int8, D.float6_e3m2], ids=lambda d: d.name)
+def test_k_chunks_put_into_a_decode_plan(M, N, K, splits, dt):
+    """The number of k chunks is the one field that an edited decode plan of 5..16 rows needs."""
+    from .test_gpu_parity import _forced
+
+    assert ops.plan(M, N, K, dt, 0, 128)["tile_m"] == 16
+    _forced(M, N, K, dt, 0, dict(splits=splits), seed=M)

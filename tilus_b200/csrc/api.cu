@@ -847,6 +847,18 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   }
   if (pl.kernel == 2 && plan_is_exact(pl))
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
+  if (pl.kernel == 2 && pl.tile_m == 16 && stream_takes(K, group) && pl.splits > 1 && (K / BLOCK_K) % pl.splits == 0) {
+    // an exact plan edited to more k chunks is one for the stream kernel, whose rings and column tiles bound the rest
+    b200q_plan_t chunks = pl;
+    const int rows = M < stream_rows_per_pass(M) ? M : stream_rows_per_pass(M);
+    if (chunks.ctas_per_split > N / BLOCK_N) chunks.ctas_per_split = N / BLOCK_N;
+    if (chunks.ctas_per_split > 0) {
+      const int t_own = stream_tiles_owned(rows, N / BLOCK_N, chunks.ctas_per_split);
+      const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info());
+      if (chunks.stages > fit && fit > 0) chunks.stages = fit;
+    }
+    return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, chunks);
+  }
   if (pl.kernel == 2)
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
   if (pl.kernel == 3) {
