@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -77,17 +78,20 @@ struct StreamBuffers {
   cudaStream_t stream;
   at::Tensor workspace;
   at::Tensor staging[2][2];
+  std::mutex host_call;  // a host call is several operations on one staging pair: one thread's at a time
 };
 std::mutex g_mutex;
-std::vector<StreamBuffers>& pool() {
-  static auto* p = new std::vector<StreamBuffers>();  // outlives the interpreter's teardown
+std::vector<std::unique_ptr<StreamBuffers>>& pool() {
+  static auto* p = new std::vector<std::unique_ptr<StreamBuffers>>();  // outlives the interpreter's teardown
   return *p;
 }
-StreamBuffers& buffers_of(int device, cudaStream_t stream) {  // g_mutex held
-  for (StreamBuffers& b : pool())
-    if (b.device == device && b.stream == stream) return b;
-  pool().push_back(StreamBuffers{device, stream, {}, {}});
-  return pool().back();
+StreamBuffers& buffers_of(int device, cudaStream_t stream) {  // g_mutex held; the entry stays where it is
+  for (const auto& b : pool())
+    if (b->device == device && b->stream == stream) return *b;
+  pool().push_back(std::make_unique<StreamBuffers>());
+  pool().back()->device = device;
+  pool().back()->stream = stream;
+  return *pool().back();
 }
 at::Tensor byte_buffer(size_t bytes, int device, bool zero) {
   const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, (c10::DeviceIndex)device);
@@ -101,6 +105,19 @@ at::Tensor workspace_of(int device, cudaStream_t stream, size_t need) {
     b.workspace = byte_buffer(need > (1u << 20) ? need : (1u << 20), device, true);
   return b.workspace;
 }
+
+// Library calls run without the interpreter lock (as through ctypes): a launch into a full queue blocks, and a copy to
+// pageable memory waits for everything queued before it.
+class NoGil {
+ public:
+  NoGil() : state_(PyEval_SaveThread()) {}
+  ~NoGil() { PyEval_RestoreThread(state_); }
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
 
 PyObject* raise_status(int st) {
   PyObject* r = PyObject_CallFunction(g_raise_status, "i", st);
@@ -157,9 +174,14 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const size_t need = g_workspace_bytes(M, l.N, l.K, l.code, l.zero_point, l.group);
     if (need == 0) return raise_unsupported(M, l.N, l.K);
     const at::Tensor ws = workspace_of(dev.index(), stream, need);
-    const int st = g_gemm(rows.const_data_ptr(), (int)rows.stride(0), qw->const_data_ptr(), scales->const_data_ptr(),
-                          out.mutable_data_ptr(), l.N, M, l.N, l.K, l.code, l.zero_point, l.group, act,
-                          ws.mutable_data_ptr(), (size_t)ws.numel(), stream);
+    const void *a = rows.const_data_ptr(), *bq = qw->const_data_ptr(), *sc = scales->const_data_ptr();
+    void *c = out.mutable_data_ptr(), *w = ws.mutable_data_ptr();
+    const int lda = (int)rows.stride(0);
+    int st;
+    {
+      const NoGil unlocked;
+      st = g_gemm(a, lda, bq, sc, c, l.N, M, l.N, l.K, l.code, l.zero_point, l.group, act, w, (size_t)ws.numel(), stream);
+    }
     if (st != 0) return raise_status(st);
   }
   if (x->dim() != 2) {
@@ -213,9 +235,11 @@ PyObject* linear_host(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (need == 0) return raise_unsupported(M, l.N, l.K);
     const at::Tensor ws = workspace_of(dev.index(), stream, need);
     at::Tensor sa, sc;
+    StreamBuffers* buffers;
     {
       std::lock_guard<std::mutex> lock(g_mutex);
-      at::Tensor* s = buffers_of(dev.index(), stream).staging[M <= 16 ? 1 : 0];
+      buffers = &buffers_of(dev.index(), stream);
+      at::Tensor* s = buffers->staging[M <= 16 ? 1 : 0];
       const size_t abytes = (size_t)M * l.K * 2, cbytes = (size_t)M * l.N * 2;
       if (!s[0].defined() || (size_t)s[0].numel() < abytes || (size_t)s[1].numel() < cbytes) {
         s[0] = byte_buffer(abytes, dev.index(), false);
@@ -224,10 +248,17 @@ PyObject* linear_host(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       sa = s[0];
       sc = s[1];
     }
-    const int st = g_gemm_host(x->const_data_ptr(), (int)x->stride(0), qw->const_data_ptr(), scales->const_data_ptr(),
-                               out->mutable_data_ptr(), (int)out->stride(0), M, l.N, l.K, l.code, l.zero_point, l.group,
-                               act, sa.mutable_data_ptr(), sc.mutable_data_ptr(), ws.mutable_data_ptr(),
-                               (size_t)ws.numel(), stream);
+    const void *a = x->const_data_ptr(), *bq = qw->const_data_ptr(), *scp = scales->const_data_ptr();
+    void *c = out->mutable_data_ptr(), *a_stage = sa.mutable_data_ptr(), *c_stage = sc.mutable_data_ptr();
+    void* w = ws.mutable_data_ptr();
+    const int lda = (int)x->stride(0), ldc = (int)out->stride(0);
+    int st;
+    {
+      const NoGil unlocked;
+      std::lock_guard<std::mutex> lock(buffers->host_call);
+      st = g_gemm_host(a, lda, bq, scp, c, ldc, M, l.N, l.K, l.code, l.zero_point, l.group, act, a_stage, c_stage, w,
+                       (size_t)ws.numel(), stream);
+    }
     if (st != 0) return raise_status(st);
   }
   Py_INCREF(args[1]);
@@ -269,11 +300,15 @@ PyObject* gate_up_cast(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const size_t need = g_workspace_bytes(M, l.N, l.K, l.code, l.zero_point, l.group);
   if (need == 0) return raise_unsupported(M, l.N, l.K);
   const at::Tensor ws = workspace_of(dev.index(), stream, need);
-  const int st = g_gemm_cast(rows.const_data_ptr(), (int)rows.stride(0), qw->const_data_ptr(), scales->const_data_ptr(),
-                             gate_up.mutable_data_ptr(), l.N, out.mutable_data_ptr(), H,
-                             static_cast<float*>(sf.mutable_data_ptr()), M, l.N, l.K, l.code, l.zero_point, l.group, act,
-                             (int)channels, clamp ? 1 : 0, (float)clamp_value, ws.mutable_data_ptr(),
-                             (size_t)ws.numel(), stream);
+  const void *a = rows.const_data_ptr(), *bq = qw->const_data_ptr(), *sc = scales->const_data_ptr();
+  void *g = gate_up.mutable_data_ptr(), *o = out.mutable_data_ptr(), *f = sf.mutable_data_ptr(), *w = ws.mutable_data_ptr();
+  const int lda = (int)rows.stride(0);
+  int st;
+  {
+    const NoGil unlocked;
+    st = g_gemm_cast(a, lda, bq, sc, g, l.N, o, H, static_cast<float*>(f), M, l.N, l.K, l.code, l.zero_point, l.group, act,
+                     (int)channels, clamp ? 1 : 0, (float)clamp_value, w, (size_t)ws.numel(), stream);
+  }
   if (st != 0) return raise_status(st);
   return PyTuple_Pack(3, THPObjectPtr(THPVariable_Wrap(std::move(out))).get(),
                       THPObjectPtr(THPVariable_Wrap(std::move(sf))).get(),
