@@ -80,3 +80,61 @@ def test_host_calls_of_several_threads_on_one_stream():
     torch.cuda.synchronize()
     for x, out, want in cases:
         assert _close(out, want)
+
+
+def test_decode_calls_of_two_threads_do_not_overtake_each_other():
+    """A fetching decode call starts before the kernel in front of it has ended only if that kernel has let go of the
+    staging buffer; whose thread queued it does not matter.  One thread's calls fetch (pinned in and out), the
+    other's do not (pageable result)."""
+    k, n = 8192, 4096
+    layer = _layer(n, k)
+    cases = []
+    for i, m in enumerate((2, 12)):
+        x = _rows(m, k, 20 + i).pin_memory()
+        outs = [torch.zeros(m, n, dtype=torch.float16) for _ in range(8)]
+        cases.append((x, [o.pin_memory() for o in outs] if i == 0 else outs, layer(x.cuda()).cpu()))
+    torch.cuda.synchronize()
+    start = threading.Barrier(2)
+
+    def work(x, outs):
+        start.wait()
+        for _ in range(25):
+            for o in outs:
+                layer.forward_host(x, o)
+
+    threads = [threading.Thread(target=work, args=c[:2]) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for x, outs, want in cases:
+        for o in outs:
+            assert _close(o, want)
+
+
+def test_a_capture_between_two_eager_host_calls_leaves_their_order_alone():
+    """What a graph captured has not run: the next eager call still waits for the one before the capture."""
+    k, n = 8192, 4096
+    layer = _layer(n, k)
+    slow, fast = _rows(12, k, 1).pin_memory(), _rows(2, k, 2).pin_memory()
+    wide = torch.zeros(12, n + 4, dtype=torch.float16).pin_memory()  # rows not 16 bytes apart: not written directly
+    out_slow, out_fast = wide[:, :n], torch.zeros(2, n, dtype=torch.float16).pin_memory()
+    want_slow, want_fast = layer(slow.cuda()).cpu(), layer(fast.cuda()).cpu()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        layer.forward_host(slow, out_slow)
+        layer.forward_host(fast, out_fast)
+        stream.synchronize()
+        for _ in range(5):
+            graph = torch.cuda.CUDAGraph()
+            out_slow.zero_()
+            out_fast.zero_()
+            torch.cuda._sleep(2_000_000)
+            layer.forward_host(slow, out_slow)
+            graph.capture_begin(capture_error_mode="thread_local")  # (torch.cuda.graph would synchronise first)
+            layer.forward_host(fast, out_fast)
+            graph.capture_end()
+            layer.forward_host(fast, out_fast)
+            stream.synchronize()
+            assert _close(out_slow, want_slow) and _close(out_fast, want_fast)

@@ -1037,22 +1037,32 @@ int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void*
 // is written exactly once, goes straight to the host buffer when that is pinned memory the GPU
 // can address (the kernel's stores are the transfer); otherwise through the second staging
 // buffer and a copy.
-// Who used a staging buffer last on a stream, as far as this thread's b200q_gemm_host calls know: a
-// decode launch that fetches its own activations has finished reading the buffer by the time its
-// successor can start; every other kernel reads it until it ends.  (Within a captured graph the order
-// of launches is the order of capture; the first launch of a graph follows everything before it.)
-struct StagingUse { cudaStream_t stream; const void* buf; bool released; };
+// Who used a staging buffer last on a stream, as far as b200q_gemm_host calls tell: a decode launch that fetches its own
+// activations has finished reading the buffer by the time its successor can start; every other kernel reads it
+// until it ends.  Threads may share a stream, so the record is the process's.  A captured graph is a record of its own,
+// by the order of capture: its first launch follows everything before the graph, and what it captures has not run
+// on the stream.
+struct StagingUse { cudaStream_t stream; const void* buf; unsigned long long capture; bool released; };
 static bool staging_released_by_last_use(cudaStream_t st, const void* buf, bool now_released) {
-  static thread_local StagingUse uses[8];
-  static thread_local int next = 0;
+  static std::mutex mu;
+  static StagingUse uses[32];
+  static int next = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0;
+  if (cudaStreamGetCaptureInfo(st, &status, &capture) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;  // (the launch will say what is wrong)
+  }
+  if (status != cudaStreamCaptureStatusActive) capture = 0;
+  std::lock_guard<std::mutex> lock(mu);
   for (StagingUse& u : uses)
-    if (u.stream == st && u.buf == buf && u.buf != nullptr) {
+    if (u.stream == st && u.buf == buf && u.capture == capture && u.buf != nullptr) {
       const bool was = u.released;
       u.released = now_released;
       return was;
     }
-  uses[next] = {st, buf, now_released};
-  next = (next + 1) % 8;
+  uses[next] = {st, buf, capture, now_released};
+  next = (next + 1) % 32;
   return false;  // unknown history: wait
 }
 
