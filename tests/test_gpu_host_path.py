@@ -138,3 +138,70 @@ def test_a_capture_between_two_eager_host_calls_leaves_their_order_alone():
             layer.forward_host(fast, out_fast)
             stream.synchronize()
             assert _close(out_slow, want_slow) and _close(out_fast, want_fast)
+
+
+def _fill_free_memory(stream, sizes):
+    """Tensors that take over whatever blocks of these sizes the allocator has free for the stream."""
+    with torch.cuda.stream(stream):
+        return [torch.full((s,), 77, dtype=torch.uint8, device="cuda") for s in sizes for _ in range(4)]
+
+
+def test_replay_after_larger_calls_on_the_stream():
+    """A captured graph keeps the workspace and the staging buffers that it names, whatever larger calls come after
+    it: its results stay right and other tensors stay untouched."""
+    k, n = 2048, 8192
+    layer = _layer(n, k)
+    host_in, host_out = _rows(2, k, 1).pin_memory(), torch.zeros(2, n, dtype=torch.float16).pin_memory()
+    mid_in, mid_out = _rows(40, k, 2).pin_memory(), torch.zeros(40, n, dtype=torch.float16)
+    dev_in = _rows(100, k, 3).cuda()
+    want = [layer(host_in.cuda()).cpu(), layer(mid_in.cuda()).cpu(), layer(dev_in).cpu()]
+    mid_pinned = mid_out.pin_memory()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+
+        def calls():
+            layer.forward_host(host_in, host_out)
+            layer.forward_host(mid_in, mid_pinned)
+            return layer(dev_in)
+
+        calls()  # warm-up on the capture stream
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            dev_out = calls()
+        # larger calls of every kind, then tensors in whatever became free
+        wide = _layer(4 * n, k, seed=9)
+        for m in (16, 128, 1000):
+            wide.forward_host(_rows(m, k, m).pin_memory(), torch.zeros(m, 4 * n, dtype=torch.float16).pin_memory())
+            wide(_rows(m, k, m).cuda())
+        stream.synchronize()
+        others = _fill_free_memory(stream, [1 << e for e in range(12, 24)] + [2 * k * 2, 40 * k * 2, 2 * n * 2, 40 * n * 2])
+        for _ in range(2):
+            host_out.zero_()
+            mid_pinned.zero_()
+            graph.replay()
+            stream.synchronize()
+            for got, ref in zip((host_out, mid_pinned, dev_out), want):
+                assert _close(got, ref)
+        assert all(bool((t == 77).all()) for t in others)
+
+
+def test_alternating_shapes_settle_on_one_pair_of_staging_buffers():
+    """Layers with long rows in and short rows out, and the other way round, in turn: after the first round the
+    calls allocate nothing."""
+    a, b = _layer(4096, 1024), _layer(1024, 4096)
+    cases = [(lay, _rows(m, lay.in_features, 1).pin_memory(), torch.zeros(m, lay.out_features, dtype=torch.float16).pin_memory())
+             for m in (4, 64) for lay in (a, b)]
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            for lay, x, out in cases:
+                lay.forward_host(x, out)
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        for _ in range(5):
+            for lay, x, out in cases:
+                lay.forward_host(x, out)
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+        stream.synchronize()
+        for lay, x, out in cases:
+            assert _close(out, lay(x.cuda()))

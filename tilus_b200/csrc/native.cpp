@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
+#include <algorithm>
 #include <memory>
 #include <mutex>
 #include <vector>
@@ -73,11 +74,14 @@ bool check_weights(const at::Tensor& qw, const at::Tensor& scales, const c10::De
 // staging pair holds the activations and results of host calls: decode batches (whose kernel fetches
 // its own activations, so that consecutive calls overlap) have a pair of their own, so that a larger
 // batch in between does not make the next decode call wait for it.
+// A buffer that has become too small is replaced by one of at least twice its size, and kept: a captured graph may
+// name its address, and b200q_gemm_host remembers staging buffers by theirs.  What is kept is less than what replaced it.
 struct StreamBuffers {
   int device;
   cudaStream_t stream;
   at::Tensor workspace;
   at::Tensor staging[2][2];
+  std::vector<at::Tensor> superseded;
   std::mutex host_call;  // a host call is several operations on one staging pair: one thread's at a time
 };
 std::mutex g_mutex;
@@ -93,17 +97,23 @@ StreamBuffers& buffers_of(int device, cudaStream_t stream) {  // g_mutex held; t
   pool().back()->stream = stream;
   return *pool().back();
 }
-at::Tensor byte_buffer(size_t bytes, int device, bool zero) {
-  const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, (c10::DeviceIndex)device);
-  return zero ? at::zeros({(int64_t)bytes}, opt) : at::empty({(int64_t)bytes}, opt);
+// One of b's buffers with room for `need` bytes; g_mutex held, b's device current and b's stream its current stream.
+at::Tensor with_room(StreamBuffers& b, at::Tensor& buffer, size_t need, bool zero) {
+  const size_t have = buffer.defined() ? (size_t)buffer.numel() : 0;
+  if (have < need || !buffer.defined()) {
+    const int64_t size = (int64_t)std::max(need, 2 * have);
+    const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, (c10::DeviceIndex)b.device);
+    at::Tensor larger = zero ? at::zeros({size}, opt) : at::empty({size}, opt);
+    if (buffer.defined()) b.superseded.push_back(std::move(buffer));
+    buffer = std::move(larger);
+  }
+  return buffer;
 }
 // `device` is current and `stream` its current stream
 at::Tensor workspace_of(int device, cudaStream_t stream, size_t need) {
   std::lock_guard<std::mutex> lock(g_mutex);
   StreamBuffers& b = buffers_of(device, stream);
-  if (!b.workspace.defined() || (size_t)b.workspace.numel() < need)
-    b.workspace = byte_buffer(need > (1u << 20) ? need : (1u << 20), device, true);
-  return b.workspace;
+  return with_room(b, b.workspace, std::max(need, (size_t)1 << 20), true);
 }
 
 // Library calls run without the interpreter lock (as through ctypes): a launch into a full queue blocks, and a copy to
@@ -240,13 +250,8 @@ PyObject* linear_host(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       std::lock_guard<std::mutex> lock(g_mutex);
       buffers = &buffers_of(dev.index(), stream);
       at::Tensor* s = buffers->staging[M <= 16 ? 1 : 0];
-      const size_t abytes = (size_t)M * l.K * 2, cbytes = (size_t)M * l.N * 2;
-      if (!s[0].defined() || (size_t)s[0].numel() < abytes || (size_t)s[1].numel() < cbytes) {
-        s[0] = byte_buffer(abytes, dev.index(), false);
-        s[1] = byte_buffer(cbytes, dev.index(), false);
-      }
-      sa = s[0];
-      sc = s[1];
+      sa = with_room(*buffers, s[0], (size_t)M * l.K * 2, false);
+      sc = with_room(*buffers, s[1], (size_t)M * l.N * 2, false);
     }
     const void *a = x->const_data_ptr(), *bq = qw->const_data_ptr(), *scp = scales->const_data_ptr();
     void *c = out->mutable_data_ptr(), *a_stage = sa.mutable_data_ptr(), *c_stage = sc.mutable_data_ptr();
