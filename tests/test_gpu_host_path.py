@@ -205,3 +205,45 @@ def test_alternating_shapes_settle_on_one_pair_of_staging_buffers():
         stream.synchronize()
         for lay, x, out in cases:
             assert _close(out, lay(x.cuda()))
+
+
+@pytest.mark.parametrize("call", ["forward", "forward_host"])
+def test_first_call_of_a_stream_inside_a_capture(call):
+    """No call has been made on the stream before it is captured, twice: each graph finds a cleared workspace whichever
+    is replayed first, and so does an eager call before any replay.  100 rows share column tiles between CTAs, 2 rows
+    with 272 columns do so in the stream kernel."""
+    k = 2048
+    shapes = [(100, 4112), (2, 272)]
+    layers = [_layer(n, k, seed=n) for _, n in shapes]
+    xs = [_rows(m, k, m) for m, _ in shapes]
+    want = [lay(x.cuda()).cpu() for lay, x in zip(layers, xs)]  # (also loads the kernels)
+    if call == "forward_host":
+        for lay, x in zip(layers, xs):
+            lay.forward_host(x.pin_memory())
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    dirty = _fill_free_memory(stream, [1 << 20, 1 << 21, 1 << 22])
+    del dirty  # what the allocator hands out next for this stream is not zero
+    ins = [x.pin_memory() if call == "forward_host" else x.cuda() for x in xs]
+    outs = [torch.zeros(w.shape, dtype=w.dtype).pin_memory() for w in want]
+    with torch.cuda.stream(stream):
+
+        def calls():
+            if call == "forward_host":
+                return [lay.forward_host(x, o) for lay, x, o in zip(layers, ins, outs)]
+            return [lay(x) for lay, x in zip(layers, ins)]
+
+        graphs, results = [], []
+        for _ in range(2):
+            graphs.append(torch.cuda.CUDAGraph())
+            with torch.cuda.graph(graphs[-1], stream=stream):
+                results.append(calls())
+        eager = calls()
+        stream.synchronize()
+        assert all(_close(g, w) for g, w in zip(eager, want))
+        for i in (1, 0, 1):
+            for r in results[i]:
+                r.zero_()
+            graphs[i].replay()
+            stream.synchronize()
+            assert all(_close(g, w) for g, w in zip(results[i], want)), i

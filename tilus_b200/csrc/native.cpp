@@ -11,6 +11,8 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -20,6 +22,7 @@
 #include <algorithm>
 #include <memory>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -97,13 +100,38 @@ StreamBuffers& buffers_of(int device, cudaStream_t stream) {  // g_mutex held; t
   pool().back()->stream = stream;
   return *pool().back();
 }
+// Device memory for b's stream, which is b's device's current stream, zeroed if asked for.  While the stream is being
+// captured the allocation and the zeroing are not part of the capture: memory of the graph's own pool would be cleared by that
+// graph's replays only, and not before the first of them.  They take place on a stream of their own then, at once.
+at::Tensor allocate(const StreamBuffers& b, int64_t size, bool zero) {
+  const c10::Device dev(at::kCUDA, (c10::DeviceIndex)b.device);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(b.stream, &capture) != cudaSuccess) (void)cudaGetLastError();  // (the launch will say what is wrong)
+  if (capture == cudaStreamCaptureStatusNone) {
+    at::Tensor t = at::detail::empty_cuda({size}, at::kByte, dev, std::nullopt);
+    if (zero) C10_CUDA_CHECK(cudaMemsetAsync(t.mutable_data_ptr(), 0, (size_t)size, b.stream));
+    return t;
+  }
+  const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  static auto* sides = new std::vector<std::pair<int, cudaStream_t>>();  // per device; g_mutex held
+  cudaStream_t side = nullptr;
+  for (const auto& s : *sides)
+    if (s.first == b.device) side = s.second;
+  if (side == nullptr) {
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    sides->emplace_back(b.device, side);
+  }
+  const c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(side, dev.index()));
+  at::Tensor t = at::detail::empty_cuda({size}, at::kByte, dev, std::nullopt);
+  if (zero) C10_CUDA_CHECK(cudaMemsetAsync(t.mutable_data_ptr(), 0, (size_t)size, side));
+  C10_CUDA_CHECK(cudaStreamSynchronize(side));
+  return t;
+}
 // One of b's buffers with room for `need` bytes; g_mutex held, b's device current and b's stream its current stream.
 at::Tensor with_room(StreamBuffers& b, at::Tensor& buffer, size_t need, bool zero) {
   const size_t have = buffer.defined() ? (size_t)buffer.numel() : 0;
   if (have < need || !buffer.defined()) {
-    const int64_t size = (int64_t)std::max(need, 2 * have);
-    const auto opt = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, (c10::DeviceIndex)b.device);
-    at::Tensor larger = zero ? at::zeros({size}, opt) : at::empty({size}, opt);
+    at::Tensor larger = allocate(b, (int64_t)std::max(need, 2 * have), zero);
     if (buffer.defined()) b.superseded.push_back(std::move(buffer));
     buffer = std::move(larger);
   }
