@@ -59,8 +59,6 @@ class QuantizedLinear(nn.Module):
             torch.empty(in_features // group_size, out_features, dtype=self.act_torch_dtype), requires_grad=False
         )
         self.register_buffer("layout_version", torch.tensor(packing.LAYOUT_VERSION, dtype=torch.int32))
-        # what every call of this layer has in common, in the order csrc/native.cpp takes it
-        self._call = (w_dtype.code, self.zero_point, group_size, in_features, out_features)
 
     # -- loading ---------------------------------------------------------------------
     def load_and_quantize(self, weight: torch.Tensor):
@@ -141,9 +139,17 @@ class QuantizedLinear(nn.Module):
     # -- compute ---------------------------------------------------------------------
     # The checks, output and workspace tensors, stream lookup and library call of the three methods below
     # are one native function each (csrc/native.cpp): a decode call takes the GPU 5..15 us.
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def _operands(self):
+        """Packed weights, scales and the layer's constants in the order csrc/native.cpp takes them, as the attributes
+        say now (weights that are no parameters any more - buffers, parametrizations - are found by name)."""
         p = self._parameters
-        return native().linear(x, p["quantized_weight"], p["scales"], self._call)
+        qw, scales = p.get("quantized_weight"), p.get("scales")
+        if qw is None or scales is None:
+            qw, scales = self.quantized_weight, self.scales
+        return qw, scales, (self.w_dtype.code, self.zero_point, self.group_size, self.in_features, self.out_features)
+
+    def forward(self, x: torch.Tensor) -> torch.Tensor:
+        return native().linear(x, *self._operands())
 
     def forward_host(self, x_host: torch.Tensor, out_host: torch.Tensor | None = None) -> torch.Tensor:
         """forward() for activations kept in host memory: ``x_host`` [M, in_features] fp16 (pinned
@@ -152,17 +158,14 @@ class QuantizedLinear(nn.Module):
         library call (b200q_gemm_host); synchronise the stream before reading the result."""
         if out_host is None:
             out_host = torch.empty(x_host.shape[0], self.out_features, dtype=self.act_torch_dtype).pin_memory()
-        p = self._parameters
-        return native().linear_host(x_host, out_host, p["quantized_weight"], p["scales"], self._call)
+        return native().linear_host(x_host, out_host, *self._operands())
 
     def forward_swiglu_cast(self, x: torch.Tensor, num_per_channels: int = 128, swiglu_clamp_value=None):
         """For a gate_up projection (out_features = 2 * hidden, gate columns first): this layer's GEMM
         followed by SwiGLU and the per-token FP8 cast, queued by one library call
         (b200q_gemm_swiglu_cast).  Returns (out float8_e4m3fn [M, hidden], out_sf float32
         [M, hidden / num_per_channels], gate_up [M, out_features])."""
-        p = self._parameters
-        return native().gate_up_cast(x, p["quantized_weight"], p["scales"], self._call, num_per_channels,
-                                     swiglu_clamp_value)
+        return native().gate_up_cast(x, *self._operands(), num_per_channels, swiglu_clamp_value)
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, x_dtype={self.x_dtype.name}, "
