@@ -247,3 +247,21 @@ def test_first_call_of_a_stream_inside_a_capture(call):
             graphs[i].replay()
             stream.synchronize()
             assert all(_close(g, w) for g, w in zip(results[i], want)), i
+
+
+def test_gate_up_inputs_of_any_shape():
+    """The gate_up call takes rows however they are shaped (heads not merged, a wider matrix's first columns) and says
+    no to rows that are too short."""
+    k, n, m = 1024, 512, 6
+    layer = _layer(n, k)
+    x = _rows(m, k, 1).cuda()
+    out, sf, gate_up = layer.forward_swiglu_cast(x)
+    want = layer(x)
+    wide = torch.cat([x, torch.ones(m, 64, dtype=torch.float16, device="cuda")], dim=1)
+    for other in (x.view(m, 8, k // 8), x.view(2, m // 2, k), x.view(-1), wide):
+        o, s, g = layer.forward_swiglu_cast(other)
+        assert torch.equal(g, gate_up) and torch.equal(s, sf) and torch.equal(o.view(torch.uint8), out.view(torch.uint8))
+    assert _close(gate_up, want)
+    for bad in (x[:, : k // 2], x[:, : k // 2].contiguous(), x[0, :7]):
+        with pytest.raises(ValueError):
+            layer.forward_swiglu_cast(bad)

@@ -314,8 +314,17 @@ PyObject* gate_up_cast(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const double clamp_value = clamp ? PyFloat_AsDouble(args[5]) : 0.0;
   if (PyErr_Occurred()) return nullptr;
   if (channels < 1) { PyErr_SetString(PyExc_ValueError, "channels per scale must be positive"); return nullptr; }
+  // rows of K values: any shape whose elements make them up ([tokens, heads, head size] of an attention output), or the
+  // first K columns of a wider matrix
   at::Tensor rows;
-  if (!as_rows(*x, l.K, &rows)) return nullptr;
+  if (x->dim() == 2 && x->size(1) >= l.K) {
+    rows = *x;
+  } else if (x->dim() != 2 && x->numel() % l.K == 0) {
+    rows = x->reshape({-1, (int64_t)l.K});
+  } else {
+    PyErr_Format(PyExc_ValueError, "expected rows of %d input features", l.K);
+    return nullptr;
+  }
   const at::ScalarType dtype = scales->scalar_type();
   const int act = act_code(dtype);
   if (!rows.is_cuda() || rows.scalar_type() != dtype || act < 0 || rows.stride(1) != 1) {
