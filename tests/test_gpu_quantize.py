@@ -33,3 +33,48 @@ def test_rounding_boundaries_groups_and_alignment(dt, k, group, aligned):
     codes_ref, scales_ref = qo.quantize_weight(w.to(torch.float16).float().numpy(), dt, group)
     np.testing.assert_array_equal(scales.cpu().numpy().view(np.uint16), scales_ref.view(np.uint16))
     assert torch.equal(packed.cpu(), packing.interleave(torch.from_numpy(codes_ref), dt))
+
+
+def _moved(layer, how):
+    from torch import nn
+
+    if how == "bfloat16":
+        layer.bfloat16()  # scales only: the packed bytes stay uint8
+    elif how == "float32":
+        layer.scales = nn.Parameter(layer.scales.data.float(), requires_grad=False)
+    elif how == "strided":
+        layer.scales = nn.Parameter(torch.zeros(*layer.scales.shape[::-1], dtype=torch.float16, device="cuda").t(),
+                                    requires_grad=False)
+    elif how == "unaligned":
+        buf = torch.zeros(layer.quantized_weight.numel() + 4, dtype=torch.uint8, device="cuda")
+        layer.quantized_weight = nn.Parameter(buf[4:], requires_grad=False)
+    elif how == "scales on the host":
+        layer.scales = nn.Parameter(layer.scales.data.cpu(), requires_grad=False)
+
+
+@pytest.mark.parametrize("how", ["as built", "bfloat16", "float32", "strided", "unaligned", "scales on the host"])
+def test_load_into_parameters_of_any_kind(how):
+    """load_and_quantize writes straight into the parameters only where the kernel may; into all others it copies,
+    with the conversion that assignment implies."""
+    from tilus_b200 import QuantizedLinear
+
+    n, k, group, dt = 96, 512, 128, D.int4b
+    w = (torch.randn(n, k, generator=torch.Generator().manual_seed(2)) * 0.1).half()
+    layer = QuantizedLinear("float16", dt, group, k, n).cuda()
+    _moved(layer, how)
+    kind = layer.scales.dtype
+    layer.load_and_quantize(w)
+    torch.cuda.synchronize()
+    codes, scales = qo.quantize_weight(w.float().numpy(), dt, group)
+    assert torch.equal(layer.quantized_weight.data.cpu(), packing.interleave(torch.from_numpy(codes), dt))
+    assert layer.scales.dtype == kind
+    want = torch.from_numpy(scales).reshape(layer.scales.shape)
+    assert torch.equal(layer.scales.data.cpu(), want.to(kind))
+
+
+def test_out_tensors_that_do_not_fit_are_refused():
+    w = torch.randn(32, 256, device="cuda").half()
+    bq, sc = quantize.quantize_and_pack(w, D.int4b, 128)
+    for out in ((bq[1:], sc), (bq, sc.float()), (bq, sc.t()), (bq.cpu(), sc), (bq[:-16], sc)):
+        with pytest.raises(ValueError):
+            quantize.quantize_and_pack(w, D.int4b, 128, out=out)

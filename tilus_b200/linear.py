@@ -68,9 +68,14 @@ class QuantizedLinear(nn.Module):
             raise ValueError("load_and_quantize is symmetric: use a signed or float weight type "
                              "(unsigned codes come in through load_codes / load_packed)")
         dev = self.quantized_weight.device
-        if dev.type == "cuda":  # on the GPU: scales, codes and packing, straight into the parameters
-            quantize.quantize_and_pack(weight.to(dev), self.w_dtype, self.group_size, self.act_torch_dtype,
-                                       out=(self.quantized_weight.data, self.scales.data))
+        if dev.type == "cuda":  # on the GPU: scales, codes and packing, straight into the parameters where they can take it
+            out = (self.quantized_weight.data, self.scales.data)
+            if not quantize.can_write(*out, weight.shape, self.w_dtype, self.group_size, self.act_torch_dtype, dev):
+                out = None
+            packed, scales = quantize.quantize_and_pack(weight.to(dev), self.w_dtype, self.group_size,
+                                                        self.act_torch_dtype, out=out)
+            if out is None:  # (a layer moved to another dtype, scales elsewhere, ...: copied, converted as needed)
+                self.load_packed(packed, scales, layout="b200")
             return
         codes, scales = quantize.quantize_weight(weight.to(dev), self.w_dtype, self.group_size, self.act_torch_dtype)
         self.load_codes(codes, scales)

@@ -67,11 +67,19 @@ def quantize_weight(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: tor
     return codes.view(in_f, out_f), scales.view(in_f // group_size, out_f)
 
 
+def can_write(bq: torch.Tensor, scales: torch.Tensor, shape, w_dtype, group_size: int, x_dtype: torch.dtype, device) -> bool:
+    """Whether the library may write the packed weight and the scales of a weight[out, in] into these two tensors."""
+    out_f, in_f = shape
+    return (bq.device == device and scales.device == device and bq.dtype == torch.uint8 and scales.dtype == x_dtype
+            and bq.numel() * 8 == out_f * in_f * weight_dtype(w_dtype).nbits and scales.numel() == in_f // group_size * out_f
+            and bq.is_contiguous() and scales.is_contiguous() and bq.data_ptr() % 16 == 0)
+
+
 def quantize_and_pack(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: torch.dtype = torch.float16,
                       out: tuple | None = None):
     """weight[out, in] on a CUDA device (fp16, bf16 or fp32) -> (packed b200 bytes uint8[K*N*b/8],
     scales x_dtype[K/group, N]) in one library call: the same arithmetic as quantize_weight followed
-    by packing.interleave, bit for bit.  ``out``: the two (contiguous) tensors to write."""
+    by packing.interleave, bit for bit.  ``out``: the two tensors to write (see can_write)."""
     from . import _lib
     from .ops import act_code
 
@@ -88,6 +96,9 @@ def quantize_and_pack(weight: torch.Tensor, w_dtype, group_size: int, x_dtype: t
         scales = torch.empty(in_f // group_size, out_f, dtype=x_dtype, device=weight.device)
     else:
         bq, scales = out
+        if not can_write(bq, scales, weight.shape, dt, group_size, x_dtype, weight.device):
+            raise ValueError("out must be a contiguous uint8 tensor of K*N*nbits/8 bytes, 16-byte aligned, and a contiguous "
+                             f"{x_dtype} tensor of K/group_size*N scales, on the weight's device")
     with torch.cuda.device(weight.device):
         st = _lib.load().b200q_quantize(weight.data_ptr(), wcode, in_f,
                                         bq.data_ptr(), scales.data_ptr(), out_f, in_f, dt.code, group_size,
