@@ -18,6 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_build")
 LIB = os.path.join(HERE, "libb200q.so")
 NATIVE = os.path.join(HERE, "_native.so")
+NATIVE_STAMP = os.path.join(HERE, "_native.stamp")  # the interpreter and torch that NATIVE was built for
+HEADER = os.path.join(os.path.dirname(HERE), "include", "b200q.h")
 NPARTS = 8
 
 # Extra -D definitions for experiments (e.g. B200Q_EXTRA_DEFS="-DB200Q_GPW=2") and an
@@ -59,11 +61,15 @@ def _jobs():
 
 def build_native(force: bool = False) -> str:
     """The host path of QuantizedLinear (csrc/native.cpp) as a CPython extension against the installed torch."""
-    src = os.path.join(CSRC, "native.cpp")
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= os.path.getmtime(src):
-        return NATIVE
     import torch
 
+    src = os.path.join(CSRC, "native.cpp")
+    # what the binary fits: the interpreter's ABI, torch's C++ classes, the C ABI whose functions it calls by address
+    stamp = f"{sysconfig.get_config_var('SOABI')} torch {torch.__version__} {os.path.dirname(torch.__file__)}"
+    newest = max(os.path.getmtime(p) for p in (src, HEADER, os.path.abspath(__file__)))
+    if (not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) >= newest
+            and os.path.exists(NATIVE_STAMP) and open(NATIVE_STAMP).read() == stamp):
+        return NATIVE
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
@@ -74,12 +80,14 @@ def build_native(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed for native.cpp:\n{r.stdout}\n{r.stderr}")
+    with open(NATIVE_STAMP, "w") as f:
+        f.write(stamp)
     return NATIVE
 
 
 def _sources_mtime() -> float:
     paths = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh", ".h"))]
-    paths.append(os.path.join(os.path.dirname(HERE), "include", "b200q.h"))
+    paths.append(HEADER)
     paths.append(os.path.abspath(__file__))
     return max(os.path.getmtime(p) for p in paths)
 

@@ -25,15 +25,14 @@
 #include <utility>
 #include <vector>
 
+#include "../../include/b200q.h"
+
 namespace {
 
-typedef int (*GemmFn)(const void*, int, const void*, const void*, void*, int, int, int, int, int, int, int, int, void*,
-                      size_t, void*);
-typedef int (*GemmHostFn)(const void*, int, const void*, const void*, void*, int, int, int, int, int, int, int, int,
-                          void*, void*, void*, size_t, void*);
-typedef int (*GemmCastFn)(const void*, int, const void*, const void*, void*, int, void*, int, float*, int, int, int, int,
-                          int, int, int, int, int, float, void*, size_t, void*);
-typedef size_t (*WorkspaceFn)(int, int, int, int, int, int);
+typedef decltype(&b200q_gemm) GemmFn;
+typedef decltype(&b200q_gemm_host) GemmHostFn;
+typedef decltype(&b200q_gemm_swiglu_cast) GemmCastFn;
+typedef decltype(&b200q_workspace_bytes) WorkspaceFn;
 
 GemmFn g_gemm = nullptr;
 GemmHostFn g_gemm_host = nullptr;
