@@ -265,3 +265,28 @@ def test_gate_up_inputs_of_any_shape():
     for bad in (x[:, : k // 2], x[:, : k // 2].contiguous(), x[0, :7]):
         with pytest.raises(ValueError):
             layer.forward_swiglu_cast(bad)
+
+
+def test_first_launches_from_several_threads():
+    """Threads that launch the same kernel for the first time with different amounts of shared memory (rows 17 .. 128 of
+    one weight type no other test here uses)."""
+    k, n = 1024, 384
+    layer = _layer(n, k, dt=D.float5_e3m1)
+    w = layer.dequantized_weight().float()
+    xs = [_rows(m, k, m).cuda() for m in (17, 40, 64, 100, 128, 33, 80, 112)]
+    torch.cuda.synchronize()
+    start, outs = threading.Barrier(len(xs)), [None] * len(xs)
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            start.wait()
+            outs[i] = layer(xs[i])
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for x, out in zip(xs, outs):
+        assert out is not None and _close(out, x.float() @ w)

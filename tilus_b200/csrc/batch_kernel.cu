@@ -465,14 +465,9 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 template <int VAR, int ACT>
 static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
   auto kern = batch_kernel<VAR, ACT>;
-  static int configured_smem[16] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
-  }
+  static std::atomic<bool> allowed[16];
+  const cudaError_t e = allow_smem(kern, allowed);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
   cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
@@ -516,7 +511,8 @@ cudaError_t B200Q_CAT(batch_launch_part, B200Q_PART)(int var, const BatchParams&
 int batch_max_clusters(int c) {
   auto kern = batch_kernel<0, 0>;
   const int smem = 200 * 1024;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
+  static std::atomic<bool> allowed[16];
+  if (allow_smem(kern, allowed) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)c, 1, 1);
   cfg.blockDim = dim3(BATCH_THREADS, 1, 1);

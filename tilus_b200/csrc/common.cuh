@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "decode.cuh"
 
 namespace b200q {
@@ -177,6 +179,22 @@ struct CastParams {
   float clamp;
   int use_clamp;
 };
+
+// Lets launches of `kern` ask for all of an SM's shared memory, once per device; `allowed` is the kernel's own flag per
+// device.  (Allowing what each launch asks for would let two threads' first launches lower each other's limit.)
+template <class Kernel>
+inline cudaError_t allow_smem(Kernel kern, std::atomic<bool> (&allowed)[16]) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 0 && dev < 16 && allowed[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+  cudaFuncAttributes fixed;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  if ((e = cudaFuncGetAttributes(&fixed, kern)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed.sharedSizeBytes);
+  if (e == cudaSuccess && dev >= 0 && dev < 16) allowed[dev].store(true, std::memory_order_relaxed);
+  return e;
+}
 
 // two fp32 values rounded to the activation dtype (ACT 0: fp16, 1: bf16), low half first
 template <int ACT>

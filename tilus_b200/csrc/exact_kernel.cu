@@ -429,14 +429,9 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
 template <int VAR, int ACT>
 static cudaError_t exact_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
   auto kern = exact_kernel<VAR, ACT>;
-  static int configured_smem[16] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
-  }
+  static std::atomic<bool> allowed[16];
+  const cudaError_t e = allow_smem(kern, allowed);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
   cfg.blockDim = dim3(EXACT_THREADS, 1, 1);

@@ -834,14 +834,9 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
 template <int VAR, int MT, int GATHER, int ACT>
 static cudaError_t launch_one(const StreamParams& p, int smem_bytes, cudaStream_t stream) {
   auto kern = stream_kernel<VAR, MT, GATHER, ACT>;
-  static int configured_smem[16] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (smem_bytes > 48 * 1024 && (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes)) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
-  }
+  static std::atomic<bool> allowed[16];
+  const cudaError_t e = allow_smem(kern, allowed);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.S * p.CPC), 1, 1);
   cfg.blockDim = dim3(stream_warps(MT) * 32, 1, 1);

@@ -549,14 +549,9 @@ template <int VAR, int ACT>
 static cudaError_t umma_launch_one(const UmmaParams& p, const CUtensorMap& tmap, int smem_bytes,
                                    cudaStream_t stream) {
   auto kern = umma_kernel<VAR, ACT>;
-  static int configured_smem[16] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16 || configured_smem[dev] < smem_bytes) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 16) configured_smem[dev] = smem_bytes;
-  }
+  static std::atomic<bool> allowed[16];
+  const cudaError_t e = allow_smem(kern, allowed);
+  if (e != cudaSuccess) return e;
   kern<<<p.grid, UMMA_THREADS, smem_bytes, stream>>>(p, tmap);
   return cudaGetLastError();
 }
