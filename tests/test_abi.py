@@ -48,12 +48,12 @@ def test_plan_static_table():
     assert ops.plan(4096, 28672, 8192, "int4b", 0, 128)["kernel"] == 1  # prefill: tcgen05 kernel
     p8 = ops.plan(8, 4096, 4096, "uint4b", 8, 128)
     assert p8["kernel"] == 2 and p8["m_tiles"] == 1 and p8["smem_bytes"] <= 113 * 1024
-    # 9..16 rows: the same kernel with two 8-row activation tiles, one CTA per SM with all of its shared memory
+    # 9..16 rows: the decode path's tcgen05 form, one CTA per SM
     for m in (9, 16):
         ps = ops.plan(m, 8192, 8192, "uint4b", 8, 128)
         assert ps["kernel"] == 2 and ps["m_tiles"] == 2 and ps["smem_bytes"] <= 227 * 1024
         assert ps["splits"] * ps["ctas_per_split"] <= 148 and ps["stages"] >= 2
-    # 17..128 rows: tcgen05 kernel with the weights on the 256-column side of the MMA
+    # 17..128 rows: tcgen05 kernel that streams the weights once
     for m in (17, 64, 128):
         pw = ops.plan(m, 4096, 4096, "uint4b", 8, 128)
         assert pw["kernel"] == 3 and pw["smem_bytes"] <= 227 * 1024

@@ -52,8 +52,8 @@ def test_dequantize_bf16_bit_exact(dt, zp, group):
                          ids=lambda x: getattr(x, "name", str(x)))
 @pytest.mark.parametrize("M", [1, 16, 40, 256])
 def test_gemm_bf16(dt, zp, M):
-    """All three kernels (M = 1 and 16: mma.sync; 40: tcgen05, weights as the 256-column operand; 256:
-    tcgen05, weights in tensor memory) with bfloat16 activations, scales and outputs."""
+    """All four kernels (M = 1: mma.sync; 16: tcgen05 with exact weights; 40: tcgen05 with scaled weights, streamed
+    once; 256: prefill) with bfloat16 activations, scales and outputs."""
     dev = torch.device("cuda:0")
     N, K, g = 384, 2048, 128
     prob = synth.make_problem(M, N, K, dt, g, seed=M + dt.nbits)
@@ -70,7 +70,7 @@ def test_gemm_bf16(dt, zp, M):
 
 def test_bf16_large_activations_do_not_overflow_the_decode_path():
     """bfloat16 reaches magnitudes fp16 cannot hold.  The tcgen05 kernels multiply in bfloat16 and
-    take them as they are; the mma.sync path (M <= 16) multiplies in fp16 and saturates
+    take them as they are; the mma.sync kernel (here M = 1) multiplies in fp16 and saturates
     activations at +-65504, which this pins down."""
     dev = torch.device("cuda:0")
     N, K, g, dt = 64, 512, 128, D.int4b
@@ -111,3 +111,25 @@ def test_quantized_linear_bf16(dt, m):
     np.testing.assert_array_equal(_bits(layer.dequantized_weight()), _bits(w))
     ref = qo.gemm_bf16(a, w).double()
     assert float((c.cpu().double() - ref).abs().max() / ref.abs().max()) <= REL_TOL
+
+
+@pytest.mark.parametrize("dt,zp", [(D.uint4b, 8), (D.int8, 0), (D.float6_e3m2, 0), (D.uint1b, 1)],
+                         ids=lambda x: getattr(x, "name", str(x)))
+@pytest.mark.parametrize("M", [2, 4, 8, 9, 16])
+@pytest.mark.parametrize("N,K,cluster", [(7168, 2048, 1), (400, 2176, 8), (5760, 1152, 3)])
+def test_exact_kernel_bf16(dt, zp, M, N, K, cluster):
+    """The exact kernel in bfloat16: few rows where the stream plan would cut K (7168 x 2048), equal runs, and column
+    tiles shared by clusters with ragged K ranges and a ragged last tile."""
+    dev = torch.device("cuda:0")
+    group, tiles = 128, (N + 127) // 128
+    prob = synth.make_problem(M, N, K, dt, group, seed=M + N)
+    a, scales = prob["a"].to(torch.bfloat16), prob["scales"].to(torch.bfloat16)
+    bq = packing.interleave(prob["codes"], dt).to(dev)
+    plan = dict(kernel=2, tile_m=16, splits=1, cluster=cluster,
+                ctas_per_split=tiles * cluster if cluster > 1 else min(148, tiles * (K // group)))
+    if cluster == 1:
+        assert ops.plan(M, N, K, dt, zp, group, act_dtype=torch.bfloat16)["tile_m"] == 16
+    ref = qo.quantized_matmul_bf16(a, prob["codes"].numpy(), scales, dt, group, zp).double()
+    for _ in range(2):
+        c = ops.quantized_matmul(a.to(dev), bq, scales.to(dev), dt, group, zp, plan_override=plan)
+        assert float((c.cpu().double() - ref).abs().max() / ref.abs().max()) <= REL_TOL

@@ -117,9 +117,8 @@ def test_stream_kernel_variants(dt, zp):
 @pytest.mark.parametrize("M,N,K,splits", [(9, 272, 2048, 1), (33, 272, 2048, 4), (64, 512, 1024, 2), (65, 256, 1024, 8),
                                           (128, 768, 1536, 3), (17, 16, 512, 1)])
 def test_wide_kernel_shapes_and_clean_workspace(M, N, K, splits):
-    """Kernel 3 (tcgen05, weights as the 256-column operand) with forced split-K factors: ragged
-    last column tile (N not a multiple of 256), every activation-stage spacing (M <= 32, <= 64,
-    <= 128), odd group counts per split."""
+    """Kernel 3 with forced numbers of CTAs (splits times tiles of an edited plan): ragged last column tile, all
+    row counts from 9 to 128, runs that start and end inside column tiles."""
     tiles = (N + 255) // 256
     _forced(M, N, K, D.int4b, 0, dict(kernel=3, splits=splits, ctas_per_split=tiles, tile_m=128))
 
@@ -132,8 +131,8 @@ def test_wide_kernel_variants(dt, zp, group):
 
 
 def test_wide_kernel_more_items_than_sms():
-    """Persistent CTAs walk over several work items each: the pipelines, accumulator buffers and
-    barrier phases carry over item boundaries."""
+    """Runs over several column tiles each: the pipelines, accumulator buffers and barrier phases carry over
+    their boundaries."""
     M, N, K = 20, 256 * 200, 512
     prob = synth.make_problem(M, N, K, D.uint4b, 128, seed=2)
     c, _, _ = _run(prob)
@@ -221,8 +220,8 @@ def test_config2_prefill_full_size_sampled_columns():
 @pytest.mark.parametrize("M", [9, 12, 16])
 @pytest.mark.parametrize("N,K", [(8192, 8192), (4096, 4096), (272, 14336)])
 def test_stream_kernel_two_row_tiles_default_plan(M, N, K):
-    """9..16 rows run the mma.sync kernel with two 8-row activation tiles, one CTA per SM: K in
-    chunks, own tiles meeting in the fp32 scratch, left-over tiles (N = 272)."""
+    """9..16 rows by the default plan (the exact tcgen05 kernel; the mma.sync kernel's two 8-row activation tiles are
+    covered by forced plans and by the host and gather calls): equal runs and clusters, a ragged last tile (N = 272)."""
     prob = synth.make_problem(M, N, K, D.uint4b, 128, seed=M + N)
     assert ops.plan(M, N, K, D.uint4b, 8, 128)["kernel"] == 2
     c, _, _ = _run(prob)

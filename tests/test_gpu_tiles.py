@@ -34,7 +34,11 @@ def test_prefill_384_row_tiles_are_planned_and_walked():
 @pytest.mark.parametrize("N,K,group", [(16, 128, 128), (272, 1024, 512), (144, 8192, 8192), (4112, 2048, 128)])
 @pytest.mark.parametrize("w,zp", [("uint4b", 8), ("int8", 0), ("float6_e3m2", 0), ("uint1b", 0)])
 def test_exact_small_batch_kernel(M, N, K, group, w, zp):
-    _forced(M, N, K, weight_dtype(w), zp, dict(), seed=M + N, group=group)
+    """By the plan of 16 rows, which is always the exact kernel's (some batches of 5..8 rows go to the stream kernel)."""
+    pl = ops.plan(16, N, K, weight_dtype(w), zp, group)
+    assert pl["tile_m"] == 16
+    plan = {f: pl[f] for f in ("kernel", "splits", "cluster", "ctas_per_split", "tile_m", "stages")}
+    _forced(M, N, K, weight_dtype(w), zp, plan, seed=M + N, group=group)
 
 
 @pytest.mark.parametrize("M", [2, 4])
