@@ -56,7 +56,8 @@ typedef struct b200q_plan {
                             the tcgen05 kernel with exact weights; 3 = tcgen05 kernels that stream the weights
                             once (M <= 128), 1 = tcgen05 kernel for larger M */
   int32_t m_tiles;       /* kernel 2: 8-row activation tiles per pass (1 or 2); kernels 1, 3: tiles along M */
-  int32_t splits;        /* k chunks (kernel 2) / split-K factor (kernel 1); kernel 3: 1 */
+  int32_t splits;        /* k chunks (kernel 2; more than 1 makes a tcgen05 plan one for the stream kernel) /
+                            split-K factor (kernel 1); kernel 3: 1 */
   int32_t cluster;       /* kernel 3 and the tcgen05 form of kernel 2: CTAs that share a column tile's K and add up
                             in distributed shared memory (ctas_per_split = column tiles * cluster); else 1 */
   int32_t ctas_per_split;/* kernel 2: CTAs per k chunk, grid = splits * ctas_per_split; kernel 3: CTAs;
@@ -97,9 +98,11 @@ size_t b200q_workspace_bytes(int M, int N, int K, int wtype, int zero_point, int
 
 /* C = A x dequant(Bq).  a: [M, K] (row stride lda elements), bq: b200-packed weights,
  * scales: [K/group, N], c: [M, N] (row stride ldc), all three of dtype act_dtype.  Replaces
- * tilus_launch for QuantizedMatmul (examples/quantization/matmul_a16wx.py:231-405).  With bf16
- * and M <= 16 the activations are converted to fp16 for the tensor core: exactly, except that
- * magnitudes above 65504 saturate there and magnitudes below 2^-24 become zero. */
+ * tilus_launch for QuantizedMatmul (examples/quantization/matmul_a16wx.py:231-405).  The tcgen05
+ * kernels multiply bf16 activations as they are.  The stream kernel (b200q_plan_for: kernel 2 with
+ * tile_m 0; bf16 batches of up to 8 rows at most shapes, and up to 16 rows of the host-buffer and gather
+ * calls) converts them to fp16 for the tensor core: exactly, except that magnitudes above
+ * 65504 saturate there and magnitudes below 2^-24 become zero. */
 int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
                int wtype, int zero_point, int group, int act_dtype, void* workspace, size_t workspace_bytes,
                void* stream);
@@ -114,7 +117,7 @@ int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void*
  *
  * How A travels depends on where it lies.  Pageable memory, or more than 256 KB: a copy operation
  * on the stream.  Pinned memory the GPU can address: a small kernel whose PCIe reads run under the
- * previous kernel of the stream.  Pinned memory and a decode batch (M <= 16 on the stream kernel, result
+ * previous kernel of the stream.  Pinned memory and a decode batch (M <= 16, by the stream kernel whatever b200q_plan says; result
  * written straight to pinned c_host): no separate operation at all - the first CTAs of the GEMV kernel
  * fetch the rows, the others wait for them (bounded, status[1] = 9), and consecutive such calls overlap on
  * the GPU: a call does not wait for the kernel before it until it writes its outputs, which therefore
@@ -290,9 +293,9 @@ int b200q_gemm_swiglu_cast(const void* a, int lda, const void* bq, const void* s
 
 /* Reads the device status header of a workspace (synchronises `stream`): status[0] is 0 or
  * B200Q_ERR_DEVICE_TIMEOUT, status[1..3] say which wait gave up (1: 2 = tcgen05 prefill pipeline,
- * 3 = decode kernel's weight ring, 5 = wait for a peer's columns, 6 = tcgen05 small-batch pipeline,
- * 7 / 8 = gather push / collect, 9 = wait for the CTAs that fetch host activations; 2: CTA; 3: warp or
- * thread).  Clears the header.  A launch that gave up may leave partial sums
+ * 3 = stream kernel's weight ring, 5 = wait for a peer's columns, 6 = tcgen05 small-batch pipeline,
+ * 7 / 8 = gather push / collect, 9 = wait for the CTAs that fetch host activations, 10 = exact
+ * small-batch kernel's pipeline; 2: CTA; 3: warp or thread).  Clears the header.  A launch that gave up may leave partial sums
  * behind: zero the workspace before it is used again.  workspace == NULL names the built-in
  * scratch of b200q_gemm_static_ws, which this call then puts back to zero itself. */
 int b200q_device_status(void* workspace, int32_t status[4], void* stream);

@@ -214,7 +214,7 @@ static int stream_ctas_per_chunk(int NT, int s, int per_sm, const DeviceInfo& di
   return full > NT ? NT : full;
 }
 static const int kStreamMaxRows = 16;  // what the kernel takes
-static const int kStreamPlanRows = 4;  // what the plan gives it (gather launches and row tails: all of the above)
+static const int kStreamPlanRows = 4;  // what the plan gives it at any shape (gather and host-buffer launches: all of the above)
 static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counter_bytes(N) + (size_t)16 * N * sizeof(float); }
 // K is cut into S chunks (a divisor of K/512, at most one per SM) so that the activation chunk
 // [M, K/S] fits next to the rings; the grid is S * CPC.  Measured preferences, in this order: all of
@@ -348,8 +348,9 @@ static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; 
 //  - equal runs of 128-row groups, one per SM: no SM idles, but the tiles' sums meet in L2;
 //  - a cluster of c CTAs per tile: sums meet in distributed shared memory (at most as many tiles as clusters fit);
 //  - one CTA per tile.
-// The times are fits to chains of launches on B200 (4-bit weights, us; 2048^2 .. 4096 x 14336, 16 .. 128 rows, each
-// form forced; within 15 %).  Fewer CTAs start and end cheaper because the next launch finds SMs free.
+// The times are fits to chains of launches on B200 (4-bit weights in fp16, us; 2048^2 .. 4096 x 14336, 16 .. 128 rows, each
+// form forced; within 15 % there) and serve every width and both activation types: for 100 x 11008 x 4224, 6 bits in
+// bf16, they say 16.1 where a call takes 20.2.  Fewer CTAs start and end cheaper because the next launch finds SMs free.
 static int max_clusters(int c) {
   static int cache[16][9];
   int dev = 0;
@@ -505,9 +506,9 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
     return st;
   }
   // Up to 4 rows the mma.sync stream kernel (to 8 rows where stream_ahead says so); above, the tcgen05 kernels, whose
-  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 / 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8
-  // rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's second 8-row tile doubles
-  // its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
+  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 /
+  // 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8 rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's
+  // second 8-row tile doubles its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
   // kernel only a conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit).
   if (M <= 8 && stream_takes(K, group)) {
     if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di) &&

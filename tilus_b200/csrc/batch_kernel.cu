@@ -39,9 +39,9 @@
 // a cluster of CTAs to itself, the launch takes the cluster form instead (batch_common.cuh; the rule is in
 // api.cu).
 //
-// Measured (4-bit, group 128, a chain of launches; the kernel before it wrote dequantized weights to
-// 256-column shared-memory operands): 64 x 28672 x 4096 44.1 -> 23.4 us, 64 x 8192 x 8192 27.6 -> 16.4,
-// 128 x 8192 x 8192 34.0 -> 22.7.  What is left at 64 rows is the dequantize warps' instructions and
+// Measured (4-bit, group 128, a chain of cold launches; the kernel before it wrote dequantized weights to
+// 256-column shared-memory operands): 64 x 28672 x 4096 44.5 -> 24.9 us, 64 x 8192 x 8192 28.2 -> 17.1,
+// 128 x 8192 x 8192 34.0 -> 19.2.  What is left at 64 rows is the dequantize warps' instructions and
 // the additions of the partial tiles in L2.
 //
 // Every mbarrier wait is bounded in time; a wait that runs out raises a CTA-wide abort flag, all loops
@@ -535,7 +535,10 @@ int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
 // Activation groups (at most as many as there are operand slots) and ring stages (a multiple of the dequantize
 // sets) in the rest.  Up to 32 rows a CTA stays within half an SM's shared memory, so that the next launch of the
 // stream becomes resident beside this one and fills its ring while this one ends (a Llama-3-8B block of
-// linears at 32 rows: 51 us, 56 with one CTA per SM).  Above, a CTA takes more than half: the activations leave
+// linears, 4 bits, at 32 rows: 51 us, 56 with one CTA per SM).  The registers allow that for 1..7-bit integers (6 bits in
+// fp16 only), 7-bit floats and float4, which take 64; 8-bit types, 5- and 6-bit floats, float3 and 6-bit integers in bf16
+// take 66..88, so they keep to the half and run one CTA per SM all the same (8 bits with two stages in the ring:
+// 24 x 8192 x 8192 24.8 us, 14.8 with 4 bits).  Above, a CTA takes more than half: the activations leave
 // too little for the ring, and launches that leave SMs free (clusters, one CTA per column tile) would meet others
 // two to an SM, where one waits for the other's tensor memory (64 rows: 81 us with the two kinds mixed, 62).
 void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {

@@ -23,16 +23,16 @@
 //     it reads the sums of the group that was there (16 columns of tensor memory) and adds them, times their
 //     scale, to its fp32 sums of the column: one wait serves the slot and the sums.  A set needs about 1200
 //     cycles per group, most of them latencies of its barriers and of tensor memory, so their number sets the
-//     rate of narrow weights (two sets with three slots each: 13.8 us for 8192 x 8192 of 1 .. 4 bits);
+//     rate of narrow weights;
 //   * four warps finish column tiles: the sets hand over their sums through shared memory, so that the
 //     decoding goes on while a tile's last contributions are counted and written;
 //   * one warp each (one elected thread) brings the activations, the packed weights, the scales;
 //   * one warp owns tensor memory and issues the MMAs: 8 (or 16 with a zero point) per group, one commit.
 //
-// Measured (4-bit, group 128, 16 rows, a chain of launches; stream_kernel.cu before): 28672 x 4096 37.2 -> 20.6 us,
-// 8192 x 8192 19.0 -> 14.2, 4096 x 4096 10.1 -> 7.9.  Without the decode the first takes 17.4 us, without
-// decode and sums 15.6, against 9.4 us of HBM time: what is left is the start and the end of a launch
-// (about 5 us) and the decode's instructions.
+// Measured (4-bit, group 128, 16 rows, a chain of cold launches; stream_kernel.cu before): 28672 x 4096 37.3 -> 20.8 us,
+// 8192 x 8192 19.5 -> 14.3, 4096 x 4096 10.2 -> 8.3, against 9.4, 5.4 and 1.4 us of HBM time.  What is left is the start and
+// the end of a launch (about 5 us: 640 threads of 91 .. 96 registers leave no room for another GEMM's CTA on the SM, so
+// nothing of it lies under the launch before) and the decode's instructions.
 //
 // Every mbarrier wait is bounded in time; a wait that runs out raises a CTA-wide abort flag, all loops
 // leave, the producers give their copies in flight a bounded chance to land, tensor memory is freed and
@@ -476,9 +476,10 @@ int exact_smem_bytes(int bits, int stages, int M) {
   return 1024 + EXACT_SLOTS * (int)EXACT_ASTAGE + stages * batch_stage_bytes(bits, 1) + EXACT_SETS * (int)exact_hand_bytes(M) +
          (int)sizeof(ExactBarriers);
 }
-// Ring stages (a multiple of the sets).  Up to 8 rows within half an SM's shared memory, like stream_kernel.cu, whose
-// launches may follow, where that holds two stages per set (nine of 4-bit weights); 7 and 8 bits get one there, whose
-// copy and decoding cannot overlap (8 x 8192 x 8192, 8 bits: 22.3 us with 3 stages, 20.4 with 9).
+// Ring stages (a multiple of the sets).  Up to 8 rows within half an SM's shared memory where that holds two stages per
+// set (nine of 4-bit weights); 7 and 8 bits get one there, whose copy and decoding cannot overlap (8 x 8192 x 8192, 8 bits:
+// 22.3 us with 3 stages, 20.4 with 9).  The half was meant for a launch that follows on the same SM; the registers
+// keep that from happening, so the limit only bounds the ring.
 int exact_stages(int bits, int max_smem, int M) {
   const int half = 113 * 1024;
   const int cap = M <= 8 && exact_smem_bytes(bits, 2 * EXACT_SETS, M) <= half ? half : max_smem;
