@@ -91,3 +91,21 @@ def test_k_chunks_put_into_a_decode_plan(M, N, K, splits, dt):
 
     assert ops.plan(M, N, K, dt, 0, 128)["tile_m"] == 16
     _forced(M, N, K, dt, 0, dict(splits=splits), seed=M)
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 6000, 1024), (329, 9280, 1024)])
+def test_prefill_with_less_scratch_than_its_plan_asks_for(M, N, K):
+    """A fixed workspace that holds what tiles of 256 rows need, where the plan's tiles of 384 rows would cut K."""
+    dev = torch.device("cuda:0")
+    dt, group = D.int4b, 128
+    gen = torch.Generator(device=dev).manual_seed(M)
+    bq = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device=dev, generator=gen)
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
+    a = torch.randn(M, K, device=dev, generator=gen).half()
+    pl = ops.plan(M, N, K, dt, 0, group)
+    assert pl["tile_m"] == 384 and pl["workspace_bytes"] > (1 << 16)
+    ws = torch.zeros(1 << 16, dtype=torch.uint8, device=dev)
+    ref = a.float() @ ops.dequantize(bq, sc, dt, group).float()
+    c = ops.quantized_matmul(a, bq, sc, dt, group, workspace=ws)
+    assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert int(ws.count_nonzero()) == 0

@@ -558,6 +558,13 @@ static int make_plan(int M, int N, int K, int var, int group, int act, b200q_pla
   return status;
 }
 
+// The plan for a call that has `scratch` bytes.  Row tiles of 384 come with a K split that 256 rows may do without, or with
+// larger slabs (300 x 9472 x 4096): where theirs do not fit, tiles of 256.
+static void plan_within(int M, int N, int K, int var, int group, size_t scratch, b200q_plan_t* pl) {
+  if (pl->workspace_bytes > (uint64_t)scratch && pl->kernel == 1 && pl->splits > 1 && pl->tile_m > 256)
+    plan_prefill(M, N, K, var, group, 256, device_info(), pl);
+}
+
 // row tiles per raster group of the transposed tcgen05 kernel: as many as keep one group's
 // activation rows (tm x K 16-bit values per tile) within 32 MB, a quarter of L2
 static int umma_m_group(int tm, int K, int m_tiles) {
@@ -1027,6 +1034,7 @@ int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void*
   b200q_plan_t pl;
   st = make_plan(M, N, K, var, group, act_dtype, &pl);
   if (st != ST_OK) return st;
+  plan_within(M, N, K, var, group, workspace_bytes, &pl);
   return run_gemm(a, lda, bq, scales, c, ldc, M, N, K, var, group, act_dtype, workspace, workspace_bytes,
                   reinterpret_cast<cudaStream_t>(stream), pl);
 }
@@ -1180,10 +1188,7 @@ int b200q_gemm_static_ws(const void* a, int lda, const void* bq, const void* sca
   b200q_plan_t pl;
   st = make_plan(M, N, K, var, group, act_dtype, &pl);
   if (st != ST_OK) return st;
-  if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES && pl.kernel == 1 && pl.splits > 1 && pl.tile_m > 256) {
-    // row tiles of 384 are chosen with a K split that 256 rows may do without, or with smaller slabs (300 x 9472 x 4096)
-    plan_prefill(M, N, K, var, group, 256, device_info(), &pl);
-  }
+  plan_within(M, N, K, var, group, B200Q_STATIC_WS_BYTES, &pl);
   if (pl.workspace_bytes > (uint64_t)B200Q_STATIC_WS_BYTES) {
     // beyond the built-in scratch - unless all that asks for the room is a K split that the kernel does
     // without when the scratch is too small (small batches; the prefill kernel's last round).  The decode path takes
