@@ -109,3 +109,15 @@ def test_prefill_with_less_scratch_than_its_plan_asks_for(M, N, K):
     c = ops.quantized_matmul(a, bq, sc, dt, group, workspace=ws)
     assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("M", [20, 37, 80, 100])
+@pytest.mark.parametrize("K", [2048, 5120])  # 5120 columns of the activations do not fit the stream kernel in one chunk
+def test_small_batch_plans_put_on_another_kernel(M, K, kernel):
+    """The kernel is the one field that needs to change: the prefill kernel takes the tile that holds the plan's rows, the
+    stream kernel rings, chunks and CTAs that fit it."""
+    from .test_gpu_parity import _forced
+
+    assert ops.plan(M, 1920, K, D.int8, 0, 128)["kernel"] == 3
+    _forced(M, 1920, K, D.int8, 0, dict(kernel=kernel), seed=M)

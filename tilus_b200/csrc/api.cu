@@ -578,7 +578,9 @@ static int umma_m_group(int tm, int K, int m_tiles) {
 static int run_umma(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
                     int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream,
                     const b200q_plan_t& pl) {
-  const int tm = pl.tile_m;
+  // (a small-batch plan edited to this kernel names its rows, a multiple of 16 up to 128: the tile that holds them)
+  const bool rows = pl.tile_m >= 16 && pl.tile_m % 16 == 0 && pl.tile_m <= 128;
+  const int tm = !rows ? pl.tile_m : pl.tile_m <= 32 ? 32 : pl.tile_m <= 64 ? 64 : 128;
   if (tm != 32 && tm != 64 && tm != 128 && tm != 256 && tm != 384) return ST_INVALID_ARG;
   const int m_tiles = (M + tm - 1) / tm, n_tiles = (N + 127) / 128;
   const int kblocks = K / 64;
@@ -855,15 +857,17 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   }
   if (pl.kernel == 2 && plan_is_exact(pl))
     return run_batch(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl);
-  if (pl.kernel == 2 && pl.tile_m == 16 && stream_takes(K, group) && pl.splits > 1 && (K / BLOCK_K) % pl.splits == 0) {
-    // an exact plan edited to more k chunks is one for the stream kernel, whose rings and column tiles bound the rest
+  if (pl.kernel == 2 && pl.tile_m != 0 && stream_takes(K, group) && pl.splits > 0 && (K / BLOCK_K) % pl.splits == 0) {
+    // a tcgen05 plan edited to more k chunks or to this kernel: the stream kernel's rings and column tiles bound the rest
     b200q_plan_t chunks = pl;
     const int rows = M < stream_rows_per_pass(M) ? M : stream_rows_per_pass(M);
     if (chunks.ctas_per_split > N / BLOCK_N) chunks.ctas_per_split = N / BLOCK_N;
+    if (chunks.ctas_per_split > 4 * device_info().sm_count / pl.splits) chunks.ctas_per_split = 4 * device_info().sm_count / pl.splits;
     if (chunks.ctas_per_split > 0) {
       const int t_own = stream_tiles_owned(rows, N / BLOCK_N, chunks.ctas_per_split);
       const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info());
-      if (chunks.stages > fit && fit > 0) chunks.stages = fit;
+      if (chunks.stages > fit) chunks.stages = fit;
+      if (fit < 1 && plan_stream(rows, N, K, var_bits(var), device_info(), &chunks) != ST_OK) return ST_UNSUPPORTED;
     }
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, chunks);
   }
