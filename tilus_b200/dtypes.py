@@ -17,6 +17,7 @@ Every value of every type with at most 8 bits is exactly representable in fp16.
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 
 KIND_UINT = 0
@@ -67,7 +68,7 @@ class WeightDType:
         top = (1 << e) - 1 - (1 if e == 5 else 0)
         return 2.0 ** (top - bias) * (2.0 - 2.0 ** (-m))
 
-    @property
+    @functools.cached_property  # (read by every call of a layer)
     def code(self) -> int:
         """Integer tag passed through the C ABI: kind<<16 | nbits<<8 | e<<4 | m."""
         return (self.kind << 16) | (self.nbits << 8) | (self.exponent_nbits << 4) | self.mantissa_nbits
