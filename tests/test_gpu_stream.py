@@ -1,0 +1,51 @@
+"""The decode kernel where its split of the work and its rings can go wrong."""
+import pytest
+import torch
+
+from tilus_b200 import dtypes as D
+from tilus_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(M, N, K, dt, group=128, seed=0):
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(seed)
+    zp = 1 << (dt.nbits - 1) if dt.kind == D.KIND_UINT else 0
+    bq = torch.randint(0, 256, (N * K * dt.nbits // 8,), dtype=torch.uint8, device=dev, generator=gen)
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
+    a = torch.randn(M, K, device=dev, generator=gen).half()
+    ref = a.float() @ ops.dequantize(bq, sc, dt, group, zp).float()
+    return a, bq, sc, zp, ref
+
+
+@pytest.mark.parametrize("dt", [D.uint8, D.int8, D.uint7b, D.uint6b, D.int5b, D.uint4b, D.int3b, D.uint2b, D.uint1b, D.float6_e3m2],
+                         ids=lambda d: d.name)
+@pytest.mark.parametrize("M", [1, 2, 8])
+def test_repeated_calls_with_the_weights_in_l2(dt, M):
+    """A ring slot is refilled soonest when the copy finds its data in L2: every call of a warm series is right (8-bit
+    types used to be read behind the refill where registers let the compiler delay their second loads)."""
+    N, K = 2048, 8192
+    a, bq, sc, zp, ref = _problem(M, N, K, dt)
+    outs = [ops.quantized_matmul(a, bq, sc, dt, 128, zp) for _ in range(40)]
+    for c in outs:  # one rounding of the output (2^-11 of it) and of each reference weight
+        assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("M,N,K,dt", [
+    (1, 2384, 512, D.uint4b),     # 149 column tiles: two per CTA, the last CTA one
+    (1, 5120, 1536, D.int3b),     # 107 CTAs of three tiles, the last two
+    (2, 11008, 1024, D.uint8),    # 138 CTAs of five, the last three
+    (1, 16, 512, D.uint4b),       # one tile: one CTA, half the warps
+    (2, 2368, 1024, D.uint2b),    # one tile per SM
+    (3, 2384, 1024, D.float4_e2m1),
+    (4, 80000, 512, D.uint1b),    # more tiles than a CTA owns: the rest item by item
+    (8, 4096, 4096, D.uint4b),    # chunks of K, sums in the scratch
+    (7, 2384, 4096, D.int6b)], ids=str)
+def test_splits_of_the_column_tiles(M, N, K, dt):
+    a, bq, sc, zp, ref = _problem(M, N, K, dt, seed=N)
+    ws = torch.zeros(max(ops.workspace_bytes(M, N, K, dt, zp, 128), 1 << 20), dtype=torch.uint8, device=a.device)
+    for _ in range(2):
+        c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws)
+        assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert int(ws.count_nonzero()) == 0

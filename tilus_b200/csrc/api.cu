@@ -164,54 +164,46 @@ static int stream_pitch(int kc) {
   return bytes / 2;
 }
 // ---- stream kernel (kernel 2) ---------------------------------------------------------------------
-// Up to 8 rows: a CTA takes at most half an SM, so that two consecutive launches share an SM (the
-// second prefetches while the first computes) or two CTAs of one launch do: (228 KB - 2 x 1 KB
-// reserved) / 2 of shared memory.  9..16 rows: one CTA per SM with all of its shared memory, so
-// that a long K chunk of the 16 activation rows fits next to the rings.
-static const int kStreamSmemCap = 113 * 1024;
+// One CTA per SM.
+static const int kStreamSmemCap = 113 * 1024;  // half an SM
+// Rings beyond this are not worth their room: every CTA fills them before its activations arrive, and what is requested first is
+// waited for first (M = 1, 4096 x 14336, 4 bits: rings of 64 / 160 KB, activations staged 2.8 / 4.6 us after the start; the
+// linears of a Llama-3-8B block 33.3 / 34.9 us).
+static const int kStreamRing = 72 * 1024;
+static const int kOneCtaSmem = 116 * 1024;  // more than half an SM
 static int stream_slot_bytes(int bits) { return stream_gi(bits) * 256 * bits; }
 // 8-row activation tiles per launch: 1 or 2 (the kernel's MT)
 static int stream_mt(int m_pass) { return m_pass <= 8 ? 1 : 2; }
-// CTAs of one launch per SM
-static int stream_per_sm(int m_pass) { return m_pass <= 8 ? 2 : 1; }
 // most activation rows one launch of the stream kernel takes
 static int stream_rows_per_pass(int M) { (void)M; return 16; }
-static int stream_smem_cap(int m_pass, const DeviceInfo& di) {
-  return m_pass <= 8 ? kStreamSmemCap : di.max_smem;
-}
-// whole column tiles a CTA owns (their sums live in at most 16 KB of shared memory)
+// Whole column tiles a CTA owns: an equal share of all of them where that leaves the last CTA at least one, else what
+// divides evenly, the rest being shared item by item (the tiles' sums live in at most 16 KB of shared memory).
 static int stream_tiles_owned(int m_pass, int NT, int cpc) {
-  const int mt = stream_mt(m_pass), cap = 32 / mt;
-  const int t = NT / cpc;
-  return t < cap ? t : cap;
+  const int cap = 32 / stream_mt(m_pass), t = (NT + cpc - 1) / cpc;
+  if (t <= cap && (long long)t * (cpc - 1) < NT) return t;
+  return NT / cpc < cap ? NT / cpc : cap;
 }
-static int stream_fixed_smem(int m_pass, int kc, int t_own) {
-  const int mt = stream_mt(m_pass);
-  // barriers, scale caches, own-tile sums, activation chunk (+ 64 zero bytes), group sums as accumulator quads
-  return stream_header_bytes(mt) + stream_warps(mt) * STREAM_SC_GROUPS * 32 + t_own * 16 * 8 * mt * 4 +
-         m_pass * stream_pitch(kc) * 2 + 64 +
-         (kc / 128) * 16 * mt * 4;
+// log2 of the warps of a CTA that owns t_own tiles of kc rows
+static int stream_warp_shift(int m_pass, int kc, int bits, int t_own) {
+  return m_pass <= 2 && t_own > 0 && t_own * (kc / BLOCK_K) * (4 / stream_gi(bits)) <= 16 ? 3 : 4;
 }
 static int stream_smem(int m_pass, int kc, int bits, int stages, int t_own) {
-  return stream_fixed_smem(m_pass, kc, t_own) + stream_warps(stream_mt(m_pass)) * stages * stream_slot_bytes(bits);
+  const int mt = stream_mt(m_pass), warps = 1 << stream_warp_shift(m_pass, kc, bits, t_own);
+  // barriers, rings and scale caches of the warps, own-tile sums, activation chunk (+ 64 zero bytes), group sums as accumulator quads
+  return STREAM_HEADER + warps * (stages * stream_slot_bytes(bits) + STREAM_SC_GROUPS * 32) + t_own * 16 * 8 * mt * 4 +
+         m_pass * stream_pitch(kc) * 2 + 64 + (kc / 128) * 16 * mt * 4;
 }
-static int stream_stages_for(int m_pass, int kc, int bits, int t_own, const DeviceInfo& di) {
-  int st = (stream_smem_cap(m_pass, di) - stream_fixed_smem(m_pass, kc, t_own)) /
-           (stream_warps(stream_mt(m_pass)) * stream_slot_bytes(bits));
-  return st > 8 ? 8 : st;
+static int stream_stages_for(int m_pass, int kc, int bits, int t_own, int smem) {
+  int st = 8;
+  while (st > 0 && stream_smem(m_pass, kc, bits, st, t_own) > smem) --st;
+  return st;
 }
-// CTAs per k chunk.  First choice (up to 8 rows): two CTAs per SM (32 warps hide the latency of the
-// decode / mma chains best) with a count that divides the column tiles evenly, so that no tile is
-// shared between CTAs and nothing goes through the global scratch; then one CTA per SM with
-// such a count; else one CTA per SM with the left-over tiles shared item-wise.
-static int stream_ctas_per_chunk(int NT, int s, int per_sm, const DeviceInfo& di) {
+// CTAs per k chunk: the fewest that finish as soon as one per SM would
+static int stream_ctas_per_chunk(int NT, int s, const DeviceInfo& di) {
   const int full = di.sm_count / s;
   if (full < 1) return 0;
-  for (int c = 2 * full; per_sm == 2 && c >= 1 && c * 5 >= full * 8; --c)
-    if (NT % c == 0) return c;
-  for (int c = full; c >= 1 && c * 5 >= full * 4; --c)
-    if (NT % c == 0) return c;
-  return full > NT ? NT : full;
+  const int t = (NT + full - 1) / full;
+  return (NT + t - 1) / t;
 }
 static const int kStreamMaxRows = 16;  // what the kernel takes
 static const int kStreamPlanRows = 4;  // what the plan gives it at any shape (gather and host-buffer launches: all of the above)
@@ -225,28 +217,38 @@ static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counte
 static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di, b200q_plan_t* pl) {
   const int KB = K / BLOCK_K, NT = N / BLOCK_N;
   int best_s = 0, best_st = 0, best_c = 0;
-  auto consider = [&](int s, int want, bool no_leftover) {
+  auto consider = [&](int s, int want, bool no_leftover, int smem) {
     if (best_s || KB % s) return;
-    const int cpc = stream_ctas_per_chunk(NT, s, stream_per_sm(m_pass), di);
+    const int cpc = stream_ctas_per_chunk(NT, s, di);
     if (cpc < 1) return;
     const int t_own = stream_tiles_owned(m_pass, NT, cpc);
-    if (no_leftover && cpc * t_own != NT) return;
-    const int st = stream_stages_for(m_pass, (KB / s) * 512, bits, t_own, di);
-    if (st >= want) { best_s = s; best_st = st; best_c = cpc; }
+    if (no_leftover && cpc * t_own < NT) return;
+    // (a CTA that would stage more than 64 KB of activations, 1.75 times the bytes of its weights: shorter chunks.  5 x 2048 x 8192,
+    // 2 bits, 1 / 2 chunks: 8.8 / 8.1 us; 4 x 4096 x 14336, single bits, 12.8 / 11.7; but 4 x 2048 x 2048, 2 bits, 4.7 / 6.0)
+    if (no_leftover && m_pass > 2 && m_pass * (KB / s) > 64 && 4 * m_pass > 7 * t_own * bits) return;
+    const int st = stream_stages_for(m_pass, (KB / s) * 512, bits, t_own, smem);
+    if (st < want) return;
+    best_s = s; best_st = st; best_c = cpc;
+    const int ring = kStreamRing / (stream_slot_bytes(bits) << stream_warp_shift(m_pass, (KB / s) * 512, bits, t_own));
+    if (best_st > ring) best_st = ring > want ? ring : want;
   };
   const int s_max = KB < di.sm_count ? KB : di.sm_count;
-  consider(1, 2, true);
-  for (int s = 1; s <= s_max; ++s) consider(s, 3, true);
-  for (int s = 1; s <= s_max; ++s) consider(s, 2, true);
+  // 7 and 8 rows: chunks that leave half of the shared memory, since every CTA stages all rows of its chunk (4096 x 4096, 1 / 4
+  // chunks: 8 rows of 4 bits 8.0 / 7.35 us, of 8 bits 9.3 / 8.5; 5 rows of 4 bits 7.0 / 7.4)
+  const int most = m_pass == 7 || m_pass == 8 ? kStreamSmemCap : di.max_smem;
+  consider(1, 2, true, kStreamSmemCap);
+  consider(1, 2, true, most);
+  for (int s = 1; s <= s_max; ++s) consider(s, 3, true, most);
+  for (int s = 1; s <= s_max; ++s) consider(s, 2, true, most);
   for (int want = 3; want >= 1; --want)
-    for (int s = 1; s <= s_max; ++s) consider(s, want, false);
+    for (int s = 1; s <= s_max; ++s) consider(s, want, false, di.max_smem);
   if (!best_s) return ST_UNSUPPORTED;
   pl->kernel = 2;
   pl->m_tiles = stream_mt(m_pass);
   pl->splits = best_s;
   pl->cluster = 1;
   pl->ctas_per_split = best_c;
-  pl->warps = stream_warps(stream_mt(m_pass));
+  pl->warps = 1 << stream_warp_shift(m_pass, (KB / best_s) * 512, bits, stream_tiles_owned(m_pass, NT, best_c));
   pl->stages = best_st;
   pl->smem_bytes = stream_smem(m_pass, (KB / best_s) * 512, bits, best_st, stream_tiles_owned(m_pass, NT, best_c));
   pl->tile_m = 0;
@@ -335,7 +337,6 @@ static void plan_umma(int M, int N, int K, int bits, int group, const DeviceInfo
 
 // small-batch tcgen05 kernel (kernel 3): equal runs of (128-column tile, 128-row group) pairs, one CTA per SM
 static const int kBatchMaxRows = 128;
-static const int kOneCtaSmem = 116 * 1024;  // more than half an SM
 static int batch_rows(int M) { return (M + 15) / 16 * 16; }
 // arrival counts and fp32 sums of the column tiles
 static size_t batch_count_bytes(int N) { return ((size_t)((N + 127) / 128) * 32 * sizeof(int) + 255) / 256 * 256; }
@@ -456,13 +457,41 @@ static void plan_prefill(int M, int N, int K, int var, int group, int max_tm, co
   pl->workspace_bytes = need;
 }
 
+// What the two rules below were fitted to: the split that the stream kernel took with 12 warps per CTA and half an SM each, the most k
+// chunks and CTAs of at most two per SM, a divisor of the column tiles.  Whether such a split exists still tells the shapes apart.
+struct PairSplit { int splits, ctas; };
+static PairSplit pair_split(int M, int NT, int KB, int bits, const DeviceInfo& di) {
+  PairSplit best = {0, 0};
+  auto consider = [&](int s, int want, bool whole) {
+    const int full = di.sm_count / s;
+    if (best.splits || KB % s || full < 1) return;
+    int c = 0;
+    for (int i = 2 * full; !c && i * 5 >= full * 8; --i) c = NT % i == 0 ? i : 0;
+    for (int i = full; !c && i >= 1 && i * 5 >= full * 4; --i) c = NT % i == 0 ? i : 0;
+    if (!c) c = full > NT ? NT : full;
+    const int own = NT / c < 32 ? NT / c : 32, kc = KB / s * 512;
+    if (whole && c * own != NT) return;
+    const int fixed = 1024 + 12 * STREAM_SC_GROUPS * 32 + own * 512 + M * stream_pitch(kc) * 2 + 64 + kc / 2;
+    int slots = (kStreamSmemCap - fixed) / (12 * stream_slot_bytes(bits));
+    if (slots > 8) slots = 8;
+    if (slots >= want) best = {s, c};
+  };
+  const int s_max = KB < di.sm_count ? KB : di.sm_count;
+  consider(1, 2, true);
+  for (int s = 1; s <= s_max; ++s) consider(s, 3, true);
+  for (int s = 1; s <= s_max; ++s) consider(s, 2, true);
+  for (int want = 3; want >= 1; --want)
+    for (int s = 1; s <= s_max; ++s) consider(s, want, false);
+  return best;
+}
+
 // A stream plan that cuts K and still has one CTA per SM at most (no divisor of the column tiles near two per SM): its
 // chunks meet in the scratch like the exact kernel's, at half the warps.  The exact kernel is then faster from two
 // rows on, and for one row from three chunks on; stream / exact, us, chains of cold launches, 4 bits: 7168 x 2048 (2
 // chunks) 9.5 / 8.7, 2448 x 11776 (23) 13.8 / 11.8, 3504 x 9728 (19) 14.9 / 12.3, 5120 x 5120 (2) 11.3 .. 11.8 / 11.6 and 10.9 at
 // one row; 3504 x 9728 in 8 bits 18.9 / 15.3.
-static bool stream_outrun(int M, const b200q_plan_t& pl, const DeviceInfo& di) {
-  return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas_per_split <= di.sm_count;
+static bool stream_outrun(int M, const PairSplit& pl, const DeviceInfo& di) {
+  return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas <= di.sm_count;
 }
 
 // fp16, 5..8 rows: the shapes where the stream kernel is still the faster one.  What the exact kernel pays is a start and
@@ -479,11 +508,11 @@ static bool stream_outrun(int M, const b200q_plan_t& pl, const DeviceInfo& di) {
 // 8-bit integers, whose bytes the exact kernel takes with the fewest instructions, only from 32 M weights on (8192 x 2048 at 6
 // rows 7.7 / 6.5, 8192 x 4096 at 5 rows 10.9 / 11.8).  The choice costs 0.2 % against the better of the two over all
 // of them and is never more than 11 % behind the stream kernel (4096 x 8192 at 5 rows, 2 bits 8.6 / 9.5).
-static bool stream_ahead(int M, int N, int K, int var, const b200q_plan_t& pl, const DeviceInfo& di) {
+static bool stream_ahead(int M, int N, int K, int var, const PairSplit& pl, const DeviceInfo& di) {
   const long long million = 1ll << 20, weights = (long long)N * K;
   if (M <= kStreamPlanRows) return true;
   if (M > 8) return false;
-  if (pl.splits * pl.ctas_per_split > di.sm_count) {
+  if (pl.splits * pl.ctas > di.sm_count) {
     const bool bytes = var_bits(var) == 8 && !var_is_float(var);
     if (pl.splits == 1) return weights >= 32 * million || (weights > 12 * million && M <= 6 && !bytes);
     if (pl.splits >= 4) return (weights <= 4 * million || (weights > 12 * million && weights <= 20 * million)) && !bytes;
@@ -511,8 +540,9 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
   // second 8-row tile doubles its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
   // kernel only a conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit).
   if (M <= 8 && stream_takes(K, group)) {
-    if (plan_stream(M, N, K, bits, di, pl) == ST_OK && !stream_outrun(M, *pl, di) &&
-        (act == B200Q_BF16 || stream_ahead(M, N, K, var, *pl, di))) {
+    const PairSplit pair = pair_split(M, N / BLOCK_N, K / BLOCK_K, bits, di);
+    if (pair.splits > 0 && !stream_outrun(M, pair, di) && (act == B200Q_BF16 || stream_ahead(M, N, K, var, pair, di)) &&
+        plan_stream(M, N, K, bits, di, pl) == ST_OK) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
       return ST_OK;
@@ -778,6 +808,7 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
   p.stages = pl.stages;
   p.pdl = pl.pdl;
   p.act = act;
+  p.zero = 0u;
   {
     const int ipt = p.KBc * (4 / stream_gi(bits));  // items per column tile inside a k chunk
     p.ipt_shift = -1;
@@ -789,7 +820,8 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
   p.a_host = nullptr; p.fetch_flag = nullptr; p.fetch_ctas = 0; p.nowait = 0;
   if (a_host) {
     if (gather || M > stream_rows_per_pass(M)) return ST_INVALID_ARG;
-    const int per_cta = stream_warps(stream_mt(M)) * 32 * 4;  // 16-byte pieces one CTA fetches
+    const int warp_shift = stream_warp_shift(M, p.KBc * 512, bits, stream_tiles_owned(M, p.NT, p.CPC));
+    const int per_cta = (32 << warp_shift) * 4;  // 16-byte pieces one CTA fetches
     p.a_host = reinterpret_cast<const __half*>(a_host);
     p.lda = lda_host;
     p.fetch_flag = reinterpret_cast<unsigned*>(workspace) + 16;  // words 16, 17 of the status header
@@ -809,10 +841,16 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
     p.c = reinterpret_cast<__half*>(c) + (size_t)m0 * ldc;
     p.M = mc;
     p.T_own = stream_tiles_owned(mc, p.NT, p.CPC);
+    p.warp_shift = stream_warp_shift(mc, p.KBc * 512, bits, p.T_own);
     // (staging_released: the previous user of the staging buffer on this stream lets go of it before it
     // releases its successor - only then may this launch write it without waiting)
     p.nowait = (a_host && staging_released && p.S == 1 && p.T_own * p.CPC == p.NT) ? 1 : 0;
-    const int smem = stream_smem(mc, p.KBc * 512, bits, pl.stages, p.T_own);
+    int smem = stream_smem(mc, p.KBc * 512, bits, pl.stages, p.T_own);
+    // CTAs that fit one per SM must not meet two to an SM while others idle, as they would where the previous launch's CTAs
+    // leave at different times (128 CTAs of 6144 x 4096 on 88 SMs: 7.2 us, one to an SM 5.4).  Launches of a few KB per CTA
+    // gain more from starting beside their predecessor (2048 x 2048, 2 bits, 8 KB: 3.1 / 3.8 us; 3 bits, 12 KB: 3.8 / 3.9).
+    const bool spread = p.S * p.CPC <= device_info().sm_count && (long long)p.T_own * p.KBc * bits > 20;
+    if (spread && smem < kOneCtaSmem) smem = kOneCtaSmem;
     if (smem > device_info().max_smem) return ST_UNSUPPORTED;
     cudaError_t e = stream_launch(var, p, stream_mt(mc), smem, stream);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
@@ -865,7 +903,7 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     if (chunks.ctas_per_split > 4 * device_info().sm_count / pl.splits) chunks.ctas_per_split = 4 * device_info().sm_count / pl.splits;
     if (chunks.ctas_per_split > 0) {
       const int t_own = stream_tiles_owned(rows, N / BLOCK_N, chunks.ctas_per_split);
-      const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info());
+      const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info().max_smem);
       if (chunks.stages > fit) chunks.stages = fit;
       if (fit < 1 && plan_stream(rows, N, K, var_bits(var), device_info(), &chunks) != ST_OK) return ST_UNSUPPORTED;
     }

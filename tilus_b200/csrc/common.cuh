@@ -38,12 +38,12 @@ constexpr size_t WS_HEADER_BYTES = 256;
 inline size_t ws_counter_bytes(int N) { return (((size_t)(N / BLOCK_N) * 4) + 255) / 256 * 256; }
 
 // ---- stream kernel (up to 16 rows per launch): item-balanced, ring-fed ------------------------------
-// warps per CTA.  Up to 8 rows (MT = 1) two CTAs share an SM: 12 warps each leave up to 85 registers per
-// thread (the loop uses 52 .. 72), which keeps it out of local memory (16 warps at 64 registers spilled and
-// measured 5-10 % slower; 10 and 14 warps were no better).  9..16 rows (MT = 2): one CTA has the SM.
-constexpr int stream_warps(int mt) { return mt == 1 ? 12 : 16; }
-// bytes of mbarriers in front of the rings: 8 slots of 8 bytes per warp, rounded up to 1 KB
-constexpr int stream_header_bytes(int mt) { return (stream_warps(mt) * 64 + 1023) / 1024 * 1024; }
+// Warps per CTA, one CTA per SM (M = 1, 4 bits, us per launch with 12 warps and two CTAs per SM / 16 / 20 / 24 warps:
+// 8192 x 8192 9.9 / 9.6 / 11.0 / 10.1, the four linears of a Llama-3-8B block 38.0 / 35.1 / 35.0 / 34.8).  The smallest calls,
+// one or two rows and at most 16 ring items per CTA, have half as many: most of 16 would only be started (1024 x 1024
+// 2.7 us with 8, 3.1 with 16).
+constexpr int STREAM_WARPS = 16;
+constexpr int STREAM_HEADER = STREAM_WARPS * 64;  // bytes of mbarriers in front of the rings: 8 slots of 8 bytes per warp
 constexpr int STREAM_SC_GROUPS = 16;  // groups per warp in the shared-memory scale cache (32 bytes each)
 // 128-row groups per ring item: items of 1..2 KB for every bit width
 constexpr int stream_gi(int bits) { return bits <= 2 ? 4 : bits <= 5 ? 2 : 1; }
@@ -89,6 +89,8 @@ struct StreamParams {
   int pitch;             // shared-memory row pitch of the activation chunk, in halfs
   int stages;            // ring slots per warp (<= 8)
   int pdl;               // launch with programmatic stream serialization
+  int warp_shift;        // log2 of the warps per CTA
+  uint32_t zero;         // 0, which the compiler does not know
   int ipt_shift;         // log2 of the items per column tile inside a k chunk when that is a power of two, else -1
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
   int trig;              // 1: CTA 0 lets the next kernel of the stream launch only after its own griddepcontrol.wait

@@ -2,16 +2,17 @@
 //
 // Data movement.  The (column tile, k block) items of the weight matrix - GI consecutive
 // 128-row groups of a 16-column x 512-row block, 1..2 KB contiguous - are cut into equal
-// contiguous runs, one per warp, and every CTA gets the same number of items whatever the
-// shape.  One elected lane of a warp keeps the warp's own shared-memory ring full with TMA bulk copies
+// contiguous runs, one per warp.  One elected lane of a warp keeps the warp's own shared-memory ring full with TMA bulk copies
 // (cp.async.bulk, completion on an mbarrier per slot).  Weights and scales are constants, so
 // the ring is filled and the warp's scales are cached in shared memory before the kernel
-// waits for its predecessor in the stream (programmatic dependent launch): the memory
-// system always has the next layer's requests queued behind the current layer's.  A CTA
-// takes at most half of an SM (16 warps at <= 64 registers, <= 113 KB of shared memory): two
-// CTAs of one launch share an SM, or - when a launch has one CTA per SM - the next launch
-// of the stream becomes resident beside it and prefetches while it computes.  K is cut into S
-// chunks when the activation chunk [M, K/S] would not fit next to the rings; a CTA works
+// waits for its predecessor in the stream (programmatic dependent launch).  A launch is one CTA of 16 warps per SM, as few CTAs as
+// finish as soon (T_own column tiles each, the last one what is left).  Two CTAs per SM, in a number that divides
+// the column tiles, left SMs idle or with one CTA where others had two, and staged the activations twice (M = 1, 4 bits, us: 6144 x
+// 4096 6.9 -> 5.4, 28672 x 4096 13.9 -> 12.7, 5120 x 5120 9.7 -> 6.3, 7168 x 2048 8.7 -> 4.8).  What a launch of M = 1 spends
+// now, 28672 x 4096, us: 0.3 from its predecessor's end to its start, 0.8 to the wait, 1.0 for the activations, 9.3
+// for the weights (6.5 TB/s), 0.7 for the outputs and the spread of the CTAs.  Launches that share an SM, so that one's start
+// lies under the other's end, measured slower: nothing keeps two CTAs of the later one off the SM that empties first.
+// K is cut into S chunks when the activation chunk [M, K/S] would not fit next to the rings; a CTA works
 // inside one chunk.
 //
 // Compute.  One 128-row group at a time.  A lane reads its two units (columns r and r+8, 32
@@ -79,6 +80,16 @@ __device__ __forceinline__ void ld_unit_words(const unsigned char* ptr, uint32_t
   }
 }
 
+// one word of every vector load of ld_unit_words
+template <int B>
+__device__ __forceinline__ uint32_t loaded_words(const uint32_t (&w)[B]) {
+  constexpr int STEP = B % 4 == 0 ? 4 : B % 2 == 0 ? 2 : 1;
+  uint32_t x = 0u;
+#pragma unroll
+  for (int q = 0; q < B; q += STEP) x |= w[q];
+  return x;
+}
+
 // 16-bit pattern of an output value in the activation dtype (ACT 0: fp16, 1: bf16)
 template <int ACT>
 __device__ __forceinline__ unsigned short out_bits(float v) {
@@ -134,18 +145,15 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
 }
 
 // Shared-memory layout (byte offsets from the dynamic smem base):
-//   [0, HDR)     mbarriers [warp][stage]   (up to 8 stages of 8 bytes per warp, HDR a multiple of 1 KB)
+//   [0, HDR)     mbarriers [warp][stage]   (up to 8 stages of 8 bytes per warp)
 //   [HDR, ...)   rings [warp][stage][ITEM_BYTES] of packed weights
 //   then         scale caches [warp][STREAM_SC_GROUPS][16] 16-bit scales: those of the warp's next groups
 //   then         tile sums of the CTA's own column tiles [T_own][16 columns][8*MT rows] floats
 //   then         activation chunk [M][pitch] halfs, then group sums [groups][8*MT] floats
 //
-// MT = 1 (up to 8 rows): at most half an SM per CTA, so that two CTAs - of this launch or of the next
-// one in the stream - share an SM.  MT = 2 (up to 16 rows): one CTA per SM with all of its registers
-// and shared memory, which keeps the two 8-row accumulator sets in registers and a K chunk of the
-// 16 activation rows next to the rings.
+// MT = 1: up to 8 rows; MT = 2: up to 16, in two 8-row accumulator sets.
 template <int VAR, int MT, int GATHER, int ACT>
-__global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream_kernel(const StreamParams p) {
+__global__ void __launch_bounds__(STREAM_WARPS * 32, 1) stream_kernel(const StreamParams p) {
   constexpr int B = var_bits(VAR);
   constexpr int MP = 8 * MT;
   constexpr int BIAS = var_bias(VAR);
@@ -153,8 +161,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
   constexpr int NI = 4 / GI;  // items per block
   constexpr int ITEM_BYTES = GI * 256 * B;
   constexpr int SLOT_BYTES = ITEM_BYTES;
-  constexpr int NWARPS = stream_warps(MT);
-  constexpr int HDR = stream_header_bytes(MT);
+  constexpr int HDR = STREAM_HEADER;
   constexpr int SCG = STREAM_SC_GROUPS;
   constexpr float F = (float)(1u << lin_factor_log2(VAR));
   // Where the linear pattern of a pair sits in the fp16 mantissa (bit T, decode.cuh int_target) sets a
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
   // 8-bit integers and the float types have T = 0 for every pair and need no such pass.
   constexpr bool PRESCALE = !var_is_float(VAR) && B != 8;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  const int NST = p.stages;
+  const int NST = p.stages, NWARPS = 1 << p.warp_shift;
   const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem_raw);
   unsigned char* sScale = smem_raw + HDR + (size_t)NWARPS * NST * SLOT_BYTES;
   float* sAcc = reinterpret_cast<float*>(sScale + (size_t)NWARPS * SCG * 32);
@@ -174,7 +181,8 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
 
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int r = lane >> 2, j = lane & 3;
-  const int chunk = blockIdx.x % p.S, ci = blockIdx.x / p.S;
+  int chunk = 0, ci = blockIdx.x;
+  if (p.S > 1) { ci = blockIdx.x / p.S; chunk = blockIdx.x - ci * p.S; }
   const int kb_base = chunk * p.KBc;
   const int IPT = p.KBc * NI;  // items per column tile inside a k chunk
   // x / IPT and x % IPT: a shift when IPT is a power of two (the host says so), which keeps integer
@@ -201,9 +209,10 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
       l1 = (int)(left_items * (ci + 1) / p.CPC);
     }
   }
-  const int n_left = l1 - l0, n_total = n_left + p.T_own * IPT;
-  // n_total < 2^26 (column tiles x k blocks x 4 of one CTA), NWARPS <= 32: the products fit in 32 bits
-  const int v0 = (int)((unsigned)n_total * (unsigned)warp / NWARPS), v1 = (int)((unsigned)n_total * (unsigned)(warp + 1) / NWARPS);
+  const int my_tiles = max(0, min(p.T_own, p.NT - own_tile0));  // (the last CTA may own fewer)
+  const int n_left = l1 - l0, n_total = n_left + my_tiles * IPT;
+  // n_total < 2^26 (column tiles x k blocks x 4 of one CTA): the products fit in 32 bits
+  const int v0 = (int)((unsigned)n_total * (unsigned)warp >> p.warp_shift), v1 = (int)((unsigned)n_total * (unsigned)(warp + 1) >> p.warp_shift);
   // this warp's two item runs: cA items of left-over tiles, then cB items of the CTA's own tiles
   const int cA = v0 < n_left ? min(v1, n_left) - v0 : 0;
   int qA = 0, qB = 0;
@@ -270,10 +279,9 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
     if (gidx < n_items * GI)
       *reinterpret_cast<uint4*>(sc_warp + (gidx % SCG) * 32 + (lane & 1) * 16) = __ldg(scale_src(gidx));
   };
-  if (lane == 0) {
-    for (int s = 0; s < NST; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + s * 8) : "memory");
+  if (lane < NST) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + lane * 8) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
   for (int s = 0; s < NST && issued < n_items; ++s) issue_next(bar0 + s * 8, ring_s + s * SLOT_BYTES);
@@ -574,19 +582,22 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
           sf0[gi] = scale_f32<ACT>(sp[0]);
           sf1[gi] = scale_f32<ACT>(sp[8]);
         }
+        uint32_t loaded = 0u;
 #pragma unroll
         for (int gi = 0; gi < GI; ++gi) {
           uint32_t w0[B], w1[B];
           ld_unit_words<B>(slot + w_lane + gi * (256 * B), w0);
           ld_unit_words<B>(slot + w_lane + gi * (256 * B) + 128 * B, w1);
+          loaded |= loaded_words<B>(w0) | loaded_words<B>(w1);
           uint32_t W0[16], W1[16];
           unit_decode_linear<VAR>(w0, W0);
           unit_decode_linear<VAR>(w1, W1);
           if (gi == GI - 1) {
-            // every lane has turned its copy of the item's last group into operands (the loads have
-            // returned: their values were used), so the warp may ask for the next item into this slot
+            // The warp asks for the next item into this slot once it has read this one.  The copy's address takes part in what
+            // was read (p.zero is zero), since nothing else keeps a load, or the decoding that first waits for it, ahead
+            // of a copy that another unit writes: with registers to spare 8-bit types had their second loads behind it.
             __syncwarp();
-            if (issued < n_items) issue_next(bar, ring_s + slot_off);
+            if (issued < n_items) issue_next(bar, ring_s + slot_off + (loaded & p.zero));
           }
           const uint32_t koff = (uint32_t)((g0 + gi) * 320);  // bytes: 128 columns + 4 x 8 of padding per group
           // two accumulation chains per 8-row tile; the first starts from the zero-point term of the group
@@ -726,7 +737,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
   if (nowait) asm volatile("griddepcontrol.wait;" ::: "memory");  // outputs of consecutive calls land in order
   if (p.T_own > 0) {
     __syncthreads();
-    const int n0 = own_tile0 * 16, ncols = p.T_own * 16;
+    const int n0 = own_tile0 * 16, ncols = my_tiles * 16;
     if (p.S == 1) {  // all of K was here: write C
       if constexpr (!gather_pairs(GATHER)) {
         for (int m = 0; m < p.M; ++m)
@@ -749,7 +760,7 @@ __global__ void __launch_bounds__(stream_warps(MT) * 32, MT == 1 ? 2 : 1) stream
       int* s_last = reinterpret_cast<int*>(sAcc);  // the tile sums are no longer needed
       if (tid == 0) __threadfence();  // cumulative over the CTA's additions (ordered by the barrier above)
       __syncthreads();
-      for (int t = tid; t < p.T_own; t += NWARPS * 32) {
+      for (int t = tid; t < my_tiles; t += NWARPS * 32) {
         const int old = atomicAdd(p.counters + own_tile0 + t, IPT);
         s_last[t] = (old + IPT == items_per_tile_total) ? 1 : 0;
       }
@@ -839,7 +850,7 @@ static cudaError_t launch_one(const StreamParams& p, int smem_bytes, cudaStream_
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.S * p.CPC), 1, 1);
-  cfg.blockDim = dim3(stream_warps(MT) * 32, 1, 1);
+  cfg.blockDim = dim3(32u << p.warp_shift, 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
