@@ -78,3 +78,29 @@ def test_out_tensors_that_do_not_fit_are_refused():
     for out in ((bq[1:], sc), (bq, sc.float()), (bq, sc.t()), (bq.cpu(), sc), (bq[:-16], sc)):
         with pytest.raises(ValueError):
             quantize.quantize_and_pack(w, D.int4b, 128, out=out)
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("kind", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("group", [32, 128, 256])
+def test_signed_codes_of_ordinary_and_special_weights(bits, kind, group):
+    """Units that need no clamping and those that do: zeros, weights so small that the least scale takes them beyond the
+    range, infinities and NaN, single outliers, against the definition on the same device (codes are whole numbers: equal)."""
+    dt, n, k = getattr(D, f"int{bits}b" if bits < 8 else "int8"), 64, 512
+    gen = torch.Generator(device="cuda").manual_seed(bits + group)
+    w = torch.randn(n, k, device="cuda", generator=gen) * 0.02
+    w[0], w[1], w[2] = 0.0, 3e-7, w[2] * 1e-5
+    w[3, 7], w[4, 9], w[5, 11] = float("inf"), float("-inf"), float("nan")
+    w[6, ::37] *= 300.0
+    w = w.to(kind)
+    packed, scales = quantize.quantize_and_pack(w, dt, group, torch.float16)
+    lo, hi = -float(1 << (bits - 1)), float((1 << (bits - 1)) - 1)
+    x = w.float().reshape(n, k // group, group)
+    amax = torch.nan_to_num(x.abs(), nan=0.0, posinf=float("inf")).amax(2)
+    s = (amax / hi if hi else amax / torch.zeros_like(amax))
+    s = torch.where(s.isnan(), s.new_tensor(1e-6), s.clamp(min=1e-6)).half()
+    assert torch.equal(scales.view(torch.int16), s.t().contiguous().view(torch.int16))
+    q = x / s.float()[:, :, None]
+    q = torch.where(q.isnan(), q.new_tensor(lo), q.clamp(lo, hi)).round().reshape(n, k)
+    codes = (q.to(torch.int32) & ((1 << bits) - 1)).to(torch.uint8).t().contiguous()
+    assert torch.equal(packed.cpu(), packing.interleave(codes.cpu(), dt))

@@ -17,12 +17,14 @@
 // neighbouring lanes of a column, so their absmax is a shuffle and the dense weight is read once; other
 // groups get their scales from a pass of their own (quant_scales_kernel, one warp per column and group).
 //
-// What bounds it: HBM (2 or 4 bytes read and b/8 written per weight), provided the arithmetic stays near ten
-// instructions per weight.  The IEEE division of the definition alone is as much, so integer codes come
+// What bounds it: HBM (2 or 4 bytes read and b/8 written per weight), provided the arithmetic stays near four
+// instructions per weight.  The IEEE division of the definition alone is ten, so integer codes come
 // from one multiplication by the reciprocal of the scale, and only a unit with a value within the
 // multiplication's error of a rounding boundary is computed again with the division: the codes are
-// those of the division in every case.  fp16 [28672, 4096] -> int4 g128: 544 us for two scalar passes plus
-// the copy into the layer, 94 us in this form (45 us at the copy rate of HBM).
+// those of the division in every case.  Signed types (signed_codes) need no clamping where the unit's largest weight
+// rounds inside the range, work on two values per instruction and pack 2, 4 and 8 bits in fp32.  fp16 [28672, 4096] ->
+// int4 g128: 94 us with clamping and bit packing per value and 1024 threads per SM, 64 us now with 2048 (68 with 1536,
+// 79 with 1024: a thread's loads are in flight for half of its life; 45 us at the copy rate of HBM).
 #include "common.cuh"
 
 namespace b200q {
@@ -37,6 +39,7 @@ struct QuantParams {
   int N, K, G, group;  // G = K / 128
   int kind, ebits, mbits;  // kind: 0 unsigned, 1 two's complement, 2 float
   int vec;                 // every row starts on a 16-byte boundary
+  int gshift;              // log2(group) if local
   int local;               // groups of 32, 64 or 128 rows: inside the four neighbouring lanes of a column
   float minv, maxv;
 };
@@ -87,6 +90,84 @@ __device__ __forceinline__ void load_weights(const QuantParams& p, size_t idx, f
   }
 }
 
+// ---- two fp32 values at a time (one instruction on sm_100) ----
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack_f2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma_f2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// max(|a|, |b|, m) of the numbers among them
+__device__ __forceinline__ float max_abs_numbers(float a, float b, float m) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(m));
+  return r;
+}
+// max(|a|, |b|, m), NaN if one of them is
+__device__ __forceinline__ float max_abs(float a, float b, float m) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(m));
+  return r;
+}
+
+// The 32 consecutive weights of a unit as they are in memory: 16-bit pairs, or fp32
+template <int WT>
+struct UnitWeights {
+  uint32_t raw[WT == 1 ? 32 : 16];
+  __device__ __forceinline__ void load(const QuantParams& p, size_t idx) {
+    if (p.vec) {
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p.w) + idx * (WT == 1 ? 4 : 2));
+#pragma unroll
+      for (int i = 0; i < (WT == 1 ? 8 : 4); ++i) {
+        const uint4 x = __ldg(src + i);
+        raw[4 * i] = x.x; raw[4 * i + 1] = x.y; raw[4 * i + 2] = x.z; raw[4 * i + 3] = x.w;
+      }
+    } else if constexpr (WT == 1) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) raw[i] = __ldg(reinterpret_cast<const uint32_t*>(p.w) + idx + i);
+    } else {
+      const unsigned short* src = reinterpret_cast<const unsigned short*>(p.w) + idx;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) raw[i] = (uint32_t)__ldg(src + 2 * i) | ((uint32_t)__ldg(src + 2 * i + 1) << 16);
+    }
+  }
+  __device__ __forceinline__ float2 pair(int i) const {
+    if constexpr (WT == 0) return __half22float2(h2_from_bits(raw[i]));
+    else if constexpr (WT == 2) return make_float2(__uint_as_float(raw[i] << 16), __uint_as_float(raw[i] & 0xffff0000u));
+    else return make_float2(__uint_as_float(raw[2 * i]), __uint_as_float(raw[2 * i + 1]));
+  }
+  __device__ __forceinline__ float operator[](int i) const { return i & 1 ? pair(i >> 1).y : pair(i >> 1).x; }
+  // largest magnitude of the numbers among them
+  __device__ __forceinline__ float largest() const {
+    if constexpr (WT == 0) {
+      __half2 m = __habs2(h2_from_bits(raw[0]));
+#pragma unroll
+      for (int i = 1; i < 16; ++i) m = __hmax2(m, __habs2(h2_from_bits(raw[i])));
+      return fmaxf(fmaxf(__low2float(m), __high2float(m)), 0.f);
+    } else if constexpr (WT == 2) {
+      __nv_bfloat162 m = __habs2(bf2_from_bits(raw[0]));
+#pragma unroll
+      for (int i = 1; i < 16; ++i) m = __hmax2(m, __habs2(bf2_from_bits(raw[i])));
+      return fmaxf(fmaxf(__low2float(m), __high2float(m)), 0.f);
+    } else {
+      float m = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) m = max_abs_numbers(pair(i).x, pair(i).y, m);
+      return m;
+    }
+  }
+};
+
 // scales of groups that are not 32, 64 or 128 rows: one warp per (column, group), 8 weights per lane and step
 template <int WT>
 __global__ void __launch_bounds__(256) quant_scales_kernel(const QuantParams p) {
@@ -134,6 +215,57 @@ __device__ __forceinline__ uint32_t encode_float_code(float x, int nbits, int e,
   return sign | ((uint32_t)exp_value << m) | (mant ^ (1u << m));
 }
 
+// Signed codes of a unit without clamping: the caller has made sure that no value rounds beyond the range.  `v`: the weights,
+// taken in pairs (even k, odd k), `rs` the scale's reciprocal.  With C = 1.5 * 2^23, t = v * rs + C rounds the quotient to the
+// integer i = t - C, and v * rs - i is how far it was from it; returns the largest of those distances.  Types of one plane (2, 4,
+// 8 bits) have the codes of a 16-bit field added up in fp32 as well, even and odd k side by side: sum of i * 2^(B f) + 2^(B - 1)
+// in every field, an integer below 2^16.  The others have them OR-ed together from the low mantissa bits.
+template <int B, int I = 0>
+__device__ __forceinline__ void put_pairs(const uint32_t (&code)[32], uint32_t (&words)[B]);
+template <int B, class Weights>
+__device__ __forceinline__ float signed_codes(const Weights& v, float rs, uint32_t (&words)[B]) {
+  constexpr float C = 12582912.0f;
+  const f32x2 rs2 = pack_f2(rs, rs), c2 = pack_f2(C, C), minus = pack_f2(-1.f, -1.f);
+  float worst = 0.f;
+  if constexpr (B == 2 || B == 4 || B == 8) {
+    constexpr int PER = 16 / B;  // pairs per word
+    constexpr uint32_t HALVES = (1u << (B - 1)) * (B == 2 ? 0x5555u : B == 4 ? 0x1111u : 0x0101u);
+    const f32x2 step = pack_f2((float)(1 << B), (float)(1 << B)), end = pack_f2(C + (float)HALVES, C + (float)HALVES);
+#pragma unroll
+    for (int w = 0; w < B; ++w) {
+      f32x2 sum = 0ull;  // minus the sum: what v * rs needs added is -i
+#pragma unroll
+      for (int f = PER - 1; f >= 0; --f) {
+        const float2 xy = v.pair(w * PER + f);
+        const f32x2 x = pack_f2(xy.x, xy.y);
+        const f32x2 neg = fma_f2(fma_f2(x, rs2, c2), minus, c2);
+        const float2 d = unpack_f2(fma_f2(x, rs2, neg));
+        worst = max_abs(d.x, d.y, worst);
+        sum = f == PER - 1 ? neg : fma_f2(sum, step, neg);
+      }
+      const float2 t = unpack_f2(fma_f2(sum, minus, end));
+      words[w] = __byte_perm(__float_as_uint(t.x), __float_as_uint(t.y), 0x5410);
+    }
+  } else {
+    const f32x2 off = pack_f2(C + (float)(1 << (B - 1)), C + (float)(1 << (B - 1)));
+    uint32_t code[32];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 xy = v.pair(i);
+      const f32x2 x = pack_f2(xy.x, xy.y), t = fma_f2(x, rs2, off);
+      const float2 d = unpack_f2(fma_f2(x, rs2, fma_f2(t, minus, off)));
+      worst = max_abs(d.x, d.y, worst);
+      const float2 c = unpack_f2(t);
+      code[2 * i] = __float_as_uint(c.x);
+      code[2 * i + 1] = __float_as_uint(c.y);
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q) words[q] = 0u;
+    put_pairs<B>(code, words);
+  }
+  return worst;
+}
+
 // code of pair position i (0..31) into the unit's plane words (widths = the set bits of B, widest first)
 template <int B, int I, int P = 0>
 __device__ __forceinline__ void put_code(uint32_t code, uint32_t (&words)[B]) {
@@ -150,28 +282,44 @@ __device__ __forceinline__ void put_codes(const F& code_of, uint32_t (&words)[B]
   if constexpr (I + 1 < 32) put_codes<B, I + 1>(code_of, words);
 }
 
+// both codes of pair I and of those behind it (low bits of `code`) into the plane words, two fields at a time
+template <int B, int I, int P = 0>
+__device__ __forceinline__ void put_pair(uint32_t both, uint32_t (&words)[B]) {
+  constexpr int pw = plane_width(B, P), per = 16 / pw;
+  constexpr int lo = plane_lo(B, P), pos = (I % per) * pw;
+  constexpr uint32_t mask = (((1u << pw) - 1u) << pos) * 0x00010001u;
+  uint32_t& w = words[plane_word_base(B, P) + I / per];
+  w |= (pos >= lo ? both << (pos >= lo ? pos - lo : 0) : both >> (pos < lo ? lo - pos : 0)) & mask;
+  if constexpr (P + 1 < plane_count(B)) put_pair<B, I, P + 1>(both, words);
+}
+template <int B, int I>
+__device__ __forceinline__ void put_pairs(const uint32_t (&code)[32], uint32_t (&words)[B]) {
+  put_pair<B, I>(__byte_perm(code[2 * I], code[2 * I + 1], 0x5410), words);
+  if constexpr (I + 1 < 16) put_pairs<B, I + 1>(code, words);
+}
+
 template <int WT, int B, bool FLOAT>
-__global__ void __launch_bounds__(256) quant_pack_kernel(const QuantParams p) {
-  // unit index = ((nt * G + g) * 2 + half) * 32 + lane,  lane = r * 4 + j,  g = 128-row group of K
-  const long long unit = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (unit >= (long long)p.N * p.K / 32) return;  // whole warps: N * K / 32 is a multiple of 64
-  const int lane = (int)(unit & 31), half = (int)((unit >> 5) & 1);
-  const long long grp = unit >> 6;
-  const int nt = (int)(grp / p.G), g = (int)(grp - (long long)nt * p.G);
+__global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const QuantParams p) {
+  // unit index = ((nt * G + g) * 2 + half) * 32 + lane,  lane = r * 4 + j,  g = 128-row group of K.  A block has four groups
+  // of one 16-column tile (a division per thread costs as much as a quarter of its weights).
+  const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1;
+  const unsigned per_tile = (unsigned)(p.G + 3) / 4;
+  const int nt = (int)(blockIdx.x / per_tile), g = (int)(blockIdx.x - nt * per_tile) * 4 + (int)(threadIdx.x >> 6);
+  if (g >= p.G) return;  // whole warps
+  const long long unit = ((long long)nt * p.G + g) * 64 + (threadIdx.x & 63);
   const int r = lane >> 2, j = lane & 3;
   const int n = nt * 16 + half * 8 + r;
   const int k0 = g * 128 + j * 32;
-  float v[32];
-  load_weights<WT, 32>(p, (size_t)n * p.ldw + k0, v);
+  UnitWeights<WT> v;
+  v.load(p, (size_t)n * p.ldw + k0);
+  const float unit_max = v.largest();
   float s;
   if (p.local) {
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) m = fmaxf(m, fabsf(v[i]));
+    float m = unit_max;
     if (p.group >= 64) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     if (p.group == 128) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
     const unsigned short sb = scale_bits(p, m);
-    if ((k0 % p.group) == 0) p.scales[(size_t)(k0 / p.group) * p.N + n] = sb;
+    if ((k0 & (p.group - 1)) == 0) p.scales[(size_t)(k0 >> p.gshift) * p.N + n] = sb;
     s = p.act == 0 ? __half2float(__ushort_as_half(sb)) : __uint_as_float((uint32_t)sb << 16);
   } else {
     s = load_scale(p, (size_t)(k0 / p.group) * p.N + n);
@@ -185,21 +333,27 @@ __global__ void __launch_bounds__(256) quant_pack_kernel(const QuantParams p) {
       return encode_float_code(q, B, p.ebits, p.mbits);
     }, words);
   } else {
-    // Offset binary code = rint(clamp(w / s)) + offset.  Estimate: x = w * (1 / s) + offset with two
-    // roundings, |x - (w / s + offset)| < 2^(B-22); adding 1.5 * 2^23 rounds it to an integer in the low bits.
-    constexpr float MAGIC = 12582912.0f;
+    // Signed types whose largest weight of the unit rounds inside the range: no clamping, see signed_codes.  A unit with a
+    // value within the products' error of a rounding boundary, or a NaN, takes the division below.
     constexpr float EPS = (float)(1 << B) * (1.0f / (1 << 22));
-    const float offset = p.kind == 1 ? (float)(1 << (B - 1)) : 0.f;
-    const float lo = p.minv + offset, hi = p.maxv + offset;
     const float rs = __fdiv_rn(1.0f, s);
-    float worst = s < 1e30f ? 0.f : 1.f;  // beyond that the reciprocal loses bits
-    put_codes<B, 0>([&](int i) {
-      const float x = fminf(fmaxf(fmaf(v[i], rs, offset), lo), hi);
-      const float t = x + MAGIC;
-      worst = fmaxf(worst, fabsf(x - (t - MAGIC)));
-      return __float_as_uint(t);
-    }, words);
-    if (worst > 0.5f - EPS) {  // some value sits on a rounding boundary: the definition's own division
+    bool done = false;
+    if (p.kind == 1 && s < 1e30f && unit_max * rs <= p.maxv + (0.5f - EPS)) {
+      done = signed_codes<B>(v, rs, words) <= 0.5f - EPS;
+    } else if (p.kind == 0 && s < 1e30f) {
+      // Unsigned types: code = rint(clamp(w / s)).  Estimate: x = w * (1 / s), |x - w / s| < 2^(B-22); adding 1.5 * 2^23
+      // rounds it to an integer in the low bits.
+      constexpr float MAGIC = 12582912.0f;
+      float worst = 0.f;
+      put_codes<B, 0>([&](int i) {
+        const float x = fminf(fmaxf(v[i] * rs, p.minv), p.maxv);
+        const float t = x + MAGIC;
+        worst = fmaxf(worst, fabsf(x - (t - MAGIC)));
+        return __float_as_uint(t);
+      }, words);
+      done = worst <= 0.5f - EPS;
+    }
+    if (!done) {  // the definition's own division
 #pragma unroll
       for (int q = 0; q < B; ++q) words[q] = 0u;
       put_codes<B, 0>([&](int i) {
@@ -225,8 +379,7 @@ __global__ void __launch_bounds__(256) quant_pack_kernel(const QuantParams p) {
 template <int WT, int B, bool FLOAT>
 static cudaError_t pack_launch(const QuantParams& p, int nbits, cudaStream_t stream) {
   if (nbits == B) {
-    const long long units = (long long)p.N * p.K / 32;
-    quant_pack_kernel<WT, B, FLOAT><<<(unsigned)((units + 255) / 256), 256, 0, stream>>>(p);
+    quant_pack_kernel<WT, B, FLOAT><<<(unsigned)(p.N / 16) * (unsigned)((p.G + 3) / 4), 256, 0, stream>>>(p);
     return cudaGetLastError();
   }
   if constexpr (B < 8) return pack_launch<WT, B + 1, FLOAT>(p, nbits, stream);
@@ -256,6 +409,7 @@ cudaError_t quantize_launch(const void* w, int w_dtype, int ldw, void* bq, void*
   p.minv = minv; p.maxv = maxv;
   p.vec = (((uintptr_t)w & 15) == 0 && ldw % (w_dtype == 1 ? 4 : 8) == 0) ? 1 : 0;
   p.local = 128 % group == 0 ? 1 : 0;
+  p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
   if (w_dtype == 1) return quantize_as<1>(p, nbits, stream);
   if (w_dtype == 2) return quantize_as<2>(p, nbits, stream);
   return quantize_as<0>(p, nbits, stream);
