@@ -5,6 +5,8 @@ import torch
 from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 
+from .test_gpu_parity import _forced
+
 pytestmark = pytest.mark.gpu
 
 
@@ -35,3 +37,17 @@ def test_runs_of_many_short_tiles_without_synchronisation(M, N, K):
         ref = xs[i % 3].float() @ w
         assert float((got.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max()), i
     assert ops.device_status(ops.get_workspace(dev, 1 << 20)) == [0, 0, 0, 0]
+
+
+@pytest.mark.parametrize("M,group", [(5, 128), (16, 512), (24, 128), (64, 32), (128, 128)])
+@pytest.mark.parametrize("tiles,ctas", [(7, 3), (9, 9), (10, 9), (23, 4)])
+@pytest.mark.parametrize("K", [2048, 2176])
+def test_whole_tiles_behind_shares_of_the_others(M, group, tiles, ctas, K):
+    """More column tiles than CTAs: whole tiles of a CTA's own behind its share of the rest, with shares of less than a
+    group, none at all, and a last column tile of 16 columns."""
+    if K % group:
+        pytest.skip("group does not divide K")
+    N, dt = tiles * 128 - 112, D.int4b
+    exact = M <= 16 and group % 128 == 0
+    plan = dict(kernel=2 if exact else 3, tile_m=16 if exact else 128, splits=1, cluster=1, ctas_per_split=ctas)
+    _forced(M, N, K, dt, 0, plan, seed=M + tiles, group=group)
