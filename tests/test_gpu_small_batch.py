@@ -40,14 +40,32 @@ def test_runs_of_many_short_tiles_without_synchronisation(M, N, K):
 
 
 @pytest.mark.parametrize("M,group", [(5, 128), (16, 512), (24, 128), (64, 32), (128, 128)])
-@pytest.mark.parametrize("tiles,ctas", [(7, 3), (9, 9), (10, 9), (23, 4)])
+@pytest.mark.parametrize("tiles,ctas", [(7, 3), (9, 9), (10, 9), (23, 4), (8, 4), (41, 40)])
 @pytest.mark.parametrize("K", [2048, 2176])
-def test_whole_tiles_behind_shares_of_the_others(M, group, tiles, ctas, K):
-    """More column tiles than CTAs: whole tiles of a CTA's own behind its share of the rest, with shares of less than a
-    group, none at all, and a last column tile of 16 columns."""
+def test_runs_of_one_to_six_column_tiles(M, group, tiles, ctas, K):
+    """At least as many column tiles as CTAs: runs that are whole tiles, runs that begin and end inside one, runs one group
+    longer than a tile, and a last column tile of 16 columns."""
     if K % group:
         pytest.skip("group does not divide K")
     N, dt = tiles * 128 - 112, D.int4b
     exact = M <= 16 and group % 128 == 0
     plan = dict(kernel=2 if exact else 3, tile_m=16 if exact else 128, splits=1, cluster=1, ctas_per_split=ctas)
     _forced(M, N, K, dt, 0, plan, seed=M + tiles, group=group)
+
+
+@pytest.mark.parametrize("M,dt,group", [(8, D.uint4b, 128), (16, D.int3b, 128), (24, D.uint4b, 128), (64, D.uint4b, 128),
+                                        (128, D.int4b, 64)], ids=str)
+@pytest.mark.parametrize("N,K", [(28672, 4096), (19072, 4096)])
+def test_wide_layers_repeat_their_results_bit_for_bit(M, dt, group, N, K):
+    """With at least as many column tiles as CTAs no run is shorter than a tile, so that two CTAs at most add to a tile: whichever
+    comes first, the sum of two numbers is the same."""
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(M)
+    bq = torch.randint(0, 256, (N * K * dt.nbits // 8,), dtype=torch.uint8, device=dev, generator=gen)
+    scales = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
+    x = torch.randn(M, K, device=dev, generator=gen).half()
+    zp = 8 if dt.kind == D.KIND_UINT else 0
+    assert ops.plan(M, N, K, dt, zp, group)["tile_m"] == (M + 15) // 16 * 16
+    outs = [ops.quantized_matmul(x, bq, scales, dt, group, zp) for _ in range(12)]
+    for c in outs[1:]:
+        assert torch.equal(c, outs[0])

@@ -707,15 +707,6 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
     p.unit = G;
     grid = n_tiles < device_info().sm_count ? n_tiles : device_info().sm_count;
   }
-  // More column tiles than CTAs: every CTA has whole tiles of its own and takes its share of the others before them, so that the sums
-  // that meet in L2 are not what the launch ends with (28672 x 4096, 4 bits, equal runs / own tiles, us: 8 rows 19.7 / 18.3, 64 rows
-  // 25.4 / 23.2; 19072 columns, 12 rows 15.6 / 14.1).  Not for short tiles, whose shares are a group or two (57344 x 1024,
-  // 3 bits, 100 rows: 21.6 / 23.2).
-  p.own = 0;
-  if (p.cluster == 1 && p.unit == 1 && n_tiles > grid && G >= 16) {
-    p.own = n_tiles / (int)grid;
-    p.work = (n_tiles - p.own * (int)grid) * G;
-  }
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return ST_CUDA;
   CUtensorMap tmaps[2];  // activations; packed weights

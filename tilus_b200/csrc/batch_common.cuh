@@ -57,37 +57,11 @@ __device__ __forceinline__ void batch_load_units(uint32_t stage, int nl, int h, 
   }
 }
 
-// The groups of CTA c, in the order in which it takes them, as positions v = 0 .. n - 1: a contiguous run of the groups counted tile by
-// tile over the whole matrix, and behind it `own` whole tiles.  The run covers at most one tile's end, whole tiles, and
-// one tile's start; what it shares with other CTAs is added up in L2 while the whole tiles are worked on.
-struct BatchRun {
-  int lo, n_left, own_lo, n, G;
-  __device__ __forceinline__ BatchRun(const BatchParams& p, int c) : own_lo(0), G(p.G) {
-    int end;
-    if (p.cluster > 1) {
-      lo = (c / p.cluster) * p.G + (c % p.cluster) * p.G / p.cluster;
-      end = (c / p.cluster) * p.G + (c % p.cluster + 1) * p.G / p.cluster;
-    } else {
-      const int first = p.own * p.grid * p.G;  // of the groups that are shared out
-      if (p.work <= 0x7fffffff / p.grid) {  // (a 64-bit division costs ~100 instructions)
-        lo = first + (int)((unsigned)p.work * (unsigned)c / (unsigned)p.grid) * p.unit;
-        end = first + (int)((unsigned)p.work * (unsigned)(c + 1) / (unsigned)p.grid) * p.unit;
-      } else {
-        lo = first + (int)((long long)p.work * c / p.grid) * p.unit;
-        end = first + (int)((long long)p.work * (c + 1) / p.grid) * p.unit;
-      }
-      own_lo = c * p.own * p.G;
-    }
-    n_left = end - lo;
-    n = n_left + p.own * p.G;
-  }
-  // group v, counted over the whole matrix
-  __device__ __forceinline__ int at(int v) const { return v < n_left ? lo + v : own_lo + v - n_left; }
-  // groups from v to the end of its column tile or of the run
-  __device__ __forceinline__ int segment(int v) const {
-    return v < n_left ? min(G - (lo + v) % G, n_left - v) : G - (v - n_left) % G;
-  }
-};
+// first group of CTA c's run
+__device__ __forceinline__ int batch_run_start(const BatchParams& p, int c) {
+  if (p.cluster > 1) return (c / p.cluster) * p.G + (c % p.cluster) * p.G / p.cluster;
+  return (int)((long long)p.work * c / p.grid) * p.unit;
+}
 
 // ---- column tiles shared by the CTAs of a cluster ------------------------------------------------
 // Cluster form of a launch (p.cluster > 1): a cluster owns one column tile, its CTAs equal ranges of K.  Every CTA

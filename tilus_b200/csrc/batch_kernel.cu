@@ -34,9 +34,7 @@
 // contiguous runs, one per CTA, whatever the shape.  A run covers at most one tile's end, whole
 // tiles, and one tile's start.  Whole tiles are written to C; a partial tile's sums are added into an
 // fp32 scratch tile (red.global.add.v4) and counted in, and whoever completes the count converts them,
-// writes C and puts the scratch back to zero (batch_epilogue).  With more tiles than CTAs a CTA has whole tiles of its
-// own and takes an equal run of the other tiles' groups before them (BatchRun), so that the launch does not end on these sums:
-// 28672 x 4096, 4 bits, 64 rows 25.4 -> 23.2 us.  The additions are the price of the form:
+// writes C and puts the scratch back to zero (batch_epilogue).  These additions are the price of the form:
 // 4.8 MB of them at 64 rows keep L2 busy for 6 us.  Where the column tiles are few enough that every one can have
 // a cluster of CTAs to itself, the launch takes the cluster form instead (batch_common.cuh; the rule is in
 // api.cu).
@@ -141,7 +139,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   volatile int* abort_flag = &bars->abort_flag;
-  const BatchRun run(p, blockIdx.x);  // this CTA's groups
+  // this CTA's run of groups, counted tile by tile over the whole matrix
+  const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
 
   if (tid == 0) {
     for (int i = 0; i < BATCH_SLOTS_MAX; ++i) { mbar_init(BAR_ADDR(slot_full, i), 4); mbar_init(BAR_ADDR(done, i), 1); }
@@ -181,10 +180,11 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   const uint32_t slots_t = tmem + (uint32_t)(batch_d_stride(NR) * 2);
 
   // one segment of the run: pos -> tile, groups
-#define SEGMENT(pos)                                                        \
-  const int tile = run.at(pos) / p.G, len = run.segment(pos);               \
-  const bool last_seg = (pos) + len == run.n;                               \
-  (void)last_seg; (void)tile;
+#define SEGMENT(pos)                                     \
+  const int tile = (pos) / p.G, g0 = (pos) - tile * p.G; \
+  const int len = min(p.G - g0, run1 - (pos));           \
+  const bool last_seg = (pos) + len == run1;             \
+  (void)last_seg;
 
   if (warp < W_EPI) {
     // ================= dequantize (and a share of the last segment's epilogue) =================
@@ -194,7 +194,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     bool good = true;
     int stage = set, slot = set;    // stages of a set: set, set + BATCH_SETS, ...; slots likewise
     uint32_t ring_phase = 0, slot_phase = 1;
-    for (int g_own = set; g_own < run.n; g_own += BATCH_SETS) {
+    for (int g_own = set; g_own < run1 - run0; g_own += BATCH_SETS) {
       if (!mbar_wait_abortable(BAR_ADDR(g_full, stage), ring_phase, abort_flag)) { good = false; break; }
       const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
       const uint32_t sc = scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u;
@@ -239,8 +239,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
     if (good && p.cluster <= 1) {
-      int pos = 0, seg = 0;  // the last segment
-      while (pos + run.segment(pos) < run.n) { pos += run.segment(pos); ++seg; }
+      int pos = run0, seg = 0;  // the last segment
+      while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
       asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
       if (mbar_wait_abortable(BAR_ADDR(run_done, 0), 0u, abort_flag)) {
@@ -255,7 +255,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
     int seg = 0;
-    for (int pos = 0; pos < run.n && p.cluster <= 1; ++seg) {
+    for (int pos = run0; pos < run1 && p.cluster <= 1; ++seg) {
       SEGMENT(pos)
       if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -273,9 +273,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       int stage = 0, n_issued = 0, slot = 0;
       uint32_t phase = 0;
       bool good = true;
-      int g = run.lo % p.G;
-      for (int pos = 0; pos < run.n; ++pos) {
-        if (pos == run.n_left) g = 0;
+      int g = run0 % p.G;
+      for (int pos = run0; pos < run1; ++pos) {
         if (n_issued >= AS) {
           if (!mbar_wait_abortable(BAR_ADDR(done, slot), phase, abort_flag)) { good = false; break; }
           if (++slot == BATCH_SETS * sps) { slot = 0; phase ^= 1u; }
@@ -304,9 +303,8 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       int stage = 0, n_issued = 0;
       uint32_t phase = 1;
       bool good = true;
-      int tile = run.lo / p.G, g = run.lo - tile * p.G;
-      for (int pos = 0; pos < run.n; ++pos) {
-        if (pos == run.n_left) { g = 0; tile = run.own_lo / p.G; }  // on to the CTA's own tiles
+      int tile = run0 / p.G, g = run0 - tile * p.G;
+      for (int pos = run0; pos < run1; ++pos) {
         if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
         const uint32_t bar = BAR_ADDR(g_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(WSTAGE) : "memory");
@@ -331,18 +329,13 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       int stage = 0, n_issued = 0;
       uint32_t phase = 1;
       bool good = true;
-      int tile = run.lo / p.G, g = run.lo - tile * p.G;
+      int tile = run0 / p.G, g = run0 - tile * p.G;
       // scale row(s) of the group: p.rpg rows per group, or one row for p.group / 128 groups
       const int groups_per_row = p.rpg == 1 ? p.group / 128 : 1;
       int in_row = g % groups_per_row;
       const __half* sc = p.scales + (size_t)(p.rpg == 1 ? g / groups_per_row : g * p.rpg) * p.N + tile * 128;
       uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
-      for (int pos = 0; pos < run.n; ++pos) {
-        if (pos == run.n_left) {
-          g = 0; in_row = 0; tile = run.own_lo / p.G;
-          sc = p.scales + tile * 128;
-          sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
-        }
+      for (int pos = run0; pos < run1; ++pos) {
         if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
         const uint32_t bar = BAR_ADDR(g_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(sc_bytes * (uint32_t)p.rpg)
@@ -378,7 +371,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
       // the look (twice 100 cycles) lies under them; only a group that was not ready then is waited for
       bool ready = false;
-      for (int pos = 0; pos < run.n && good; ++seg) {
+      for (int pos = run0; pos < run1 && good; ++seg) {
         SEGMENT(pos)
         if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -460,7 +453,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     cluster_arrive();
     cluster_wait();
     if (warp < W_ACT && !*abort_flag)
-      cluster_finish<ACT, 1>(p, smem_base, 0u, blockIdx.x % p.cluster, run.lo / p.G, (warp & 3) * 32 + lane, lane,
+      cluster_finish<ACT, 1>(p, smem_base, 0u, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
                           warp >> 2, 3);
     cluster_arrive();  // nobody leaves while its sums are being read
     cluster_wait();

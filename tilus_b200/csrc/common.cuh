@@ -152,8 +152,7 @@ struct BatchParams {
   int work, unit;        // work units of the launch and 128-row groups per unit (1, or G: whole column tiles)
   int stages;            // packed 128-row groups in the shared-memory ring
   int a_stages;          // 128-row activation groups in shared memory
-  int grid;              // CTAs: each takes an equal contiguous run of work units, or
-  int own;               // > 0: this many whole column tiles, after an equal run of the tiles left over
+  int grid;              // CTAs: each takes an equal contiguous run of work units
   int cluster;           // > 1: CTAs per column tile, which share its K and add up in distributed shared memory
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
 };

@@ -93,7 +93,8 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   volatile int* abort_flag = &bars->abort_flag;
-  const BatchRun run(p, blockIdx.x);  // this CTA's groups
+  // this CTA's run of groups, counted tile by tile over the whole matrix
+  const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
 
   if (tid == 0) {
     for (int i = 0; i < EXACT_SLOTS; ++i) {
@@ -149,12 +150,12 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     float sq[EXACT_SPS];  // scales of the groups in the set's slots
     int stage = set;      // the set's stages: set, set + EXACT_SETS, ...
     uint32_t ring_phase = 0, hand_phase = 1;
-    const int n_own = (run.n - set + EXACT_SETS - 1) / EXACT_SETS;
+    const int n_own = (run1 - run0 - set + EXACT_SETS - 1) / EXACT_SETS;
     const bool more = p.M > 4, most = p.M > 8;
     const bool alone = p.cluster <= 1;
-    int seg_end = run.segment(0);  // of the segment the sums belong to
-    int pos = set;                 // group whose sums are added next
-    while (pos >= seg_end && seg_end < run.n) seg_end += run.segment(seg_end);  // (first segments without a group of this set)
+    int seg_end = min((run0 / p.G + 1) * p.G, run1);  // of the segment the sums belong to
+    int pos = run0 + set;                             // group whose sums are added next
+    while (pos >= seg_end && seg_end < run1) seg_end = min(seg_end + p.G, run1);  // (first segments without a group of this set)
     bool good = true;
     for (int i0 = 0; i0 < n_own + EXACT_SPS && good; i0 += EXACT_SPS) {
 #pragma unroll
@@ -193,10 +194,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR_ADDR(hand_full, set));
             // (segments without a group of this set are passed over)
-            while (seg_end < run.n) {
-              seg_end += run.segment(seg_end);
-              if (pos + EXACT_SETS < seg_end) break;
-            }
+            do seg_end = min(seg_end + p.G, run1); while (pos + EXACT_SETS >= seg_end && seg_end < run1);
           }
           pos += EXACT_SETS;
         }
@@ -236,14 +234,14 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
     uint32_t phase = 0u;  // bit s: of set s
     bool good = true;
-    for (int pos = 0; pos < run.n && good && p.cluster <= 1;) {
-      const int tile = run.at(pos) / p.G, len = run.segment(pos);
+    for (int pos = run0; pos < run1 && good && p.cluster <= 1;) {
+      const int tile = pos / p.G, len = min((tile + 1) * p.G, run1) - pos;
       float4 f[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) f[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int set = 0; set < EXACT_SETS; ++set) {
-        if ((set + EXACT_SETS - pos % EXACT_SETS) % EXACT_SETS >= len) continue;  // no group of this set
+        if ((set + EXACT_SETS - (pos - run0) % EXACT_SETS) % EXACT_SETS >= len) continue;  // no group of this set
         if (!mbar_wait_abortable(BAR_ADDR(hand_full, set), (phase >> set) & 1u, abort_flag)) { good = false; break; }
         phase ^= 1u << set;
         const float4* hand = reinterpret_cast<const float4*>(smem_al + hand_off + (uint32_t)set * HAND) + nl;
@@ -279,9 +277,8 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       int stage = 0, n_issued = 0;
       uint32_t phase = 1;  // of the group that held the stage, whose MMAs report on its slot's barrier
       bool good = true;
-      int g = run.lo % p.G;
-      for (int pos = 0; pos < run.n; ++pos) {
-        if (pos == run.n_left) g = 0;
+      int g = run0 % p.G;
+      for (int pos = run0; pos < run1; ++pos) {
         if (n_issued >= EXACT_SLOTS && !mbar_wait_abortable(BAR_ADDR(done, stage), phase, abort_flag)) { good = false; break; }
         const uint32_t bar = BAR_ADDR(a_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(EXACT_ASTAGE) : "memory");
@@ -308,17 +305,12 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       int stage = 0, n_issued = 0;
       uint32_t phase = 1;
       bool good = true;
-      int tile = run.lo / p.G, g = run.lo - tile * p.G;
+      int tile = run0 / p.G, g = run0 - tile * p.G;
       const int groups_per_row = p.group / 128;  // 128-row groups per scale row
       int in_row = g % groups_per_row;
       const __half* sc = p.scales + (size_t)(g / groups_per_row) * p.N + tile * 128;
       uint32_t sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
-      for (int pos = 0; pos < run.n; ++pos) {
-        if (pos == run.n_left) {  // on to the CTA's own tiles
-          g = 0; in_row = 0; tile = run.own_lo / p.G;
-          sc = p.scales + tile * 128;
-          sc_bytes = (uint32_t)min(128, p.N - tile * 128) * 2u;
-        }
+      for (int pos = run0; pos < run1; ++pos) {
         if (!mbar_wait_abortable(BAR_ADDR(g_empty, stage), phase, abort_flag)) { good = false; break; }
         const uint32_t bar = BAR_ADDR(g_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(weights ? WSTAGE : sc_bytes)
@@ -358,7 +350,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
       // the looks lies under them; only a group that was not ready then is waited for
       bool ready = false;
-      for (int pos = 0; pos < run.n; ++pos) {
+      for (int pos = run0; pos < run1; ++pos) {
         if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), phase, abort_flag) ||
                        !mbar_wait_abortable(BAR_ADDR(a_full, slot), phase, abort_flag))) break;
         const int slot1 = slot + 1 == EXACT_SLOTS ? 0 : slot + 1;
@@ -426,7 +418,7 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     cluster_arrive();
     cluster_wait();
     if (warp < W_EPI && !*abort_flag)
-      cluster_finish<ACT, EXACT_SETS>(p, smem_base + hand_off, HAND, blockIdx.x % p.cluster, run.lo / p.G, (warp & 3) * 32 + lane, lane,
+      cluster_finish<ACT, EXACT_SETS>(p, smem_base + hand_off, HAND, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
                           warp >> 2, EXACT_SETS);
     cluster_arrive();  // nobody leaves while its sums are being read
     cluster_wait();
