@@ -5,7 +5,7 @@ import time
 import pytest
 import torch
 
-from tilus_b200 import QuantizedLinear, float16
+from tilus_b200 import QuantizedLinear, _lib, float16, ops
 from tilus_b200 import dtypes as D
 
 pytestmark = pytest.mark.gpu
@@ -290,3 +290,59 @@ def test_first_launches_from_several_threads():
         t.join()
     for x, out in zip(xs, outs):
         assert out is not None and _close(out, x.float() @ w)
+
+
+class _HostCalls:
+    """A series of host calls through the C ABI: weights of several layers, pinned rows and results of each call."""
+
+    def __init__(self, m, n, k, dt, layers, calls):
+        gen = torch.Generator(device="cuda").manual_seed(n + m)
+        self.m, self.n, self.k, self.dt, self.zp = m, n, k, dt, 1 << (dt.nbits - 1) if dt.kind == D.KIND_UINT else 0
+        self.weights = [(torch.randint(0, 256, (n * k * dt.nbits // 8,), dtype=torch.uint8, device="cuda", generator=gen),
+                         (torch.rand(k // 128, n, device="cuda", generator=gen) * 0.01 + 0.005).half()) for _ in range(layers)]
+        self.xs = [_rows(m, k, i).pin_memory() for i in range(calls)]
+        self.outs = [torch.zeros(m, n, dtype=torch.float16).pin_memory() for _ in range(calls)]
+        self.staging = torch.zeros(m * (n + k), dtype=torch.float16, device="cuda")
+        self.ws = torch.zeros(ops.workspace_bytes(16, n, k, dt, self.zp, 128), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+
+    def run(self):
+        lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+        for i, (x, out) in enumerate(zip(self.xs, self.outs)):
+            bq, sc = self.weights[i % len(self.weights)]
+            _lib.check(lib.b200q_gemm_host(x.data_ptr(), self.k, bq.data_ptr(), sc.data_ptr(), out.data_ptr(), self.n, self.m,
+                                           self.n, self.k, self.dt.code, self.zp, 128, _lib.ACT_F16, self.staging.data_ptr(),
+                                           self.staging.data_ptr() + 2 * self.m * self.k, self.ws.data_ptr(), self.ws.numel(),
+                                           stream))
+
+    def check(self):
+        torch.cuda.synchronize()
+        for i, (x, out) in enumerate(zip(self.xs, self.outs)):
+            w = ops.dequantize(*self.weights[i % len(self.weights)], self.dt, 128, self.zp).float()
+            assert _close(out, x.cuda().float() @ w), i
+        assert int(self.ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 28672, 1024), (4, 11008, 2048), (2, 17216, 1024), (1, 5120, 5120)])
+def test_chained_host_calls_whose_last_cta_owns_fewer_column_tiles(m, n, k):
+    calls = _HostCalls(m, n, k, D.uint4b, 3, 18)
+    for _ in range(3):
+        calls.run()
+    calls.check()
+
+
+def test_host_calls_overlap_whether_or_not_the_last_cta_is_full():
+    """28672 columns leave the last CTA fewer column tiles than 28704 do: nothing is left over in either, so both fetch
+    their rows under the call before (13 us a call; 18 without)."""
+    chains = [_HostCalls(1, n, 4096, D.uint4b, 4, 40) for n in (28672, 28704)]
+    best = [1e9, 1e9]
+    for _ in range(6):
+        for i, chain in enumerate(chains):
+            chain.run()
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            chain.run()
+            e1.record()
+            torch.cuda.synchronize()
+            best[i] = min(best[i], e0.elapsed_time(e1))
+    assert best[0] <= 1.2 * best[1], best

@@ -844,7 +844,7 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
     p.warp_shift = stream_warp_shift(mc, p.KBc * 512, bits, p.T_own);
     // (staging_released: the previous user of the staging buffer on this stream lets go of it before it
     // releases its successor - only then may this launch write it without waiting)
-    p.nowait = (a_host && staging_released && p.S == 1 && p.T_own * p.CPC == p.NT) ? 1 : 0;
+    p.nowait = (a_host && staging_released && p.S == 1 && p.T_own * p.CPC >= p.NT) ? 1 : 0;  // (the last CTA may own fewer tiles)
     int smem = stream_smem(mc, p.KBc * 512, bits, pl.stages, p.T_own);
     // CTAs that fit one per SM must not meet two to an SM while others idle, as they would where the previous launch's CTAs
     // leave at different times (128 CTAs of 6144 x 4096 on 88 SMs: 7.2 us, one to an SM 5.4).  Launches of a few KB per CTA
