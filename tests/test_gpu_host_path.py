@@ -346,3 +346,16 @@ def test_host_calls_overlap_whether_or_not_the_last_cta_is_full():
             torch.cuda.synchronize()
             best[i] = min(best[i], e0.elapsed_time(e1))
     assert best[0] <= 1.2 * best[1], best
+
+
+@pytest.mark.parametrize("m,n,k,dt", [(4, 48, 14336, D.uint4b), (6, 32, 8192, D.uint4b), (5, 64, 13312, D.int3b), (1, 16, 20480, D.uint2b),
+                                      (2, 16, 6144, D.uint2b), (8, 16, 512, D.int8), (16, 16, 7680, D.int8)], ids=str)
+def test_narrow_layers_with_more_activations_than_their_ctas_fetch(m, n, k, dt):
+    """Calls whose launch has too few CTAs to fetch the rows, and calls that have enough in between: a kernel of its own brings
+    them."""
+    calls = [_HostCalls(m, n, k, dt, 2, 6), _HostCalls(1, 256, 1024, D.uint4b, 2, 6)]
+    for _ in range(2):
+        for c in calls:
+            c.run()
+    for c in calls:
+        c.check()

@@ -198,6 +198,12 @@ static int stream_stages_for(int m_pass, int kc, int bits, int t_own, int smem) 
   while (st > 0 && stream_smem(m_pass, kc, bits, st, t_own) > smem) --st;
   return st;
 }
+// The first CTAs of a launch on host buffers fetch the activations, four 16-byte pieces per thread: how many of them that takes
+static int stream_fetch_ctas(int M, int N, int K, int bits, const b200q_plan_t& pl) {
+  const int kc = K / pl.splits, t_own = stream_tiles_owned(M, N / BLOCK_N, pl.ctas_per_split);
+  const int per_cta = (32 << stream_warp_shift(M, kc, bits, t_own)) * 4;
+  return (M * (K / 8) + per_cta - 1) / per_cta;
+}
 // CTAs per k chunk: the fewest that finish as soon as one per SM would
 static int stream_ctas_per_chunk(int NT, int s, const DeviceInfo& di) {
   const int full = di.sm_count / s;
@@ -820,12 +826,10 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
   p.a_host = nullptr; p.fetch_flag = nullptr; p.fetch_ctas = 0; p.nowait = 0;
   if (a_host) {
     if (gather || M > stream_rows_per_pass(M)) return ST_INVALID_ARG;
-    const int warp_shift = stream_warp_shift(M, p.KBc * 512, bits, stream_tiles_owned(M, p.NT, p.CPC));
-    const int per_cta = (32 << warp_shift) * 4;  // 16-byte pieces one CTA fetches
     p.a_host = reinterpret_cast<const __half*>(a_host);
     p.lda = lda_host;
     p.fetch_flag = reinterpret_cast<unsigned*>(workspace) + 16;  // words 16, 17 of the status header
-    p.fetch_ctas = (M * (K / 8) + per_cta - 1) / per_cta;
+    p.fetch_ctas = stream_fetch_ctas(M, N, K, bits, pl);
     if (p.fetch_ctas > p.S * p.CPC) return ST_INVALID_ARG;
   }
   if (gather) {
@@ -1136,14 +1140,16 @@ int b200q_gemm_host(const void* a_host, int lda, const void* bq, const void* sca
       (void)cudaGetLastError();  // an unregistered host pointer is not an error here
   }
   // Decode batches: the GEMV kernel's own first CTAs fetch the rows (one kernel, no copy operation at
-  // all) when the result can also go straight to the host buffer.
+  // all) when the result can also go straight to the host buffer and the launch has CTAs enough for them (a layer of a few
+  // column tiles with a long K has not: 4 x 48 x 14336 is three CTAs, its rows take four).
   if (a_mapped && act_ok(act_dtype) && (ldc % 8) == 0 && (size_t)M * N * 2 <= (1u << 20)) {
     int var;
     b200q_plan_t pl;
     cudaPointerAttributes cattr;
     if (check_problem(M, N, K, wtype, zero_point, group, true, &var) == ST_OK &&
         make_plan(M, N, K, var, group, kStreamForm, &pl) == ST_OK &&
-        pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M)) {
+        pl.splits * pl.ctas_per_split <= 2 * device_info().sm_count / stream_mt(M) &&
+        stream_fetch_ctas(M, N, K, var_bits(var), pl) <= pl.splits * pl.ctas_per_split) {
       if (cudaPointerGetAttributes(&cattr, c_host) == cudaSuccess && cattr.type == cudaMemoryTypeHost &&
           cattr.devicePointer && (((uintptr_t)cattr.devicePointer) & 15) == 0) {
         if (!bq || !scales) return ST_INVALID_ARG;
