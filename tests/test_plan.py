@@ -65,3 +65,12 @@ def test_static_workspace_takes_prefill_batches_that_256_row_tiles_fit(lib, m, n
     uint4 = 4 << 8
     assert ops.plan(m, n, k, "uint4b", 8, 128)["workspace_bytes"] > lib.b200q_static_workspace_limit()
     assert not _static_ws_refused(lib, m, n, k, uint4, 8)
+
+
+@pytest.mark.parametrize("m", [7, 8])
+@pytest.mark.parametrize("n", [2048, 8192, 14336, 18944, 28672, 32768])
+@pytest.mark.parametrize("w", ["uint4b", "int8", "uint2b"])
+def test_seven_and_eight_rows_do_not_cut_short_layers(m, n, w):
+    """2048 rows of weights are one chunk, whose sums stay in shared memory (28672 columns in two chunks: a fifth slower)."""
+    pl = ops.plan(m, n, 2048, w, 1 << (int(w[4]) - 1) if w[0] == "u" else 0, 128, act_dtype=torch.bfloat16)
+    assert (pl["tile_m"], pl["splits"]) == (0, 1)

@@ -240,8 +240,10 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
   };
   const int s_max = KB < di.sm_count ? KB : di.sm_count;
   // 7 and 8 rows: chunks that leave half of the shared memory, since every CTA stages all rows of its chunk (4096 x 4096, 1 / 4
-  // chunks: 8 rows of 4 bits 8.0 / 7.35 us, of 8 bits 9.3 / 8.5; 5 rows of 4 bits 7.0 / 7.4)
-  const int most = m_pass == 7 || m_pass == 8 ? kStreamSmemCap : di.max_smem;
+  // chunks: 8 rows of 4 bits 8.0 / 7.35 us, of 8 bits 9.3 / 8.5; 5 rows of 4 bits 7.0 / 7.4).  Not up to 2048 rows of weights, where
+  // the sums through the scratch cost more than the staging (1 / 2 chunks, 8 rows, bfloat16, 4 bits: 8192 x 2048 6.9 / 7.6 us, 28672 x
+  // 2048 11.2 / 14.5, of 8 bits 14.4 / 17.9; 2048 and 4096 columns within 3 %)
+  const int most = (m_pass == 7 || m_pass == 8) && KB > 4 ? kStreamSmemCap : di.max_smem;
   consider(1, 2, true, kStreamSmemCap);
   consider(1, 2, true, most);
   for (int s = 1; s <= s_max; ++s) consider(s, 3, true, most);
