@@ -65,7 +65,7 @@ typedef struct b200q_plan {
   int32_t smem_bytes;    /* dynamic shared memory per CTA */
   int32_t tile_m;        /* kernel 1: activation rows per CTA tile (32, 64, 128, 256 or 384); kernel 3: M rounded
                             up to 16; kernel 2: 0 for the stream kernel, 16 for the tcgen05 form */
-  int32_t stages;        /* pipeline depth (kernel 2: ring slots per warp; kernel 1: activation stages;
+  int32_t stages;        /* pipeline depth (kernel 2: ring slots per warp, 1 .. 8, of which those that fit are used; kernel 1: activation stages;
                             kernel 3: 128-row weight groups in the packed ring) */
   int32_t warps;         /* warps per CTA (output only) */
   int32_t passes;        /* launches: 2 when kernel 1 takes the multiple of 256 rows and kernel 2 the last 1..16 rows */

@@ -49,3 +49,16 @@ def test_splits_of_the_column_tiles(M, N, K, dt):
         c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws)
         assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
     assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("M,N,K,dt,stages", [(1, 8192, 8192, D.uint4b, 6), (1, 8192, 8192, D.uint4b, 8), (8, 4096, 4096, D.int8, 8),
+                                             (4, 4096, 14336, D.uint4b, 5), (16, 2048, 2048, D.int6b, 8), (20, 2048, 2048, D.int3b, 8)], ids=str)
+def test_plans_edited_to_deeper_rings(M, N, K, dt, stages):
+    """Up to eight slots per warp may be asked for; as many are used as the launch has room for."""
+    a, bq, sc, zp, ref = _problem(M, N, K, dt, seed=stages)
+    pl = ops.plan(min(M, 4), N, K, dt, zp, 128)
+    assert pl["tile_m"] == 0 and pl["stages"] < stages
+    ws = torch.zeros(ops.workspace_bytes(16, N, K, dt, zp, 128), dtype=torch.uint8, device=a.device)
+    c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws, plan_override={**pl, "stages": stages})
+    assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert int(ws.count_nonzero()) == 0

@@ -851,13 +851,16 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
     // (staging_released: the previous user of the staging buffer on this stream lets go of it before it
     // releases its successor - only then may this launch write it without waiting)
     p.nowait = (a_host && staging_released && p.S == 1 && p.T_own * p.CPC >= p.NT) ? 1 : 0;  // (the last CTA may own fewer tiles)
-    int smem = stream_smem(mc, p.KBc * 512, bits, pl.stages, p.T_own);
+    // (rings of a plan edited to more slots than the launch has room for: as many as fit)
+    const int fit = stream_stages_for(mc, p.KBc * 512, bits, p.T_own, device_info().max_smem);
+    if (fit < 1) return ST_UNSUPPORTED;
+    p.stages = pl.stages < fit ? pl.stages : fit;
+    int smem = stream_smem(mc, p.KBc * 512, bits, p.stages, p.T_own);
     // CTAs that fit one per SM must not meet two to an SM while others idle, as they would where the previous launch's CTAs
     // leave at different times (128 CTAs of 6144 x 4096 on 88 SMs: 7.2 us, one to an SM 5.4).  Launches of a few KB per CTA
     // gain more from starting beside their predecessor (2048 x 2048, 2 bits, 8 KB: 3.1 / 3.8 us; 3 bits, 12 KB: 3.8 / 3.9).
     const bool spread = p.S * p.CPC <= device_info().sm_count && (long long)p.T_own * p.KBc * bits > 20;
     if (spread && smem < kOneCtaSmem) smem = kOneCtaSmem;
-    if (smem > device_info().max_smem) return ST_UNSUPPORTED;
     cudaError_t e = stream_launch(var, p, stream_mt(mc), smem, stream);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
   }
@@ -907,10 +910,10 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     const int rows = M < stream_rows_per_pass(M) ? M : stream_rows_per_pass(M);
     if (chunks.ctas_per_split > N / BLOCK_N) chunks.ctas_per_split = N / BLOCK_N;
     if (chunks.ctas_per_split > 4 * device_info().sm_count / pl.splits) chunks.ctas_per_split = 4 * device_info().sm_count / pl.splits;
+    if (chunks.stages > 8) chunks.stages = 8;
     if (chunks.ctas_per_split > 0) {
       const int t_own = stream_tiles_owned(rows, N / BLOCK_N, chunks.ctas_per_split);
       const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info().max_smem);
-      if (chunks.stages > fit) chunks.stages = fit;
       if (fit < 1 && plan_stream(rows, N, K, var_bits(var), device_info(), &chunks) != ST_OK) return ST_UNSUPPORTED;
     }
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, chunks);
