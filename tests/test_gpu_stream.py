@@ -9,14 +9,27 @@ pytestmark = pytest.mark.gpu
 
 
 def _problem(M, N, K, dt, group=128, seed=0):
+    """A problem that the decode kernel takes: with fp16 activations, or with bfloat16 where fp16 goes to the exact kernel.  The
+    bfloat16 scales are fp16 numbers too, so that the reference's weights are rounded to fp16 in either case."""
     dev = torch.device("cuda:0")
     gen = torch.Generator(device=dev).manual_seed(seed)
     zp = 1 << (dt.nbits - 1) if dt.kind == D.KIND_UINT else 0
+    act = next((t for t in (torch.float16, torch.bfloat16) if ops.plan(min(M, 16), N, K, dt, zp, group, act_dtype=t)["tile_m"] == 0),
+               torch.float16)
     bq = torch.randint(0, 256, (N * K * dt.nbits // 8,), dtype=torch.uint8, device=dev, generator=gen)
-    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).half()
-    a = torch.randn(M, K, device=dev, generator=gen).half()
-    ref = a.float() @ ops.dequantize(bq, sc, dt, group, zp).float()
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).to(act)
+    a = torch.randn(M, K, device=dev, generator=gen).to(act)
+    ref = a.float() @ ops.dequantize(bq, sc.half(), dt, group, zp).float()
     return a, bq, sc, zp, ref
+
+
+def _close(c, ref):
+    """One rounding of the output (2^-11 of it, bfloat16 2^-9) and one of each reference weight (2^-11)."""
+    return float((c.float() - ref).abs().max()) <= (2e-3 if c.dtype == torch.float16 else 4e-3) * float(ref.abs().max())
+
+
+def _is_stream(a, N, dt, zp, group=128):
+    return ops.plan(a.shape[0], N, a.shape[1], dt, zp, group, act_dtype=a.dtype)["tile_m"] == 0
 
 
 @pytest.mark.parametrize("dt", [D.uint8, D.int8, D.uint7b, D.uint6b, D.int5b, D.uint4b, D.int3b, D.uint2b, D.uint1b, D.float6_e3m2],
@@ -27,27 +40,36 @@ def test_repeated_calls_with_the_weights_in_l2(dt, M):
     types used to be read behind the refill where registers let the compiler delay their second loads)."""
     N, K = 2048, 8192
     a, bq, sc, zp, ref = _problem(M, N, K, dt)
+    assert _is_stream(a, N, dt, zp)
     outs = [ops.quantized_matmul(a, bq, sc, dt, 128, zp) for _ in range(40)]
-    for c in outs:  # one rounding of the output (2^-11 of it) and of each reference weight
-        assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    for c in outs:
+        assert _close(c, ref)
 
 
 @pytest.mark.parametrize("M,N,K,dt", [
-    (1, 2384, 512, D.uint4b),     # 149 column tiles: two per CTA, the last CTA one
+    (1, 2384, 1024, D.int8),      # 149 column tiles, two CTAs on one SM
+    (1, 2384, 4096, D.int8),      # two tiles per CTA, the last CTA one
     (1, 5120, 1536, D.int3b),     # 107 CTAs of three tiles, the last two
     (2, 11008, 1024, D.uint8),    # 138 CTAs of five, the last three
     (1, 16, 512, D.uint4b),       # one tile: one CTA, half the warps
+    (1, 16384, 1024, D.uint2b),   # two CTAs of 8 warps per SM
+    (3, 12112, 1024, D.int5b),    # 253 such CTAs of three tiles, the last one
+    (2, 4736, 2048, D.uint4b),    # one tile for each of two CTAs on every SM
+    (4, 1040, 1024, D.float6_e3m2),  # 8 warps for four rows
+    (8, 8192, 512, D.uint2b),     # and for eight (bfloat16)
     (2, 2368, 1024, D.uint2b),    # one tile per SM
     (3, 2384, 1024, D.float4_e2m1),
-    (4, 80000, 512, D.uint1b),    # more tiles than a CTA owns: the rest item by item
+    (4, 160000, 512, D.uint1b),   # more tiles than a CTA owns: the rest item by item
     (8, 4096, 4096, D.uint4b),    # chunks of K, sums in the scratch
-    (7, 2384, 4096, D.int6b)], ids=str)
+    (8, 8192, 4096, D.int6b),     # the same, with fewer tiles for the last CTA of a chunk (bfloat16)
+    (7, 28672, 2048, D.int8)], ids=str)
 def test_splits_of_the_column_tiles(M, N, K, dt):
     a, bq, sc, zp, ref = _problem(M, N, K, dt, seed=N)
+    assert _is_stream(a, N, dt, zp)
     ws = torch.zeros(max(ops.workspace_bytes(M, N, K, dt, zp, 128), 1 << 20), dtype=torch.uint8, device=a.device)
     for _ in range(2):
         c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws)
-        assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+        assert _close(c, ref)
     assert int(ws.count_nonzero()) == 0
 
 
@@ -60,5 +82,5 @@ def test_plans_edited_to_deeper_rings(M, N, K, dt, stages):
     assert pl["tile_m"] == 0 and pl["stages"] < stages
     ws = torch.zeros(ops.workspace_bytes(16, N, K, dt, zp, 128), dtype=torch.uint8, device=a.device)
     c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws, plan_override={**pl, "stages": stages})
-    assert float((c.float() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    assert _close(c, ref)
     assert int(ws.count_nonzero()) == 0

@@ -164,13 +164,14 @@ static int stream_pitch(int kc) {
   return bytes / 2;
 }
 // ---- stream kernel (kernel 2) ---------------------------------------------------------------------
-// One CTA per SM.
+// One CTA of 16 warps per SM, or two of 8.
 static const int kStreamSmemCap = 113 * 1024;  // half an SM
 // Rings beyond this are not worth their room: every CTA fills them before its activations arrive, and what is requested first is
 // waited for first (M = 1, 4096 x 14336, 4 bits: rings of 64 / 160 KB, activations staged 2.8 / 4.6 us after the start; the
 // linears of a Llama-3-8B block 33.3 / 34.9 us).
 static const int kStreamRing = 72 * 1024;
 static const int kOneCtaSmem = 116 * 1024;  // more than half an SM
+static const int kTwoCtaSmem = 80 * 1024;   // more than a third
 static int stream_slot_bytes(int bits) { return stream_gi(bits) * 256 * bits; }
 // 8-row activation tiles per launch: 1 or 2 (the kernel's MT)
 static int stream_mt(int m_pass) { return m_pass <= 8 ? 1 : 2; }
@@ -183,25 +184,41 @@ static int stream_tiles_owned(int m_pass, int NT, int cpc) {
   if (t <= cap && (long long)t * (cpc - 1) < NT) return t;
   return NT / cpc < cap ? NT / cpc : cap;
 }
-// log2 of the warps of a CTA that owns t_own tiles of kc rows
-static int stream_warp_shift(int m_pass, int kc, int bits, int t_own) {
-  return m_pass <= 2 && t_own > 0 && t_own * (kc / BLOCK_K) * (4 / stream_gi(bits)) <= 16 ? 3 : 4;
+// log2 of the warps of a CTA that owns t_own tiles of kc rows, in a launch of `ctas` CTAs.  Launches of more CTAs than SMs: 8, of which two
+// share an SM (16 would leave the second one no registers).  At most 16 ring items per CTA: 8, since most of 16 would only be
+// started - for one and two rows always, for more rows as long as there is not much to stage, which 16 warps do faster (16 / 8 warps,
+// us, 4 bits: 4 x 1024 x 1024 3.60 / 3.34, 3 x 2048 x 1024 3.81 / 3.27, 8 x 8192 x 512 4.45 / 3.94; but 4 x 2048 x 2048 4.32 / 4.45; 2
+// bits, four items: 4 x 4096 x 1024 4.45 / 3.60, 4 x 2048 x 2048 4.62 / 4.41, two items: 8 x 1024 x 1024 4.37 / 4.54).
+static int stream_warp_shift(int m_pass, int kc, int bits, int t_own, int ctas) {
+  if (stream_mt(m_pass) == 1 && ctas > device_info().sm_count) return 3;
+  const int KBc = kc / BLOCK_K, items = t_own * KBc * (4 / stream_gi(bits));
+  if (t_own < 1 || items > 16 || m_pass > 8) return 4;
+  return m_pass <= 2 || m_pass * KBc <= (items == 3 || items == 4 ? 16 : 12) ? 3 : 4;
 }
-static int stream_smem(int m_pass, int kc, int bits, int stages, int t_own) {
-  const int mt = stream_mt(m_pass), warps = 1 << stream_warp_shift(m_pass, kc, bits, t_own);
+static int stream_smem(int m_pass, int kc, int bits, int stages, int t_own, int ctas) {
+  const int mt = stream_mt(m_pass), warps = 1 << stream_warp_shift(m_pass, kc, bits, t_own, ctas);
   // barriers, rings and scale caches of the warps, own-tile sums, activation chunk (+ 64 zero bytes), group sums as accumulator quads
   return STREAM_HEADER + warps * (stages * stream_slot_bytes(bits) + STREAM_SC_GROUPS * 32) + t_own * 16 * 8 * mt * 4 +
          m_pass * stream_pitch(kc) * 2 + 64 + (kc / 128) * 16 * mt * 4;
 }
-static int stream_stages_for(int m_pass, int kc, int bits, int t_own, int smem) {
+// What a launch of `ctas` CTAs asks for.  CTAs that fit one per SM must not meet two to an SM while others idle, as they would where the
+// previous launch's CTAs leave at different times (128 CTAs of 6144 x 4096 on 88 SMs: 7.2 us, one to an SM 5.4).  Launches of a few KB
+// per CTA gain more from starting beside their predecessor (2048 x 2048, 2 bits, 8 KB: 3.1 / 3.8 us; 3 bits, 12 KB: 3.8 / 3.9).
+// Likewise three of two (M = 1, 8192 x 1024: 4 bits 3.77 us, 3.51 so; 28672 x 2048, 3 bits, 15.4 / 11.5).
+static int stream_launch_smem(int m_pass, int kc, int bits, int stages, int t_own, int ctas) {
+  const int smem = stream_smem(m_pass, kc, bits, stages, t_own, ctas), sms = device_info().sm_count;
+  const int least = ctas <= sms ? (t_own * (kc / BLOCK_K) * bits > 20 ? kOneCtaSmem : 0) : stream_mt(m_pass) == 1 ? kTwoCtaSmem : 0;
+  return smem > least ? smem : least;
+}
+static int stream_stages_for(int m_pass, int kc, int bits, int t_own, int ctas, int smem) {
   int st = 8;
-  while (st > 0 && stream_smem(m_pass, kc, bits, st, t_own) > smem) --st;
+  while (st > 0 && stream_smem(m_pass, kc, bits, st, t_own, ctas) > smem) --st;
   return st;
 }
 // The first CTAs of a launch on host buffers fetch the activations, four 16-byte pieces per thread: how many of them that takes
 static int stream_fetch_ctas(int M, int N, int K, int bits, const b200q_plan_t& pl) {
   const int kc = K / pl.splits, t_own = stream_tiles_owned(M, N / BLOCK_N, pl.ctas_per_split);
-  const int per_cta = (32 << stream_warp_shift(M, kc, bits, t_own)) * 4;
+  const int per_cta = (32 << stream_warp_shift(M, kc, bits, t_own, pl.splits * pl.ctas_per_split)) * 4;
   return (M * (K / 8) + per_cta - 1) / per_cta;
 }
 // CTAs per k chunk: the fewest that finish as soon as one per SM would
@@ -210,6 +227,18 @@ static int stream_ctas_per_chunk(int NT, int s, const DeviceInfo& di) {
   if (full < 1) return 0;
   const int t = (NT + full - 1) / full;
   return (NT + t - 1) / t;
+}
+// Small layers, few rows: two CTAs of 8 warps per SM, each with its own share of the column tiles, which start, wait and finish beside
+// each other.  For rings that one CTA fills for most of its life: column tiles of at most 21 KB, or layers of 8 MB in all, 8-bit types
+// only the latter, activations of at most 8 KB, and not where two equal shares make the fullest SM do an eighth more.  M = 1, us, one CTA of
+// 16 warps / two of 8: 16384 x 1024, 4 bits 5.0 / 4.4, 2 bits 4.4 / 4.0; 12288 x 2048, 2 bits 5.7 / 5.0; 8192 x 2048, 4 bits 4.9 / 4.5;
+// 12288 x 1536, 5 bits 7.4 / 6.2; 8192 x 1024, 8 bits 4.7 / 4.4; 4096 x 4096, 4 bits 5.1 / 4.9.  Beyond those lines: 14336 x 4096, 4 bits
+// 9.0 / 9.3; 16384 x 2048, 8 bits 8.5 / 8.8; 4 x 4096 x 2048, 4 bits 4.7 / 5.0; 5120 x 4096, 3 bits (two tiles on 160 CTAs) 6.6 / 8.0.
+static int stream_paired_ctas(int m_pass, int NT, int K, int bits, const DeviceInfo& di) {
+  const int tile = 2 * K * bits;  // bytes
+  if (m_pass > 4 || m_pass * (K / BLOCK_K) > 8 || ((bits == 8 || tile > 21 << 10) && (long long)NT * tile > 8 << 20)) return 0;
+  const int t = (NT + 2 * di.sm_count - 1) / (2 * di.sm_count), ctas = (NT + t - 1) / t;
+  return ctas > di.sm_count && 2 * t * 7 <= (NT + di.sm_count - 1) / di.sm_count * 8 ? ctas : 0;
 }
 static const int kStreamMaxRows = 16;  // what the kernel takes
 static const int kStreamPlanRows = 4;  // what the plan gives it at any shape (gather and host-buffer launches: all of the above)
@@ -223,19 +252,19 @@ static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counte
 static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di, b200q_plan_t* pl) {
   const int KB = K / BLOCK_K, NT = N / BLOCK_N;
   int best_s = 0, best_st = 0, best_c = 0;
-  auto consider = [&](int s, int want, bool no_leftover, int smem) {
+  auto consider = [&](int s, int want, bool no_leftover, int smem, int cpc = 0) {
     if (best_s || KB % s) return;
-    const int cpc = stream_ctas_per_chunk(NT, s, di);
+    if (cpc < 1) cpc = stream_ctas_per_chunk(NT, s, di);
     if (cpc < 1) return;
     const int t_own = stream_tiles_owned(m_pass, NT, cpc);
     if (no_leftover && cpc * t_own < NT) return;
     // (a CTA that would stage more than 64 KB of activations, 1.75 times the bytes of its weights: shorter chunks.  5 x 2048 x 8192,
     // 2 bits, 1 / 2 chunks: 8.8 / 8.1 us; 4 x 4096 x 14336, single bits, 12.8 / 11.7; but 4 x 2048 x 2048, 2 bits, 4.7 / 6.0)
     if (no_leftover && m_pass > 2 && m_pass * (KB / s) > 64 && 4 * m_pass > 7 * t_own * bits) return;
-    const int st = stream_stages_for(m_pass, (KB / s) * 512, bits, t_own, smem);
+    const int st = stream_stages_for(m_pass, (KB / s) * 512, bits, t_own, s * cpc, smem);
     if (st < want) return;
     best_s = s; best_st = st; best_c = cpc;
-    const int ring = kStreamRing / (stream_slot_bytes(bits) << stream_warp_shift(m_pass, (KB / s) * 512, bits, t_own));
+    const int ring = kStreamRing / (stream_slot_bytes(bits) << stream_warp_shift(m_pass, (KB / s) * 512, bits, t_own, s * cpc));
     if (best_st > ring) best_st = ring > want ? ring : want;
   };
   const int s_max = KB < di.sm_count ? KB : di.sm_count;
@@ -244,6 +273,8 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
   // the sums through the scratch cost more than the staging (1 / 2 chunks, 8 rows, bfloat16, 4 bits: 8192 x 2048 6.9 / 7.6 us, 28672 x
   // 2048 11.2 / 14.5, of 8 bits 14.4 / 17.9; 2048 and 4096 columns within 3 %)
   const int most = (m_pass == 7 || m_pass == 8) && KB > 4 ? kStreamSmemCap : di.max_smem;
+  const int pairs = stream_paired_ctas(m_pass, NT, K, bits, di);
+  if (pairs) consider(1, 2, true, kStreamSmemCap, pairs);
   consider(1, 2, true, kStreamSmemCap);
   consider(1, 2, true, most);
   for (int s = 1; s <= s_max; ++s) consider(s, 3, true, most);
@@ -256,9 +287,10 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
   pl->splits = best_s;
   pl->cluster = 1;
   pl->ctas_per_split = best_c;
-  pl->warps = 1 << stream_warp_shift(m_pass, (KB / best_s) * 512, bits, stream_tiles_owned(m_pass, NT, best_c));
+  const int t_own = stream_tiles_owned(m_pass, NT, best_c), kc = (KB / best_s) * 512;
+  pl->warps = 1 << stream_warp_shift(m_pass, kc, bits, t_own, best_s * best_c);
   pl->stages = best_st;
-  pl->smem_bytes = stream_smem(m_pass, (KB / best_s) * 512, bits, best_st, stream_tiles_owned(m_pass, NT, best_c));
+  pl->smem_bytes = stream_smem(m_pass, kc, bits, best_st, t_own, best_s * best_c);
   pl->tile_m = 0;
   pl->pdl = 1;
   return ST_OK;
@@ -847,20 +879,15 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
     p.c = reinterpret_cast<__half*>(c) + (size_t)m0 * ldc;
     p.M = mc;
     p.T_own = stream_tiles_owned(mc, p.NT, p.CPC);
-    p.warp_shift = stream_warp_shift(mc, p.KBc * 512, bits, p.T_own);
+    p.warp_shift = stream_warp_shift(mc, p.KBc * 512, bits, p.T_own, p.S * p.CPC);
     // (staging_released: the previous user of the staging buffer on this stream lets go of it before it
     // releases its successor - only then may this launch write it without waiting)
     p.nowait = (a_host && staging_released && p.S == 1 && p.T_own * p.CPC >= p.NT) ? 1 : 0;  // (the last CTA may own fewer tiles)
     // (rings of a plan edited to more slots than the launch has room for: as many as fit)
-    const int fit = stream_stages_for(mc, p.KBc * 512, bits, p.T_own, device_info().max_smem);
+    const int fit = stream_stages_for(mc, p.KBc * 512, bits, p.T_own, p.S * p.CPC, device_info().max_smem);
     if (fit < 1) return ST_UNSUPPORTED;
     p.stages = pl.stages < fit ? pl.stages : fit;
-    int smem = stream_smem(mc, p.KBc * 512, bits, p.stages, p.T_own);
-    // CTAs that fit one per SM must not meet two to an SM while others idle, as they would where the previous launch's CTAs
-    // leave at different times (128 CTAs of 6144 x 4096 on 88 SMs: 7.2 us, one to an SM 5.4).  Launches of a few KB per CTA
-    // gain more from starting beside their predecessor (2048 x 2048, 2 bits, 8 KB: 3.1 / 3.8 us; 3 bits, 12 KB: 3.8 / 3.9).
-    const bool spread = p.S * p.CPC <= device_info().sm_count && (long long)p.T_own * p.KBc * bits > 20;
-    if (spread && smem < kOneCtaSmem) smem = kOneCtaSmem;
+    const int smem = stream_launch_smem(mc, p.KBc * 512, bits, p.stages, p.T_own, p.S * p.CPC);
     cudaError_t e = stream_launch(var, p, stream_mt(mc), smem, stream);
     if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
   }
@@ -913,7 +940,7 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
     if (chunks.stages > 8) chunks.stages = 8;
     if (chunks.ctas_per_split > 0) {
       const int t_own = stream_tiles_owned(rows, N / BLOCK_N, chunks.ctas_per_split);
-      const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, device_info().max_smem);
+      const int fit = stream_stages_for(rows, K / pl.splits, var_bits(var), t_own, pl.splits * chunks.ctas_per_split, device_info().max_smem);
       if (fit < 1 && plan_stream(rows, N, K, var_bits(var), device_info(), &chunks) != ST_OK) return ST_UNSUPPORTED;
     }
     return run_stream(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, chunks);

@@ -38,10 +38,9 @@ constexpr size_t WS_HEADER_BYTES = 256;
 inline size_t ws_counter_bytes(int N) { return (((size_t)(N / BLOCK_N) * 4) + 255) / 256 * 256; }
 
 // ---- stream kernel (up to 16 rows per launch): item-balanced, ring-fed ------------------------------
-// Warps per CTA, one CTA per SM (M = 1, 4 bits, us per launch with 12 warps and two CTAs per SM / 16 / 20 / 24 warps:
-// 8192 x 8192 9.9 / 9.6 / 11.0 / 10.1, the four linears of a Llama-3-8B block 38.0 / 35.1 / 35.0 / 34.8).  The smallest calls,
-// one or two rows and at most 16 ring items per CTA, have half as many: most of 16 would only be started (1024 x 1024
-// 2.7 us with 8, 3.1 with 16).
+// Most warps per CTA, one CTA per SM (M = 1, 4 bits, us per launch with 12 warps and two CTAs per SM / 16 / 20 / 24 warps:
+// 8192 x 8192 9.9 / 9.6 / 11.0 / 10.1, the four linears of a Llama-3-8B block 38.0 / 35.1 / 35.0 / 34.8).  Small launches have
+// CTAs of half as many, one or two per SM (api.cu, stream_warp_shift and stream_paired_ctas).
 constexpr int STREAM_WARPS = 16;
 constexpr int STREAM_HEADER = STREAM_WARPS * 64;  // bytes of mbarriers in front of the rings: 8 slots of 8 bytes per warp
 constexpr int STREAM_SC_GROUPS = 16;  // groups per warp in the shared-memory scale cache (32 bytes each)

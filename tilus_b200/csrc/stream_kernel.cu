@@ -6,7 +6,8 @@
 // (cp.async.bulk, completion on an mbarrier per slot).  Weights and scales are constants, so
 // the ring is filled and the warp's scales are cached in shared memory before the kernel
 // waits for its predecessor in the stream (programmatic dependent launch).  A launch is one CTA of 16 warps per SM, as few CTAs as
-// finish as soon (T_own column tiles each, the last one what is left).  Two CTAs per SM, in a number that divides
+// finish as soon (T_own column tiles each, the last one what is left); small launches have CTAs of 8 warps, one or two per
+// SM (api.cu: stream_warp_shift, stream_paired_ctas).  For the others two CTAs per SM, of 12 warps, in a number that divides
 // the column tiles, left SMs idle or with one CTA where others had two, and staged the activations twice (M = 1, 4 bits, us: 6144 x
 // 4096 6.9 -> 5.4, 28672 x 4096 13.9 -> 12.7, 5120 x 5120 9.7 -> 6.3, 7168 x 2048 8.7 -> 4.8).  What a launch of M = 1 spends
 // now, 28672 x 4096, us: 0.3 from its predecessor's end to its start, 0.8 to the wait, 1.0 for the activations, 9.3
