@@ -331,10 +331,12 @@ def test_chained_host_calls_whose_last_cta_owns_fewer_column_tiles(m, n, k):
     calls.check()
 
 
-def test_host_calls_overlap_whether_or_not_the_last_cta_is_full():
-    """28672 columns leave the last CTA fewer column tiles than 28704 do: nothing is left over in either, so both fetch
-    their rows under the call before (13 us a call; 18 without)."""
-    chains = [_HostCalls(1, n, 4096, D.uint4b, 4, 40) for n in (28672, 28704)]
+@pytest.mark.parametrize("m,n,other", [(1, 28672, 28704), (9, 32768, 28672)])
+def test_host_calls_are_as_fast_as_those_of_a_similar_width(m, n, other):
+    """One row: 28672 columns leave the last CTA fewer column tiles than 28704 do; nothing is left over in either, so both fetch
+    their rows under the call before (13 us a call; 18 without).  Nine rows: 32768 columns on 128 CTAs (27 us, 28672 columns
+    25; 36 on 147 CTAs, whose warps end inside column tiles)."""
+    chains = [_HostCalls(m, width, 4096, D.uint4b, 4, 40) for width in (n, other)]
     best = [1e9, 1e9]
     for _ in range(6):
         for i, chain in enumerate(chains):
@@ -345,7 +347,7 @@ def test_host_calls_overlap_whether_or_not_the_last_cta_is_full():
             e1.record()
             torch.cuda.synchronize()
             best[i] = min(best[i], e0.elapsed_time(e1))
-    assert best[0] <= 1.2 * best[1], best
+    assert best[0] <= 1.25 * best[1], best
 
 
 @pytest.mark.parametrize("m,n,k,dt", [(4, 48, 14336, D.uint4b), (6, 32, 8192, D.uint4b), (5, 64, 13312, D.int3b), (1, 16, 20480, D.uint2b),

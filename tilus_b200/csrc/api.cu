@@ -221,10 +221,15 @@ static int stream_fetch_ctas(int M, int N, int K, int bits, const b200q_plan_t& 
   const int per_cta = (32 << stream_warp_shift(M, kc, bits, t_own, pl.splits * pl.ctas_per_split)) * 4;
   return (M * (K / 8) + per_cta - 1) / per_cta;
 }
-// CTAs per k chunk: the fewest that finish as soon as one per SM would
-static int stream_ctas_per_chunk(int NT, int s, const DeviceInfo& di) {
+// CTAs per k chunk: the fewest that finish as soon as one per SM would.  9 to 16 rows: a number near all SMs that divides the column
+// tiles, where there is one, since every warp then ends on the end of a tile and hands over its two sets of sums once (host
+// calls, 4 bits, us, such a number / the fewest: 9 x 8192 x 8192 23.6 / 29.0, 9 x 32768 x 4096 27.2 / 36.4, 16 x 16384 x 8192 53.9 / 58.9;
+// 9 x 28672 x 4096 25.1 / 25.0).
+static int stream_ctas_per_chunk(int m_pass, int NT, int s, const DeviceInfo& di) {
   const int full = di.sm_count / s;
   if (full < 1) return 0;
+  for (int c = full; m_pass > 8 && c * 5 >= full * 4; --c)
+    if (NT % c == 0) return c;
   const int t = (NT + full - 1) / full;
   return (NT + t - 1) / t;
 }
@@ -254,7 +259,7 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
   int best_s = 0, best_st = 0, best_c = 0;
   auto consider = [&](int s, int want, bool no_leftover, int smem, int cpc = 0) {
     if (best_s || KB % s) return;
-    if (cpc < 1) cpc = stream_ctas_per_chunk(NT, s, di);
+    if (cpc < 1) cpc = stream_ctas_per_chunk(m_pass, NT, s, di);
     if (cpc < 1) return;
     const int t_own = stream_tiles_owned(m_pass, NT, cpc);
     if (no_leftover && cpc * t_own < NT) return;
