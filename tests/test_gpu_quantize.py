@@ -104,3 +104,38 @@ def test_signed_codes_of_ordinary_and_special_weights(bits, kind, group):
     q = torch.where(q.isnan(), q.new_tensor(lo), q.clamp(lo, hi)).round().reshape(n, k)
     codes = (q.to(torch.int32) & ((1 << bits) - 1)).to(torch.uint8).t().contiguous()
     assert torch.equal(packed.cpu(), packing.interleave(codes.cpu(), dt))
+
+
+@pytest.mark.parametrize("n,k", [(16, 128), (48, 128), (80, 384), (16, 640), (144, 1152)])
+@pytest.mark.parametrize("dt", [D.int4b, D.uint3b, D.float6_e3m2], ids=lambda d: d.name)
+def test_groups_that_do_not_fill_the_last_block(n, k, dt):
+    """A block takes four 128-row groups, of several column tiles where their number is odd; the last block has fewer."""
+    w = (torch.randn(n, k, generator=torch.Generator().manual_seed(n + k)) * 0.1).half()
+    guard = torch.full((n * k * dt.nbits // 8 + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+    scales = torch.empty(k // 128, n, dtype=torch.float16, device="cuda")
+    packed, scales = quantize.quantize_and_pack(w.cuda(), dt, 128, out=(guard[: -4096], scales))
+    codes_ref, scales_ref = qo.quantize_weight(w.float().numpy(), dt, 128)
+    np.testing.assert_array_equal(scales.cpu().numpy().view(np.uint16), scales_ref.view(np.uint16))
+    assert torch.equal(packed.cpu(), packing.interleave(torch.from_numpy(codes_ref), dt))
+    assert bool((guard[-4096:] == 0x5a).all())
+
+
+def test_short_rows_take_no_longer_than_long_ones():
+    """The same weights as rows of 128 and of 512: all threads of a block have work in both (26 us; 31 with three quarters of
+    each block idle)."""
+    best = {}
+    dt, count = D.float6_e3m2, 65536 * 128
+    w = [(torch.randn(count, device="cuda") * 0.02).half() for _ in range(4)]
+    outs = {k: (torch.empty(count * 6 // 8, dtype=torch.uint8, device="cuda"), torch.empty(k // 128, count // k, dtype=torch.float16, device="cuda"))
+            for k in (128, 512)}
+    for _ in range(6):
+        for k, out in outs.items():
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(2_000_000)  # the launches queue up behind it
+            e0.record()
+            for i in range(24):
+                quantize.quantize_and_pack(w[i % 4].view(-1, k), dt, 128, out=out)
+            e1.record()
+            torch.cuda.synchronize()
+            best[k] = min(best.get(k, 1e9), e0.elapsed_time(e1))
+    assert best[128] <= 1.1 * best[512], best

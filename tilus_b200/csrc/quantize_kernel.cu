@@ -23,8 +23,11 @@
 // multiplication's error of a rounding boundary is computed again with the division: the codes are
 // those of the division in every case.  Signed types (signed_codes) need no clamping where the unit's largest weight
 // rounds inside the range, work on two values per instruction and pack 2, 4 and 8 bits in fp32.  fp16 [28672, 4096] ->
-// int4 g128: 94 us with clamping and bit packing per value and 1024 threads per SM, 64 us now with 2048 (68 with 1536,
-// 79 with 1024: a thread's loads are in flight for half of its life; 45 us at the copy rate of HBM).
+// int4 g128: 94 us with clamping and bit packing per value and 1024 threads per SM, 62 us now with 2048 (66 with 1536,
+// 79 with 1024: a thread's loads are in flight for half of its life; 45 us at the copy rate of HBM).  2048 threads leave 32
+// registers: the 16-bit builds of 3 and of 5 to 8 bits spill 12 .. 52 bytes to the stack and are still ahead of 1536 threads with 40
+// and no spills (28672 x 4096: int3 72 / 75 us, int5 69 / 71, int6 67 / 68, int7 71 / 72, int8 60 / 61; small layers up to 4 % behind,
+// 2048 x 2048, int8: 6.4 / 6.1).
 #include "common.cuh"
 
 namespace b200q {
@@ -300,13 +303,19 @@ __device__ __forceinline__ void put_pairs(const uint32_t (&code)[32], uint32_t (
 
 template <int WT, int B, bool FLOAT>
 __global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const QuantParams p) {
-  // unit index = ((nt * G + g) * 2 + half) * 32 + lane,  lane = r * 4 + j,  g = 128-row group of K.  A block has four groups
-  // of one 16-column tile (a division per thread costs as much as a quarter of its weights).
+  // unit index = ((nt * G + g) * 2 + half) * 32 + lane,  lane = r * 4 + j,  g = 128-row group of K.  A block has four groups,
+  // of one 16-column tile where G allows it (a 64-bit division per thread costs as much as a quarter of its weights).
   const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1;
-  const unsigned per_tile = (unsigned)(p.G + 3) / 4;
-  const int nt = (int)(blockIdx.x / per_tile), g = (int)(blockIdx.x - nt * per_tile) * 4 + (int)(threadIdx.x >> 6);
-  if (g >= p.G) return;  // whole warps
-  const long long unit = ((long long)nt * p.G + g) * 64 + (threadIdx.x & 63);
+  const unsigned grp = blockIdx.x * 4 + (threadIdx.x >> 6);
+  int nt;
+  if ((p.G & 3) == 0) {
+    nt = (int)(blockIdx.x / ((unsigned)p.G >> 2));
+  } else {
+    nt = (int)(grp / (unsigned)p.G);
+    if (nt >= p.N >> 4) return;  // whole warps
+  }
+  const int g = (int)(grp - (unsigned)nt * p.G);
+  const long long unit = (long long)grp * 64 + (threadIdx.x & 63);
   const int r = lane >> 2, j = lane & 3;
   const int n = nt * 16 + half * 8 + r;
   const int k0 = g * 128 + j * 32;
@@ -379,7 +388,7 @@ __global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const 
 template <int WT, int B, bool FLOAT>
 static cudaError_t pack_launch(const QuantParams& p, int nbits, cudaStream_t stream) {
   if (nbits == B) {
-    quant_pack_kernel<WT, B, FLOAT><<<(unsigned)(p.N / 16) * (unsigned)((p.G + 3) / 4), 256, 0, stream>>>(p);
+    quant_pack_kernel<WT, B, FLOAT><<<(unsigned)(((long long)(p.N / 16) * p.G + 3) / 4), 256, 0, stream>>>(p);
     return cudaGetLastError();
   }
   if constexpr (B < 8) return pack_launch<WT, B + 1, FLOAT>(p, nbits, stream);
