@@ -62,10 +62,12 @@ typedef struct b200q_plan {
                             in distributed shared memory (ctas_per_split = column tiles * cluster); else 1 */
   int32_t ctas_per_split;/* kernel 2: CTAs per k chunk, grid = splits * ctas_per_split; kernel 3: CTAs;
                             kernel 1: output tiles */
-  int32_t smem_bytes;    /* dynamic shared memory per CTA */
+  int32_t smem_bytes;    /* dynamic shared memory per CTA (output only); the stream kernel's is what a CTA uses, of which a launch may
+                            reserve more to keep its CTAs one or two to an SM */
   int32_t tile_m;        /* kernel 1: activation rows per CTA tile (32, 64, 128, 256 or 384); kernel 3: M rounded
                             up to 16; kernel 2: 0 for the stream kernel, 16 for the tcgen05 form */
-  int32_t stages;        /* pipeline depth (kernel 2: ring slots per warp, 1 .. 8, of which those that fit are used; kernel 1: activation stages;
+  int32_t stages;        /* pipeline depth (kernel 2: ring slots per warp, 1 .. 8, of which as many as fit are used;
+                            kernel 1: activation stages;
                             kernel 3: 128-row weight groups in the packed ring) */
   int32_t warps;         /* warps per CTA (output only) */
   int32_t passes;        /* launches: 2 when kernel 1 takes the multiple of 256 rows and kernel 2 the last 1..16 rows */

@@ -252,8 +252,8 @@ static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counte
 // [M, K/S] fits next to the rings; the grid is S * CPC.  Measured preferences, in this order: all of
 // K in one chunk with two ring slots per warp (the CTAs then write their own tiles without meeting
 // anybody in the global scratch); the fewest chunks with three slots and no column tiles left over
-// (left-over tiles are shared item-wise through the scratch, 40 % slower on the 28672-column layer
-// at M = 8); the fewest chunks with two slots and none left over; then whatever fits.
+// (left-over tiles are shared item-wise through the scratch: the linears of a Llama-3-8B block on 148 CTAs so, one row,
+// 41 us, 33 with whole tiles); the fewest chunks with two slots and none left over; then whatever fits.
 static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di, b200q_plan_t* pl) {
   const int KB = K / BLOCK_K, NT = N / BLOCK_N;
   int best_s = 0, best_st = 0, best_c = 0;
@@ -502,8 +502,13 @@ static void plan_prefill(int M, int N, int K, int var, int group, int max_tm, co
   pl->workspace_bytes = need;
 }
 
-// What the two rules below were fitted to: the split that the stream kernel took with 12 warps per CTA and half an SM each, the most k
-// chunks and CTAs of at most two per SM, a divisor of the column tiles.  Whether such a split exists still tells the shapes apart.
+// What the two rules below were fitted to: the split of an earlier form of the stream kernel (12 warps per CTA and half an SM each, the most
+// k chunks and CTAs of at most two per SM, a divisor of the column tiles), and its times.  They have not been fitted again to
+// the present form (stream_ctas_per_chunk, stream_paired_ctas), which is faster mostly where that split was a bad one.  Both kernels
+// forced now, fp16, 13 widths 1024 .. 28672 x 4 depths 2048 .. 8192: the kernel picked is behind the faster one by 6 / 12 / 7 / 10 / 10
+// / 6 % on average at 1 / 2 / 4 / 5 / 6 / 8 rows in 4 bits, by 3 % in 8 bits.  Nearly all of it is the stream kernel not being
+// picked, at worst 1 x 2560 x 2048 in 4 bits, 5.1 us for 3.2, 1 x 3584 x 4096 7.5 for 4.9, 5 x 1024 x 2048 5.7 for 4.4; the other way
+// 4 x 2048 x 5120 in 8 bits, 7.4 us for 6.6.
 struct PairSplit { int splits, ctas; };
 static PairSplit pair_split(int M, int NT, int KB, int bits, const DeviceInfo& di) {
   PairSplit best = {0, 0};
@@ -530,18 +535,17 @@ static PairSplit pair_split(int M, int NT, int KB, int bits, const DeviceInfo& d
   return best;
 }
 
-// A stream plan that cuts K and still has one CTA per SM at most (no divisor of the column tiles near two per SM): its
-// chunks meet in the scratch like the exact kernel's, at half the warps.  The exact kernel is then faster from two
-// rows on, and for one row from three chunks on; stream / exact, us, chains of cold launches, 4 bits: 7168 x 2048 (2
-// chunks) 9.5 / 8.7, 2448 x 11776 (23) 13.8 / 11.8, 3504 x 9728 (19) 14.9 / 12.3, 5120 x 5120 (2) 11.3 .. 11.8 / 11.6 and 10.9 at
-// one row; 3504 x 9728 in 8 bits 18.9 / 15.3.
+// Where that split cut K and still had one CTA per SM at most (no divisor of the column tiles near two per SM), its chunks met in the
+// scratch like the exact kernel's, at half the warps, and the exact kernel was faster from two rows on, for one row from three
+// chunks on (earlier form / exact, us, 4 bits: 7168 x 2048 9.5 / 8.7, 2448 x 11776 13.8 / 11.8, 5120 x 5120 11.3 .. 11.8 / 11.6).  The
+// present form does not cut K there: 4 x 7168 x 2048 5.5 / 7.0, 2 x 5120 x 5120 7.2 / 9.2.
 static bool stream_outrun(int M, const PairSplit& pl, const DeviceInfo& di) {
   return pl.splits > (M == 1 ? 2 : 1) && pl.splits * pl.ctas <= di.sm_count;
 }
 
-// fp16, 5..8 rows: the shapes where the stream kernel is still the faster one.  What the exact kernel pays is a start and
+// fp16, 5..8 rows: the shapes where the stream kernel's earlier form was the faster one.  What the exact kernel pays is a start and
 // an end of 5-6 us and, where equal runs share column tiles, sums in L2; what the stream kernel pays is the staging of the
-// activations, once per CTA, and a second pass through the scratch where it cuts K.  Measured, stream / exact, us, cold
+// activations, once per CTA, and a second pass through the scratch where it cuts K.  Measured, earlier form / exact, us, cold
 // chains, 11 types x 17 shapes x 5..8 rows:
 //  - two CTAs per SM without cutting K, layers of more than 12 M weights, up to 6 rows (4096 x 4096 at 5 rows: 4 bits 7.2 /
 //    7.9, float6 7.3 / 9.2), from 32 M weights up to 8 rows (32768 x 2048 at 8 rows: 4 bits 12.1 / 14.0); at 7 and 8 rows below
@@ -551,8 +555,7 @@ static bool stream_outrun(int M, const PairSplit& pl, const DeviceInfo& di) {
 //    again not between 4 M and 12 M (2048 x 4096 6.3 / 5.5);
 //  - up to 4 M float weights and 6 rows (1024 x 4096 at 5 rows, float8 4.8 / 6.2).
 // 8-bit integers, whose bytes the exact kernel takes with the fewest instructions, only from 32 M weights on (8192 x 2048 at 6
-// rows 7.7 / 6.5, 8192 x 4096 at 5 rows 10.9 / 11.8).  The choice costs 0.2 % against the better of the two over all
-// of them and is never more than 11 % behind the stream kernel (4096 x 8192 at 5 rows, 2 bits 8.6 / 9.5).
+// rows 7.7 / 6.5, 8192 x 4096 at 5 rows 10.9 / 11.8).
 static bool stream_ahead(int M, int N, int K, int var, const PairSplit& pl, const DeviceInfo& di) {
   const long long million = 1ll << 20, weights = (long long)N * K;
   if (M <= kStreamPlanRows) return true;
@@ -580,10 +583,10 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
     return st;
   }
   // Up to 4 rows the mma.sync stream kernel (to 8 rows where stream_ahead says so); above, the tcgen05 kernels, whose
-  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 36.8 / 40.0 / 45.8 /
-  // 52.9 / 53.0 us at 1 / 2 / 4 / 6 / 8 rows, the tcgen05 kernel 47.4 / 47.2 / 47.3 / 48.5 / 48.4; at 9 rows the former's
+  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 34.9 / 37.7 / 42.8 /
+  // 46.9 / 46.5 us at 1 / 2 / 4 / 6 / 8 rows, the tcgen05 kernel 48.2 / 48.7 / 48.9 / 49.8 / 50.2; at 9 rows the former's
   // second 8-row tile doubles its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
-  // kernel only a conversion of the activations: up to 8 rows the latter is 6 % faster (8192 x 8192, 4-bit).
+  // kernel only a conversion of the activations: at 8 rows the latter is 13 % faster (8192 x 8192, 4-bit, 14.0 / 16.1 us).
   if (M <= 8 && stream_takes(K, group)) {
     const PairSplit pair = pair_split(M, N / BLOCK_N, K / BLOCK_K, bits, di);
     if (pair.splits > 0 && !stream_outrun(M, pair, di) && (act == B200Q_BF16 || stream_ahead(M, N, K, var, pair, di)) &&
