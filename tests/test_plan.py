@@ -87,3 +87,15 @@ def test_small_decode_launches_have_ctas_of_eight_warps(m, n, k, w, ctas, warps)
     pl = ops.plan(m, n, k, w, 1 << (int(w[4]) - 1) if w[0] == "u" else 0, 128, act_dtype=torch.bfloat16)
     assert (pl["tile_m"], pl["splits"], pl["ctas_per_split"], pl["warps"]) == (0, 1, ctas, warps)
     assert pl["smem_bytes"] <= (113 if ctas > 148 else 227) * 1024
+
+
+@pytest.mark.parametrize("m,n,k,w,splits", [
+    (4, 1024, 14336, "uint4b", (4, 7, 14)), (3, 1024, 13824, "int8", (3, 9)), (6, 3072, 9216, "uint4b", (3, 6)), (6, 1536, 7168, "int8", (7,)),
+    (5, 2048, 14336, "uint4b", (4, 7)), (6, 8192, 8192, "uint4b", (2, 4)), (8, 4096, 4096, "uint4b", (4,)),
+    (4, 4096, 4096, "uint4b", (1,)), (6, 28672, 4096, "uint4b", (1,)), (5, 16384, 8192, "uint4b", (1,)), (2, 8192, 8192, "uint4b", (1,)),
+    (1, 1024, 14336, "uint4b", (1,))])
+def test_k_chunks_of_two_to_eight_rows(m, n, k, w, splits):
+    """Narrow layers with long rows are cut, which saves staging; wide ones are not.  Any of the numbers given is within 6 % of the
+    best that was timed."""
+    pl = ops.plan(m, n, k, w, 8 if w[0] == "u" else 0, 128, act_dtype=torch.bfloat16)
+    assert pl["tile_m"] == 0 and pl["splits"] in splits, pl

@@ -188,11 +188,12 @@ static int stream_tiles_owned(int m_pass, int NT, int cpc) {
 // share an SM (16 would leave the second one no registers).  At most 16 ring items per CTA: 8, since most of 16 would only be
 // started - for one and two rows always, for more rows as long as there is not much to stage, which 16 warps do faster (16 / 8 warps,
 // us, 4 bits: 4 x 1024 x 1024 3.60 / 3.34, 3 x 2048 x 1024 3.81 / 3.27, 8 x 8192 x 512 4.45 / 3.94; but 4 x 2048 x 2048 4.32 / 4.45; 2
-// bits, four items: 4 x 4096 x 1024 4.45 / 3.60, 4 x 2048 x 2048 4.62 / 4.41, two items: 8 x 1024 x 1024 4.37 / 4.54).
+// bits, four items: 4 x 4096 x 1024 4.45 / 3.60, 4 x 2048 x 2048 4.62 / 4.41, two items: 8 x 1024 x 1024 4.37 / 4.54; single bits, 14 items:
+// 6 x 16384 x 1024 5.30 / 5.96).
 static int stream_warp_shift(int m_pass, int kc, int bits, int t_own, int ctas) {
   if (stream_mt(m_pass) == 1 && ctas > device_info().sm_count) return 3;
   const int KBc = kc / BLOCK_K, items = t_own * KBc * (4 / stream_gi(bits));
-  if (t_own < 1 || items > 16 || m_pass > 8) return 4;
+  if (t_own < 1 || items > (m_pass <= 4 ? 16 : 8) || m_pass > 8) return 4;
   return m_pass <= 2 || m_pass * KBc <= (items == 3 || items == 4 ? 16 : 12) ? 3 : 4;
 }
 static int stream_smem(int m_pass, int kc, int bits, int stages, int t_own, int ctas) {
@@ -248,9 +249,17 @@ static int stream_paired_ctas(int m_pass, int NT, int K, int bits, const DeviceI
 static const int kStreamMaxRows = 16;  // what the kernel takes
 static const int kStreamPlanRows = 4;  // what the plan gives it at any shape (gather and host-buffer launches: all of the above)
 static size_t stream_workspace_bytes(int N) { return WS_HEADER_BYTES + ws_counter_bytes(N) + (size_t)16 * N * sizeof(float); }
+// What a number of k chunks costs a launch of 2 to 8 rows, in activations that a CTA stages (82 us per million): those of its chunk, and
+// with several chunks 9500 for meeting in the scratch and 0.075 for each sum that goes through it.  Fitted to all divisors
+// of K up to 16 forced at 622 shapes (1024 .. 57344 columns, K = 2048 .. 14336, 2, 4 and 8 bits): the choice is behind the best one by 0.7 % on
+// average and 14 % at most.  What it replaced - one chunk where it fits, at 7 and 8 rows half of the shared memory - was 7 % behind
+// on average, 68 % at most (us, that / now: 4 x 1024 x 14336, 4 bits 11.0 / 6.6, 6 x 3072 x 9216 12.5 / 8.1, 6 x 8192 x 8192 14.6 / 12.3).
+static double stream_chunk_cost(int m_pass, int N, int K, int s) {
+  return (double)m_pass * K / s + (s > 1 ? 9500.0 + 0.075 * N * m_pass * s : 0.0);
+}
 // K is cut into S chunks (a divisor of K/512, at most one per SM) so that the activation chunk
-// [M, K/S] fits next to the rings; the grid is S * CPC.  Measured preferences, in this order: all of
-// K in one chunk with two ring slots per warp (the CTAs then write their own tiles without meeting
+// [M, K/S] fits next to the rings; the grid is S * CPC.  2 to 8 rows: the number with the least of what depends on it, see
+// stream_chunk_cost.  Otherwise, measured preferences, in this order: all of K in one chunk with two ring slots per warp (the CTAs then write their own tiles without meeting
 // anybody in the global scratch); the fewest chunks with three slots and no column tiles left over
 // (left-over tiles are shared item-wise through the scratch: the linears of a Llama-3-8B block on 148 CTAs so, one row,
 // 41 us, 33 with whole tiles); the fewest chunks with two slots and none left over; then whatever fits.
@@ -263,9 +272,6 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
     if (cpc < 1) return;
     const int t_own = stream_tiles_owned(m_pass, NT, cpc);
     if (no_leftover && cpc * t_own < NT) return;
-    // (a CTA that would stage more than 64 KB of activations, 1.75 times the bytes of its weights: shorter chunks.  5 x 2048 x 8192,
-    // 2 bits, 1 / 2 chunks: 8.8 / 8.1 us; 4 x 4096 x 14336, single bits, 12.8 / 11.7; but 4 x 2048 x 2048, 2 bits, 4.7 / 6.0)
-    if (no_leftover && m_pass > 2 && m_pass * (KB / s) > 64 && 4 * m_pass > 7 * t_own * bits) return;
     const int st = stream_stages_for(m_pass, (KB / s) * 512, bits, t_own, s * cpc, smem);
     if (st < want) return;
     best_s = s; best_st = st; best_c = cpc;
@@ -273,17 +279,22 @@ static int plan_stream(int m_pass, int N, int K, int bits, const DeviceInfo& di,
     if (best_st > ring) best_st = ring > want ? ring : want;
   };
   const int s_max = KB < di.sm_count ? KB : di.sm_count;
-  // 7 and 8 rows: chunks that leave half of the shared memory, since every CTA stages all rows of its chunk (4096 x 4096, 1 / 4
-  // chunks: 8 rows of 4 bits 8.0 / 7.35 us, of 8 bits 9.3 / 8.5; 5 rows of 4 bits 7.0 / 7.4).  Not up to 2048 rows of weights, where
-  // the sums through the scratch cost more than the staging (1 / 2 chunks, 8 rows, bfloat16, 4 bits: 8192 x 2048 6.9 / 7.6 us, 28672 x
-  // 2048 11.2 / 14.5, of 8 bits 14.4 / 17.9; 2048 and 4096 columns within 3 %)
-  const int most = (m_pass == 7 || m_pass == 8) && KB > 4 ? kStreamSmemCap : di.max_smem;
   const int pairs = stream_paired_ctas(m_pass, NT, K, bits, di);
   if (pairs) consider(1, 2, true, kStreamSmemCap, pairs);
+  if (m_pass >= 2 && m_pass <= 8 && !best_s) {
+    int cheapest = 0;
+    for (int s = 1; s <= s_max; ++s) {
+      if (cheapest && stream_chunk_cost(m_pass, N, K, s) >= stream_chunk_cost(m_pass, N, K, cheapest)) continue;
+      consider(s, 2, true, di.max_smem);
+      if (best_s) cheapest = s;
+      best_s = 0;
+    }
+    if (cheapest) consider(cheapest, 2, true, di.max_smem);
+  }
   consider(1, 2, true, kStreamSmemCap);
-  consider(1, 2, true, most);
-  for (int s = 1; s <= s_max; ++s) consider(s, 3, true, most);
-  for (int s = 1; s <= s_max; ++s) consider(s, 2, true, most);
+  consider(1, 2, true, di.max_smem);
+  for (int s = 1; s <= s_max; ++s) consider(s, 3, true, di.max_smem);
+  for (int s = 1; s <= s_max; ++s) consider(s, 2, true, di.max_smem);
   for (int want = 3; want >= 1; --want)
     for (int s = 1; s <= s_max; ++s) consider(s, want, false, di.max_smem);
   if (!best_s) return ST_UNSUPPORTED;
