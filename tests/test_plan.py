@@ -77,9 +77,9 @@ def test_seven_and_eight_rows_do_not_cut_short_layers(m, n, w):
 
 
 @pytest.mark.parametrize("m,n,k,w,ctas,warps", [
-    (1, 16384, 1024, "uint2b", 256, 8), (2, 16384, 1024, "uint4b", 256, 8), (4, 8192, 1024, "uint2b", 256, 8), (1, 12288, 2048, "uint2b", 256, 8),
+    (1, 16384, 1024, "uint2b", 256, 8), (2, 16384, 1024, "uint4b", 256, 8), (4, 16384, 1024, "uint4b", 256, 8), (8, 16384, 512, "uint4b", 256, 8), (1, 12288, 2048, "uint2b", 256, 8),
     (1, 8192, 1024, "int8", 256, 8), (1, 12288, 1536, "int5b", 256, 8),  # two CTAs of 8 warps per SM
-    (4, 1024, 1024, "uint4b", 64, 8), (3, 2048, 1024, "uint4b", 128, 8), (5, 8192, 512, "uint2b", 128, 8),  # one, with little to stage
+    (4, 1024, 1024, "uint4b", 64, 8), (3, 2048, 1024, "uint4b", 128, 8), (5, 8192, 512, "uint2b", 128, 8), (4, 8192, 1024, "uint2b", 128, 8),  # one, with little to stage
     (1, 16384, 2048, "int8", 147, 16), (4, 4096, 2048, "uint4b", 128, 16), (1, 5120, 4096, "int3b", 107, 16),  # beyond those lines
     (8, 1024, 1024, "uint2b", 64, 16), (1, 8192, 8192, "uint4b", 128, 16)])
 def test_small_decode_launches_have_ctas_of_eight_warps(m, n, k, w, ctas, warps):

@@ -186,14 +186,14 @@ static int stream_tiles_owned(int m_pass, int NT, int cpc) {
 }
 // log2 of the warps of a CTA that owns t_own tiles of kc rows, in a launch of `ctas` CTAs.  Launches of more CTAs than SMs: 8, of which two
 // share an SM (16 would leave the second one no registers).  At most 16 ring items per CTA: 8, since most of 16 would only be
-// started - for one and two rows always, for more rows as long as there is not much to stage, which 16 warps do faster (16 / 8 warps,
-// us, 4 bits: 4 x 1024 x 1024 3.60 / 3.34, 3 x 2048 x 1024 3.81 / 3.27, 8 x 8192 x 512 4.45 / 3.94; but 4 x 2048 x 2048 4.32 / 4.45; 2
-// bits, four items: 4 x 4096 x 1024 4.45 / 3.60, 4 x 2048 x 2048 4.62 / 4.41, two items: 8 x 1024 x 1024 4.37 / 4.54; single bits, 14 items:
-// 6 x 16384 x 1024 5.30 / 5.96).
+// started - for one and two rows always, for more rows with at most 8 items and as long as there is not much to stage, which 16 warps
+// do faster (16 / 8 warps, us, 4 bits: 4 x 1024 x 1024 3.60 / 3.34, 3 x 2048 x 1024 3.81 / 3.27, 8 x 8192 x 512 4.45 / 3.94; but 4 x
+// 2048 x 2048 4.32 / 4.45; 2 bits, four items: 4 x 4096 x 1024 4.45 / 3.60, 4 x 2048 x 2048 4.62 / 4.41, two items: 8 x 1024 x 1024 4.37
+// / 4.54; single bits, 14 items: 6 x 16384 x 1024 5.30 / 5.96).
 static int stream_warp_shift(int m_pass, int kc, int bits, int t_own, int ctas) {
   if (stream_mt(m_pass) == 1 && ctas > device_info().sm_count) return 3;
   const int KBc = kc / BLOCK_K, items = t_own * KBc * (4 / stream_gi(bits));
-  if (t_own < 1 || items > (m_pass <= 4 ? 16 : 8) || m_pass > 8) return 4;
+  if (t_own < 1 || items > (m_pass <= 2 ? 16 : 8) || m_pass > 8) return 4;
   return m_pass <= 2 || m_pass * KBc <= (items == 3 || items == 4 ? 16 : 12) ? 3 : 4;
 }
 static int stream_smem(int m_pass, int kc, int bits, int stages, int t_own, int ctas) {
@@ -236,15 +236,20 @@ static int stream_ctas_per_chunk(int m_pass, int NT, int s, const DeviceInfo& di
 }
 // Small layers, few rows: two CTAs of 8 warps per SM, each with its own share of the column tiles, which start, wait and finish beside
 // each other.  For rings that one CTA fills for most of its life: column tiles of at most 21 KB, or layers of 8 MB in all, 8-bit types
-// only the latter, activations of at most 8 KB, and not where two equal shares make the fullest SM do an eighth more.  M = 1, us, one CTA of
+// only the latter, activations of at most 12 KB, not where two equal shares make the fullest SM do an eighth more, and from three rows on
+// not where one CTA would have 8 warps.  M = 1, us, one CTA of
 // 16 warps / two of 8: 16384 x 1024, 4 bits 5.0 / 4.4, 2 bits 4.4 / 4.0; 12288 x 2048, 2 bits 5.7 / 5.0; 8192 x 2048, 4 bits 4.9 / 4.5;
 // 12288 x 1536, 5 bits 7.4 / 6.2; 8192 x 1024, 8 bits 4.7 / 4.4; 4096 x 4096, 4 bits 5.1 / 4.9.  Beyond those lines: 14336 x 4096, 4 bits
-// 9.0 / 9.3; 16384 x 2048, 8 bits 8.5 / 8.8; 4 x 4096 x 2048, 4 bits 4.7 / 5.0; 5120 x 4096, 3 bits (two tiles on 160 CTAs) 6.6 / 8.0.
+// 9.0 / 9.3; 16384 x 2048, 8 bits 8.5 / 8.8; 4 x 4096 x 2048, 4 bits 4.7 / 5.0; 5120 x 4096, 3 bits (two tiles on 160 CTAs) 6.6 / 8.0;
+// 8 x 8192 x 512, single bits (8 warps) 4.3 / 4.5.  More rows: 3 x 12288 x 2048, 2 bits 6.4 / 6.0; 6 x 16384 x 1024, 4 bits 6.2 / 5.8; 8 x
+// 16384 x 512 5.2 / 5.0; 4 x 16384 x 1536 7.0 / 6.6.
 static int stream_paired_ctas(int m_pass, int NT, int K, int bits, const DeviceInfo& di) {
   const int tile = 2 * K * bits;  // bytes
-  if (m_pass > 4 || m_pass * (K / BLOCK_K) > 8 || ((bits == 8 || tile > 21 << 10) && (long long)NT * tile > 8 << 20)) return 0;
+  if (m_pass > 8 || m_pass * (K / BLOCK_K) > 12 || ((bits == 8 || tile > 21 << 10) && (long long)NT * tile > 8 << 20)) return 0;
   const int t = (NT + 2 * di.sm_count - 1) / (2 * di.sm_count), ctas = (NT + t - 1) / t;
-  return ctas > di.sm_count && 2 * t * 7 <= (NT + di.sm_count - 1) / di.sm_count * 8 ? ctas : 0;
+  const int t1 = (NT + di.sm_count - 1) / di.sm_count, ctas1 = (NT + t1 - 1) / t1;
+  if (m_pass > 2 && stream_warp_shift(m_pass, K, bits, t1, ctas1) == 3) return 0;
+  return ctas > di.sm_count && 2 * t * 7 <= t1 * 8 ? ctas : 0;
 }
 static const int kStreamMaxRows = 16;  // what the kernel takes
 static const int kStreamPlanRows = 4;  // what the plan gives it at any shape (gather and host-buffer launches: all of the above)
