@@ -235,17 +235,19 @@ static int stream_ctas_per_chunk(int m_pass, int NT, int s, const DeviceInfo& di
   return (NT + t - 1) / t;
 }
 // Small layers, few rows: two CTAs of 8 warps per SM, each with its own share of the column tiles, which start, wait and finish beside
-// each other.  For rings that one CTA fills for most of its life: column tiles of at most 21 KB, or layers of 8 MB in all, 8-bit types
-// only the latter, activations of at most 12 KB, not where two equal shares make the fullest SM do an eighth more, and from three rows on
-// not where one CTA would have 8 warps.  M = 1, us, one CTA of
-// 16 warps / two of 8: 16384 x 1024, 4 bits 5.0 / 4.4, 2 bits 4.4 / 4.0; 12288 x 2048, 2 bits 5.7 / 5.0; 8192 x 2048, 4 bits 4.9 / 4.5;
-// 12288 x 1536, 5 bits 7.4 / 6.2; 8192 x 1024, 8 bits 4.7 / 4.4; 4096 x 4096, 4 bits 5.1 / 4.9.  Beyond those lines: 14336 x 4096, 4 bits
-// 9.0 / 9.3; 16384 x 2048, 8 bits 8.5 / 8.8; 4 x 4096 x 2048, 4 bits 4.7 / 5.0; 5120 x 4096, 3 bits (two tiles on 160 CTAs) 6.6 / 8.0;
-// 8 x 8192 x 512, single bits (8 warps) 4.3 / 4.5.  More rows: 3 x 12288 x 2048, 2 bits 6.4 / 6.0; 6 x 16384 x 1024, 4 bits 6.2 / 5.8; 8 x
-// 16384 x 512 5.2 / 5.0; 4 x 16384 x 1536 7.0 / 6.6.
+// each other.  For rings that one CTA fills for most of its life: column tiles of at most 21 KB, or up to 2048 rows layers of 8 MB in
+// all, 8-bit types only the latter; activations of at most 12 KB; not where two equal shares make the fullest SM do an eighth more;
+// from three rows on not where one CTA would have 8 warps.  us, one CTA of 16 warps / two of 8: M = 1: 16384 x 1024, 4 bits 5.0 / 4.4, 2
+// bits 4.4 / 4.0; 12288 x 2048, 2 bits 5.7 / 5.0; 8192 x 2048, 4 bits 4.9 / 4.5; 12288 x 1536, 5 bits 7.4 / 6.2; 8192 x 1024, 8 bits 4.7
+// / 4.4; more rows: 3 x 12288 x 2048, 2 bits 6.4 / 6.0; 6 x 16384 x 1024, 4 bits 6.2 / 5.8; 8 x 16384 x 512 5.2 / 5.0; 4 x 16384 x 1536
+// 7.0 / 6.6.  Beyond those lines: 14336 x 4096, 4 bits 9.0 / 9.3; 4096 x 4096 5.1 / 4.9 in a chain of its own, but 0.2 us more among
+// the other linears of a block; 16384 x 2048, 8 bits 8.5 / 8.8; 4 x 4096 x 2048, 4 bits 4.7 / 5.0; 5120 x 4096, 3 bits (two tiles on 160
+// CTAs) 6.6 / 8.0; 8 x 8192 x 512, single bits (8 warps) 4.3 / 4.5.
 static int stream_paired_ctas(int m_pass, int NT, int K, int bits, const DeviceInfo& di) {
   const int tile = 2 * K * bits;  // bytes
-  if (m_pass > 8 || m_pass * (K / BLOCK_K) > 12 || ((bits == 8 || tile > 21 << 10) && (long long)NT * tile > 8 << 20)) return 0;
+  if (m_pass > 8 || m_pass * (K / BLOCK_K) > 12) return 0;
+  if (tile > 21 << 10 && K > 2048) return 0;
+  if ((bits == 8 || tile > 21 << 10) && (long long)NT * tile > 8 << 20) return 0;
   const int t = (NT + 2 * di.sm_count - 1) / (2 * di.sm_count), ctas = (NT + t - 1) / t;
   const int t1 = (NT + di.sm_count - 1) / di.sm_count, ctas1 = (NT + t1 - 1) / t1;
   if (m_pass > 2 && stream_warp_shift(m_pass, K, bits, t1, ctas1) == 3) return 0;
