@@ -524,9 +524,10 @@ static void plan_prefill(int M, int N, int K, int var, int group, int max_tm, co
 // k chunks and CTAs of at most two per SM, a divisor of the column tiles), and its times.  They have not been fitted again to
 // the present form (stream_ctas_per_chunk, stream_paired_ctas), which is faster mostly where that split was a bad one.  Both kernels
 // forced now, fp16, 13 widths 1024 .. 28672 x 4 depths 2048 .. 8192: the kernel picked is behind the faster one by 6 / 12 / 7 / 10 / 10
-// / 6 % on average at 1 / 2 / 4 / 5 / 6 / 8 rows in 4 bits, by 3 % in 8 bits.  Nearly all of it is the stream kernel not being
+// / 6 % on average at 1 / 2 / 4 / 5 / 6 / 8 rows in 4 bits, by 2 to 3 % in 8 bits.  Nearly all of it is the stream kernel not being
 // picked, at worst 1 x 2560 x 2048 in 4 bits, 5.1 us for 3.2, 1 x 3584 x 4096 7.5 for 4.9, 5 x 1024 x 2048 5.7 for 4.4; the other way
-// 4 x 2048 x 5120 in 8 bits, 7.4 us for 6.6.
+// 4 x 2048 x 5120 in 8 bits, 7.2 us for 6.5.  (Speed is not all there is to it: the stream kernel stages fp16 activations times 2^-T, T up to
+// 10 - bits, so that those below 2^(T-14) lose low bits there and not in the exact kernel.)
 struct PairSplit { int splits, ctas; };
 static PairSplit pair_split(int M, int NT, int KB, int bits, const DeviceInfo& di) {
   PairSplit best = {0, 0};
@@ -601,10 +602,10 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
     return st;
   }
   // Up to 4 rows the mma.sync stream kernel (to 8 rows where stream_ahead says so); above, the tcgen05 kernels, whose
-  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 34.9 / 37.7 / 42.8 /
-  // 46.9 / 46.5 us at 1 / 2 / 4 / 6 / 8 rows, the tcgen05 kernel 48.2 / 48.7 / 48.9 / 49.8 / 50.2; at 9 rows the former's
+  // cost hardly depends on the rows.  A Llama-3-8B block of linears (4-bit) takes the stream kernel 34.6 / 38.6 / 41.1 /
+  // 44.9 / 45.7 us at 1 / 2 / 4 / 6 / 8 rows, the tcgen05 kernel 48.6 / 48.8 / 48.8 / 49.9 / 49.8; at 9 rows the former's
   // second 8-row tile doubles its staging and MMAs.  bfloat16 costs the exact kernel one more half instruction per pair of weights and the stream
-  // kernel only a conversion of the activations: at 8 rows the latter is 13 % faster (8192 x 8192, 4-bit, 14.0 / 16.1 us).
+  // kernel only a conversion of the activations: at 8 rows the latter is 22 % faster (8192 x 8192, 4-bit, 12.6 / 16.1 us).
   if (M <= 8 && stream_takes(K, group)) {
     const PairSplit pair = pair_split(M, N / BLOCK_N, K / BLOCK_K, bits, di);
     if (pair.splits > 0 && !stream_outrun(M, pair, di) && (act == B200Q_BF16 || stream_ahead(M, N, K, var, pair, di)) &&

@@ -13,8 +13,8 @@
 // now, 28672 x 4096, us: 0.3 from its predecessor's end to its start, 0.8 to the wait, 1.0 for the activations, 9.3
 // for the weights (6.5 TB/s), 0.7 for the outputs and the spread of the CTAs.  Launches that share an SM, so that one's start
 // lies under the other's end, measured slower: nothing keeps two CTAs of the later one off the SM that empties first.
-// K is cut into S chunks when the activation chunk [M, K/S] would not fit next to the rings; a CTA works
-// inside one chunk.
+// K is cut into S chunks where that saves more staging than it costs, or where the activation chunk [M, K/S] would not
+// fit next to the rings (api.cu, plan_stream); a CTA works inside one chunk.
 //
 // Compute.  One 128-row group at a time.  A lane reads its two units (columns r and r+8, 32
 // rows each) with one vector load per unit, turns them into tensor-core operands with the
