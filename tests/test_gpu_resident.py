@@ -1,0 +1,135 @@
+"""The decode kernel with the activations in registers, where its split of the work can go wrong."""
+import pytest
+import torch
+
+from tilus_b200 import dtypes as D
+from tilus_b200 import ops
+from tilus_b200.variants import supported_weight_dtypes
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(M, N, K, dt, group, act=torch.float16, mean=0.0, seed=0):
+    dev = torch.device("cuda:0")
+    gen = torch.Generator(device=dev).manual_seed(seed)
+    zp = 1 << (dt.nbits - 1) if dt.kind == D.KIND_UINT else 0
+    bq = torch.randint(0, 256, (N * K * dt.nbits // 8,), dtype=torch.uint8, device=dev, generator=gen)
+    if dt.is_float() and dt.exponent_nbits == 5:
+        bq &= 0xBF  # no Inf / NaN patterns
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).to(act)
+    a = (torch.randn(M, K, device=dev, generator=gen) + mean).to(act)
+    values = ops.dequantize(bq, torch.ones(1, N, dtype=torch.float16, device=dev), dt, K, zp).double()  # exact in fp16
+    ref = a.double() @ (values * sc.double().repeat_interleave(group, 0))
+    return a, bq, sc, zp, ref
+
+
+def _close(c, ref):
+    """No weight is rounded: one rounding of the output (2^-11, bfloat16 2^-8) and the fp32 sums, whose terms are up to
+    a hundred times the result where the activations have a mean (a few 2^-24 of them: 2e-5 of the largest result)."""
+    eps = 2.0 ** -11 if c.dtype == torch.float16 else 2.0 ** -8
+    return bool(((c.double() - ref).abs() <= eps * ref.abs() + 2e-5 * ref.abs().max()).all())
+
+
+def _run(a, bq, sc, dt, zp, group, S, ws, out=None):
+    N, K = sc.shape[1], a.shape[1]
+    assert ops.plan(a.shape[0], N, K, dt, zp, group, act_dtype=a.dtype)["kernel"] in (2, 3)
+    return ops.quantized_matmul(a, bq, sc, dt, group, zp, workspace=ws, plan_override=dict(resident=S), out=out)
+
+
+def _check(M, N, K, dt, group, S, act=torch.float16, mean=0.0):
+    a, bq, sc, zp, ref = _problem(M, N, K, dt, group, act, mean, seed=M + N)
+    ws = torch.zeros(max(ops.workspace_bytes(M, N, K, dt, zp, group), 1 << 16), dtype=torch.uint8, device=a.device)
+    c = _run(a, bq, sc, dt, zp, group, S, ws)
+    assert _close(c, ref)
+    assert torch.equal(_run(a, bq, sc, dt, zp, group, S, ws), c)  # the sums are added in order
+    assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("dt", supported_weight_dtypes(), ids=lambda d: d.name)
+@pytest.mark.parametrize("M,K,S", [(5, 1024, 1), (16, 1152, 1), (8, 7168, 1), (3, 2432, 4)])
+def test_every_weight_type(dt, M, K, S):
+    _check(M, 1040, K, dt, 128, S, mean=3.0 if M == 5 else 0.0)
+
+
+@pytest.mark.parametrize("M,N,K,group,S", [
+    (1, 16, 128, 128, 1),          # one group of one tile: one warp has work
+    (2, 16, 512, 512, 4),          # a cluster with one group each
+    (8, 32, 8192, 128, 1),         # four groups per warp
+    (8, 2368, 4096, 4096, 1),      # a tile per SM, one scale per column
+    (7, 2384, 5120, 128, 1),       # two tiles, the last CTA one; some warps with a third group
+    (4, 28672, 1024, 256, 1),      # sets of warps that take turns with 13 tiles
+    (1, 14336, 2048, 128, 1),      # two sets with four and three tiles
+    (16, 6144, 4096, 128, 1),      # 16 rows, three tiles
+    (9, 4112, 2048, 1024, 1),      # 9 rows, the last CTA with one tile
+    (16, 2064, 2176, 128, 2),      # 16 rows in clusters, 8.5 groups per CTA
+    (8, 4096, 14336, 128, 4),
+    (6, 4096, 14336, 7168, 2),     # seven groups for two warps
+    (8, 75776, 1024, 128, 1),      # 32 tiles per CTA
+    (3, 16400, 11008, 128, 2),     # 86 groups
+])
+def test_splits(M, N, K, group, S):
+    _check(M, N, K, D.uint4b, group, S)
+
+
+@pytest.mark.parametrize("M,K,S", [(1, 4096, 1), (8, 2048, 1), (8, 8192, 2), (5, 7680, 1)])
+def test_bfloat16(M, K, S):
+    _check(M, 1040, K, D.int4b, 128, S, act=torch.bfloat16)
+
+
+def test_bfloat16_out_of_range():
+    """Magnitudes that fp16 does not have saturate (infinities too); NaN stays NaN."""
+    a, bq, sc, zp, _ = _problem(4, 64, 1024, D.int4b, 128, torch.bfloat16)
+    a[0, 5], a[1, 7], a[2, 9] = 1e6, float("inf"), float("nan")
+    c = ops.quantized_matmul(a, bq, sc, D.int4b, 128, zp, plan_override=dict(resident=1))
+    b = a.clone()
+    b[0, 5] = b[1, 7] = 65504.0
+    ref = b.double() @ ops.dequantize(bq, sc, D.int4b, 128, zp).double()
+    assert float((c - ref)[[0, 1, 3]].abs().max() / ref[[0, 1, 3]].abs().max()) <= 2.0 ** -7
+    assert bool(c[2].isnan().all())
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -20, 2.0 ** -9, 400.0])
+def test_activations_of_any_magnitude_are_multiplied_as_they_are(scale):
+    """No power of two is taken off the activations beforehand: small fp16 values keep their bits."""
+    a, bq, sc, zp, _ = _problem(3, 272, 2048, D.uint4b, 128)
+    a = (a.float() * scale).half()
+    sc = sc.float().div(scale if scale < 1 else 1).clamp(max=60000).half()
+    values = ops.dequantize(bq, torch.ones(1, 272, dtype=torch.float16, device=a.device), D.uint4b, 2048, zp).double()
+    ref = a.double() @ (values * sc.double().repeat_interleave(128, 0))
+    assert _close(ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=dict(resident=1)), ref)
+
+
+@pytest.mark.parametrize("M,gap", [(1, 1), (8, 3), (16, 8)])
+def test_outputs_inside_a_wider_tensor(M, gap):
+    a, bq, sc, zp, ref = _problem(M, 272, 1024, D.uint4b, 128)
+    wide = torch.full((M, 272 + gap), 7.0, dtype=torch.float16, device=a.device)
+    ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, out=wide[:, :272], plan_override=dict(resident=1))
+    assert _close(wide[:, :272], ref) and bool((wide[:, 272:] == 7.0).all())
+
+
+def test_edits_of_other_fields_leave_the_kernel():
+    a, bq, sc, zp, ref = _problem(8, 4096, 4096, D.uint4b, 128)
+    pl = ops.plan(8, 4096, 4096, D.uint4b, zp, 128)
+    assert pl["resident"] == 1
+    c = ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp)
+    assert torch.equal(ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=pl), c)
+    for edit in (dict(resident=0), dict(splits=2), dict(stages=2, ctas_per_split=100), dict(kernel=3, tile_m=16, splits=1, ctas_per_split=90)):
+        assert float((ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=edit).double() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    rows = torch.randn(20, 4096, device=a.device).half()  # a plan put on more rows than the kernel takes
+    got = ops.quantized_matmul(rows, bq, sc, D.uint4b, 128, zp, plan_override=pl)
+    want = rows.float() @ ops.dequantize(bq, sc, D.uint4b, 128, zp).float()
+    assert float((got.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,N,K,dt", [
+    (1, 2384, 1024, D.int8), (1, 5120, 1536, D.int3b), (2, 11008, 1024, D.uint8), (1, 16, 512, D.uint4b), (3, 12112, 1024, D.int5b),
+    (4, 1040, 1024, D.float6_e3m2), (4, 160000, 512, D.uint1b), (8, 4096, 4096, D.uint4b), (1, 28672, 8192, D.uint4b),
+    (8, 6144, 4096, D.uint4b), (16, 4096, 4096, D.int8), (12, 2064, 1152, D.uint2b), (5, 1040, 1408, D.float6_e3m2)], ids=str)
+def test_the_kernels_beside_it(M, N, K, dt):
+    """The stream and exact kernels at shapes that the table gives to this one: other callers (host buffers, gathers,
+    edited plans) still have them."""
+    a, bq, sc, zp, ref = _problem(M, N, K, dt, 128)
+    ws = torch.zeros(max(ops.workspace_bytes(M, N, K, dt, zp, 128), 1 << 16), dtype=torch.uint8, device=a.device)
+    for _ in range(2):
+        assert _close(_run(a, bq, sc, dt, zp, 128, 0, ws), ref)
+        assert int(ws.count_nonzero()) == 0

@@ -55,7 +55,7 @@ class Plan(ctypes.Structure):
         ("warps", ctypes.c_int32),
         ("passes", ctypes.c_int32),
         ("pdl", ctypes.c_int32),
-        ("reserved", ctypes.c_int32),
+        ("resident", ctypes.c_int32),
         ("workspace_bytes", ctypes.c_uint64),
     ]
 

@@ -45,6 +45,8 @@ def _jobs():
     for part in range(NPARTS):
         jobs.append(("stream_kernel.cu", f"stream_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
     for part in range(NPARTS):
+        jobs.append(("resident_kernel.cu", f"resident_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
+    for part in range(NPARTS):
         jobs.append(("batch_kernel.cu", f"batch_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))
     for part in range(NPARTS):
         jobs.append(("exact_kernel.cu", f"exact_part{part}.o", [f"-DB200Q_NPARTS={NPARTS}", f"-DB200Q_PART={part}"]))

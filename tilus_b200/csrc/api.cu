@@ -42,6 +42,10 @@ B200Q_DECL_BPART(4) B200Q_DECL_BPART(5) B200Q_DECL_BPART(6) B200Q_DECL_BPART(7)
   cudaError_t exact_launch_part##i(int, const BatchParams&, const void*, int, cudaStream_t);
 B200Q_DECL_EPART(0) B200Q_DECL_EPART(1) B200Q_DECL_EPART(2) B200Q_DECL_EPART(3)
 B200Q_DECL_EPART(4) B200Q_DECL_EPART(5) B200Q_DECL_EPART(6) B200Q_DECL_EPART(7)
+#define B200Q_DECL_RPART(i) \
+  cudaError_t resident_launch_part##i(int, const ResidentParams&, int, int, int, cudaStream_t);
+B200Q_DECL_RPART(0) B200Q_DECL_RPART(1) B200Q_DECL_RPART(2) B200Q_DECL_RPART(3)
+B200Q_DECL_RPART(4) B200Q_DECL_RPART(5) B200Q_DECL_RPART(6) B200Q_DECL_RPART(7)
 int exact_smem_bytes(int bits, int stages, int M);
 int exact_stages(int bits, int max_smem, int M);
 int batch_max_clusters(int c);
@@ -62,6 +66,19 @@ static cudaError_t stream_launch(int var, const StreamParams& p, int mt, int sme
     case 5: return stream_launch_part5(var, p, mt, smem, s);
     case 6: return stream_launch_part6(var, p, mt, smem, s);
     default: return stream_launch_part7(var, p, mt, smem, s);
+  }
+}
+
+static cudaError_t resident_launch(int var, const ResidentParams& p, int mt, int ng, int smem, cudaStream_t s) {
+  switch (var % B200Q_NPARTS) {
+    case 0: return resident_launch_part0(var, p, mt, ng, smem, s);
+    case 1: return resident_launch_part1(var, p, mt, ng, smem, s);
+    case 2: return resident_launch_part2(var, p, mt, ng, smem, s);
+    case 3: return resident_launch_part3(var, p, mt, ng, smem, s);
+    case 4: return resident_launch_part4(var, p, mt, ng, smem, s);
+    case 5: return resident_launch_part5(var, p, mt, ng, smem, s);
+    case 6: return resident_launch_part6(var, p, mt, ng, smem, s);
+    default: return resident_launch_part7(var, p, mt, ng, smem, s);
   }
 }
 
@@ -588,6 +605,87 @@ static bool stream_ahead(int M, int N, int K, int var, const PairSplit& pl, cons
   return var_is_float(var) && M <= 6 && weights <= 4 * million;
 }
 
+// ---- decode kernel with the activations in registers (resident_kernel.cu) ---------------------------
+struct ResidentSplit { int S, T_own, wk_shift, n_max, stages, slab_shift, smem, grid; };
+// How S CTAs per cluster share the work: column tiles per cluster, and the warps that share K.  16 of them where that gives each two
+// groups of 128 rows or more; for fewer rows of K the warps may form two or four sets that take turns with the column tiles, each with
+// the activations of all of K: fewer parts per column tile to add up, more activations to load.  us per launch (4 bits, fits): 0.23
+// per group and 0.25 per tile of a warp, 12.5 per MB of activations (1 x 28672 x 2048, 16 / 8 warps 9.3 / 8.0; 8 x 4096 x 2048 3.3 / 3.7;
+// four groups per warp are slower than two of twice the warps, 1 x 28672 x 4096 14.9 / 13.4).
+static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInfo& di, ResidentSplit* rs) {
+  const int G = K / 128, NT = N / BLOCK_N, mt = stream_mt(M), ng_max = mt == 1 ? 4 : 2;
+  if (M > 16 || S < 1 || S > 8 || G < S) return false;
+  int clusters = di.sm_count / S;
+  if (S > 1 && max_clusters(S) < clusters) clusters = max_clusters(S);
+  if (clusters < 1) return false;
+  rs->S = S;
+  rs->T_own = (NT + clusters - 1) / clusters;
+  rs->grid = S * ((NT + rs->T_own - 1) / rs->T_own);
+  const int Gc = (G + S - 1) / S;
+  double least = 0.0;
+  for (int sh = 4; sh >= 2; --sh) {
+    const int n = (Gc + (1 << sh) - 1) >> sh, sets = RES_WARPS >> sh;
+    if (n > (sh == 4 ? ng_max : 2)) continue;
+    const double cost = ((rs->T_own + sets - 1) / sets) * (0.23 * n + 0.25) + 12.5e-6 * 2.0 * M * Gc * 128 * sets;
+    if (least > 0.0 && cost >= least) continue;
+    least = cost;
+    rs->wk_shift = sh;
+    rs->n_max = n;
+  }
+  if (least <= 0.0) return false;
+  const int ng = rs->n_max <= 2 ? 2 : 4, slot = res_gi(bits, ng) * 256 * bits;
+  const int sets = RES_WARPS >> rs->wk_shift, Tw = (rs->T_own + sets - 1) / sets;
+  rs->slab_shift = Tw <= 1 ? 0 : Tw <= 2 ? 1 : 2;
+  const long long fixed = RES_HEADER + (long long)RES_WARPS * ng * Tw * 32 + (RES_WARPS << rs->slab_shift) * mt * 512 +
+                          (S > 1 ? (long long)rs->T_own * mt * 512 : 0);
+  if (fixed > di.max_smem) return false;
+  int st = kStreamRing / (RES_WARPS * slot);
+  st = st > 8 ? 8 : st < 2 ? 2 : st;
+  while (st > 2 && fixed + st * RES_WARPS * slot > di.max_smem) --st;
+  rs->stages = st;
+  rs->smem = (int)fixed + st * RES_WARPS * slot;
+  if (rs->smem > di.max_smem) return false;
+  if (rs->smem < kOneCtaSmem) rs->smem = kOneCtaSmem;  // (never two to an SM while others idle, see stream_launch_smem)
+  return true;
+}
+// Where the resident kernel takes a decode call that the table gives to the stream kernel (tile_m 0) or the exact kernel: the CTAs
+// per cluster, or 0.  Measured against those, cold chains, 11 widths x 6 depths (1024 .. 14336) x 1 .. 16 rows in 4 bits, 5 x 5 in
+// 1, 2, 3, 6 and 8 bits; time here over time there:
+//  - 5 to 8 rows 0.44 .. 0.98; 2 to 4 rows 0.49 .. 1.0, except where rows of K leave some warps a third group (K = 5120, 1.02 .. 1.11
+//    from 8192 columns on) and 5 to 7 bits beyond 8192 rows of K (up to 1.03);
+//  - one row: up to 4096 rows of K 0.71 .. 0.99, for 1 and 2 bits up to 8192 columns, 3 bits up to 16384 (2 bits, 28672 x 4096 1.06);
+//    up to 8192 rows of K two column tiles per CTA, 1 and 2 bits one (4096 x 8192, 4 bits 0.98, 6144 x 8192 1.03);
+//    beyond, 8-bit integers (0.94 .. 0.97) and 4 bits up to 3072 columns (0.82 .. 0.96);
+//  - 9 to 16 rows (fp16 only: the exact kernel takes bfloat16 as it is), whose second set of sums makes the loop 1.5 times longer: up to
+//    4096 rows of K in the ranges below 0.63 .. 0.96; beyond 1.0 .. 1.3.
+// S: one CTA per cluster where a warp's activations fit its registers, and where K is long or the columns few; us, 8 rows,
+// S = 1 / 2 / 4: 8192 x 8192 11.5 / 10.6 / 12.7, 4096 x 14336 - / 12.1 / 10.5, 28672 x 14336 - / 45.1 / 45.2.
+static int resident_cluster(int M, int N, int K, int var, int group, int act, bool stream_form, const DeviceInfo& di) {
+  if (M > 16 || group % 128 != 0 || (act == B200Q_BF16 && !stream_form)) return 0;
+  const int G = K / 128, bits = var_bits(var);
+  int S;
+  if (M > 8) {
+    if (G > 32 || N > (G > 16 ? 11008 : G == 16 ? 6144 : 4096) || (G > 16 && N < 3072 && M > 12)) return 0;
+    S = 1;
+  } else {
+    S = G <= 40 || (G <= 64 && M < 5 && N < 8192) ? 1 : G <= 64 || (N >= 16384 && G <= 128) ? 2 : 4;
+    const bool integer = !var_is_float(var);
+    if (M == 1 && G <= 32) {
+      if (N > (bits <= 2 ? 8192 : bits == 3 ? 16384 : 1 << 30)) return 0;
+    } else if (M == 1 && G <= 64) {
+      if (N > (bits <= 2 ? 2048 : 4096)) return 0;
+    } else if (M == 1) {
+      if (!(integer && bits == 8) && !(bits == 4 && N <= 3072)) return 0;
+    } else if (M <= 4 && stream_form) {
+      const int n = (G + 16 * S - 1) / (16 * S);
+      if (N >= 8192 && G * 20 < n * 16 * S * 17) return 0;
+      if (G > 64 && bits >= 5 && bits <= 7) return 0;
+    }
+  }
+  ResidentSplit rs;
+  return resident_split(M, N, K, bits, S, di, &rs) ? S : 0;
+}
+
 static const int kStreamForm = -1;  // in place of an activation type: the stream kernel's plan for any M that it takes
 
 static int make_plan_uncached(int M, int N, int K, int var, int group, int act, b200q_plan_t* pl) {
@@ -612,6 +710,7 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
         plan_stream(M, N, K, bits, di, pl) == ST_OK) {
       pl->passes = 1;
       pl->workspace_bytes = stream_workspace_bytes(N);  // fp32 scratch [N][8 or 16]
+      pl->resident = resident_cluster(M, N, K, var, group, act, true, di);
       return ST_OK;
     }
     std::memset(pl, 0, sizeof(*pl));
@@ -620,6 +719,7 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
   if (M <= kBatchMaxRows) {
     plan_batch(M, N, K, bits, group, di, pl);
     pl->workspace_bytes = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M, N);
+    if (batch_exact(M, group)) pl->resident = resident_cluster(M, N, K, var, group, act, false, di);
     if (M <= kStreamMaxRows && stream_takes(K, group)) {  // the decode path's other form, see b200q_plan_t
       pl->kernel = 2;
       pl->m_tiles = stream_mt(M);
@@ -921,6 +1021,30 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
   return ST_OK;
 }
 
+static int run_resident(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
+                        int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream, const b200q_plan_t& pl,
+                        const ResidentSplit& rs) {
+  // (the workspace that the plan's other form asks for, so that the same calls are refused; only the status word is used)
+  const size_t need = pl.tile_m == 0 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
+  if (!workspace || ws_bytes < need || ((uintptr_t)workspace & 255)) return ST_WORKSPACE;
+  if (((uintptr_t)scales) & 15) return ST_INVALID_ARG;
+  ResidentParams p;
+  p.a = reinterpret_cast<const __half*>(a);
+  p.bq = bq;
+  p.scales = reinterpret_cast<const __half*>(scales);
+  p.c = reinterpret_cast<__half*>(c);
+  p.status = reinterpret_cast<int*>(workspace);
+  p.M = M; p.N = N; p.lda = lda; p.ldc = ldc;
+  p.G = K / 128; p.NT = N / BLOCK_N;
+  p.gshift = gshift_of(group); p.gdiv = group / 128;
+  p.S = rs.S; p.T_own = rs.T_own; p.wk_shift = rs.wk_shift;
+  p.stages = rs.stages; p.slab_shift = rs.slab_shift; p.grid = rs.grid;
+  p.act = act; p.zero = 0u;
+  const cudaError_t e = resident_launch(var, p, stream_mt(M), rs.n_max, rs.smem, stream);
+  if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
+  return ST_OK;
+}
+
 // the form of the decode path (kernel 2) that exact_kernel.cu runs
 static bool plan_is_exact(const b200q_plan_t& pl) { return pl.tile_m == 16 && pl.splits == 1; }
 
@@ -931,6 +1055,12 @@ static int run_gemm(const void* a, int lda, const void* bq, const void* scales, 
   if (((uintptr_t)a | (uintptr_t)bq | (uintptr_t)c) & 15) return ST_INVALID_ARG;
   if (((uintptr_t)scales) & 1) return ST_INVALID_ARG;
   if (lda < K || ldc < N || (lda % 8) != 0) return ST_INVALID_ARG;
+  // (a call that the resident kernel does not take - a plan put on more rows, or a tcgen05 plan on bfloat16, whose range fp16 does not
+  // have - runs on the plan's other form)
+  ResidentSplit rs;
+  if (pl.resident > 0 && (pl.kernel == 2 || (pl.kernel == 3 && pl.tile_m == 16)) && group % 128 == 0 && !(act == B200Q_BF16 && (M > 8 || pl.tile_m != 0)) &&
+      resident_split(M, N, K, var_bits(var), pl.resident, device_info(), &rs))
+    return run_resident(a, lda, bq, scales, c, ldc, M, N, K, var, group, act, workspace, ws_bytes, stream, pl, rs);
   if (pl.kernel == 1 && pl.passes == 2) {
     // the full 256-row tiles on the tcgen05 kernel, the short last tile on the decode kernel
     const int tail = M % 256;
@@ -1039,8 +1169,16 @@ int b200q_gemm_planned(const void* a, int lda, const void* bq, const void* scale
   int var;
   int st = check_problem(M, N, K, wtype, zero_point, group, true, &var);
   if (st != ST_OK) return st;
+  b200q_plan_t pl = *plan;
+  if (pl.resident > 0) {  // an edit of any other field names one of the other kernels
+    b200q_plan_t own;
+    const int rows = M < 16 ? M : 16;
+    if (make_plan(rows, N, K, var, group, act_dtype, &own) != ST_OK || own.kernel != pl.kernel || own.tile_m != pl.tile_m ||
+        own.splits != pl.splits || own.cluster != pl.cluster || own.ctas_per_split != pl.ctas_per_split || own.stages != pl.stages)
+      pl.resident = 0;
+  }
   return run_gemm(a, lda, bq, scales, c, ldc, M, N, K, var, group, act_dtype, workspace, workspace_bytes,
-                  reinterpret_cast<cudaStream_t>(stream), *plan);
+                  reinterpret_cast<cudaStream_t>(stream), pl);
 }
 
 int b200q_gemm_gather(const void* a, int lda, const void* bq, const void* scales, int M, int N, int K, int wtype,

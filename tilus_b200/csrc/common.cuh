@@ -111,6 +111,30 @@ struct StreamParams {
   GatherArgs ga;
 };
 
+// ---- decode kernel with the activations in registers (up to 16 rows) ----------------------------------
+constexpr int RES_WARPS = 16;
+constexpr int RES_HEADER = 1024 + 256;  // bytes of barriers in front of the rings: 8 slots per warp; slabs of up to four sets
+// 128-row groups per ring slot: at most 2 KB
+__host__ __device__ constexpr int res_gi(int bits, int ng) { return ng >= 4 && bits <= 2 ? 4 : bits <= 4 ? 2 : 1; }
+struct ResidentParams {
+  const __half* a;       // [M, K] row-major, leading dimension lda
+  const void* bq;        // b200 layout
+  const __half* scales;  // [K/group, N], 16-byte aligned
+  __half* c;             // [M, N], leading dimension ldc
+  int* status;           // workspace status header
+  int M, N, lda, ldc;
+  int G, NT;             // K/128, N/16
+  int gshift, gdiv;      // as StreamParams
+  int S;                 // CTAs of a cluster, which share K; 1: no cluster
+  int T_own;             // column tiles per cluster
+  int wk_shift;          // log2 of the warps that share K; the 16 / that sets of warps take turns with the column tiles
+  int stages;            // ring slots per warp (<= 8)
+  int slab_shift;        // log2 of the column tiles whose partial sums have room in shared memory
+  int grid;
+  int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
+  uint32_t zero;         // 0, which the compiler does not know
+};
+
 // ---- tcgen05 kernel with the weights in tensor memory (any M; used for M > 128) ----------------
 struct UmmaParams {
   const uint4* bq;       // b200 layout

@@ -1,0 +1,486 @@
+// Decode batches of up to 16 rows with the activations in registers: C[M, N] = A[M, K] x dequant(Bq[K, N]).
+//
+// What bounds it: HBM, and around a launch 3 us of start, activations and end.  In stream_kernel.cu a warp reads the
+// activations of each 128-row group from shared memory, 2 KB for every 1 KB of 4-bit weights: 32 of the 45 cycles that HBM leaves
+// an SM per 16 x 128 group went to shared memory, and every CTA staged and converted the activations before its first product.
+// Here K is split over the warps of a CTA instead of the column tiles: a warp owns up to four 128-row groups of K and loads
+// their activations once, as tensor-core operands (the operand's k order is the packed layout's: lane (r, j) holds 64 contiguous
+// bytes of row r per group), and then takes the CTA's column tiles one after the other.  Shared memory carries the weights only,
+// and nothing is staged.  us, cold chains, 4 bits, group 128, before (stream or exact kernel) / here: 8 x 4096 x 4096 7.1 / 4.7, 8 x
+// 28672 x 4096 19.8 / 13.6, 8 x 4096 x 14336 13.1 / 10.6, 1 x 4096 x 4096 4.6 / 3.9, 1 x 28672 x 4096 13.7 / 12.7; 16 x 4096 x 4096
+// 8.2 / 7.1, but 16 x 28672 x 4096 20.3 / 20.6 (two sets of sums per warp: 185 instructions per group, 121 with one).
+//
+// Weights.  One elected thread of a warp keeps the warp's ring full with TMA bulk copies, as in stream_kernel.cu: slots of one, two or
+// four groups of a column tile, about 64 KB per CTA (three slots of 2 KB instead of two: no gain).  All loads of a slot come first, then the
+// request for the next one, then the products (loads group by group: 28672 x 4096 14.0 us, 13.6 so).
+//
+// Products.  mma.sync.m16n8k16, 16 columns of weights against 8 rows of activations: 8 cycles per SM quadrant, so that one
+// group costs 16 of the SM's 45 cycles.  An integer code sits in the mantissa of an fp16 subnormal at one of two places (res_target), an
+// accumulator each, whose sums are added with the factor between the places: the activations are multiplied as they are (the
+// stream kernel multiplies them by 2^-T beforehand, which costs those below 2^(T-14) low bits), for half of the shifts of a single place.
+// The zero point: both accumulators start from a quarter of -zero_point * sum(a), and the other half is added behind the group's
+// products, so that sums of activations with a mean stay around zero on the way (the sums over a come from eight MMAs per group with a
+// constant operand, once per launch).  Per group the sums are multiplied by the scale in fp32: no weight is rounded.
+//
+// Sums.  The 16 warps' parts of a column tile meet in shared memory (four tiles of room, an mbarrier that counts the warps and one
+// that frees the room), and one of the warps, in turn, adds them up in order and writes C: results repeat bit for bit.  Where the
+// activations do not fit the registers - more than 8192 rows of K for up to 8 rows of A, 4096 for 16 - a cluster of S CTAs
+// shares K and adds its sums up in distributed shared memory.
+//
+// Every wait is bounded; one that runs out leaves the loops, waits (bounded) for the copies in flight and is reported in the workspace's
+// status word.
+#include "common.cuh"
+
+#ifndef B200Q_PART
+#define B200Q_PART 0
+#endif
+#ifndef B200Q_NPARTS
+#define B200Q_NPARTS 1
+#endif
+
+namespace b200q {
+
+// ---- where the codes of a pair sit in the operand's mantissa: two places per width, half of the pairs each ----
+// (the places that need the fewest shifts; a pair's products carry the factor 2^T, one accumulator per place)
+B200Q_HD constexpr int res_class(int b, int h) {
+  return b == 3 || b == 7 ? (h >> 1) & 1 : b == 5 ? (h ^ (h >> 2)) & 1 : h & 1;
+}
+B200Q_HD constexpr int res_target(int b, int cls) {
+  switch (b) {
+    case 1: return cls;
+    case 2: case 6: return 2 * cls;
+    case 3: case 7: return 1 + 2 * cls;
+    case 4: case 5: return 4 * cls;
+    default: return 0;
+  }
+}
+// the i-th pair of a class, i = 0 .. 7
+B200Q_HD constexpr int res_pair(int b, int cls, int i) {
+  int n = 0;
+  for (int h = 0; h < 16; ++h)
+    if (res_class(b, h) == cls && n++ == i) return h;
+  return 0;
+}
+template <int VAR, int H>
+__device__ __forceinline__ uint32_t res_operand(const uint32_t* w) {
+  constexpr int B = var_bits(VAR);
+  if constexpr (var_is_float(VAR)) return pair_raw<VAR, H>(w);
+  else {
+    constexpr int T = res_target(B, res_class(B, H));
+    if constexpr (lin_uniform_inverted(VAR)) return gather_pair<B, H, T>(w, 0u) ^ (0x00010001u << T);
+    else return gather_pair<B, H, T>(w, 0u);
+  }
+}
+
+template <int ACT>
+__device__ __forceinline__ unsigned short res_out_bits(float v) {
+  if constexpr (ACT == 0) return __half_as_ushort(__float2half_rn(v));
+  else return __bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+template <int ACT>
+__device__ __forceinline__ float res_scale(unsigned short bits) {
+  if constexpr (ACT == 0) return __half2float(__ushort_as_half(bits));
+  else return __uint_as_float((uint32_t)bits << 16);
+}
+// two bf16 values as fp16: exact inside fp16's range, larger magnitudes saturate, those below 2^-24 vanish, NaN stays
+__device__ __forceinline__ uint32_t res_bf16x2_to_f16x2(uint32_t w) {
+  uint32_t h;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(__uint_as_float(w & 0xffff0000u)), "f"(__uint_as_float(w << 16)));
+  return h;
+}
+// the words of a unit, and one word of every vector load
+template <int B>
+__device__ __forceinline__ uint32_t res_unit(const unsigned char* ptr, uint32_t (&w)[B]) {
+  if constexpr (B % 4 == 0) {
+    uint32_t x = 0u;
+#pragma unroll
+    for (int q = 0; q < B / 4; ++q) {
+      const uint4 v = reinterpret_cast<const uint4*>(ptr)[q];
+      w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+      x |= v.x;
+    }
+    return x;
+  } else if constexpr (B % 2 == 0) {
+    uint32_t x = 0u;
+#pragma unroll
+    for (int q = 0; q < B / 2; ++q) {
+      const uint2 v = reinterpret_cast<const uint2*>(ptr)[q];
+      w[2 * q] = v.x; w[2 * q + 1] = v.y;
+      x |= v.x;
+    }
+    return x;
+  } else {
+    uint32_t x = 0u;
+#pragma unroll
+    for (int q = 0; q < B; ++q) { w[q] = reinterpret_cast<const uint32_t*>(ptr)[q]; x |= w[q]; }
+    return x;
+  }
+}
+
+__device__ __forceinline__ unsigned long long f2_pack(float x, float y) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ void f2_unpack(unsigned long long v, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// d = a * b + c with c in registers of its own
+__device__ __forceinline__ void mma_m16n8k16_from(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                                  uint32_t b1, float c0, float c1, float c2, float c3) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// Shared memory: barriers of the rings [warp][8] and of the slabs [set][full 4, empty 4]; rings [warp][slot]; scales
+// [warp][tile][NG][16]; slabs [set][slot][warp][MT][32 lanes] float4; with a cluster the CTA's sums [tile][MT][32 lanes] float4.
+// Columns of `af`, `nb`: rows of A come in sets of eight (MT of them), 128-row groups of K in NG.
+template <int VAR, int MT, int NG, int ACT>
+__global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const ResidentParams p) {
+  constexpr int B = var_bits(VAR);
+  constexpr int BIAS = lin_uniform_bias(VAR);
+  constexpr int GI = res_gi(B, NG);
+  constexpr int IPT = NG / GI;             // slots per column tile
+  constexpr uint32_t GROUP = 256u * B, SLOT = GI * GROUP;
+  constexpr int T0 = var_is_float(VAR) ? 0 : res_target(B, 0), T1 = var_is_float(VAR) ? 0 : res_target(B, 1);
+  constexpr int FL = lin_factor_log2(VAR) - T0;
+  constexpr float F = (lin_uniform_inverted(VAR) ? -1.0f : 1.0f) * (float)(1u << FL);
+  constexpr int NBQ = MT * NG <= 2 ? 4 : 2;  // registers of a zero-point term: as the accumulators have it, or once
+  constexpr float R10 = (float)(1 << (T1 - T0)), R01 = 1.0f / R10;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int r = lane >> 2, j = lane & 3;
+  const int NST = p.stages, WK = 1 << p.wk_shift, WT = RES_WARPS >> p.wk_shift;
+  const int set = warp >> p.wk_shift, wi = warp & (WK - 1);
+
+  int ci = blockIdx.x, chunk = 0;
+  if (p.S > 1) { ci = blockIdx.x / p.S; chunk = blockIdx.x - ci * p.S; }
+  const int gc0 = p.S > 1 ? p.G * chunk / p.S : 0, gc1 = p.S > 1 ? p.G * (chunk + 1) / p.S : p.G;
+  const int Gc = gc1 - gc0, base = Gc >> p.wk_shift, rem = Gc & (WK - 1);
+  const int n = base + (wi < rem ? 1 : 0), g0 = gc0 + wi * base + min(wi, rem);  // this warp's groups of K
+  const int active = min(WK, Gc);                                                 // warps of a set that have any
+  const int tile0 = ci * p.T_own, tiles = min(p.T_own, p.NT - tile0);
+  const int my = n > 0 && tiles > set ? (tiles - set + WT - 1) >> (4 - p.wk_shift) : 0;  // tiles of this set
+
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  // ---- shared memory ----
+  const uint32_t bar0 = smem_base + (uint32_t)warp * 64u;
+  const uint32_t full0 = smem_base + 1024u + (uint32_t)set * 64u, empty0 = full0 + 32u;  // [slab slot]
+  const uint32_t ring_off = RES_HEADER + (uint32_t)(warp * NST) * SLOT, ring_s = smem_base + ring_off;
+  const uint32_t sc_off = RES_HEADER + (uint32_t)(RES_WARPS * NST) * SLOT;
+  const int Tw = (p.T_own + WT - 1) >> (4 - p.wk_shift);
+  unsigned char* sc_warp = smem_raw + sc_off + (size_t)warp * NG * Tw * 32;
+  const uint32_t slab_off = sc_off + (uint32_t)(RES_WARPS * NG * Tw * 32);
+  const int D = 1 << p.slab_shift;
+  float4* slab = reinterpret_cast<float4*>(smem_raw + slab_off) + (size_t)set * D * WK * MT * 32;
+  float4* csum = reinterpret_cast<float4*>(smem_raw + slab_off + (uint32_t)(WT * D * WK * MT * 512));
+
+  // ---- weights: the warp's own ring ----
+  const int ipt = (n + GI - 1) / GI, n_items = my * ipt;
+  const uint32_t last_bytes = (uint32_t)(n - (ipt - 1) * GI) * GROUP;
+  const unsigned char* src = reinterpret_cast<const unsigned char*>(p.bq) + ((size_t)(tile0 + set) * p.G + g0) * GROUP;
+  const size_t tile_skip = (size_t)WT * p.G * GROUP - (size_t)(ipt - 1) * SLOT;
+  int issued = 0, pq = 0;
+  auto issue_next = [&](uint32_t bar, uint32_t dst) {
+    const bool last = IPT == 1 || pq == ipt - 1;
+    const uint32_t bytes = last ? last_bytes : SLOT;
+    if (elect_one()) {
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+          "r"(bytes), "r"(bar)
+          : "memory");
+    }
+    ++issued;
+    if (last) { src += tile_skip; pq = 0; } else { src += SLOT; ++pq; }
+  };
+  if (lane < NST) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + lane * 8) : "memory");
+  if (wi == 0 && lane < 4) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full0 + lane * 8), "r"(active) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + lane * 8) : "memory");
+  }
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncwarp();
+  for (int s = 0; s < NST && issued < n_items; ++s) issue_next(bar0 + s * 8, ring_s + s * SLOT);
+
+  // ---- scales of all of the warp's tiles and groups: [tile][group][16] ----
+  for (int gi = 0; gi < n; ++gi) {
+    const int row = p.gshift >= 0 ? (g0 + gi) >> p.gshift : (g0 + gi) / p.gdiv;
+    const unsigned short* srow = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)row * p.N + tile0 * 16;
+    for (int x = lane; x < my * 2; x += 32) {
+      const uint32_t dst = smem_base + (uint32_t)(sc_warp - smem_raw) + (uint32_t)(((x >> 1) * NG + gi) * 32 + (x & 1) * 16);
+      const unsigned short* s = srow + (set + (x >> 1) * WT) * 16 + (x & 1) * 8;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(s) : "memory");
+    }
+  }
+
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // ---- activations: operand fragments of the warp's groups, kept for all column tiles ----
+  uint32_t af[NG][MT][16];
+#pragma unroll
+  for (int g = 0; g < NG; ++g)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const bool valid = g < n && mt * 8 + r < p.M;
+      const uint4* pa = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned short*>(p.a) +
+                                                       (size_t)(mt * 8 + r) * p.lda + (size_t)(g0 + g) * 128 + j * 32);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 v = valid ? __ldg(pa + q) : make_uint4(0u, 0u, 0u, 0u);
+        af[g][mt][4 * q] = v.x; af[g][mt][4 * q + 1] = v.y; af[g][mt][4 * q + 2] = v.z; af[g][mt][4 * q + 3] = v.w;
+      }
+    }
+  // a quarter of the zero-point term of every group and row, in the accumulators' unit (row 2j, 2j + 1 of each 8)
+  float nb[BIAS != 0 ? NG : 1][BIAS != 0 ? MT : 1][NBQ];
+#pragma unroll
+  for (int g = 0; g < NG; ++g)
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      if constexpr (ACT == 1) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) af[g][mt][q] = res_bf16x2_to_f16x2(af[g][mt][q]);
+      }
+      if constexpr (BIAS != 0) {
+        float d[4];
+        constexpr uint32_t ONE = 0x3c003c00u;
+        mma_m16n8k16_init(d, ONE, ONE, ONE, ONE, af[g][mt][0], af[g][mt][1]);
+#pragma unroll
+        for (int q = 2; q < 16; q += 2) mma_m16n8k16(d, ONE, ONE, ONE, ONE, af[g][mt][q], af[g][mt][q + 1]);
+        constexpr float Q = -0.25f * (float)BIAS / (float)(1u << FL);
+#pragma unroll
+        for (int q = 0; q < NBQ; ++q) nb[g][mt][q] = d[q] * Q;
+      }
+    }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();  // barriers of the slabs
+
+  // ---- column tiles ----
+  bool ok = true;
+  int next_read = wi;
+  auto finish = [&](int ti) {  // adds up the warps' sums of tile ti of this set
+    const uint32_t bar = full0 + (uint32_t)(ti & (D - 1)) * 8u;
+    if (!mbar_wait_bounded(bar, (uint32_t)(ti >> p.slab_shift) & 1u)) { ok = false; return; }
+    const float4* s = slab + (size_t)(ti & (D - 1)) * WK * MT * 32 + lane;
+    const int tile = set + ti * WT;
+    float4 v[MT];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) v[mt] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int w = 0; w < active; ++w)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const float4 x = s[(w * MT + mt) * 32];
+        v[mt].x += x.x; v[mt].y += x.y; v[mt].z += x.z; v[mt].w += x.w;
+      }
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + (uint32_t)(ti & (D - 1)) * 8u) : "memory");
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      v[mt].x *= F; v[mt].y *= F; v[mt].z *= F; v[mt].w *= F;
+      if (p.S > 1) {
+        csum[(tile * MT + mt) * 32 + lane] = v[mt];
+      } else {
+        const int m = mt * 8 + 2 * j, col = (tile0 + tile) * 16 + r;
+        unsigned short* c = reinterpret_cast<unsigned short*>(p.c) + (size_t)m * p.ldc + col;
+        if (m < p.M) { c[0] = res_out_bits<ACT>(v[mt].x); c[8] = res_out_bits<ACT>(v[mt].z); }
+        if (m + 1 < p.M) { c[p.ldc] = res_out_bits<ACT>(v[mt].y); c[p.ldc + 8] = res_out_bits<ACT>(v[mt].w); }
+      }
+    }
+  };
+  uint32_t slot_off = 0, bar = bar0, parity = 0;
+  const unsigned char* ring_g = smem_raw + ring_off;
+  const uint32_t w_lane = (uint32_t)(lane * B * 4);
+  const unsigned short* sc_lane = reinterpret_cast<const unsigned short*>(sc_warp) + r;
+  for (int ti = 0; ti < my && ok; ++ti, sc_lane += NG * 16) {
+    unsigned long long acc[MT][2];  // rows 2j, 2j + 1 of columns r and r + 8
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = 0ull;
+#pragma unroll
+    for (int q = 0; q < IPT; ++q) {
+      if (q * GI >= n) break;
+      if (!__all_sync(0xffffffffu, mbar_test(bar, parity) ? 1 : 0)) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity) ? 1 : 0)) { ok = false; break; }
+      }
+      const unsigned char* slot = ring_g + slot_off;
+      uint32_t loaded = 0u, w0[GI][B], w1[GI][B];
+#pragma unroll
+      for (int gi = 0; gi < GI; ++gi) {
+        loaded |= res_unit<B>(slot + w_lane + gi * GROUP, w0[gi]);
+        loaded |= res_unit<B>(slot + w_lane + gi * GROUP + GROUP / 2, w1[gi]);
+      }
+      __syncwarp();
+      if (issued < n_items) issue_next(bar, ring_s + slot_off + (loaded & p.zero));
+#pragma unroll
+      for (int gi = 0; gi < GI; ++gi) {
+        const int g = q * GI + gi;
+        if (gi > 0 && g >= n) break;
+        const float sf0 = res_scale<ACT>(sc_lane[g * 16]), sf1 = res_scale<ACT>(sc_lane[g * 16 + 8]);
+        float d0[MT][4], d1[MT][4];
+        unsigned long long z0[MT], z1[MT];
+        if constexpr (BIAS != 0) {
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            z0[mt] = f2_pack(nb[g][mt][0], nb[g][mt][1]);
+            z1[mt] = NBQ == 4 ? f2_pack(nb[g][mt][NBQ - 2], nb[g][mt][NBQ - 1]) : z0[mt];
+          }
+        }
+#define RES_STEP(I)                                                                                                  \
+  {                                                                                                                  \
+    constexpr int H0 = res_pair(B, 0, 2 * I), H1 = res_pair(B, 0, 2 * I + 1), H2 = res_pair(B, 1, 2 * I),            \
+                  H3 = res_pair(B, 1, 2 * I + 1);                                                                    \
+    const uint32_t x0 = res_operand<VAR, H0>(w0[gi]), x1 = res_operand<VAR, H0>(w1[gi]), x2 = res_operand<VAR, H1>(w0[gi]),      \
+                   x3 = res_operand<VAR, H1>(w1[gi]);                                                                    \
+    const uint32_t y0 = res_operand<VAR, H2>(w0[gi]), y1 = res_operand<VAR, H2>(w1[gi]), y2 = res_operand<VAR, H3>(w0[gi]),      \
+                   y3 = res_operand<VAR, H3>(w1[gi]);                                                                    \
+    _Pragma("unroll") for (int mt = 0; mt < MT; ++mt) {                                                              \
+      if constexpr (I > 0) {                                                                                         \
+        mma_m16n8k16(d0[mt], x0, x1, x2, x3, af[g][mt][H0], af[g][mt][H1]);                                          \
+        mma_m16n8k16(d1[mt], y0, y1, y2, y3, af[g][mt][H2], af[g][mt][H3]);                                          \
+      } else if constexpr (BIAS == 0) {                                                                              \
+        mma_m16n8k16_init(d0[mt], x0, x1, x2, x3, af[g][mt][H0], af[g][mt][H1]);                                     \
+        mma_m16n8k16_init(d1[mt], y0, y1, y2, y3, af[g][mt][H2], af[g][mt][H3]);                                     \
+      } else {                                                                                                       \
+        float c0, c1, c2, c3, e0, e1, e2, e3;                                                                        \
+        f2_unpack(z0[mt], c0, c1); f2_unpack(z1[mt], c2, c3);                                                        \
+        mma_m16n8k16_from(d0[mt], x0, x1, x2, x3, af[g][mt][H0], af[g][mt][H1], c0, c1, c2, c3);                     \
+        f2_unpack(T1 != T0 ? f2_mul(z0[mt], f2_pack(R10, R10)) : z0[mt], e0, e1);                                    \
+        f2_unpack(T1 != T0 ? f2_mul(z1[mt], f2_pack(R10, R10)) : z1[mt], e2, e3);                                    \
+        mma_m16n8k16_from(d1[mt], y0, y1, y2, y3, af[g][mt][H2], af[g][mt][H3], e0, e1, e2, e3);                     \
+      }                                                                                                              \
+    }                                                                                                                \
+  }
+        RES_STEP(0) RES_STEP(1) RES_STEP(2) RES_STEP(3)
+#undef RES_STEP
+        const unsigned long long s0 = f2_pack(sf0, sf0), s1 = f2_pack(sf1, sf1), r01 = f2_pack(R01, R01), two = f2_pack(2.f, 2.f);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const unsigned long long lo0 = f2_pack(d0[mt][0], d0[mt][1]), hi0 = f2_pack(d0[mt][2], d0[mt][3]);
+          const unsigned long long lo1 = f2_pack(d1[mt][0], d1[mt][1]), hi1 = f2_pack(d1[mt][2], d1[mt][3]);
+          unsigned long long lo = T1 != T0 ? f2_fma(lo1, r01, lo0) : f2_add(lo1, lo0);
+          unsigned long long hi = T1 != T0 ? f2_fma(hi1, r01, hi0) : f2_add(hi1, hi0);
+          if constexpr (BIAS != 0) { lo = f2_fma(z0[mt], two, lo); hi = f2_fma(z1[mt], two, hi); }
+          acc[mt][0] = f2_fma(s0, lo, acc[mt][0]);
+          acc[mt][1] = f2_fma(s1, hi, acc[mt][1]);
+        }
+      }
+      slot_off += SLOT; bar += 8;
+      if (slot_off == (uint32_t)NST * SLOT) { slot_off = 0; bar = bar0; parity ^= 1u; }
+    }
+    if (!ok) break;
+    const int sl = ti & (D - 1);
+    if (ti >= D && !mbar_wait_bounded(empty0 + (uint32_t)sl * 8u, (uint32_t)((ti >> p.slab_shift) - 1) & 1u)) { ok = false; break; }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+    {
+      float4 v;
+      f2_unpack(acc[mt][0], v.x, v.y);
+      f2_unpack(acc[mt][1], v.z, v.w);
+      slab[(sl * WK + wi) * MT * 32 + mt * 32 + lane] = v;
+    }
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(full0 + (uint32_t)sl * 8u) : "memory");
+    if (ti > 0 && ti - 1 == next_read) { finish(ti - 1); next_read += active; }
+  }
+  ok = __all_sync(0xffffffffu, ok ? 1 : 0);
+  if (ok && my > 0 && next_read == my - 1) finish(my - 1);
+  if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
+    if (lane == 0) {
+      atomicExch(p.status, ST_DEVICE_TIMEOUT);
+      p.status[1] = 10;  // where: resident kernel
+      p.status[2] = blockIdx.x;
+      p.status[3] = warp;
+    }
+    for (int s = 0; s < NST; ++s) mbar_wait_bounded(bar0 + s * 8, 0);
+  }
+  if (p.S > 1) {  // the cluster's CTAs hold parts of the same tiles
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t csum_s = smem_base + (uint32_t)(reinterpret_cast<unsigned char*>(csum) - smem_raw);
+    for (int t = chunk + warp * p.S; t < tiles; t += RES_WARPS * p.S) {
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < p.S; ++c) {
+          uint32_t addr;
+          float4 x;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(csum_s + (uint32_t)((t * MT + mt) * 512 + lane * 16)), "r"(c));
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(addr) : "memory");
+          v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+        }
+        const int m = mt * 8 + 2 * j, col = (tile0 + t) * 16 + r;
+        unsigned short* c = reinterpret_cast<unsigned short*>(p.c) + (size_t)m * p.ldc + col;
+        if (m < p.M) { c[0] = res_out_bits<ACT>(v.x); c[8] = res_out_bits<ACT>(v.z); }
+        if (m + 1 < p.M) { c[p.ldc] = res_out_bits<ACT>(v.y); c[p.ldc + 8] = res_out_bits<ACT>(v.w); }
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+template <int VAR, int MT, int NG, int ACT>
+static cudaError_t launch_one(const ResidentParams& p, int smem_bytes, cudaStream_t stream) {
+  auto kern = resident_kernel<VAR, MT, NG, ACT>;
+  static std::atomic<bool> allowed[16];
+  const cudaError_t e = allow_smem(kern, allowed);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
+  cfg.blockDim = dim3(RES_WARPS * 32, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)p.S;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.S > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+template <int VAR>
+static cudaError_t launch_var(int var, const ResidentParams& p, int mt, int ng, int smem_bytes, cudaStream_t stream) {
+  if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
+    if (var == VAR) {
+      if (mt == 2 && ng <= 2 && p.act == 0) return launch_one<VAR, 2, 2, 0>(p, smem_bytes, stream);
+      if (mt != 1 || ng > 4) return cudaErrorInvalidValue;
+      if (p.act == 0)
+        return ng <= 2 ? launch_one<VAR, 1, 2, 0>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 0>(p, smem_bytes, stream);
+      return ng <= 2 ? launch_one<VAR, 1, 2, 1>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 1>(p, smem_bytes, stream);
+    }
+  }
+  if constexpr (VAR + 1 < VAR_COUNT) return launch_var<VAR + 1>(var, p, mt, ng, smem_bytes, stream);
+  else return cudaErrorInvalidValue;
+}
+
+#define B200Q_CAT2(a, b) a##b
+#define B200Q_CAT(a, b) B200Q_CAT2(a, b)
+cudaError_t B200Q_CAT(resident_launch_part, B200Q_PART)(int var, const ResidentParams& p, int mt, int ng, int smem_bytes,
+                                                         cudaStream_t stream) {
+  return launch_var<0>(var, p, mt, ng, smem_bytes, stream);
+}
+
+}  // namespace b200q
