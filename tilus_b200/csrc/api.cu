@@ -49,8 +49,8 @@ B200Q_DECL_RPART(4) B200Q_DECL_RPART(5) B200Q_DECL_RPART(6) B200Q_DECL_RPART(7)
 int exact_smem_bytes(int bits, int stages, int M);
 int exact_stages(int bits, int max_smem, int M);
 int batch_max_clusters(int c);
-int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg);
-void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages);
+int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg, int cluster);
+void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int* stages, int* a_stages);
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg);
 int umma_a_stages(int tm, int bits, int max_smem, int rpg);
 
@@ -429,9 +429,10 @@ static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; 
 //  - equal runs of 128-row groups, one per SM: no SM idles, but the tiles' sums meet in L2;
 //  - a cluster of c CTAs per tile: sums meet in distributed shared memory (at most as many tiles as clusters fit);
 //  - one CTA per tile.
-// The times are fits to chains of launches on B200 (4-bit weights in fp16, us; 2048^2 .. 4096 x 14336, 16 .. 128 rows, each
+// The times are fits to chains of launches on B200 (4-bit weights in fp16, us; 1024 x 4096 .. 4096 x 14336, 16 .. 128 rows, each
 // form forced; within 15 % there) and serve every width and both activation types: for 100 x 11008 x 4224, 6 bits in
-// bf16, they say 16.1 where a call takes 20.2.  Fewer CTAs start and end cheaper because the next launch finds SMs free.
+// bf16, they say 16.1 where a call takes 20.2.  Fewer CTAs start and end cheaper because the next launch finds SMs free (17 x 2048 x
+// 4096, 4 / 6 CTAs per tile, that is 64 / 96 CTAs, 4.5 / 5.7 us, equal runs 6.0; 64 x 4096 x 4096, 2 / 3 / 4 per tile 8.5 / 8.6 / 8.6).
 static int max_clusters(int c) {
   static int cache[16][9];
   int dev = 0;
@@ -446,16 +447,25 @@ static int max_clusters(int c) {
 static void batch_split(int M, int group, int n_tiles, int G, const DeviceInfo& di, int* ctas, int* cluster) {
   long long grid = ((long long)n_tiles * G + 1) / 2;  // at least two groups per CTA
   if (grid > di.sm_count) grid = di.sm_count;
-  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * ((double)n_tiles * G / grid);
+  const bool exact = batch_exact(M, group), shares = !exact && batch_shares_sm(batch_rows(M));
+  const double groups = (double)n_tiles * G / grid;
+  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * groups;
   *ctas = (int)grid;
   *cluster = 1;
-  // (kernels whose CTAs share SMs stay with equal runs: CTAs of such launches must not meet two to an SM while
-  // others idle; the exact kernel's registers allow one CTA per SM)
-  const bool one_per_sm = batch_exact(M, group) || !batch_shares_sm(batch_rows(M));
-  for (int c = 1; c <= 8 && one_per_sm; ++c) {
+  // (Kernels whose CTAs share SMs stay with equal runs: CTAs of cluster launches must not meet two to an SM while others idle, and the
+  // two kinds mixed wait for each other's SMs - a Llama-3-8B block at 17 rows 69 us with clusters for its narrow layers, 49 without.
+  // The exact kernel's registers allow one CTA per SM.)
+  for (int c = 1; c <= 8 && !shares; ++c) {
     if ((c > 1 && G < 2 * c) || n_tiles * c > di.sm_count || (c > 1 && n_tiles > max_clusters(c))) continue;
-    const double start = 0.05 * (n_tiles * c) - 1.1;
-    const double t = (start > 2.3 ? start : 2.3) + 0.033 * M + 0.29 * ((G + c - 1) / c);
+    const int each = (G + c - 1) / c;
+    double t;
+    if (exact) {
+      const double start = 0.05 * (n_tiles * c) - 1.1;
+      t = (start > 2.3 ? start : 2.3) + 0.033 * M + 0.29 * each;
+    } else {
+      const bool overlap = 2 * n_tiles * c <= di.sm_count;  // the next launch finds SMs free
+      t = 0.03 * M + (c == 1 ? (overlap ? 2.0 : 3.5) + 0.28 * each : overlap ? 2.0 + 0.29 * each : 4.0 + 0.33 * each) + (c > 6 ? 0.8 : 0.0);
+    }
     if (t < best) {
       best = t;
       *ctas = n_tiles * c;
@@ -477,8 +487,8 @@ static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInf
     pl->smem_bytes = exact_smem_bytes(bits, pl->stages, M);
   } else {
     int a_stages;
-    batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), &pl->stages, &a_stages);
-    pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group));
+    batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), cluster, &pl->stages, &a_stages);
+    pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group), cluster);
   }
   if (!exact && !batch_shares_sm(batch_rows(M)) && pl->smem_bytes < kOneCtaSmem) pl->smem_bytes = kOneCtaSmem;
   pl->tile_m = batch_rows(M);
@@ -657,7 +667,10 @@ static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInf
 //    up to 8192 rows of K two column tiles per CTA, 1 and 2 bits one (4096 x 8192, 4 bits 0.98, 6144 x 8192 1.03);
 //    beyond, 8-bit integers (0.94 .. 0.97) and 4 bits up to 3072 columns (0.82 .. 0.96);
 //  - 9 to 16 rows (fp16 only: the exact kernel takes bfloat16 as it is), whose second set of sums makes the loop 1.5 times longer: up to
-//    4096 rows of K in the ranges below 0.63 .. 0.96; beyond 1.0 .. 1.3.
+//    4096 rows of K in the ranges below 0.63 .. 0.96; beyond 1.0 .. 1.3.  Among layers that stay with the exact kernel, whose launches
+//    leave SMs to their successors, a launch on all SMs costs those up to 2 us: with 4096 x 4096 here a Llama-3-8B block takes, us, at 9
+//    / 13 / 16 rows 47.2 / 49.3 / 51.1 in 4 bits (50.1 / 51.1 / 50.3 without), 54.0 / 54.8 / 57.7 in 8 bits (54.5 / 54.9 / 55.7), 58.1 /
+//    60.2 / 61.2 in 3 bits (62.5 / 63.1 / 62.2), 59.8 / 61.6 / 63.4 in float6 (62.9 / 63.5 / 62.8): 8 bits up to 12 rows, 4 bits up to 14.
 // S: one CTA per cluster where a warp's activations fit its registers, and where K is long or the columns few; us, 8 rows,
 // S = 1 / 2 / 4: 8192 x 8192 11.5 / 10.6 / 12.7, 4096 x 14336 - / 12.1 / 10.5, 28672 x 14336 - / 45.1 / 45.2.
 static int resident_cluster(int M, int N, int K, int var, int group, int act, bool stream_form, const DeviceInfo& di) {
@@ -665,7 +678,8 @@ static int resident_cluster(int M, int N, int K, int var, int group, int act, bo
   const int G = K / 128, bits = var_bits(var);
   int S;
   if (M > 8) {
-    if (G > 32 || N > (G > 16 ? 11008 : G == 16 ? 6144 : 4096) || (G > 16 && N < 3072 && M > 12)) return 0;
+    if (G > 32 || N > (G > 16 ? (M > 12 ? 4096 : 11008) : G == 16 ? 6144 : 4096) || (G > 16 && N < 3072 && M > 12)) return 0;
+    if (G > 16 && ((bits == 8 && M > 12) || (bits == 4 && M > 14))) return 0;
     S = 1;
   } else {
     S = G <= 40 || (G <= 64 && M < 5 && N < 8192) ? 1 : G <= 64 || (N >= 16384 && G <= 128) ? 2 : 4;
@@ -901,11 +915,11 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   p.rpg = rpg_of(group);
   p.rows = rows;
   const bool exact = batch_exact(M, group);
-  batch_stages(bits, device_info().max_smem, rows, p.rpg, &p.stages, &p.a_stages);
+  batch_stages(bits, device_info().max_smem, rows, p.rpg, p.cluster, &p.stages, &p.a_stages);
   if (exact) p.stages = exact_stages(bits, device_info().max_smem, M);
   p.grid = (int)grid;
   p.act = act;
-  int smem = exact ? exact_smem_bytes(bits, p.stages, M) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg);
+  int smem = exact ? exact_smem_bytes(bits, p.stages, M) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg, p.cluster);
   if (!exact && (p.cluster > 1 || !batch_shares_sm(rows)) && smem < kOneCtaSmem) smem = kOneCtaSmem;
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
   cudaError_t e = exact ? exact_launch(var, p, tmaps, smem, stream) : batch_launch(var, p, tmaps, smem, stream);

@@ -73,6 +73,10 @@ __device__ __forceinline__ void cluster_arrive() {  // orders shared memory acce
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive_relaxed() {  // orders nothing
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() {
   __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -74,9 +74,20 @@ struct BatchBarriers {
   uint64_t g_full[BATCH_STAGES_MAX], g_empty[BATCH_STAGES_MAX];
   uint64_t d_full[2], d_empty[2];
   uint64_t run_done;  // the MMAs of the whole run have completed
+  uint64_t sums_full[4];  // cluster form, per lane quadrant: all CTAs' sums of this CTA's rows are here
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+constexpr int BATCH_BARRIERS = (int)(offsetof(BatchBarriers, tmem_base) / 8);
+// arrivals that complete a phase of the i-th barrier
+__host__ __device__ constexpr int batch_barrier_count(int i) {
+  return i < (int)(offsetof(BatchBarriers, done) / 8) ? 4
+       : i < (int)(offsetof(BatchBarriers, g_full) / 8) ? 1
+       : i < (int)(offsetof(BatchBarriers, g_empty) / 8) ? 2
+       : i < (int)(offsetof(BatchBarriers, d_full) / 8) ? 4
+       : i < (int)(offsetof(BatchBarriers, d_empty) / 8) ? 1
+       : i < (int)(offsetof(BatchBarriers, run_done) / 8) ? 4 : 1;
+}
 
 // tensor memory (all 512 columns): two D accumulators of nr columns, then as many operand slots as fit
 __host__ __device__ constexpr int batch_d_stride(int nr) { return nr <= 64 ? 64 : 128; }
@@ -118,9 +129,80 @@ __device__ __forceinline__ void batch_epilogue(const BatchParams& p, uint32_t d_
   if (!whole) batch_finish<ACT>(p, tile, len, wq, lane, part, parts);
 }
 
-template <int VAR, int ACT>
-__global__ void __launch_bounds__(BATCH_THREADS, 1)
-batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
+// The end of a column tile whose K a cluster shares, by the twelve warps that know of tensor memory.  The rows are cut into quads of four,
+// of which the CTAs own equal shares (the last ones what is left).  A warp takes 16 rows of its 32 columns at a time from tensor
+// memory to the CTA's own shared memory (over the activations: all MMAs have completed), [quad][32] float4, and sends each owner
+// its quads with one bulk copy, which counts its bytes in on the owner's barrier of the lane quadrant.  The owner adds the
+// CTAs' sums in rank order and writes C.  A CTA that has all of its sums says so on the cluster's barrier and waits for the others
+// before it leaves, since until then its own copies may not have been read.  (64 x 4096 x 4096, three CTAs per tile, us per launch: sums
+// left in place and fetched by their owners between two barriers of the cluster 9.8, the last 3 of them; sent word by word 9.2.)
+__host__ __device__ constexpr int batch_own_quads(int quads, int cluster) { return (quads + cluster - 1) / cluster; }
+template <int ACT>
+__device__ __forceinline__ void cluster_epilogue(const BatchParams& p, uint32_t tmem, const unsigned char* smem, uint32_t smem_s,
+                                                 uint32_t sums_off, uint32_t run_done, uint32_t full, int tile, int warp, int lane,
+                                                 volatile int* abort_flag) {
+  const int wq = warp & 3, part = warp >> 2, rank = blockIdx.x % p.cluster;
+  const int quads = (p.M + 3) / 4, own = batch_own_quads(quads, p.cluster);
+  const int q0 = min(quads, rank * own), q1 = min(quads, q0 + own);  // this CTA's
+  const uint32_t sent = smem_s + (uint32_t)(wq * quads) * 512u;
+  const uint32_t got_off = sums_off + (uint32_t)(wq * p.cluster * own) * 512u;  // [CTA][owned quad][32]
+  bool ok = mbar_wait_abortable(run_done, 0u, abort_flag);
+  if (__all_sync(0xffffffffu, ok ? 1 : 0)) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (part == 0 && lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)((q1 - q0) * p.cluster) * 512u)
+                   : "memory");
+    for (int c0 = part * 4; c0 < quads; c0 += 12) {
+      uint32_t v[16];
+      tmem_ld_16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(c0 * 4), v);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (c0 + u < quads)
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sent + (uint32_t)((c0 + u) * 512 + lane * 16)), "r"(v[4 * u]),
+                       "r"(v[4 * u + 1]), "r"(v[4 * u + 2]), "r"(v[4 * u + 3])
+                       : "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (elect_one()) {
+      for (int c0 = part * 4; c0 < quads; c0 += 12) {
+        const int c1 = min(quads, c0 + 4);
+        for (int q = c0, owner = c0 / own; q < c1; ++owner) {
+          const int next = min(c1, (owner + 1) * own);
+          uint32_t dst, bar;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
+                       : "r"(smem_s + got_off + (uint32_t)(rank * own + q - owner * own) * 512u), "r"(owner));
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(full), "r"(owner));
+          asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                       "r"(sent + (uint32_t)q * 512u), "r"((uint32_t)(next - q) * 512u), "r"(bar)
+                       : "memory");
+          q = next;
+        }
+      }
+    }
+    __syncwarp();
+    ok = mbar_wait_abortable(full, 0u, abort_flag);
+    ok = __all_sync(0xffffffffu, ok ? 1 : 0);
+  } else {
+    ok = false;
+  }
+  cluster_arrive_relaxed();
+  if (!ok) return;
+  const float4* parts = reinterpret_cast<const float4*>(smem + got_off) + lane;
+#pragma unroll 2
+  for (int q = part; q < q1 - q0; q += 3) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int r = 0; r < p.cluster; ++r) {
+      const float4 x = parts[(r * own + q) * 32];
+      sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+    }
+    batch_store4<ACT>(p, tile * 128 + wq * 32 + lane, lane, (q0 + q) * 4, sum);
+  }
+}
+
+template <int VAR, int ACT, bool CLUSTER>
+__device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorMap& tmap_a, const CUtensorMap& tmap_w) {
   constexpr int B = var_bits(VAR);
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_unaligned = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -132,6 +214,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   const uint32_t ring_off = (uint32_t)AS * ASTAGE, scales_off = ring_off + (uint32_t)WS * WSTAGE;
   const uint32_t ring_s = smem_base + ring_off, scales_s = smem_base + scales_off;
   const uint32_t bars_off = scales_off + (uint32_t)WS * SSTAGE;
+  const uint32_t sums_off = bars_off + (uint32_t)((sizeof(BatchBarriers) + 127) / 128 * 128);  // what a cluster's CTAs send
   BatchBarriers* bars = reinterpret_cast<BatchBarriers*>(smem_al + bars_off);
   const uint32_t bars_s = smem_base + bars_off;
 #define BAR_ADDR(field, i) (bars_s + (uint32_t)offsetof(BatchBarriers, field) + (uint32_t)(i) * 8u)
@@ -142,24 +225,28 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   // this CTA's run of groups, counted tile by tile over the whole matrix
   const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
 
-  if (tid == 0) {
-    for (int i = 0; i < BATCH_SLOTS_MAX; ++i) { mbar_init(BAR_ADDR(slot_full, i), 4); mbar_init(BAR_ADDR(done, i), 1); }
-    for (int i = 0; i < AS; ++i) mbar_init(BAR_ADDR(a_full, i), 1);
-    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
-    for (int i = 0; i < 2; ++i) { mbar_init(BAR_ADDR(d_full, i), 1); mbar_init(BAR_ADDR(d_empty, i), 4); }
-    mbar_init(BAR_ADDR(run_done, 0), 1);
-    bars->abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
-  }
-  __syncthreads();
-  // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
-  // this SM may still hold it)
   constexpr int TM_THREADS = BATCH_SETS * 128 + 160;
   constexpr int W_EPI = BATCH_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
                 W_SCALES = W_EPI + 7;
+  // (The descriptors are on their way while the barriers are set up, by the lanes of one warp.  Thread 0 alone took 1800 cycles
+  // for both, ahead of the first copies.)
+  if (warp == W_WEIGHTS && lane == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+  }
+  if (warp == 0) {
+    for (int i = lane; i < BATCH_BARRIERS; i += 32) mbar_init(bars_s + (uint32_t)i * 8u, (uint32_t)batch_barrier_count(i));
+    if (lane == 0) bars->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  if constexpr (CLUSTER) {  // (the peers' barriers are there before anything is sent to them)
+    cluster_arrive();
+    cluster_wait();
+  }
+  // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
+  // this SM may still hold it)
   if (warp == W_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      bars_s + (uint32_t)offsetof(BatchBarriers, tmem_base))
@@ -238,7 +325,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
       stage += BATCH_SETS;
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
-    if (good && p.cluster <= 1) {
+    if (!CLUSTER && good) {
       int pos = run0, seg = 0;  // the last segment
       while (pos / p.G != (run1 - 1) / p.G) { pos = (pos / p.G + 1) * p.G; ++seg; }
       SEGMENT(pos)
@@ -255,7 +342,7 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
     int seg = 0;
-    for (int pos = run0; pos < run1 && p.cluster <= 1; ++seg) {
+    for (int pos = run0; pos < run1 && !CLUSTER; ++seg) {
       SEGMENT(pos)
       if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -416,22 +503,14 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     }
   }
 
-  if (p.cluster > 1 && warp < W_ACT) {
-    // the tile's sums to shared memory, over activations and ring (all MMAs have completed: nobody reads them)
+  if constexpr (CLUSTER) {
     __syncwarp();
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
-    if (mbar_wait_abortable(BAR_ADDR(run_done, 0), 0u, abort_flag)) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float4* sums = reinterpret_cast<float4*>(smem_al) + (warp & 3) * 32 + lane;
-      for (int c0 = (warp >> 2) * 16; c0 < p.M; c0 += 48) {
-        uint32_t v[16];
-        tmem_ld_16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (c0 + 4 * i < p.M)
-            sums[(c0 / 4 + i) * 128] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                                   __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-      }
+    if (warp < W_ACT) {
+      asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
+      cluster_epilogue<ACT>(p, tmem, smem_al, smem_base, sums_off, BAR_ADDR(run_done, 0), BAR_ADDR(sums_full, warp & 3), run0 / p.G,
+                            warp, lane, abort_flag);
+    } else {
+      cluster_arrive_relaxed();
     }
   }
 
@@ -449,22 +528,28 @@ batch_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
-  if (p.cluster > 1) {
-    cluster_arrive();
-    cluster_wait();
-    if (warp < W_ACT && !*abort_flag)
-      cluster_finish<ACT, 1>(p, smem_base, 0u, blockIdx.x % p.cluster, run0 / p.G, (warp & 3) * 32 + lane, lane,
-                          warp >> 2, 3);
-    cluster_arrive();  // nobody leaves while its sums are being read
-    cluster_wait();
-  }
+  if constexpr (CLUSTER) cluster_wait();  // everybody has what was sent from here, and nothing more is on its way here
 #undef BAR_ADDR
 #undef SEGMENT
 }
 
+// Equal runs, and a cluster of CTAs per column tile.  Two CTAs of the former have registers on an SM (64, see batch_stages) for the types
+// named there; 7-bit integers in bfloat16 have to be told (72 otherwise).
 template <int VAR, int ACT>
+__global__ void __launch_bounds__(BATCH_THREADS, !var_is_float(VAR) && var_bits(VAR) == 7 ? 2 : 1)
+batch_kernel(const __grid_constant__ BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
+  batch_body<VAR, ACT, false>(p, tmap_a, tmap_w);
+}
+template <int VAR, int ACT>
+__global__ void __launch_bounds__(BATCH_THREADS, 1)
+tile_cluster_kernel(const __grid_constant__ BatchParams p, const __grid_constant__ CUtensorMap tmap_a,
+                    const __grid_constant__ CUtensorMap tmap_w) {
+  batch_body<VAR, ACT, true>(p, tmap_a, tmap_w);
+}
+
+template <int VAR, int ACT, bool CLUSTER>
 static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
-  auto kern = batch_kernel<VAR, ACT>;
+  auto kern = CLUSTER ? tile_cluster_kernel<VAR, ACT> : batch_kernel<VAR, ACT>;
   static std::atomic<bool> allowed[16];
   const cudaError_t e = allow_smem(kern, allowed);
   if (e != cudaSuccess) return e;
@@ -489,9 +574,13 @@ template <int VAR>
 static cudaError_t batch_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
                                     cudaStream_t stream) {
   if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
-    if (var == VAR)
-      return p.act == 0 ? batch_launch_one<VAR, 0>(p, tmaps, smem_bytes, stream)
-                        : batch_launch_one<VAR, 1>(p, tmaps, smem_bytes, stream);
+    if (var == VAR) {
+      if (p.cluster > 1)
+        return p.act == 0 ? batch_launch_one<VAR, 0, true>(p, tmaps, smem_bytes, stream)
+                          : batch_launch_one<VAR, 1, true>(p, tmaps, smem_bytes, stream);
+      return p.act == 0 ? batch_launch_one<VAR, 0, false>(p, tmaps, smem_bytes, stream)
+                        : batch_launch_one<VAR, 1, false>(p, tmaps, smem_bytes, stream);
+    }
   }
   if constexpr (VAR + 1 < VAR_COUNT) return batch_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
   else return cudaErrorInvalidValue;
@@ -509,7 +598,7 @@ cudaError_t B200Q_CAT(batch_launch_part, B200Q_PART)(int var, const BatchParams&
 #if B200Q_PART == 0
 // clusters of c CTAs that the current device holds at a time with one CTA per SM; 0 without a device
 int batch_max_clusters(int c) {
-  auto kern = batch_kernel<0, 0>;
+  auto kern = tile_cluster_kernel<0, 0>;
   const int smem = 200 * 1024;
   static std::atomic<bool> allowed[16];
   if (allow_smem(kern, allowed) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
@@ -528,9 +617,10 @@ int batch_max_clusters(int c) {
   if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
   return n;
 }
-// dynamic shared memory: alignment slack + activation groups + packed ring + scales + barriers
-int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
-  return 1024 + a_stages * rows * 256 + stages * batch_stage_bytes(bits, rpg) + (int)sizeof(BatchBarriers);
+// dynamic shared memory: alignment slack + activation groups + packed ring + scales + barriers + what a cluster's CTAs send
+int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg, int cluster) {
+  return 1024 + a_stages * rows * 256 + stages * batch_stage_bytes(bits, rpg) + (int)sizeof(BatchBarriers) +
+         (cluster > 1 ? 128 + batch_own_quads(rows / 4, cluster) * cluster * 2048 : 0);
 }
 // Activation groups (at most as many as there are operand slots) and ring stages (a multiple of the dequantize
 // sets) in the rest.  Up to 32 rows a CTA stays within half an SM's shared memory, so that the next launch of the
@@ -541,11 +631,12 @@ int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg) {
 // 24 x 8192 x 8192 24.8 us, 14.8 with 4 bits).  Above, a CTA takes more than half: the activations leave
 // too little for the ring, and launches that leave SMs free (clusters, one CTA per column tile) would meet others
 // two to an SM, where one waits for the other's tensor memory (64 rows: 81 us with the two kinds mixed, 62).
-void batch_stages(int bits, int max_smem, int rows, int rpg, int* stages, int* a_stages) {
-  const int cap = batch_shares_sm(rows) ? 113 * 1024 : max_smem;
+void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int* stages, int* a_stages) {
+  const int cap = batch_shares_sm(rows) && cluster <= 1 ? 113 * 1024 : max_smem;
   *a_stages = rows <= 64 ? 6 : 4;
+  while (*a_stages > 2 && batch_smem_bytes(bits, BATCH_SETS, *a_stages, rows, rpg, cluster) > cap) --*a_stages;  // (8 bits, 128 rows, a cluster)
   int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
-  while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg) > cap) st -= BATCH_SETS;
+  while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg, cluster) > cap) st -= BATCH_SETS;
   *stages = st;
 }
 #endif

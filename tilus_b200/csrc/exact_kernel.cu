@@ -68,6 +68,13 @@ struct ExactBarriers {
   uint32_t tmem_base;
   volatile int abort_flag;
 };
+constexpr int EXACT_BARRIERS = (int)(offsetof(ExactBarriers, tmem_base) / 8);
+// arrivals that complete a phase of the i-th barrier
+__host__ __device__ constexpr int exact_barrier_count(int i) {
+  return i < (int)(offsetof(ExactBarriers, done) / 8) ? 4
+       : i < (int)(offsetof(ExactBarriers, g_full) / 8) ? 1
+       : i < (int)(offsetof(ExactBarriers, g_empty) / 8) ? 2 : 4;
+}
 
 template <int VAR, int ACT>
 __global__ void __launch_bounds__(EXACT_THREADS, 1)
@@ -96,24 +103,21 @@ exact_kernel(const BatchParams p, const __grid_constant__ CUtensorMap tmap_a, co
   // this CTA's run of groups, counted tile by tile over the whole matrix
   const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
 
-  if (tid == 0) {
-    for (int i = 0; i < EXACT_SLOTS; ++i) {
-      mbar_init(BAR_ADDR(slot_full, i), 4);
-      mbar_init(BAR_ADDR(done, i), 1);
-      mbar_init(BAR_ADDR(a_full, i), 1);
-    }
-    for (int i = 0; i < WS; ++i) { mbar_init(BAR_ADDR(g_full, i), 2); mbar_init(BAR_ADDR(g_empty, i), 4); }
-    for (int i = 0; i < EXACT_SETS; ++i) { mbar_init(BAR_ADDR(hand_full, i), 4); mbar_init(BAR_ADDR(hand_empty, i), 4); }
-    bars->abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  constexpr int W_EPI = EXACT_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6;
+  // (by the lanes of one warp while the descriptors are on their way, as in batch_kernel.cu)
+  if (warp == W_WEIGHTS && lane == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+  }
+  if (warp == 0) {
+    for (int i = lane; i < EXACT_BARRIERS; i += 32) mbar_init(bars_s + (uint32_t)i * 8u, (uint32_t)exact_barrier_count(i));
+    if (lane == 0) bars->abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
   // the producers may start; the roles that use tensor memory wait for it below (the previous launch's CTA on
   // this SM may still hold it)
-  constexpr int W_EPI = EXACT_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6;
   if (warp == W_MMA) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      bars_s + (uint32_t)offsetof(ExactBarriers, tmem_base))
