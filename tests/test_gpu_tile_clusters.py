@@ -45,3 +45,30 @@ def test_rings_beside_the_sums(M, dt, zp, group, act):
 def test_clusters_of_few_rows_by_an_edited_plan(M):
     """Up to 16 rows the exact kernel's clusters, up to 32 a form that no plan has."""
     _check(M, 1040, 2048, D.int4b, 0, 64, 4)
+
+
+@pytest.mark.parametrize("M,N,K,dt,group,act", [
+    (40, 36864, 512, D.uint4b, 128, torch.float16),   # 288 column tiles, two for each of 144 CTAs
+    (17, 20000, 512, D.uint4b, 128, torch.float16),   # 157 tiles, whole ones, 79 CTAs of which one has a single tile
+    (32, 16384, 1024, D.uint2b, 128, torch.float16),  # 128 whole tiles, two CTAs to an SM
+    (65, 2064, 1024, D.int6b, 64, torch.bfloat16),    # one tile per CTA beyond 64 rows: three sets, one accumulator
+    (128, 1168, 2048, D.uint8, 64, torch.float16),    # the same with a ring too short for three sets
+    (24, 4112, 2048, D.int8, 128, torch.float16),     # few rows of a wide type: three sets, the SM to itself
+    (32, 2064, 8192, D.float6_e3m2, 8192, torch.bfloat16),
+    (9, 1040, 1152, D.int3b, 32, torch.float16)], ids=str)
+def test_whole_tiles_and_sets(M, N, K, dt, group, act):
+    """Splits of the planned launches where CTAs have whole column tiles, and the number of dequantizing sets."""
+    dev = torch.device("cuda:0")
+    zp = 1 << (dt.nbits - 1) if dt.kind == D.KIND_UINT else 0
+    gen = torch.Generator(device=dev).manual_seed(M)
+    bq = torch.randint(0, 256, (N * K * dt.nbits // 8,), dtype=torch.uint8, device=dev, generator=gen)
+    sc = (torch.rand(K // group, N, device=dev, generator=gen) * 0.01 + 0.005).to(act)
+    a = torch.randn(M, K, device=dev, generator=gen).to(act)
+    ref = a.double() @ ops.dequantize(bq, sc, dt, group, zp).double()
+    ws = torch.zeros(ops.workspace_bytes(M, N, K, dt, zp, group), dtype=torch.uint8, device=dev)
+    outs = [ops.quantized_matmul(a, bq, sc, dt, group, zp, workspace=ws) for _ in range(10)]
+    eps = 2.0 ** -11 if act == torch.float16 else 2.0 ** -8  # as above
+    assert bool(((outs[0].double() - ref).abs() <= eps * ref.abs() + 2e-5 * ref.abs().max()).all())
+    for c in outs[1:]:
+        assert torch.equal(c, outs[0])
+    assert int(ws.count_nonzero()) == 0

@@ -50,7 +50,7 @@ int exact_smem_bytes(int bits, int stages, int M);
 int exact_stages(int bits, int max_smem, int M);
 int batch_max_clusters(int c);
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg, int cluster);
-void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int* stages, int* a_stages);
+void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int sets, int* stages, int* a_stages);
 int umma_smem_bytes(int tm, int bits, int a_stages, int rpg);
 int umma_a_stages(int tm, int bits, int max_smem, int rpg);
 
@@ -428,7 +428,7 @@ static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; 
 // How the column tiles are shared out, as (CTAs, CTAs per cluster):
 //  - equal runs of 128-row groups, one per SM: no SM idles, but the tiles' sums meet in L2;
 //  - a cluster of c CTAs per tile: sums meet in distributed shared memory (at most as many tiles as clusters fit);
-//  - one CTA per tile.
+//  - whole tiles, as many per CTA as one round takes.
 // The times are fits to chains of launches on B200 (4-bit weights in fp16, us; 1024 x 4096 .. 4096 x 14336, 16 .. 128 rows, each
 // form forced; within 15 % there) and serve every width and both activation types: for 100 x 11008 x 4224, 6 bits in
 // bf16, they say 16.1 where a call takes 20.2.  Fewer CTAs start and end cheaper because the next launch finds SMs free (17 x 2048 x
@@ -444,40 +444,63 @@ static int max_clusters(int c) {
   if (dev < 16) cache[dev][c] = n + 1;
   return n;
 }
-static void batch_split(int M, int group, int n_tiles, int G, const DeviceInfo& di, int* ctas, int* cluster) {
+// Dequantizing sets of a CTA of batch_kernel.cu: three, since two leave a third of the time to latencies (64 x 16384 x 4096,
+// 4 bits 15.6 / 14.6 us, 100 x 11008 x 4224, 6 bits in bfloat16 20.3 / 18.7), but beyond 64 rows only where every CTA has one column tile to
+// itself and the ring two stages per set: tensor memory then holds a single accumulator next to three sets' slots (128 x 28672 x 4096
+// 32.4 / 34.7), and a cluster's ring gets too short (128 x 4096 x 14336 18.7 / 20.7; in 8 bits with scales per 64 rows 119 x 9920 x 4096 19.6 /
+// 21.9).  Two for types of which two CTAs share an SM.
+static int batch_sets(int var, int rows, int rpg, int cluster, bool one_tile, const DeviceInfo& di) {
+  if (rows <= 64) return batch_shares_sm(rows, var) && cluster <= 1 ? 2 : 3;
+  int stages, a_stages;
+  batch_stages(var_bits(var), di.max_smem, rows, rpg, 1, 3, &stages, &a_stages);
+  return cluster == 1 && one_tile && stages >= 6 ? 3 : 2;
+}
+static void batch_split(int M, int var, int group, int n_tiles, int G, const DeviceInfo& di, int* ctas, int* cluster) {
   long long grid = ((long long)n_tiles * G + 1) / 2;  // at least two groups per CTA
   if (grid > di.sm_count) grid = di.sm_count;
-  const bool exact = batch_exact(M, group), shares = !exact && batch_shares_sm(batch_rows(M));
+  const bool exact = batch_exact(M, group), shares = !exact && batch_shares_sm(batch_rows(M), var);
   const double groups = (double)n_tiles * G / grid;
-  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * groups;
+  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * groups + (!exact && groups > 24 ? 0.12 * (groups - 24) : 0.0);
   *ctas = (int)grid;
   *cluster = 1;
-  // (Kernels whose CTAs share SMs stay with equal runs: CTAs of cluster launches must not meet two to an SM while others idle, and the
-  // two kinds mixed wait for each other's SMs - a Llama-3-8B block at 17 rows 69 us with clusters for its narrow layers, 49 without.
-  // The exact kernel's registers allow one CTA per SM.)
-  for (int c = 1; c <= 8 && !shares; ++c) {
-    if ((c > 1 && G < 2 * c) || n_tiles * c > di.sm_count || (c > 1 && n_tiles > max_clusters(c))) continue;
-    const int each = (G + c - 1) / c;
+  // Kernels whose CTAs share SMs have no clusters: CTAs of cluster launches must not meet two to an SM while others idle, and the
+  // two kinds mixed wait for each other's SMs (a Llama-3-8B block at 17 rows 69 us with clusters for its narrow layers, 49 without).
+  // The exact kernel's registers allow one CTA per SM.
+  for (int c = 1; c <= (shares ? 1 : 8); ++c) {
+    const int tiles = c == 1 && !exact ? (n_tiles + di.sm_count - 1) / di.sm_count : 1;  // whole column tiles of a CTA
+    const int n = (n_tiles + tiles - 1) / tiles * c;
+    if (shares && 2 * n <= di.sm_count) continue;  // (the next launch's CTAs would meet these, 28 x 3200 x 1280 on 25 CTAs 6.2 us for 5.4)
+    if ((c > 1 && G < 2 * c) || n > di.sm_count || (c > 1 && n_tiles > max_clusters(c))) continue;
+    const int each = tiles * ((G + c - 1) / c);
     double t;
     if (exact) {
-      const double start = 0.05 * (n_tiles * c) - 1.1;
+      const double start = 0.05 * n - 1.1;
       t = (start > 2.3 ? start : 2.3) + 0.033 * M + 0.29 * each;
     } else {
-      const bool overlap = 2 * n_tiles * c <= di.sm_count;  // the next launch finds SMs free
-      t = 0.03 * M + (c == 1 ? (overlap ? 2.0 : 3.5) + 0.28 * each : overlap ? 2.0 + 0.29 * each : 4.0 + 0.33 * each) + (c > 6 ? 0.8 : 0.0);
+      const bool overlap = 2 * n <= di.sm_count;  // the next launch finds SMs free
+      t = 0.03 * M + (c > 6 ? 0.8 : 0.0);
+      if (c == 1) t += (overlap ? 2.0 : 3.5) + 0.28 * each + (each > 32 ? 0.08 * (each - 32) : 0.0);
+      else t += (overlap ? 2.0 + 0.29 * each : 4.0 + 0.33 * each) + (M > 64 ? 0.05 * (M - 64) / c : 0.0);
     }
     if (t < best) {
       best = t;
-      *ctas = n_tiles * c;
+      *ctas = n;
       *cluster = c;
     }
   }
 }
-static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInfo& di, b200q_plan_t* pl) {
+// Equal runs on so many CTAs are whole column tiles, none of which is shared.
+static bool batch_whole_tiles(int n_tiles, int ctas, int cluster, const DeviceInfo& di) {
+  const int tiles = (n_tiles + di.sm_count - 1) / di.sm_count;
+  return cluster <= 1 && ctas == (n_tiles + tiles - 1) / tiles;
+}
+static void plan_batch(int M, int N, int K, int var, int group, const DeviceInfo& di, b200q_plan_t* pl) {
   int ctas, cluster;
-  batch_split(M, group, (N + 127) / 128, K / 128, di, &ctas, &cluster);
+  const int bits = var_bits(var);
+  batch_split(M, var, group, (N + 127) / 128, K / 128, di, &ctas, &cluster);
   pl->kernel = 3;
   const bool exact = batch_exact(M, group);
+  const int sets = batch_sets(var, batch_rows(M), rpg_of(group), cluster, ctas == (N + 127) / 128, di);
   pl->m_tiles = 1;
   pl->splits = 1;
   pl->cluster = cluster;
@@ -487,12 +510,12 @@ static void plan_batch(int M, int N, int K, int bits, int group, const DeviceInf
     pl->smem_bytes = exact_smem_bytes(bits, pl->stages, M);
   } else {
     int a_stages;
-    batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), cluster, &pl->stages, &a_stages);
+    batch_stages(bits, di.max_smem, batch_rows(M), rpg_of(group), cluster, sets, &pl->stages, &a_stages);
     pl->smem_bytes = batch_smem_bytes(bits, pl->stages, a_stages, batch_rows(M), rpg_of(group), cluster);
   }
-  if (!exact && !batch_shares_sm(batch_rows(M)) && pl->smem_bytes < kOneCtaSmem) pl->smem_bytes = kOneCtaSmem;
+  if (!exact && (cluster > 1 || !batch_shares_sm(batch_rows(M), var)) && pl->smem_bytes < kOneCtaSmem) pl->smem_bytes = kOneCtaSmem;
   pl->tile_m = batch_rows(M);
-  pl->warps = exact ? 20 : 16;
+  pl->warps = exact || sets == 3 ? 20 : 16;
   pl->passes = 1;
   pl->pdl = 1;  // always launched as a programmatic dependent
 }
@@ -731,7 +754,7 @@ static int make_plan_uncached(int M, int N, int K, int var, int group, int act, 
   }
   // up to 128 rows the small-batch kernels (weights streamed once); beyond, the prefill kernel
   if (M <= kBatchMaxRows) {
-    plan_batch(M, N, K, bits, group, di, pl);
+    plan_batch(M, N, K, var, group, di, pl);
     pl->workspace_bytes = WS_HEADER_BYTES + ws_counter_bytes(N) + batch_scratch_bytes(M, N);
     if (batch_exact(M, group)) pl->resident = resident_cluster(M, N, K, var, group, act, false, di);
     if (M <= kStreamMaxRows && stream_takes(K, group)) {  // the decode path's other form, see b200q_plan_t
@@ -873,6 +896,7 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   const int rows = batch_rows(M), n_tiles = (N + 127) / 128, G = K / 128;
   const size_t fixed = WS_HEADER_BYTES + ws_counter_bytes(N);
   if (!workspace || ws_bytes < fixed || ((uintptr_t)workspace & 255)) return ST_WORKSPACE;
+  const bool exact = batch_exact(M, group);
   BatchParams p;
   p.work = n_tiles * G;
   p.unit = 1;
@@ -883,6 +907,9 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   p.cluster = pl.cluster > 1 && pl.cluster <= 8 && grid == (long long)n_tiles * pl.cluster && G >= 2 * pl.cluster ? pl.cluster : 1;
   if (p.cluster > 1) {
     // (distributed shared memory needs no scratch)
+  } else if (!exact && batch_whole_tiles(n_tiles, (int)grid, 1, device_info())) {
+    p.work = n_tiles;
+    p.unit = G;
   } else if (ws_bytes < fixed + batch_scratch_bytes(M, N)) {  // a caller with a smaller workspace: whole tiles need none
     p.work = n_tiles;
     p.unit = G;
@@ -914,13 +941,13 @@ static int run_batch(const void* a, int lda, const void* bq, const void* scales,
   p.group = group;
   p.rpg = rpg_of(group);
   p.rows = rows;
-  const bool exact = batch_exact(M, group);
-  batch_stages(bits, device_info().max_smem, rows, p.rpg, p.cluster, &p.stages, &p.a_stages);
+  p.sets = batch_sets(var, rows, p.rpg, p.cluster, grid == n_tiles, device_info());
+  batch_stages(bits, device_info().max_smem, rows, p.rpg, p.cluster, p.sets, &p.stages, &p.a_stages);
   if (exact) p.stages = exact_stages(bits, device_info().max_smem, M);
   p.grid = (int)grid;
   p.act = act;
   int smem = exact ? exact_smem_bytes(bits, p.stages, M) : batch_smem_bytes(bits, p.stages, p.a_stages, rows, p.rpg, p.cluster);
-  if (!exact && (p.cluster > 1 || !batch_shares_sm(rows)) && smem < kOneCtaSmem) smem = kOneCtaSmem;
+  if (!exact && (p.cluster > 1 || !batch_shares_sm(rows, var)) && smem < kOneCtaSmem) smem = kOneCtaSmem;
   if (smem > device_info().max_smem) return ST_UNSUPPORTED;
   cudaError_t e = exact ? exact_launch(var, p, tmaps, smem, stream) : batch_launch(var, p, tmaps, smem, stream);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }

@@ -61,10 +61,9 @@
 
 namespace b200q {
 
-constexpr int BATCH_SETS = 2;                      // dequantize sets of four warps
-constexpr int BATCH_THREADS = BATCH_SETS * 128 + 256;  // + four epilogue warps, three producers, MMA warp
-constexpr int BATCH_SLOTS_MAX = 3 * BATCH_SETS;    // 128-row operand slots
-constexpr int BATCH_STAGES_MAX = 16;               // 128-row groups in the packed ring, a multiple of BATCH_SETS
+constexpr int batch_threads(int sets) { return sets * 128 + 256; }  // + four epilogue warps, three producers, MMA warp
+constexpr int BATCH_SLOTS_MAX = 6;                 // 128-row operand slots, of 64 tensor-memory columns
+constexpr int BATCH_STAGES_MAX = 16;               // 128-row groups in the packed ring, a multiple of the sets
 constexpr int BATCH_A_MAX = 6;                     // 128-row activation groups in shared memory, at most the slots
 
 struct BatchBarriers {
@@ -80,18 +79,21 @@ struct BatchBarriers {
 };
 constexpr int BATCH_BARRIERS = (int)(offsetof(BatchBarriers, tmem_base) / 8);
 // arrivals that complete a phase of the i-th barrier
-__host__ __device__ constexpr int batch_barrier_count(int i) {
+__host__ __device__ constexpr int batch_barrier_count(int i, int sets) {
   return i < (int)(offsetof(BatchBarriers, done) / 8) ? 4
        : i < (int)(offsetof(BatchBarriers, g_full) / 8) ? 1
        : i < (int)(offsetof(BatchBarriers, g_empty) / 8) ? 2
        : i < (int)(offsetof(BatchBarriers, d_full) / 8) ? 4
        : i < (int)(offsetof(BatchBarriers, d_empty) / 8) ? 1
-       : i < (int)(offsetof(BatchBarriers, run_done) / 8) ? 4 : 1;
+       : i < (int)(offsetof(BatchBarriers, run_done) / 8) ? 4
+       : i < (int)(offsetof(BatchBarriers, sums_full) / 8) ? 1 : sets + 1;
 }
 
-// tensor memory (all 512 columns): two D accumulators of nr columns, then as many operand slots as fit
+// tensor memory (all 512 columns): two D accumulators of nr columns - one for three sets beyond 64 rows, whose CTAs have a single
+// column tile - then the operand slots
 __host__ __device__ constexpr int batch_d_stride(int nr) { return nr <= 64 ? 64 : 128; }
-__host__ __device__ constexpr int batch_slots_per_set(int nr) { return nr <= 64 ? 3 : 2; }
+__host__ __device__ constexpr int batch_d_count(int nr, int sets) { return sets == 3 && nr > 64 ? 1 : 2; }
+__host__ __device__ constexpr int batch_slots(int nr, int sets) { return (512 - batch_d_count(nr, sets) * batch_d_stride(nr)) / 64; }
 
 // The epilogue of one segment, shared out over `parts` groups of four warps (this warp belongs to group
 // `part`): rows in chunks of 16 from tensor memory, to C (a whole tile) or added into the tile's scratch.
@@ -132,12 +134,13 @@ __device__ __forceinline__ void batch_epilogue(const BatchParams& p, uint32_t d_
 // The end of a column tile whose K a cluster shares, by the twelve warps that know of tensor memory.  The rows are cut into quads of four,
 // of which the CTAs own equal shares (the last ones what is left).  A warp takes 16 rows of its 32 columns at a time from tensor
 // memory to the CTA's own shared memory (over the activations: all MMAs have completed), [quad][32] float4, and sends each owner
-// its quads with one bulk copy, which counts its bytes in on the owner's barrier of the lane quadrant.  The owner adds the
+// its quads with one bulk copy, which counts its bytes in on the owner's barrier of the lane quadrant, as the owner's own warps
+// count themselves in.  The owner adds the
 // CTAs' sums in rank order and writes C.  A CTA that has all of its sums says so on the cluster's barrier and waits for the others
 // before it leaves, since until then its own copies may not have been read.  (64 x 4096 x 4096, three CTAs per tile, us per launch: sums
 // left in place and fetched by their owners between two barriers of the cluster 9.8, the last 3 of them; sent word by word 9.2.)
 __host__ __device__ constexpr int batch_own_quads(int quads, int cluster) { return (quads + cluster - 1) / cluster; }
-template <int ACT>
+template <int ACT, int SETS>
 __device__ __forceinline__ void cluster_epilogue(const BatchParams& p, uint32_t tmem, const unsigned char* smem, uint32_t smem_s,
                                                  uint32_t sums_off, uint32_t run_done, uint32_t full, int tile, int warp, int lane,
                                                  volatile int* abort_flag) {
@@ -145,14 +148,11 @@ __device__ __forceinline__ void cluster_epilogue(const BatchParams& p, uint32_t 
   const int quads = (p.M + 3) / 4, own = batch_own_quads(quads, p.cluster);
   const int q0 = min(quads, rank * own), q1 = min(quads, q0 + own);  // this CTA's
   const uint32_t sent = smem_s + (uint32_t)(wq * quads) * 512u;
-  const uint32_t got_off = sums_off + (uint32_t)(wq * p.cluster * own) * 512u;  // [CTA][owned quad][32]
+  const uint32_t got_off = sums_off + (uint32_t)(wq * (p.cluster - 1) * own) * 512u;  // [other CTA][owned quad][32]
   bool ok = mbar_wait_abortable(run_done, 0u, abort_flag);
   if (__all_sync(0xffffffffu, ok ? 1 : 0)) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (part == 0 && lane == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)((q1 - q0) * p.cluster) * 512u)
-                   : "memory");
-    for (int c0 = part * 4; c0 < quads; c0 += 12) {
+    for (int c0 = part * 4; c0 < quads; c0 += 4 * (SETS + 1)) {
       uint32_t v[16];
       tmem_ld_16(tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)(c0 * 4), v);
 #pragma unroll
@@ -165,13 +165,19 @@ __device__ __forceinline__ void cluster_epilogue(const BatchParams& p, uint32_t 
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (elect_one()) {
-      for (int c0 = part * 4; c0 < quads; c0 += 12) {
+      if (part == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full), "r"((uint32_t)((q1 - q0) * (p.cluster - 1)) * 512u)
+                     : "memory");
+      else
+        mbar_arrive(full);
+      for (int c0 = part * 4; c0 < quads; c0 += 4 * (SETS + 1)) {
         const int c1 = min(quads, c0 + 4);
         for (int q = c0, owner = c0 / own; q < c1; ++owner) {
-          const int next = min(c1, (owner + 1) * own);
+          const int next = min(c1, (owner + 1) * own), place = rank - (rank > owner ? 1 : 0);
+          if (owner == rank) { q = next; continue; }
           uint32_t dst, bar;
           asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
-                       : "r"(smem_s + got_off + (uint32_t)(rank * own + q - owner * own) * 512u), "r"(owner));
+                       : "r"(smem_s + got_off + (uint32_t)(place * own + q - owner * own) * 512u), "r"(owner));
           asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(full), "r"(owner));
           asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                        "r"(sent + (uint32_t)q * 512u), "r"((uint32_t)(next - q) * 512u), "r"(bar)
@@ -189,19 +195,20 @@ __device__ __forceinline__ void cluster_epilogue(const BatchParams& p, uint32_t 
   cluster_arrive_relaxed();
   if (!ok) return;
   const float4* parts = reinterpret_cast<const float4*>(smem + got_off) + lane;
+  const float4* mine = reinterpret_cast<const float4*>(smem) + (wq * quads + q0) * 32 + lane;
 #pragma unroll 2
-  for (int q = part; q < q1 - q0; q += 3) {
+  for (int q = part; q < q1 - q0; q += SETS + 1) {
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
     for (int r = 0; r < p.cluster; ++r) {
-      const float4 x = parts[(r * own + q) * 32];
+      const float4 x = r == rank ? mine[q * 32] : parts[((r - (r > rank ? 1 : 0)) * own + q) * 32];
       sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
     }
     batch_store4<ACT>(p, tile * 128 + wq * 32 + lane, lane, (q0 + q) * 4, sum);
   }
 }
 
-template <int VAR, int ACT, bool CLUSTER>
+template <int VAR, int ACT, bool CLUSTER, int SETS>
 __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorMap& tmap_a, const CUtensorMap& tmap_w) {
   constexpr int B = var_bits(VAR);
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -225,8 +232,8 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
   // this CTA's run of groups, counted tile by tile over the whole matrix
   const int run0 = batch_run_start(p, blockIdx.x), run1 = batch_run_start(p, blockIdx.x + 1);
 
-  constexpr int TM_THREADS = BATCH_SETS * 128 + 160;
-  constexpr int W_EPI = BATCH_SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
+  constexpr int TM_THREADS = SETS * 128 + 160;
+  constexpr int W_EPI = SETS * 4, W_ACT = W_EPI + 4, W_WEIGHTS = W_EPI + 5, W_MMA = W_EPI + 6,
                 W_SCALES = W_EPI + 7;
   // (The descriptors are on their way while the barriers are set up, by the lanes of one warp.  Thread 0 alone took 1800 cycles
   // for both, ahead of the first copies.)
@@ -235,7 +242,7 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
     asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
   }
   if (warp == 0) {
-    for (int i = lane; i < BATCH_BARRIERS; i += 32) mbar_init(bars_s + (uint32_t)i * 8u, (uint32_t)batch_barrier_count(i));
+    for (int i = lane; i < BATCH_BARRIERS; i += 32) mbar_init(bars_s + (uint32_t)i * 8u, (uint32_t)batch_barrier_count(i, SETS));
     if (lane == 0) bars->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -263,8 +270,8 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
   const uint32_t tmem = (warp < W_ACT || warp == W_MMA) ? __shfl_sync(0xffffffffu, bars->tmem_base, 0) : 0u;
-  const int sps = batch_slots_per_set(NR);
-  const uint32_t slots_t = tmem + (uint32_t)(batch_d_stride(NR) * 2);
+  const int nslots = batch_slots(NR, SETS), n_d = batch_d_count(NR, SETS), d_stride = batch_d_stride(NR);
+  const uint32_t slots_t = tmem + (uint32_t)(n_d * d_stride);
 
   // one segment of the run: pos -> tile, groups
 #define SEGMENT(pos)                                     \
@@ -279,9 +286,9 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
     const int nl = wq * 32 + lane;  // lane of tensor memory = column inside the tile
     const uint32_t lane_t = (uint32_t)(wq * 32) << 16;
     bool good = true;
-    int stage = set, slot = set;    // stages of a set: set, set + BATCH_SETS, ...; slots likewise
+    int stage = set, slot = set;    // stages of a set: set, set + SETS, ...; slots likewise
     uint32_t ring_phase = 0, slot_phase = 1;
-    for (int g_own = set; g_own < run1 - run0; g_own += BATCH_SETS) {
+    for (int g_own = set; g_own < run1 - run0; g_own += SETS) {
       if (!mbar_wait_abortable(BAR_ADDR(g_full, stage), ring_phase, abort_flag)) { good = false; break; }
       const uint32_t st = ring_s + (uint32_t)stage * WSTAGE;
       const uint32_t sc = scales_s + (uint32_t)stage * SSTAGE + (uint32_t)nl * 2u;
@@ -320,9 +327,9 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(BAR_ADDR(slot_full, slot));
-      slot += BATCH_SETS;
-      if (slot >= BATCH_SETS * sps) { slot = set; slot_phase ^= 1u; }
-      stage += BATCH_SETS;
+      slot += SETS;
+      if (slot >= nslots) { slot = set; slot_phase ^= 1u; }
+      stage += SETS;
       if (stage >= WS) { stage = set; ring_phase ^= 1u; }
     }
     if (!CLUSTER && good) {
@@ -332,8 +339,8 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
       asm volatile("griddepcontrol.wait;" ::: "memory");  // C and the scratch may still be in use by the previous kernel
       if (mbar_wait_abortable(BAR_ADDR(run_done, 0), 0u, abort_flag)) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), 0u, tile, len, wq, lane, set,
-                            BATCH_SETS + 1);
+        batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg % n_d) * d_stride), 0u, tile, len, wq, lane, set,
+                            SETS + 1);
       }
     }
   } else if (warp < W_ACT) {
@@ -344,10 +351,10 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
     int seg = 0;
     for (int pos = run0; pos < run1 && !CLUSTER; ++seg) {
       SEGMENT(pos)
-      if (!mbar_wait_abortable(BAR_ADDR(d_full, seg & 1), (uint32_t)(seg >> 1) & 1u, abort_flag)) break;
+      if (!mbar_wait_abortable(BAR_ADDR(d_full, seg % n_d), (uint32_t)(seg / n_d) & 1u, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg & 1) * batch_d_stride(NR)), BAR_ADDR(d_empty, seg & 1), tile,
-                          len, wq, lane, last_seg ? BATCH_SETS : 0, last_seg ? BATCH_SETS + 1 : 1);
+      batch_epilogue<ACT>(p, tmem + lane_t + (uint32_t)((seg % n_d) * d_stride), BAR_ADDR(d_empty, seg % n_d), tile,
+                          len, wq, lane, last_seg ? SETS : 0, last_seg ? SETS + 1 : 1);
       pos += len;
     }
   } else if (warp == W_ACT) {
@@ -364,7 +371,7 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
       for (int pos = run0; pos < run1; ++pos) {
         if (n_issued >= AS) {
           if (!mbar_wait_abortable(BAR_ADDR(done, slot), phase, abort_flag)) { good = false; break; }
-          if (++slot == BATCH_SETS * sps) { slot = 0; phase ^= 1u; }
+          if (++slot == nslots) { slot = 0; phase ^= 1u; }
         }
         const uint32_t bar = BAR_ADDR(a_full, stage);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(ASTAGE) : "memory");
@@ -453,16 +460,15 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
       const uint32_t idesc = umma_idesc<ACT>(NR);
       bool good = true;
       int slot = 0, stage = 0, seg = 0;
-      const int nslots = BATCH_SETS * sps;
       uint32_t slot_phase = 0, a_phase = 0;
       // the next group's barriers are looked at before this group's MMAs are issued, so that the latency of
       // the look (twice 100 cycles) lies under them; only a group that was not ready then is waited for
       bool ready = false;
       for (int pos = run0; pos < run1 && good; ++seg) {
         SEGMENT(pos)
-        if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg & 1), ((uint32_t)(seg >> 1) & 1u) ^ 1u, abort_flag)) { good = false; break; }
+        if (!mbar_wait_abortable(BAR_ADDR(d_empty, seg % n_d), ((uint32_t)(seg / n_d) & 1u) ^ 1u, abort_flag)) { good = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t d_t = tmem + (uint32_t)((seg & 1) * batch_d_stride(NR));
+        const uint32_t d_t = tmem + (uint32_t)((seg % n_d) * d_stride);
         for (int i = 0; i < len && good; ++i) {
           if (!ready && (!mbar_wait_abortable(BAR_ADDR(slot_full, slot), slot_phase, abort_flag) ||
                          !mbar_wait_abortable(BAR_ADDR(a_full, stage), a_phase, abort_flag))) { good = false; break; }
@@ -492,7 +498,7 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
         }
         if (good)
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                           BAR_ADDR(d_full, seg & 1))
+                           BAR_ADDR(d_full, seg % n_d))
                        : "memory");
         pos += len;
       }
@@ -507,7 +513,7 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
     __syncwarp();
     if (warp < W_ACT) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // C may still be in use by the previous kernel
-      cluster_epilogue<ACT>(p, tmem, smem_al, smem_base, sums_off, BAR_ADDR(run_done, 0), BAR_ADDR(sums_full, warp & 3), run0 / p.G,
+      cluster_epilogue<ACT, SETS>(p, tmem, smem_al, smem_base, sums_off, BAR_ADDR(run_done, 0), BAR_ADDR(sums_full, warp & 3), run0 / p.G,
                             warp, lane, abort_flag);
     } else {
       cluster_arrive_relaxed();
@@ -533,29 +539,38 @@ __device__ __forceinline__ void batch_body(const BatchParams& p, const CUtensorM
 #undef SEGMENT
 }
 
-// Equal runs, and a cluster of CTAs per column tile.  Two CTAs of the former have registers on an SM (64, see batch_stages) for the types
-// named there; 7-bit integers in bfloat16 have to be told (72 otherwise).
+// Equal runs with two sets: of up to 32 rows, of which two CTAs have registers on an SM (64, see batch_stages), and of more than 64.
+// Equal runs with three sets, and a cluster of CTAs per column tile (api.cu, batch_sets).
+// (float4, and 7-bit integers in bfloat16, would take 69 to 72 registers and do with 64 without spills; the others' code is slower for
+// being told.)
+constexpr bool batch_told_registers(int var, int act) { return var == VAR_F4E2M1 || (!var_is_float(var) && var_bits(var) == 7 && act == 1); }
 template <int VAR, int ACT>
-__global__ void __launch_bounds__(BATCH_THREADS, !var_is_float(VAR) && var_bits(VAR) == 7 ? 2 : 1)
+__global__ void __launch_bounds__(batch_threads(2), batch_told_registers(VAR, ACT) ? 2 : 1)
 batch_kernel(const __grid_constant__ BatchParams p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w) {
-  batch_body<VAR, ACT, false>(p, tmap_a, tmap_w);
+  batch_body<VAR, ACT, false, 2>(p, tmap_a, tmap_w);
 }
 template <int VAR, int ACT>
-__global__ void __launch_bounds__(BATCH_THREADS, 1)
+__global__ void __launch_bounds__(batch_threads(3), 1)
+tile_run_kernel(const __grid_constant__ BatchParams p, const __grid_constant__ CUtensorMap tmap_a,
+                const __grid_constant__ CUtensorMap tmap_w) {
+  batch_body<VAR, ACT, false, 3>(p, tmap_a, tmap_w);
+}
+template <int VAR, int ACT, int SETS>
+__global__ void __launch_bounds__(batch_threads(SETS), 1)
 tile_cluster_kernel(const __grid_constant__ BatchParams p, const __grid_constant__ CUtensorMap tmap_a,
                     const __grid_constant__ CUtensorMap tmap_w) {
-  batch_body<VAR, ACT, true>(p, tmap_a, tmap_w);
+  batch_body<VAR, ACT, true, SETS>(p, tmap_a, tmap_w);
 }
 
-template <int VAR, int ACT, bool CLUSTER>
+template <int VAR, int ACT, bool CLUSTER, int SETS>
 static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
-  auto kern = CLUSTER ? tile_cluster_kernel<VAR, ACT> : batch_kernel<VAR, ACT>;
+  auto kern = CLUSTER ? tile_cluster_kernel<VAR, ACT, SETS> : SETS == 3 ? tile_run_kernel<VAR, ACT> : batch_kernel<VAR, ACT>;
   static std::atomic<bool> allowed[16];
   const cudaError_t e = allow_smem(kern, allowed);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)p.grid, 1, 1);
-  cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
+  cfg.blockDim = dim3((unsigned)batch_threads(SETS), 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -570,16 +585,20 @@ static cudaError_t batch_launch_one(const BatchParams& p, const CUtensorMap* tma
   return cudaLaunchKernelEx(&cfg, kern, p, tmaps[0], tmaps[1]);
 }
 
+template <int VAR, bool CLUSTER, int SETS>
+static cudaError_t batch_launch_act(const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes, cudaStream_t stream) {
+  return p.act == 0 ? batch_launch_one<VAR, 0, CLUSTER, SETS>(p, tmaps, smem_bytes, stream)
+                    : batch_launch_one<VAR, 1, CLUSTER, SETS>(p, tmaps, smem_bytes, stream);
+}
+
 template <int VAR>
 static cudaError_t batch_launch_var(int var, const BatchParams& p, const CUtensorMap* tmaps, int smem_bytes,
                                     cudaStream_t stream) {
   if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
     if (var == VAR) {
       if (p.cluster > 1)
-        return p.act == 0 ? batch_launch_one<VAR, 0, true>(p, tmaps, smem_bytes, stream)
-                          : batch_launch_one<VAR, 1, true>(p, tmaps, smem_bytes, stream);
-      return p.act == 0 ? batch_launch_one<VAR, 0, false>(p, tmaps, smem_bytes, stream)
-                        : batch_launch_one<VAR, 1, false>(p, tmaps, smem_bytes, stream);
+        return p.sets == 3 ? batch_launch_act<VAR, true, 3>(p, tmaps, smem_bytes, stream) : batch_launch_act<VAR, true, 2>(p, tmaps, smem_bytes, stream);
+      return p.sets == 3 ? batch_launch_act<VAR, false, 3>(p, tmaps, smem_bytes, stream) : batch_launch_act<VAR, false, 2>(p, tmaps, smem_bytes, stream);
     }
   }
   if constexpr (VAR + 1 < VAR_COUNT) return batch_launch_var<VAR + 1>(var, p, tmaps, smem_bytes, stream);
@@ -598,13 +617,13 @@ cudaError_t B200Q_CAT(batch_launch_part, B200Q_PART)(int var, const BatchParams&
 #if B200Q_PART == 0
 // clusters of c CTAs that the current device holds at a time with one CTA per SM; 0 without a device
 int batch_max_clusters(int c) {
-  auto kern = tile_cluster_kernel<0, 0>;
+  auto kern = tile_cluster_kernel<0, 0, 3>;
   const int smem = 200 * 1024;
   static std::atomic<bool> allowed[16];
   if (allow_smem(kern, allowed) != cudaSuccess) { (void)cudaGetLastError(); return 0; }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)c, 1, 1);
-  cfg.blockDim = dim3(BATCH_THREADS, 1, 1);
+  cfg.blockDim = dim3((unsigned)batch_threads(3), 1, 1);
   cfg.dynamicSmemBytes = (size_t)smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -620,23 +639,25 @@ int batch_max_clusters(int c) {
 // dynamic shared memory: alignment slack + activation groups + packed ring + scales + barriers + what a cluster's CTAs send
 int batch_smem_bytes(int bits, int stages, int a_stages, int rows, int rpg, int cluster) {
   return 1024 + a_stages * rows * 256 + stages * batch_stage_bytes(bits, rpg) + (int)sizeof(BatchBarriers) +
-         (cluster > 1 ? 128 + batch_own_quads(rows / 4, cluster) * cluster * 2048 : 0);
+         (cluster > 1 ? 128 + batch_own_quads(rows / 4, cluster) * (cluster - 1) * 2048 : 0);
 }
 // Activation groups (at most as many as there are operand slots) and ring stages (a multiple of the dequantize
-// sets) in the rest.  Up to 32 rows a CTA stays within half an SM's shared memory, so that the next launch of the
-// stream becomes resident beside this one and fills its ring while this one ends (a Llama-3-8B block of
-// linears, 4 bits, at 32 rows: 51 us, 56 with one CTA per SM).  The registers allow that for 1..7-bit integers (6 bits in
-// fp16 only), 7-bit floats and float4, which take 64; 8-bit types, 5- and 6-bit floats, float3 and 6-bit integers in bf16
-// take 66..88, so they keep to the half and run one CTA per SM all the same (8 bits with two stages in the ring:
-// 24 x 8192 x 8192 24.8 us, 14.8 with 4 bits).  Above, a CTA takes more than half: the activations leave
-// too little for the ring, and launches that leave SMs free (clusters, one CTA per column tile) would meet others
-// two to an SM, where one waits for the other's tensor memory (64 rows: 81 us with the two kinds mixed, 62).
-void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int* stages, int* a_stages) {
-  const int cap = batch_shares_sm(rows) && cluster <= 1 ? 113 * 1024 : max_smem;
+// sets) in the rest.  Up to 32 rows of 1-, 2- and 4-bit integers and float4 (batch_shares_sm: two sets) a CTA stays within half an SM's
+// shared memory and 64 registers, so that the next launch of the stream becomes resident beside this one and fills its ring while
+// this one ends (a Llama-3-8B block of linears, 4 bits, at 32 rows: 51 us, 56 with one CTA per SM).  The other types gain more from three sets
+// and an SM's whole shared memory (the block at 32 rows, us, so / sharing: 8 bits 57 / 82, whose ring had two stages in a half; 6 bits 59 /
+// 61, 3 bits 59 / 60, float6 62 / 66), and more rows leave too little for the ring; launches that leave SMs free (clusters, one CTA per
+// column tile) would meet others two to an SM, where one waits for the other's tensor memory (64 rows: 81 us with the two kinds
+// mixed, 62).
+void batch_stages(int bits, int max_smem, int rows, int rpg, int cluster, int sets, int* stages, int* a_stages) {
+  const int cap = rows <= 32 && sets == 2 ? 113 * 1024 : max_smem;
   *a_stages = rows <= 64 ? 6 : 4;
-  while (*a_stages > 2 && batch_smem_bytes(bits, BATCH_SETS, *a_stages, rows, rpg, cluster) > cap) --*a_stages;  // (8 bits, 128 rows, a cluster)
-  int st = BATCH_STAGES_MAX / BATCH_SETS * BATCH_SETS;
-  while (st > BATCH_SETS && batch_smem_bytes(bits, st, *a_stages, rows, rpg, cluster) > cap) st -= BATCH_SETS;
+  int st = 0;
+  for (;; --*a_stages) {  // (wide types in clusters of many rows: activations make room for a ring of two stages per set)
+    st = BATCH_STAGES_MAX / sets * sets;
+    while (st > sets && batch_smem_bytes(bits, st, *a_stages, rows, rpg, cluster) > cap) st -= sets;
+    if (cluster <= 1 || *a_stages == 2 || (st >= 2 * sets && batch_smem_bytes(bits, st, *a_stages, rows, rpg, cluster) <= cap)) break;
+  }
   *stages = st;
 }
 #endif

@@ -178,10 +178,13 @@ struct BatchParams {
   int grid;              // CTAs: each takes an equal contiguous run of work units
   int cluster;           // > 1: CTAs per column tile, which share its K and add up in distributed shared memory
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
+  int sets;              // dequantizing sets of four warps: 2 or 3 (batch_kernel.cu)
 };
 
 // batch_kernel.cu: whether a CTA leaves room for a second one on its SM (see batch_stages)
-inline bool batch_shares_sm(int rows) { return rows <= 32; }
+constexpr bool batch_shares_sm(int rows, int var) {
+  return rows <= 32 && (var_is_float(var) ? var == VAR_F4E2M1 : var_bits(var) == 1 || var_bits(var) == 2 || var_bits(var) == 4);
+}
 
 // ---- dequantize kernel -----------------------------------------------------------------------
 struct DequantParams {
