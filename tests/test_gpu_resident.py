@@ -61,7 +61,9 @@ def test_every_weight_type(dt, M, K, S):
     (1, 14336, 2048, 128, 1),      # two sets with four and three tiles
     (16, 6144, 4096, 128, 1),      # 16 rows, three tiles
     (9, 4112, 2048, 1024, 1),      # 9 rows, the last CTA with one tile
-    (16, 2064, 2176, 128, 2),      # 16 rows in clusters, 8.5 groups per CTA
+    (8, 2064, 2176, 128, 2),       # 8.5 groups per CTA
+    (5, 4096, 1024, 128, 8),       # eight CTAs to a cluster, a group each
+    (2, 80, 9216, 128, 3),         # clusters of three, five tiles in all
     (8, 4096, 14336, 128, 4),
     (6, 4096, 14336, 7168, 2),     # seven groups for two warps
     (8, 75776, 1024, 128, 1),      # 32 tiles per CTA

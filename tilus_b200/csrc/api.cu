@@ -647,7 +647,7 @@ struct ResidentSplit { int S, T_own, wk_shift, n_max, stages, slab_shift, smem, 
 // four groups per warp are slower than two of twice the warps, 1 x 28672 x 4096 14.9 / 13.4).
 static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInfo& di, ResidentSplit* rs) {
   const int G = K / 128, NT = N / BLOCK_N, mt = stream_mt(M), ng_max = mt == 1 ? 4 : 2;
-  if (M > 16 || S < 1 || S > 8 || G < S) return false;
+  if (M > 16 || S < 1 || S > 8 || G < S || (S > 1 && mt > 1)) return false;
   int clusters = di.sm_count / S;
   if (S > 1 && max_clusters(S) < clusters) clusters = max_clusters(S);
   if (clusters < 1) return false;
@@ -670,7 +670,7 @@ static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInf
   const int sets = RES_WARPS >> rs->wk_shift, Tw = (rs->T_own + sets - 1) / sets;
   rs->slab_shift = Tw <= 1 ? 0 : Tw <= 2 ? 1 : 2;
   const long long fixed = RES_HEADER + (long long)RES_WARPS * ng * Tw * 32 + (RES_WARPS << rs->slab_shift) * mt * 512 +
-                          (S > 1 ? (long long)rs->T_own * mt * 512 : 0);
+                          (S > 1 ? (long long)(rs->T_own + S - 1) / S * S * mt * 512 : 0);  // sums that a cluster's CTAs get
   if (fixed > di.max_smem) return false;
   int st = kStreamRing / (RES_WARPS * slot);
   st = st > 8 ? 8 : st < 2 ? 2 : st;
@@ -682,20 +682,22 @@ static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInf
   return true;
 }
 // Where the resident kernel takes a decode call that the table gives to the stream kernel (tile_m 0) or the exact kernel: the CTAs
-// per cluster, or 0.  Measured against those, cold chains, 11 widths x 6 depths (1024 .. 14336) x 1 .. 16 rows in 4 bits, 5 x 5 in
-// 1, 2, 3, 6 and 8 bits; time here over time there:
-//  - 5 to 8 rows 0.44 .. 0.98; 2 to 4 rows 0.49 .. 1.0, except where rows of K leave some warps a third group (K = 5120, 1.02 .. 1.11
-//    from 8192 columns on) and 5 to 7 bits beyond 8192 rows of K (up to 1.03);
+// per cluster, or 0.  Measured against those, cold chains, 9 widths x 13 depths (1024 .. 14336) x 1, 2, 4 and 8 rows in 4 bits, 5 x 6 in 1, 2, 3,
+// 6 and 8 bits; time here over time there:
+//  - 5 to 8 rows 0.44 .. 0.97, except 5 to 7 bits on 16384 columns and more beyond 4096 rows of K (1.00 .. 1.03); 2 to 4 rows 0.49 .. 1.0,
+//    except where 4096 to 6144 rows of K, in two or three groups per warp, meet many columns (2 x 28672 x 4608 1.16), and 5 to 7 bits beyond
+//    8192 rows of K (1.00 .. 1.03);
 //  - one row: up to 4096 rows of K 0.71 .. 0.99, for 1 and 2 bits up to 8192 columns, 3 bits up to 16384 (2 bits, 28672 x 4096 1.06);
-//    up to 8192 rows of K two column tiles per CTA, 1 and 2 bits one (4096 x 8192, 4 bits 0.98, 6144 x 8192 1.03);
-//    beyond, 8-bit integers (0.94 .. 0.97) and 4 bits up to 3072 columns (0.82 .. 0.96);
+//    up to 8192 rows of K two column tiles per CTA 0.76 .. 0.99 (1 and 2 bits one), and from 7168 on wide layers 0.94 .. 1.02
+//    (6144 x 8192 1.02, 28672 x 4608 1.20); beyond, 0.75 .. 1.0 but for 5 to 7 bits (1.1);
 //  - 9 to 16 rows (fp16 only: the exact kernel takes bfloat16 as it is), whose second set of sums makes the loop 1.5 times longer: up to
 //    4096 rows of K in the ranges below 0.63 .. 0.96; beyond 1.0 .. 1.3.  Among layers that stay with the exact kernel, whose launches
 //    leave SMs to their successors, a launch on all SMs costs those up to 2 us: with 4096 x 4096 here a Llama-3-8B block takes, us, at 9
 //    / 13 / 16 rows 47.2 / 49.3 / 51.1 in 4 bits (50.1 / 51.1 / 50.3 without), 54.0 / 54.8 / 57.7 in 8 bits (54.5 / 54.9 / 55.7), 58.1 /
 //    60.2 / 61.2 in 3 bits (62.5 / 63.1 / 62.2), 59.8 / 61.6 / 63.4 in float6 (62.9 / 63.5 / 62.8): 8 bits up to 12 rows, 4 bits up to 14.
-// S: one CTA per cluster where a warp's activations fit its registers, and where K is long or the columns few; us, 8 rows,
-// S = 1 / 2 / 4: 8192 x 8192 11.5 / 10.6 / 12.7, 4096 x 14336 - / 12.1 / 10.5, 28672 x 14336 - / 45.1 / 45.2.
+// S: one CTA per cluster where a warp's activations fit its registers, and where the columns are few or the decoding dear; us, 8 rows,
+// 4 bits, S = 1 / 2 / 4: 4096 x 5120 6.3 / 5.9 / 5.9 (6 bits 8.0 / 8.3 / 8.6), 8192 x 8192 11.7 / 10.3 / 10.6, 4096 x 14336 - / 11.1 / 9.8,
+// 28672 x 14336 - / 43.8 / 45.2.
 static int resident_cluster(int M, int N, int K, int var, int group, int act, bool stream_form, const DeviceInfo& di) {
   if (M > 16 || group % 128 != 0 || (act == B200Q_BF16 && !stream_form)) return 0;
   const int G = K / 128, bits = var_bits(var);
@@ -705,18 +707,22 @@ static int resident_cluster(int M, int N, int K, int var, int group, int act, bo
     if (G > 16 && ((bits == 8 && M > 12) || (bits == 4 && M > 14))) return 0;
     S = 1;
   } else {
-    S = G <= 40 || (G <= 64 && M < 5 && N < 8192) ? 1 : G <= 64 || (N >= 16384 && G <= 128) ? 2 : 4;
-    const bool integer = !var_is_float(var);
+    if (G <= 32) S = 1;
+    else if (G <= 40) S = M >= 5 && bits <= 4 ? 2 : 1;
+    else if (G <= 64) S = M == 1 && G < 56 && N < 8192 ? 1 : 2;
+    else S = G <= 128 && (N >= 16384 || (G <= 96 && N >= 8192)) ? 2 : 4;
+    const bool dear = bits >= 5 && bits <= 7;
     if (M == 1 && G <= 32) {
       if (N > (bits <= 2 ? 8192 : bits == 3 ? 16384 : 1 << 30)) return 0;
     } else if (M == 1 && G <= 64) {
-      if (N > (bits <= 2 ? 2048 : 4096)) return 0;
+      if (bits <= 2 ? N > 2048 : N > 4096 && !(N >= 8192 && G >= 56)) return 0;
     } else if (M == 1) {
-      if (!(integer && bits == 8) && !(bits == 4 && N <= 3072)) return 0;
+      if (dear && stream_form) return 0;
     } else if (M <= 4 && stream_form) {
-      const int n = (G + 16 * S - 1) / (16 * S);
-      if (N >= 8192 && G * 20 < n * 16 * S * 17) return 0;
-      if (G > 64 && bits >= 5 && bits <= 7) return 0;
+      if (G > 32 && G < 48 && N >= (M == 2 ? 6144 : 14336)) return 0;
+      if (G > 64 && dear && N >= 6144) return 0;
+    } else if (M >= 5 && dear && G > 32 && N >= 16384) {
+      return 0;
     }
   }
   ResidentSplit rs;

@@ -7,7 +7,7 @@
 // their activations once, as tensor-core operands (the operand's k order is the packed layout's: lane (r, j) holds 64 contiguous
 // bytes of row r per group), and then takes the CTA's column tiles one after the other.  Shared memory carries the weights only,
 // and nothing is staged.  us, cold chains, 4 bits, group 128, before (stream or exact kernel) / here: 8 x 4096 x 4096 7.1 / 4.7, 8 x
-// 28672 x 4096 19.8 / 13.6, 8 x 4096 x 14336 13.1 / 10.6, 1 x 4096 x 4096 4.6 / 3.9, 1 x 28672 x 4096 13.7 / 12.7; 16 x 4096 x 4096
+// 28672 x 4096 19.8 / 13.3, 8 x 4096 x 14336 13.1 / 9.8, 1 x 4096 x 4096 4.6 / 3.6, 1 x 28672 x 4096 13.7 / 12.3; 16 x 4096 x 4096
 // 8.2 / 7.1, but 16 x 28672 x 4096 20.3 / 20.6 (two sets of sums per warp: 185 instructions per group, 121 with one).
 //
 // Weights.  One elected thread of a warp keeps the warp's ring full with TMA bulk copies, as in stream_kernel.cu: slots of one, two or
@@ -25,7 +25,8 @@
 // Sums.  The 16 warps' parts of a column tile meet in shared memory (four tiles of room, an mbarrier that counts the warps and one
 // that frees the room), and one of the warps, in turn, adds them up in order and writes C: results repeat bit for bit.  Where the
 // activations do not fit the registers - more than 8192 rows of K for up to 8 rows of A, 4096 for 16 - a cluster of S CTAs
-// shares K and adds its sums up in distributed shared memory.
+// shares K.  The warp that adds up a tile sends the CTA's sum to the CTA that writes the tile (every S-th), which waits for the bytes
+// it expects at the end: no CTA reads another's memory, so none has to wait for the others before it leaves.
 //
 // Every wait is bounded; one that runs out leaves the loops, waits (bounded) for the copies in flight and is reported in the workspace's
 // status word.
@@ -87,6 +88,15 @@ __device__ __forceinline__ uint32_t res_bf16x2_to_f16x2(uint32_t w) {
   uint32_t h;
   asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(__uint_as_float(w & 0xffff0000u)), "f"(__uint_as_float(w << 16)));
   return h;
+}
+// 16 bytes of an activation row, or zeros where there is no row.  In program order, so that all of a warp's loads are in flight at once:
+// left to the compiler, some waited for the first conversions (8 x 6144 x 4096 5.55 us, 5.49 so).
+__device__ __forceinline__ uint4 res_load_row(const uint4* p, bool valid) {
+  uint4 v;
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+               "@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((uint32_t)valid));
+  return v;
 }
 // the words of a unit, and one word of every vector load
 template <int B>
@@ -151,7 +161,7 @@ __device__ __forceinline__ void mma_m16n8k16_from(float (&d)[4], uint32_t a0, ui
 // Shared memory: barriers of the rings [warp][8] and of the slabs [set][full 4, empty 4]; rings [warp][slot]; scales
 // [warp][tile][NG][16]; slabs [set][slot][warp][MT][32 lanes] float4; with a cluster the CTA's sums [tile][MT][32 lanes] float4.
 // Columns of `af`, `nb`: rows of A come in sets of eight (MT of them), 128-row groups of K in NG.
-template <int VAR, int MT, int NG, int ACT>
+template <int VAR, int MT, int NG, int ACT, bool CLUSTER>
 __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const ResidentParams p) {
   constexpr int B = var_bits(VAR);
   constexpr int BIAS = lin_uniform_bias(VAR);
@@ -171,8 +181,8 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
   const int set = warp >> p.wk_shift, wi = warp & (WK - 1);
 
   int ci = blockIdx.x, chunk = 0;
-  if (p.S > 1) { ci = blockIdx.x / p.S; chunk = blockIdx.x - ci * p.S; }
-  const int gc0 = p.S > 1 ? p.G * chunk / p.S : 0, gc1 = p.S > 1 ? p.G * (chunk + 1) / p.S : p.G;
+  if constexpr (CLUSTER) { ci = blockIdx.x / p.S; chunk = blockIdx.x - ci * p.S; }
+  const int gc0 = CLUSTER ? p.G * chunk / p.S : 0, gc1 = CLUSTER ? p.G * (chunk + 1) / p.S : p.G;
   const int Gc = gc1 - gc0, base = Gc >> p.wk_shift, rem = Gc & (WK - 1);
   const int n = base + (wi < rem ? 1 : 0), g0 = gc0 + wi * base + min(wi, rem);  // this warp's groups of K
   const int active = min(WK, Gc);                                                 // warps of a set that have any
@@ -191,7 +201,22 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
   const uint32_t slab_off = sc_off + (uint32_t)(RES_WARPS * NG * Tw * 32);
   const int D = 1 << p.slab_shift;
   float4* slab = reinterpret_cast<float4*>(smem_raw + slab_off) + (size_t)set * D * WK * MT * 32;
-  float4* csum = reinterpret_cast<float4*>(smem_raw + slab_off + (uint32_t)(WT * D * WK * MT * 512));
+  const uint32_t got_off = slab_off + (uint32_t)(WT * D * WK * MT * 512), got_bar = smem_base + RES_HEADER - 8u;  // cluster: see finish
+
+  // ---- scales of all of the warp's tiles and groups: [tile][group][16]; requested first, as the products wait for them
+  // longest (1 x 4096 x 4096, behind the rings' set-up 3.85 us, here 3.63; behind the activations' loads 4.4) ----
+  {
+    const unsigned char* srow = reinterpret_cast<const unsigned char*>(p.scales) + (size_t)(unsigned)(tile0 + set) * 32u + (lane & 1) * 16;
+    const uint32_t row_bytes = (uint32_t)p.N * 2u, dst0 = smem_base + (uint32_t)(sc_warp - smem_raw) + (lane & 1) * 16;
+#pragma unroll
+    for (int gi = 0; gi < NG; ++gi) {
+      if (gi >= n) break;
+      const uint32_t row = p.gshift >= 0 ? (uint32_t)(g0 + gi) >> p.gshift : (uint32_t)(g0 + gi) / (uint32_t)p.gdiv;
+      const unsigned char* src_row = srow + (size_t)row * row_bytes;
+      for (int x = lane >> 1; x < my; x += 16)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst0 + (uint32_t)((x * NG + gi) * 32)), "l"(src_row + ((uint32_t)x * 32u << (4 - p.wk_shift))) : "memory");
+    }
+  }
 
   // ---- weights: the warp's own ring ----
   const int ipt = (n + GI - 1) / GI, n_items = my * ipt;
@@ -217,20 +242,16 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full0 + lane * 8), "r"(active) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(empty0 + lane * 8) : "memory");
   }
+  if (CLUSTER && tid == 0) {
+    // what the cluster's CTAs send for the tiles that this one writes (every S-th)
+    const uint32_t bytes = (uint32_t)((max(tiles, 0) - chunk + p.S - 1) / p.S * p.S * MT) * 512u;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(got_bar) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(got_bar), "r"(bytes) : "memory");
+  }
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   __syncwarp();
+  if constexpr (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   for (int s = 0; s < NST && issued < n_items; ++s) issue_next(bar0 + s * 8, ring_s + s * SLOT);
-
-  // ---- scales of all of the warp's tiles and groups: [tile][group][16] ----
-  for (int gi = 0; gi < n; ++gi) {
-    const int row = p.gshift >= 0 ? (g0 + gi) >> p.gshift : (g0 + gi) / p.gdiv;
-    const unsigned short* srow = reinterpret_cast<const unsigned short*>(p.scales) + (size_t)row * p.N + tile0 * 16;
-    for (int x = lane; x < my * 2; x += 32) {
-      const uint32_t dst = smem_base + (uint32_t)(sc_warp - smem_raw) + (uint32_t)(((x >> 1) * NG + gi) * 32 + (x & 1) * 16);
-      const unsigned short* s = srow + (set + (x >> 1) * WT) * 16 + (x & 1) * 8;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(s) : "memory");
-    }
-  }
 
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
@@ -245,7 +266,7 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
                                                        (size_t)(mt * 8 + r) * p.lda + (size_t)(g0 + g) * 128 + j * 32);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const uint4 v = valid ? __ldg(pa + q) : make_uint4(0u, 0u, 0u, 0u);
+        const uint4 v = res_load_row(pa + q, valid);
         af[g][mt][4 * q] = v.x; af[g][mt][4 * q + 1] = v.y; af[g][mt][4 * q + 2] = v.z; af[g][mt][4 * q + 3] = v.w;
       }
     }
@@ -271,7 +292,8 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
       }
     }
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();  // barriers of the slabs
+  if constexpr (CLUSTER) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // everybody's barriers are there
+  else __syncthreads();
 
   // ---- column tiles ----
   bool ok = true;
@@ -296,8 +318,15 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
       v[mt].x *= F; v[mt].y *= F; v[mt].z *= F; v[mt].w *= F;
-      if (p.S > 1) {
-        csum[(tile * MT + mt) * 32 + lane] = v[mt];
+      if constexpr (CLUSTER) {  // to the CTA that writes the tile: [its tile][CTA][MT][32 lanes]
+        const int owner = tile % p.S;
+        uint32_t dst, bar;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst)
+                     : "r"(smem_base + got_off + (uint32_t)(((tile - owner + chunk) * MT + mt) * 512 + lane * 16)), "r"(owner));
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(got_bar), "r"(owner));
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(v[mt].x),
+                     "f"(v[mt].y), "f"(v[mt].z), "f"(v[mt].w), "r"(bar)
+                     : "memory");
       } else {
         const int m = mt * 8 + 2 * j, col = (tile0 + tile) * 16 + r;
         unsigned short* c = reinterpret_cast<unsigned short*>(p.c) + (size_t)m * p.ldc + col;
@@ -411,20 +440,15 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
     }
     for (int s = 0; s < NST; ++s) mbar_wait_bounded(bar0 + s * 8, 0);
   }
-  if (p.S > 1) {  // the cluster's CTAs hold parts of the same tiles
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const uint32_t csum_s = smem_base + (uint32_t)(reinterpret_cast<unsigned char*>(csum) - smem_raw);
-    for (int t = chunk + warp * p.S; t < tiles; t += RES_WARPS * p.S) {
+  if constexpr (CLUSTER) {
+    for (int t = chunk + warp * p.S; t < tiles && ok; t += RES_WARPS * p.S) {
+      if (!__all_sync(0xffffffffu, mbar_wait_bounded(got_bar, 0u) ? 1 : 0)) { ok = false; break; }
+      const float4* got = reinterpret_cast<const float4*>(smem_raw + got_off) + (t - chunk) * MT * 32 + lane;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int c = 0; c < p.S; ++c) {
-          uint32_t addr;
-          float4 x;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(csum_s + (uint32_t)((t * MT + mt) * 512 + lane * 16)), "r"(c));
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(addr) : "memory");
+          const float4 x = got[(c * MT + mt) * 32];
           v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
         }
         const int m = mt * 8 + 2 * j, col = (tile0 + t) * 16 + r;
@@ -433,15 +457,18 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
         if (m + 1 < p.M) { c[p.ldc] = res_out_bits<ACT>(v.y); c[p.ldc + 8] = res_out_bits<ACT>(v.w); }
       }
     }
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
+      if (lane == 0) { atomicExch(p.status, ST_DEVICE_TIMEOUT); p.status[1] = 10; p.status[2] = blockIdx.x; p.status[3] = warp; }
+      // peers may still send their sums: they have left, or are here as well, when this ends
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
   }
 }
 
-template <int VAR, int MT, int NG, int ACT>
+template <int VAR, int MT, int NG, int ACT, bool CLUSTER>
 static cudaError_t launch_one(const ResidentParams& p, int smem_bytes, cudaStream_t stream) {
-  auto kern = resident_kernel<VAR, MT, NG, ACT>;
+  auto kern = resident_kernel<VAR, MT, NG, ACT, CLUSTER>;
   static std::atomic<bool> allowed[16];
   const cudaError_t e = allow_smem(kern, allowed);
   if (e != cudaSuccess) return e;
@@ -457,19 +484,24 @@ static cudaError_t launch_one(const ResidentParams& p, int smem_bytes, cudaStrea
   attr[1].val.clusterDim.x = (unsigned)p.S;
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.S > 1 ? 2 : 1;
+  cfg.numAttrs = CLUSTER ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
+template <int VAR, bool CLUSTER>
+static cudaError_t launch_rows8(const ResidentParams& p, int ng, int smem_bytes, cudaStream_t stream) {
+  if (ng > 4) return cudaErrorInvalidValue;
+  if (p.act == 0)
+    return ng <= 2 ? launch_one<VAR, 1, 2, 0, CLUSTER>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 0, CLUSTER>(p, smem_bytes, stream);
+  return ng <= 2 ? launch_one<VAR, 1, 2, 1, CLUSTER>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 1, CLUSTER>(p, smem_bytes, stream);
 }
 
 template <int VAR>
 static cudaError_t launch_var(int var, const ResidentParams& p, int mt, int ng, int smem_bytes, cudaStream_t stream) {
   if constexpr (VAR % B200Q_NPARTS == B200Q_PART) {
     if (var == VAR) {
-      if (mt == 2 && ng <= 2 && p.act == 0) return launch_one<VAR, 2, 2, 0>(p, smem_bytes, stream);
-      if (mt != 1 || ng > 4) return cudaErrorInvalidValue;
-      if (p.act == 0)
-        return ng <= 2 ? launch_one<VAR, 1, 2, 0>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 0>(p, smem_bytes, stream);
-      return ng <= 2 ? launch_one<VAR, 1, 2, 1>(p, smem_bytes, stream) : launch_one<VAR, 1, 4, 1>(p, smem_bytes, stream);
+      if (mt == 2) return ng <= 2 && p.act == 0 && p.S == 1 ? launch_one<VAR, 2, 2, 0, false>(p, smem_bytes, stream) : cudaErrorInvalidValue;
+      return p.S > 1 ? launch_rows8<VAR, true>(p, ng, smem_bytes, stream) : launch_rows8<VAR, false>(p, ng, smem_bytes, stream);
     }
   }
   if constexpr (VAR + 1 < VAR_COUNT) return launch_var<VAR + 1>(var, p, mt, ng, smem_bytes, stream);
