@@ -102,10 +102,10 @@ def test_k_chunks_of_two_to_eight_rows(m, n, k, w, splits):
 
 
 @pytest.mark.parametrize("m,n,k,w,act,resident", [
-    (1, 28672, 4096, "uint4b", 0, 1), (1, 4096, 5120, "uint4b", 0, 1), (1, 6144, 5120, "uint4b", 0, 0), (1, 4096, 8192, "uint4b", 0, 2), (1, 6144, 8192, "uint4b", 0, 0),
-    (1, 8192, 8192, "uint4b", 0, 2), (1, 8192, 6144, "uint4b", 0, 0), (1, 8192, 2048, "uint2b", 0, 1), (1, 11008, 2048, "uint2b", 0, 0), (1, 16384, 4096, "int3b", 0, 1),
-    (1, 28672, 4096, "int3b", 0, 0), (1, 4096, 14336, "uint4b", 0, 4), (1, 4096, 14336, "float6_e3m2", 0, 0), (1, 28672, 14336, "int8", 0, 2), (1, 8192, 11008, "uint4b", 0, 2),
-    (2, 4096, 4608, "uint4b", 0, 1), (2, 6144, 4608, "uint4b", 0, 0), (4, 8192, 5120, "uint4b", 0, 1), (4, 16384, 5120, "uint4b", 0, 0), (4, 8192, 14336, "float6_e3m2", 0, 0),
+    (1, 28672, 4096, "uint4b", 0, 1), (1, 4096, 5120, "uint4b", 0, 1), (1, 6144, 5120, "uint4b", 0, 1), (1, 8192, 6144, "uint4b", 0, 0), (1, 4096, 8192, "uint4b", 0, 1), (1, 6144, 8192, "uint4b", 0, 1),
+    (1, 8192, 8192, "uint4b", 0, 2), (1, 8192, 6144, "uint4b", 0, 0), (1, 8192, 2048, "uint2b", 0, 1), (1, 11008, 2048, "uint2b", 0, 0), (1, 16384, 4096, "int3b", 0, 1), (1, 28672, 14336, "uint4b", 0, 0), (1, 8192, 14336, "int3b", 0, 0),
+    (1, 28672, 6144, "int3b", 0, 0), (1, 4096, 14336, "uint4b", 0, 4), (1, 4096, 14336, "float6_e3m2", 0, 0), (1, 28672, 14336, "int8", 0, 4), (1, 8192, 11008, "uint4b", 0, 2),
+    (2, 4096, 4608, "uint4b", 0, 1), (2, 6144, 4608, "uint4b", 0, 1), (2, 8192, 4608, "uint4b", 0, 0), (4, 8192, 5120, "uint4b", 0, 1), (4, 16384, 5120, "uint4b", 0, 0), (4, 8192, 14336, "float6_e3m2", 0, 0),
     (8, 28672, 4096, "uint4b", 0, 1), (8, 4096, 5120, "uint4b", 0, 2), (8, 4096, 5120, "int8", 0, 1), (8, 8192, 8192, "uint4b", 0, 2), (8, 4096, 14336, "float6_e3m2", 0, 4),
     (8, 16384, 14336, "float6_e3m2", 0, 0), (8, 1024, 4224, "int6b", 0, 1), (8, 16384, 14336, "uint4b", 0, 2),
     (9, 11008, 4096, "uint4b", 0, 1), (9, 14336, 4096, "uint4b", 0, 0), (13, 4096, 4096, "uint4b", 0, 1), (13, 6144, 4096, "uint4b", 0, 0),

@@ -687,9 +687,11 @@ static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInf
 //  - 5 to 8 rows 0.44 .. 0.97, except 5 to 7 bits on 16384 columns and more beyond 4096 rows of K (1.00 .. 1.03); 2 to 4 rows 0.49 .. 1.0,
 //    except where 4096 to 6144 rows of K, in two or three groups per warp, meet many columns (2 x 28672 x 4608 1.16), and 5 to 7 bits beyond
 //    8192 rows of K (1.00 .. 1.03);
-//  - one row: up to 4096 rows of K 0.71 .. 0.99, for 1 and 2 bits up to 8192 columns, 3 bits up to 16384 (2 bits, 28672 x 4096 1.06);
-//    up to 8192 rows of K two column tiles per CTA 0.76 .. 0.99 (1 and 2 bits one), and from 7168 on wide layers 0.94 .. 1.02
-//    (6144 x 8192 1.02, 28672 x 4608 1.20); beyond, 0.75 .. 1.0 but for 5 to 7 bits (1.1);
+//  - one row: up to 4096 rows of K 0.68 .. 1.0 (2 bits, 28672 x 2048 1.02); up to 8192 rows of K 0.81 .. 1.0 in 5 bits and more, one CTA
+//    per cluster (two: 0.85 .. 1.09), 0.85 .. 0.98 in 1 and 2 bits up to 8192 columns (28672 x 6144 1.04), and in 3 and 4 bits 0.83 .. 1.0 up to
+//    6144 columns and, two CTAs per cluster, 0.95 .. 0.99 on wide layers of 7168 rows of K and more (4 bits, 8192 x 4608 1.05, 28672 x 4608
+//    1.17); beyond, 0.87 .. 0.95 in 8 bits, 0.72 .. 0.98 in 4 bits (28672 x 14336 1.0), 0.88 .. 1.0 in fewer up to 4096 columns (3 bits,
+//    28672 x 14336 1.04, 2 bits 1.08), 1.0 .. 1.1 in 5 to 7 bits;
 //  - 9 to 16 rows (fp16 only: the exact kernel takes bfloat16 as it is), whose second set of sums makes the loop 1.5 times longer: up to
 //    4096 rows of K in the ranges below 0.63 .. 0.96; beyond 1.0 .. 1.3.  Among layers that stay with the exact kernel, whose launches
 //    leave SMs to their successors, a launch on all SMs costs those up to 2 us: with 4096 x 4096 here a Llama-3-8B block takes, us, at 9
@@ -707,19 +709,22 @@ static int resident_cluster(int M, int N, int K, int var, int group, int act, bo
     if (G > 16 && ((bits == 8 && M > 12) || (bits == 4 && M > 14))) return 0;
     S = 1;
   } else {
-    if (G <= 32) S = 1;
-    else if (G <= 40) S = M >= 5 && bits <= 4 ? 2 : 1;
-    else if (G <= 64) S = M == 1 && G < 56 && N < 8192 ? 1 : 2;
-    else S = G <= 128 && (N >= 16384 || (G <= 96 && N >= 8192)) ? 2 : 4;
     const bool dear = bits >= 5 && bits <= 7;
+    if (G <= 32) S = 1;
+    else if (M == 1 && G <= 64) S = N < 8192 || bits <= 2 || bits >= 5 ? 1 : 2;
+    else if (G <= 40) S = M >= 5 && bits <= 4 ? 2 : 1;
+    else if (G <= 64) S = 2;
+    else if (M == 1) S = G <= 128 && N >= 8192 && bits <= 4 ? 2 : 4;
+    else S = G <= 128 && (N >= 16384 || (G <= 96 && N >= 8192)) ? 2 : 4;
     if (M == 1 && G <= 32) {
-      if (N > (bits <= 2 ? 8192 : bits == 3 ? 16384 : 1 << 30)) return 0;
+      if (bits <= 2 && N > 8192 && G <= 16) return 0;
     } else if (M == 1 && G <= 64) {
-      if (bits <= 2 ? N > 2048 : N > 4096 && !(N >= 8192 && G >= 56)) return 0;
+      if (bits <= 4 && (bits <= 2 ? N > 8192 : N >= 8192 && G < 56)) return 0;
     } else if (M == 1) {
-      if (dear && stream_form) return 0;
+      if (bits <= 4 ? N > (bits <= 3 ? 4096 : 16384) : dear && stream_form) return 0;
     } else if (M <= 4 && stream_form) {
-      if (G > 32 && G < 48 && N >= (M == 2 ? 6144 : 14336)) return 0;
+      if (G > 32 && G < 48 && N >= (M == 2 ? 8192 : 14336)) return 0;
+      if (M == 2 && G >= 48 && G < 56 && N >= 16384) return 0;
       if (G > 64 && dear && N >= 6144) return 0;
     } else if (M >= 5 && dear && G > 32 && N >= 16384) {
       return 0;
