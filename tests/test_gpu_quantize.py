@@ -35,6 +35,34 @@ def test_rounding_boundaries_groups_and_alignment(dt, k, group, aligned):
     assert torch.equal(packed.cpu(), packing.interleave(torch.from_numpy(codes_ref), dt))
 
 
+@pytest.mark.parametrize("dt", [D.float3_e1m1, D.float4_e2m1, D.float5_e2m2, D.float6_e3m2, D.float6_e2m3, D.float7_e3m3, D.float5_e1m3, D.float8_e5m2, D.int3b, D.uint5b],
+                         ids=lambda d: d.name)
+@pytest.mark.parametrize("wdtype", [torch.float16, torch.bfloat16, torch.float32], ids=["f16", "bf16", "f32"])
+@pytest.mark.parametrize("xdtype,group", [(torch.float16, 128), (torch.bfloat16, 96)])
+def test_quotients_next_to_every_rounding_boundary(dt, wdtype, xdtype, group):
+    """Quotients at every tie of the type and the fp32 numbers next to it, below the smallest number, at zeros of both signs and beyond the
+    largest number (the scale's own rounding); scales that are powers of two and scales that are not.  Bit for bit."""
+    n, k = 48, 384
+    top = float(dt.max_value)
+    steps = 64 if dt.nbits > 4 else 16
+    gen = torch.Generator().manual_seed(dt.nbits)
+    tie = (torch.randint(0, 2 * steps, (n, k), generator=gen) * 2 + 1).float() / (4 * steps) * 2.0 ** torch.randint(-18, 1, (n, k), generator=gen).float()
+    w = tie * top * torch.where(torch.rand(n, k, generator=gen) < 0.5, -1.0, 1.0)
+    w *= 1.0 + torch.randint(-2, 3, (n, k), generator=gen).float() * 2.0 ** -23
+    w[:, 5::7] *= 2.0 ** -30
+    w[:, 3::group] = 0.0
+    w[:, 4::group] = -0.0
+    w[:, ::group] = top
+    w *= torch.where(torch.arange(n) % 2 == 0, torch.tensor(2.0 ** -6), 0.013 + torch.rand(n, generator=gen)).view(n, 1)
+    w[7] *= 0.0
+    wd = w.to(wdtype)
+    packed, scales = quantize.quantize_and_pack(wd.cuda(), dt, group, xdtype)
+    torch.cuda.synchronize()
+    codes, want = quantize.quantize_weight(wd, dt, group, xdtype)
+    assert torch.equal(scales.cpu().view(torch.int16), want.view(torch.int16))
+    assert torch.equal(packed.cpu(), packing.interleave(codes, dt))
+
+
 def _moved(layer, how):
     from torch import nn
 

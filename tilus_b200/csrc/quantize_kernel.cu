@@ -15,19 +15,21 @@
 // with 16-byte loads, quantizes them, builds the unit's plane words in registers (signed integers in
 // offset binary) and stores them at the unit's place.  Scale groups of 32, 64 and 128 rows lie inside the four
 // neighbouring lanes of a column, so their absmax is a shuffle and the dense weight is read once; other
-// groups get their scales from a pass of their own (quant_scales_kernel, one warp per column and group).
+// groups get their scales from a pass of their own (quant_scales_kernel; a warp per column and group, 8 weights per lane, left most of its lanes
+// waiting: 14336 x 4096 int4 in groups of 256 85 us, with 32 weights per lane and as many lanes as the group needs 60).
 //
 // What bounds it: HBM (2 or 4 bytes read and b/8 written per weight), provided the arithmetic stays near four
-// instructions per weight.  The IEEE division of the definition alone is ten, so integer codes come
-// from one multiplication by the reciprocal of the scale, and only a unit with a value within the
-// multiplication's error of a rounding boundary is computed again with the division: the codes are
-// those of the division in every case.  Signed types (signed_codes) need no clamping where the unit's largest weight
-// rounds inside the range, work on two values per instruction and pack 2, 4 and 8 bits in fp32.  fp16 [28672, 4096] ->
-// int4 g128: 94 us with clamping and bit packing per value and 1024 threads per SM, 62 us now with 2048 (66 with 1536,
-// 79 with 1024: a thread's loads are in flight for half of its life; 45 us at the copy rate of HBM).  2048 threads leave 32
-// registers: the 16-bit builds of 3 and of 5 to 8 bits spill 12 .. 52 bytes to the stack and are still ahead of 1536 threads with 40
-// and no spills (28672 x 4096: int3 72 / 75 us, int5 69 / 71, int6 67 / 68, int7 71 / 72, int8 60 / 61; small layers up to 4 % behind,
-// 2048 x 2048, int8: 6.4 / 6.1).
+// instructions per weight.  The IEEE division of the definition alone is ten and the float types' encode thirty, so integer codes come
+// from one multiplication by the reciprocal of the scale, and only a unit with a value within the multiplication's error of a rounding
+// boundary is computed again from correctly rounded quotients (quotient_f2, three instructions for two weights); float codes come from such
+// quotients at once (float_codes).  The codes are those of the division in every case; a scale of 1e30 and more, or a NaN among the weights of a
+// float type, takes the definition as it stands.  Signed types (signed_codes) need no clamping where the unit's largest weight
+// rounds inside the range, work on two values per instruction and pack 2, 4 and 8 bits in fp32.  [28672, 4096], group 128, us (45 at the copy
+// rate of HBM, int4), before the quotients / now: fp16 -> int4 67 / 60, int3 78 / 64, float6 304 / 76, float4 320 / 68; bf16 -> int4 88 / 66,
+// int3, whose quotients meet the boundaries more often, 109 / 78.  A ring of cp.async stages, 1024 threads per SM, instead of plain loads: int4
+// 63, float6 84 (fp32 weights, 14336 x 4096, 55 instead of 63).  2048 threads leave 32 registers: the 16-bit builds of 5 to 8
+// bits spill 32 .. 64 bytes to the stack and are still ahead of 1536 threads with 40 and no spills (28672 x 4096: int5 69 / 71 us, int6 67 / 68,
+// int7 71 / 72, int8 60 / 61); float types of two planes and more are not (float6 82 / 76).
 #include "common.cuh"
 
 namespace b200q {
@@ -43,6 +45,7 @@ struct QuantParams {
   int kind, ebits, mbits;  // kind: 0 unsigned, 1 two's complement, 2 float
   int vec;                 // every row starts on a 16-byte boundary
   int gshift;              // log2(group) if local
+  int lshift;              // log2 of the lanes that find a group's scale, if not local
   int local;               // groups of 32, 64 or 128 rows: inside the four neighbouring lanes of a column
   float minv, maxv;
 };
@@ -55,42 +58,6 @@ __device__ __forceinline__ float load_scale(const QuantParams& p, size_t idx) {
 __device__ __forceinline__ unsigned short scale_bits(const QuantParams& p, float amax) {
   const float sc = fmaxf(__fdiv_rn(amax, p.maxv), 1e-6f);
   return p.act == 0 ? __half_as_ushort(__float2half_rn(sc)) : __bfloat16_as_ushort(__float2bfloat16_rn(sc));
-}
-
-// E consecutive weights from element idx on, E a multiple of 8, as fp32.  WT: 0 fp16, 1 fp32, 2 bf16;
-// p.vec: rows are 16-byte aligned
-template <int WT, int E>
-__device__ __forceinline__ void load_weights(const QuantParams& p, size_t idx, float (&v)[E]) {
-  if (p.vec) {
-    constexpr int PER = WT == 1 ? 4 : 8;  // weights per 16 bytes
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p.w) + idx * (WT == 1 ? 4 : 2));
-    uint4 raw[E / PER];
-#pragma unroll
-    for (int i = 0; i < E / PER; ++i) raw[i] = __ldg(src + i);
-#pragma unroll
-    for (int i = 0; i < E / PER; ++i) {
-      const uint32_t x[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if constexpr (WT == 0) {
-          const float2 f = __half22float2(h2_from_bits(x[q]));
-          v[i * 8 + 2 * q] = f.x; v[i * 8 + 2 * q + 1] = f.y;
-        } else if constexpr (WT == 2) {
-          v[i * 8 + 2 * q] = __uint_as_float(x[q] << 16);
-          v[i * 8 + 2 * q + 1] = __uint_as_float(x[q] & 0xffff0000u);
-        } else {
-          v[i * 4 + q] = __uint_as_float(x[q]);
-        }
-      }
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < E; ++i) {
-      if constexpr (WT == 0) v[i] = __half2float(reinterpret_cast<const __half*>(p.w)[idx + i]);
-      else if constexpr (WT == 2) v[i] = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.w)[idx + i]);
-      else v[i] = reinterpret_cast<const float*>(p.w)[idx + i];
-    }
-  }
 }
 
 // ---- two fp32 values at a time (one instruction on sm_100) ----
@@ -171,26 +138,24 @@ struct UnitWeights {
   }
 };
 
-// scales of groups that are not 32, 64 or 128 rows: one warp per (column, group), 8 weights per lane and step
+// scales of groups that are not 32, 64 or 128 rows: p.lanes lanes per (column, group), 32 weights each and step
 template <int WT>
 __global__ void __launch_bounds__(256) quant_scales_kernel(const QuantParams p) {
-  const int lane = threadIdx.x & 31;
-  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int groups = p.K / p.group;
-  if (wid >= (long long)p.N * groups) return;
-  const int n = (int)(wid / groups), g = (int)(wid % groups);
-  const size_t base = (size_t)n * p.ldw + (size_t)g * p.group;
+  const long long id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> p.lshift;
+  const int lane = threadIdx.x & ((1 << p.lshift) - 1), groups = p.K / p.group;
   float m = 0.f;
-#pragma unroll 2
-  for (int i = lane * 8; i < p.group; i += 256) {  // group is a multiple of 32
-    float v[8];
-    load_weights<WT, 8>(p, base + i, v);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) m = fmaxf(m, fabsf(v[q]));
+  int n = 0, g = 0;
+  if (id < (long long)p.N * groups) {
+    n = (int)(id / groups), g = (int)(id - (long long)n * groups);
+    const size_t base = (size_t)n * p.ldw + (size_t)g * p.group;
+    for (int i = lane * 32; i < p.group; i += 32 << p.lshift) {
+      UnitWeights<WT> v;
+      v.load(p, base + i);
+      m = fmaxf(m, v.largest());
+    }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) p.scales[(size_t)g * p.N + n] = scale_bits(p, m);
+  for (int o = 1 << p.lshift >> 1; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0 && id < (long long)p.N * groups) p.scales[(size_t)g * p.N + n] = scale_bits(p, m);
 }
 
 // fp32 -> sub-byte float code (sign / e exponent bits / m mantissa bits)
@@ -295,14 +260,58 @@ __device__ __forceinline__ void put_pair(uint32_t both, uint32_t (&words)[B]) {
   w |= (pos >= lo ? both << (pos >= lo ? pos - lo : 0) : both >> (pos < lo ? lo - pos : 0)) & mask;
   if constexpr (P + 1 < plane_count(B)) put_pair<B, I, P + 1>(both, words);
 }
+// put_pair of both_of(i) for every pair i of a unit
+template <int B, int I = 0, class F>
+__device__ __forceinline__ void put_pairs_of(const F& both_of, uint32_t (&words)[B]) {
+  put_pair<B, I>(both_of(I), words);
+  if constexpr (I + 1 < 16) put_pairs_of<B, I + 1>(both_of, words);
+}
 template <int B, int I>
 __device__ __forceinline__ void put_pairs(const uint32_t (&code)[32], uint32_t (&words)[B]) {
   put_pair<B, I>(__byte_perm(code[2 * I], code[2 * I + 1], 0x5410), words);
   if constexpr (I + 1 < 16) put_pairs<B, I + 1>(code, words);
 }
 
+// x / s for a pair, correctly rounded: q = x * rs with rs = rn(1 / s), then q + rn(x - q * s) * rs (Markstein, IBM J. Res. Dev. 34(1), 1990).
+// s is a 16-bit scale, 11 significant bits at most: the remainder is exact (q is off by two units at most, so that it has 13 bits), and
+// a quotient by s stays 2^-36 of itself away from the midpoint of two fp32 numbers, where the sum is off by 2^-46 before it is rounded.
+// For 1e-6 <= s < 1e30; quotients below 2^-80, whose remainder may underflow, have code 0 either way.
+// `q` is the first product: it has the sign of the quotient where that is zero, too.
+__device__ __forceinline__ f32x2 quotient_f2(float2 x, f32x2 rs, f32x2 minus_s, f32x2& q) {
+  const f32x2 v = pack_f2(x.x, x.y);
+  q = fma_f2(v, rs, 0x8000000080000000ull);
+  return fma_f2(fma_f2(q, minus_s, v), rs, q);
+}
+
+// Codes of a unit of a float type (E exponent bits, M mantissa bits) without clamping; returns the largest quotient, NaN if one is.
+// encode_float_code rounds to M + 1 significant bits and then cuts off what the type's subnormals lack: here the first is
+// (q + c) - c with c = 1.5 * 2^(23 - M) times q's power of two, the second a product with 2^(bias - 127), after which exponent and
+// mantissa stand in fp32's fields as in the code (subnormal where the code is).
+template <int B, class Weights>
+__device__ __forceinline__ float float_codes(const QuantParams& p, const Weights& v, float s, float rs, uint32_t (&words)[B]) {
+  const f32x2 rs2 = pack_f2(rs, rs), ms2 = pack_f2(-s, -s);
+  const float c = 1.5f * (float)(1 << (23 - p.mbits)), bias = __uint_as_float(p.ebits == 1 ? 1u << 22 : ((1u << (p.ebits - 1)) - 1u) << 23);
+  const f32x2 c2 = pack_f2(c, c), mc2 = pack_f2(-c, -c), b2 = pack_f2(bias, bias);
+  const uint32_t mags = ((1u << (B - 1)) - 1u) * 0x00010001u;
+  float top = 0.f;
+#pragma unroll
+  for (int q = 0; q < B; ++q) words[q] = 0u;
+  put_pairs_of<B>([&](int i) {
+    f32x2 q0;
+    const f32x2 q = quotient_f2(v.pair(i), rs2, ms2, q0);
+    const float2 qf = unpack_f2(q), sf = unpack_f2(q0);
+    top = max_abs(qf.x, qf.y, top);
+    const f32x2 e = q & 0x7f8000007f800000ull;
+    const float2 r = unpack_f2(fma_f2(fma_f2(e, mc2, fma_f2(e, c2, q)), b2, 0x8000000080000000ull));
+    const uint32_t w = __byte_perm(__float_as_uint(r.x), __float_as_uint(r.y), 0x7632);
+    const uint32_t signs = __byte_perm(__float_as_uint(sf.x), __float_as_uint(sf.y), 0x7632);
+    return ((w >> (7 - p.mbits)) & mags) | ((signs >> (16 - B)) & ((1u << (B - 1)) * 0x00010001u));
+  }, words);
+  return top;
+}
+
 template <int WT, int B, bool FLOAT>
-__global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(256, WT == 1 ? 4 : FLOAT && plane_count(B) > 1 ? 6 : 8) quant_pack_kernel(const QuantParams p) {
   // unit index = ((nt * G + g) * 2 + half) * 32 + lane,  lane = r * 4 + j,  g = 128-row group of K.  A block has four groups,
   // of one 16-column tile where G allows it (a 64-bit division per thread costs as much as a quarter of its weights).
   const int lane = threadIdx.x & 31, half = (threadIdx.x >> 5) & 1;
@@ -336,23 +345,21 @@ __global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const 
   uint32_t words[B];
 #pragma unroll
   for (int q = 0; q < B; ++q) words[q] = 0u;
+  const float rs = __fdiv_rn(1.0f, s);
+  const bool plain = s < 1e30f;
+  bool done = false;
   if constexpr (FLOAT) {
-    put_codes<B, 0>([&](int i) {
-      const float q = fminf(fmaxf(__fdiv_rn(v[i], s), p.minv), p.maxv);
-      return encode_float_code(q, B, p.ebits, p.mbits);
-    }, words);
+    // a largest quotient that rounds to the type's largest number needs no clamping
+    if (plain) done = float_codes<B>(p, v, s, rs, words) <= p.maxv + p.maxv * __uint_as_float((124u - p.mbits) << 23);
   } else {
     // Signed types whose largest weight of the unit rounds inside the range: no clamping, see signed_codes.  A unit with a
-    // value within the products' error of a rounding boundary, or a NaN, takes the division below.
-    constexpr float EPS = (float)(1 << B) * (1.0f / (1 << 22));
-    const float rs = __fdiv_rn(1.0f, s);
-    bool done = false;
-    if (p.kind == 1 && s < 1e30f && unit_max * rs <= p.maxv + (0.5f - EPS)) {
+    // value within the products' error of a rounding boundary, or a NaN, takes the quotients below.
+    constexpr float EPS = (float)(1 << B) * (1.0f / (1 << 22)), MAGIC = 12582912.0f;
+    if (p.kind == 1 && plain && unit_max * rs <= p.maxv + (0.5f - EPS)) {
       done = signed_codes<B>(v, rs, words) <= 0.5f - EPS;
-    } else if (p.kind == 0 && s < 1e30f) {
+    } else if (p.kind == 0 && plain) {
       // Unsigned types: code = rint(clamp(w / s)).  Estimate: x = w * (1 / s), |x - w / s| < 2^(B-22); adding 1.5 * 2^23
       // rounds it to an integer in the low bits.
-      constexpr float MAGIC = 12582912.0f;
       float worst = 0.f;
       put_codes<B, 0>([&](int i) {
         const float x = fminf(fmaxf(v[i] * rs, p.minv), p.maxv);
@@ -362,14 +369,26 @@ __global__ void __launch_bounds__(256, WT == 1 ? 4 : 8) quant_pack_kernel(const 
       }, words);
       done = worst <= 0.5f - EPS;
     }
-    if (!done) {  // the definition's own division
+    if (!done && plain) {
+      const f32x2 rs2 = pack_f2(rs, rs), ms2 = pack_f2(-s, -s);
+      const float off = MAGIC + (p.kind == 1 ? (float)(1 << (B - 1)) : 0.f);
 #pragma unroll
       for (int q = 0; q < B; ++q) words[q] = 0u;
-      put_codes<B, 0>([&](int i) {
-        const float q = fminf(fmaxf(__fdiv_rn(v[i], s), p.minv), p.maxv);
-        return (uint32_t)((int)rintf(q) + (p.kind == 1 ? (1 << (B - 1)) : 0));
+      put_pairs_of<B>([&](int i) {
+        f32x2 q0;
+        const float2 q = unpack_f2(quotient_f2(v.pair(i), rs2, ms2, q0));
+        return __byte_perm(__float_as_uint(fminf(fmaxf(q.x, p.minv), p.maxv) + off), __float_as_uint(fminf(fmaxf(q.y, p.minv), p.maxv) + off), 0x5410);
       }, words);
+      done = true;
     }
+  }
+  if (!done) {  // the definition as it stands
+#pragma unroll
+    for (int q = 0; q < B; ++q) words[q] = 0u;
+    put_codes<B, 0>([&](int i) {
+      const float q = fminf(fmaxf(__fdiv_rn(v[i], s), p.minv), p.maxv);
+      return FLOAT ? encode_float_code(q, B, p.ebits, p.mbits) : (uint32_t)((int)rintf(q) + (p.kind == 1 ? (1 << (B - 1)) : 0));
+    }, words);
   }
   uint32_t* dst = p.bq + (size_t)unit * B;
   if constexpr (B % 4 == 0) {
@@ -397,8 +416,8 @@ static cudaError_t pack_launch(const QuantParams& p, int nbits, cudaStream_t str
 template <int WT>
 static cudaError_t quantize_as(const QuantParams& p, int nbits, cudaStream_t stream) {
   if (!p.local) {
-    const long long warps = (long long)p.N * (p.K / p.group);
-    quant_scales_kernel<WT><<<(unsigned)((warps * 32 + 255) / 256), 256, 0, stream>>>(p);
+    const long long threads = ((long long)p.N * (p.K / p.group)) << p.lshift;
+    quant_scales_kernel<WT><<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(p);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -419,6 +438,7 @@ cudaError_t quantize_launch(const void* w, int w_dtype, int ldw, void* bq, void*
   p.vec = (((uintptr_t)w & 15) == 0 && ldw % (w_dtype == 1 ? 4 : 8) == 0) ? 1 : 0;
   p.local = 128 % group == 0 ? 1 : 0;
   p.gshift = group == 32 ? 5 : group == 64 ? 6 : 7;
+  for (p.lshift = 0; p.lshift < 5 && 32 << p.lshift < group;) ++p.lshift;  // a lane has 32 rows or more, a group up to a warp
   if (w_dtype == 1) return quantize_as<1>(p, nbits, stream);
   if (w_dtype == 2) return quantize_as<2>(p, nbits, stream);
   return quantize_as<0>(p, nbits, stream);
