@@ -648,7 +648,7 @@ def run_b200(args) -> None:
                          "frac": achieved / hbm,
                          "traffic": traffic["dram_bytes_per_launch"] if traffic else None,
                          "traffic_capture": {k: traffic[k] for k in ("commit", "command")} if traffic else None,
-                         "peak_source": peaks["source"], "kernel": "stream_kernel<u4 zp8, MT=1>",
+                         "peak_source": peaks["source"], "kernel": "resident_kernel<u4 zp8, up to 8 rows, clusters of 2>",
                          "bytes_per_launch": nbytes, "us_per_launch": per_launch_s * 1e6},
             "cpu_baseline": cpu_baseline,
             "e2e": {"value": e2e_val, "unit": "GB/s", "h2d_bytes_per_step": R_LAYERS * M * K * 2,

@@ -104,9 +104,9 @@ size_t b200q_workspace_bytes(int M, int N, int K, int wtype, int zero_point, int
 /* C = A x dequant(Bq).  a: [M, K] (row stride lda elements), bq: b200-packed weights,
  * scales: [K/group, N], c: [M, N] (row stride ldc), all three of dtype act_dtype.  Replaces
  * tilus_launch for QuantizedMatmul (examples/quantization/matmul_a16wx.py:231-405).  The tcgen05
- * kernels multiply bf16 activations as they are.  The stream kernel (b200q_plan_for: kernel 2 with
+ * kernels multiply bf16 activations as they are.  The mma.sync kernels (b200q_plan_for: kernel 2 with
  * tile_m 0; bf16 batches of up to 8 rows at most shapes, and up to 16 rows of the host-buffer and gather
- * calls) converts them to fp16 for the tensor core: exactly, except that magnitudes above
+ * calls) convert them to fp16 for the tensor core: exactly, except that magnitudes above
  * 65504 saturate there and magnitudes below 2^-24 become zero. */
 int b200q_gemm(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
                int wtype, int zero_point, int group, int act_dtype, void* workspace, size_t workspace_bytes,

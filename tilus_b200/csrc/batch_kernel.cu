@@ -7,25 +7,26 @@
 // time of the weights up to about 80 rows of 4-bit weights, and nothing the weights pass through is
 // wider than their packed form: global -> (tiled copy) -> shared -> registers -> tensor memory.
 //
-// Roles of the 16 warps of a CTA:
-//   * warps 0-7 dequantize, in two sets of four (a set covers the 128 lanes; lane L is column L of the
-//     tile).  Set s takes the 128-row groups s, s + 2, ... of the CTA: a lane reads its column's four
+// Roles of the warps of a CTA, 16 with two dequantizing sets, 20 with three (api.cu, batch_sets):
+//   * the first 8 or 12 dequantize, in sets of four (a set covers the 128 lanes; lane L is column L of the
+//     tile).  Set s takes the 128-row groups s, s + sets, ... of the CTA: a lane reads its column's four
 //     units, decodes and scales them (decode.cuh, unit_decode_scaled: the weights the reference
 //     multiplies by, examples/quantization/matmul_a16wx.py:316-320) and writes 64 tensor-memory columns.
 //     Each set has operand slots and ring stages of its own, so that every waiter of a ring barrier sees each
-//     of its phases in turn (a third set measured slower: 12.9 -> 12.3 us at 16 x 4096 x 14336 without it);
-//   * warps 8-11 are the epilogue; the dequantize warps take a share of the run's last segment.  They
+//     of its phases in turn.  Two sets leave a third of the time to latencies: 620 cycles per group, 416 of them
+//     instructions (64 x 16384 x 4096, 4 bits 15.6 us, with three sets 14.6);
+//   * the next four warps are the epilogue; the dequantize warps take a share of the run's last segment.  They
 //     do not follow the accumulators' barriers (d_full) from segment to segment - with few groups per tile they are
 //     several segments ahead of the MMAs, and a phase of two segments ago would pass for the last one's -
 //     but wait for a barrier of one phase, run_done, that the last MMA of the run completes;
-//   * warp 12 brings the activations, two 2-D tiled TMA copies (128-byte swizzle) per group;
-//   * warp 13 brings packed weights, a 128-row group of the 128 columns at a time: one 3-D tiled
+//   * one warp brings the activations, two 2-D tiled TMA copies (128-byte swizzle) per group;
+//   * one warp brings packed weights, a 128-row group of the 128 columns at a time: one 3-D tiled
 //     TMA copy for the eight 16-column pieces.  For 2, 4 and 8 bits it swizzles 16-byte chunks by
 //     128-byte line, which spreads eight neighbouring columns over all shared-memory banks (columns are
 //     16 * b bytes apart: unswizzled, 4-bit loads would collide four ways); other widths are left dense
 //     (two-way);
-//   * warp 14 owns tensor memory and issues eight tcgen05.mma per group;
-//   * warp 15 brings the scales.
+//   * one warp owns tensor memory and issues eight tcgen05.mma per group;
+//   * the last warp brings the scales.
 // The four single-thread roles run under elect.sync: copies and MMAs take their operands from uniform
 // registers.  (Eight lanes issuing one 1 KB bulk copy each took 1100 cycles per group; the copies of a
 // group may take 360 at the HBM rate of 4-bit weights.)
@@ -36,8 +37,8 @@
 // fp32 scratch tile (red.global.add.v4) and counted in, and whoever completes the count converts them,
 // writes C and puts the scratch back to zero (batch_epilogue).  These additions are the price of the form:
 // 4.8 MB of them at 64 rows keep L2 busy for 6 us.  Where the column tiles are few enough that every one can have
-// a cluster of CTAs to itself, the launch takes the cluster form instead (batch_common.cuh; the rule is in
-// api.cu).
+// a cluster of CTAs to itself, the launch takes the cluster form instead, whose CTAs send their sums to one another in bulk
+// copies (cluster_epilogue); where they fill one round of SMs, whole column tiles (the rule is in api.cu).
 //
 // Measured (4-bit, group 128, a chain of cold launches; the kernel before it wrote dequantized weights to
 // 256-column shared-memory operands): 64 x 28672 x 4096 44.5 -> 24.9 us, 64 x 8192 x 8192 28.2 -> 17.1,

@@ -1,4 +1,5 @@
 // Batches of up to 16 rows on tcgen05: C[M, N] = A[M, K] x dequant(Bq[K, N]) with exact weights.
+// Serves 9 to 16 rows and those of 5 to 8 that resident_kernel.cu does not take (api.cu, resident_cluster).
 //
 // Same product and work split as batch_kernel.cu (weights of 128 columns in tensor memory, equal runs of 128-row
 // groups per CTA), but the scale is not applied to the weights.  Every group's product is a sum of its own,

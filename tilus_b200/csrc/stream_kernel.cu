@@ -1,4 +1,5 @@
 // Decode path: C[M<=16, N] = A[M, K] x dequant(Bq[K, N]) - the memory-bound GEMV / skinny GEMM.
+// Serves host-buffer and gather calls, and of the others what resident_kernel.cu does not take (api.cu, resident_cluster).
 //
 // Data movement.  The (column tile, k block) items of the weight matrix - GI consecutive
 // 128-row groups of a 16-column x 512-row block, 1..2 KB contiguous - are cut into equal
