@@ -108,7 +108,7 @@ def test_k_chunks_of_two_to_eight_rows(m, n, k, w, splits):
     (2, 4096, 4608, "uint4b", 0, 1), (2, 6144, 4608, "uint4b", 0, 1), (2, 8192, 4608, "uint4b", 0, 0), (4, 8192, 5120, "uint4b", 0, 1), (4, 16384, 5120, "uint4b", 0, 0), (4, 8192, 14336, "float6_e3m2", 0, 0),
     (8, 28672, 4096, "uint4b", 0, 1), (8, 4096, 5120, "uint4b", 0, 2), (8, 4096, 5120, "int8", 0, 1), (8, 8192, 8192, "uint4b", 0, 2), (8, 4096, 14336, "float6_e3m2", 0, 4),
     (8, 16384, 14336, "float6_e3m2", 0, 0), (8, 1024, 4224, "int6b", 0, 1), (8, 16384, 14336, "uint4b", 0, 2),
-    (9, 11008, 4096, "uint4b", 0, 1), (9, 14336, 4096, "uint4b", 0, 0), (13, 4096, 4096, "uint4b", 0, 1), (13, 6144, 4096, "uint4b", 0, 0),
+    (9, 11008, 4096, "uint4b", 0, 1), (9, 16384, 4096, "uint4b", 0, 1), (9, 18432, 4096, "uint4b", 0, 0), (9, 12288, 4096, "float6_e3m2", 0, 0), (13, 4096, 4096, "uint4b", 0, 1), (13, 6144, 4096, "uint4b", 0, 0),
     (15, 4096, 4096, "uint4b", 0, 0), (12, 4096, 4096, "int8", 0, 1), (13, 4096, 4096, "int8", 0, 0), (16, 4096, 2048, "int8", 0, 1), (16, 4096, 4096, "float6_e3m2", 0, 1),
     (16, 2048, 4096, "uint4b", 0, 0), (16, 8192, 1024, "uint4b", 0, 0), (16, 4096, 8192, "uint4b", 0, 0), (17, 4096, 4096, "uint4b", 0, 0),
     (8, 4096, 4096, "uint4b", 1, 1), (9, 4096, 4096, "uint4b", 1, 0), (8, 4096, 4224, "uint4b", 1, 0)])
