@@ -101,6 +101,20 @@ def test_activations_of_any_magnitude_are_multiplied_as_they_are(scale):
     assert _close(ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=dict(resident=1)), ref)
 
 
+@pytest.mark.parametrize("M,dt,mean", [
+    (8, D.uint8, 3.0), (8, D.int8, 0.0), (16, D.int8, 3.0), (8, D.uint7b, 3.0), (16, D.int7b, 3.0), (8, D.int7b, 0.0), (4, D.uint5b, 0.0),
+    (4, D.int6b, 0.0), (4, D.uint4b, 0.0), (8, D.int4b, 0.0), (8, D.uint3b, 0.0), (4, D.uint8, 3.0), (8, D.uint2b, 0.0)], ids=str)
+def test_results_as_near_as_those_of_the_kernel_beside_it(M, dt, mean):
+    """The share of results that are not the nearest fp16 value measures the error of the sums: 2^11 times that error.  Next to the
+    stream (M <= 4) and exact kernels' on the same operands, plus four standard deviations of a count of that size."""
+    N, K, group = 16384, 2048, 128
+    a, bq, sc, zp, ref = _problem(M, N, K, dt, group, mean=mean, seed=3)
+    nearest = ref.half()
+    ws = torch.zeros(ops.workspace_bytes(M, N, K, dt, zp, group), dtype=torch.uint8, device=a.device)
+    here, there = (int((_run(a, bq, sc, dt, zp, group, S, ws) != nearest).sum()) for S in (1, 0))
+    assert here <= there + 4 * there ** 0.5
+
+
 @pytest.mark.parametrize("M,gap", [(1, 1), (8, 3), (16, 8)])
 def test_outputs_inside_a_wider_tensor(M, gap):
     a, bq, sc, zp, ref = _problem(M, 272, 1024, D.uint4b, 128)

@@ -20,7 +20,12 @@
 // stream kernel multiplies them by 2^-T beforehand, which costs those below 2^(T-14) low bits), for half of the shifts of a single place.
 // The zero point: both accumulators start from a quarter of -zero_point * sum(a), and the other half is added behind the group's
 // products, so that sums of activations with a mean stay around zero on the way (the sums over a come from eight MMAs per group with a
-// constant operand, once per launch).  Per group the sums are multiplied by the scale in fp32: no weight is rounded.
+// constant operand, once per launch).  For 7 and 8 bits that is not enough: their running sums still reach a quarter of (zero point) * sum(a),
+// and activations around 3 at 5 to 16 rows left twice as many results off the nearest value as exact_kernel.cu does (0.20 and 0.55 %, there
+// 0.09 and 0.30).  8 bits are multiplied as code - zero_point instead, a byte permute and a half subtraction per pair (0.05 .. 0.08 %; us, as a
+// subnormal / so: 8 x 4096 x 4096 5.60 / 5.77, 8 x 28672 x 4096 21.0 / 21.1, 16 x 4096 x 2048 5.44 / 5.16); 7 bits, whose codes take six
+// instructions per pair already (28672 x 4096 25.7 us, so 29.2), have the zero point taken off by an MMA behind each 16 rows, as in the exact
+// kernel (27.2; 0.08 %).  Per group the sums are multiplied by the scale in fp32: no weight is rounded.
 //
 // Sums.  The 16 warps' parts of a column tile meet in shared memory (four tiles of room, an mbarrier that counts the warps and one
 // that frees the room), and one of the warps, in turn, adds them up in order and writes C: results repeat bit for bit.  Where the
@@ -45,7 +50,8 @@ namespace b200q {
 // (Places that need the fewest shifts.  Of those 1 and 2 bits take the highest: the tensor core keeps a subnormal's leading zeros, so that a
 // code at bit 0 costs the sums ten bits.  Error beyond the rounding of the results, rms of the results, 4096 to 14336 rows of K, 1 to 4 / 5 to 16
 // rows: 2 bits at 0 and 2 2.6e-6 / 2.2e-6, at 6 and 8 7e-8 / 1.1e-7; the stream / exact kernel 1.5e-6 / 2.1e-6.  8 bits at 2 instead of 0:
-// no difference, 1 % slower.  A pair's products carry the factor 2^T, one accumulator per place.)
+// no difference, 1 % slower.  5 and 6 bits from one and two places up: 0.30 and 0.17 % of the results off the nearest value, from here 0.14 and
+// 0.09, for two shifts per unit.  A pair's products carry the factor 2^T, one accumulator per place.)
 B200Q_HD constexpr int res_class(int b, int h) {
   return b == 2 ? ~h & 1 : b == 3 || b == 7 ? (h >> 1) & 1 : b == 5 ? (h ^ (h >> 2)) & 1 : h & 1;
 }
@@ -53,9 +59,10 @@ B200Q_HD constexpr int res_target(int b, int cls) {
   switch (b) {
     case 1: return 8 + cls;
     case 2: return 6 + 2 * cls;
-    case 6: return 2 * cls;
+    case 6: return 4 - 2 * cls;
     case 3: case 7: return 1 + 2 * cls;
-    case 4: case 5: return 4 * cls;
+    case 4: return 4 * cls;
+    case 5: return 1 + 4 * cls;
     default: return 0;
   }
 }
@@ -66,11 +73,17 @@ B200Q_HD constexpr int res_pair(int b, int cls, int i) {
     if (res_class(b, h) == cls && n++ == i) return h;
   return 0;
 }
+// types whose operand is the value code - zero_point, and those whose zero point has MMAs of its own
+B200Q_HD constexpr bool res_by_value(int v) { return !var_is_float(v) && var_bits(v) == 8 && var_bias(v) != 0; }
+B200Q_HD constexpr bool res_zero_mma(int v) { return !var_is_float(v) && var_bits(v) == 7 && var_bias(v) != 0; }
 template <int VAR, int H>
 __device__ __forceinline__ uint32_t res_operand(const uint32_t* w) {
   constexpr int B = var_bits(VAR);
   if constexpr (var_is_float(VAR)) return pair_raw<VAR, H>(w);
-  else {
+  else if constexpr (res_by_value(VAR)) {
+    const uint32_t code = __byte_perm(w[H >> 1], 0x64646464u, H & 1 ? 0x4341u : 0x4240u);  // 1024 + code
+    return bits_from_h2(__hsub2(h2_from_bits(code), h2_from_bits(dup16(half_bits_of_uint(1024u + var_bias(VAR))))));
+  } else {
     constexpr int T = res_target(B, res_class(B, H));
     if constexpr (lin_uniform_inverted(VAR)) return gather_pair<B, H, T>(w, 0u) ^ (0x00010001u << T);
     else return gather_pair<B, H, T>(w, 0u);
@@ -168,15 +181,17 @@ __device__ __forceinline__ void mma_m16n8k16_from(float (&d)[4], uint32_t a0, ui
 template <int VAR, int MT, int NG, int ACT, bool CLUSTER>
 __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const ResidentParams p) {
   constexpr int B = var_bits(VAR);
-  constexpr int BIAS = lin_uniform_bias(VAR);
+  constexpr bool ZERO_MMA = res_zero_mma(VAR);
+  constexpr int BIAS = res_by_value(VAR) || ZERO_MMA ? 0 : lin_uniform_bias(VAR);  // the zero point of the accumulators' start
   constexpr int GI = res_gi(B, NG);
   constexpr int IPT = NG / GI;             // slots per column tile
   constexpr uint32_t GROUP = 256u * B, SLOT = GI * GROUP;
   constexpr int T0 = var_is_float(VAR) ? 0 : res_target(B, 0), T1 = var_is_float(VAR) ? 0 : res_target(B, 1);
-  constexpr int FL = lin_factor_log2(VAR) - T0;
+  constexpr uint32_t ZP0 = (0x8000u | (uint32_t)(var_bias(VAR) << T0)) * 0x00010001u, ZP1 = (0x8000u | (uint32_t)(var_bias(VAR) << T1)) * 0x00010001u;
+  constexpr int FL = res_by_value(VAR) ? 0 : lin_factor_log2(VAR) - T0;
   constexpr float F = (lin_uniform_inverted(VAR) ? -1.0f : 1.0f) * (float)(1u << FL);
   constexpr int NBQ = MT * NG <= 2 ? 4 : 2;  // registers of a zero-point term: as the accumulators have it, or once
-  constexpr float R10 = (float)(1 << (T1 - T0)), R01 = 1.0f / R10;
+  constexpr float R10 = (float)(1 << T1) / (float)(1 << T0), R01 = 1.0f / R10;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -398,6 +413,10 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
         f2_unpack(T1 != T0 ? f2_mul(z0[mt], f2_pack(R10, R10)) : z0[mt], e0, e1);                                    \
         f2_unpack(T1 != T0 ? f2_mul(z1[mt], f2_pack(R10, R10)) : z1[mt], e2, e3);                                    \
         mma_m16n8k16_from(d1[mt], y0, y1, y2, y3, af[g][mt][H2], af[g][mt][H3], e0, e1, e2, e3);                     \
+      }                                                                                                              \
+      if constexpr (ZERO_MMA) {                                                                                      \
+        mma_m16n8k16(d0[mt], ZP0, ZP0, ZP0, ZP0, af[g][mt][H0], af[g][mt][H1]);                                      \
+        mma_m16n8k16(d1[mt], ZP1, ZP1, ZP1, ZP1, af[g][mt][H2], af[g][mt][H3]);                                      \
       }                                                                                                              \
     }                                                                                                                \
   }
