@@ -72,11 +72,11 @@ typedef struct b200q_plan {
   int32_t warps;         /* warps per CTA (output only) */
   int32_t passes;        /* launches: 2 when kernel 1 takes the multiple of 256 rows and kernel 2 the last 1..16 rows */
   int32_t pdl;           /* 1: launch with programmatic stream serialization (overlap with the previous kernel);
-                            kernel 3 always is, kernel 1 never */
+                            the tcgen05 kernels of kernels 2 and 3 always are, kernel 1 never */
   int32_t resident;      /* > 0 (kernel 2, and kernel 3 up to 16 rows): the call runs on the mma.sync kernel that keeps the
-                            activations in registers, with this many CTAs to a cluster that shares K (1, 2, 4); the other
-                            fields then describe the kernel that takes the call where it is 0, which an edit of any
-                            of them makes it */
+                            activations in registers, with this many CTAs to a cluster that shares K (1, 2, 4); of the other
+                            fields pdl applies to it, and kernel, splits, cluster, ctas_per_split, tile_m and stages describe
+                            the kernel that takes the call where this is 0, which an edit of any of these six makes it */
   uint64_t workspace_bytes;
 } b200q_plan_t;
 

@@ -6,6 +6,8 @@ from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 from tilus_b200.variants import supported_weight_dtypes
 
+from .launches import kernels, launches
+
 pytestmark = pytest.mark.gpu
 
 
@@ -135,6 +137,18 @@ def test_edits_of_other_fields_leave_the_kernel():
     got = ops.quantized_matmul(rows, bq, sc, D.uint4b, 128, zp, plan_override=pl)
     want = rows.float() @ ops.dequantize(bq, sc, D.uint4b, 128, zp).float()
     assert float((got.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (1, 8192, 8192), (16, 4096, 2048)])
+def test_a_plan_says_whether_the_launch_overlaps_the_one_before(M, N, K):
+    """pdl = 0 is for callers whose previous kernel writes weights or scales and releases its dependents early."""
+    a, bq, sc, zp, ref = _problem(M, N, K, D.uint4b, 128)
+    pl = ops.plan(M, N, K, D.uint4b, zp, 128)
+    assert pl["resident"] > 0 and pl["pdl"] == 1
+    early, late = (lambda pdl=pdl: ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=dict(pdl=pdl)) for pdl in (1, 0))
+    assert _close(late(), ref) and torch.equal(early(), late())
+    assert [e for _, e in launches(early, early, late, early, late)] == [False, True, False, True, False]
+    assert set(kernels(early, late)) == {"resident_kernel"}
 
 
 @pytest.mark.parametrize("M,N,K,dt", [

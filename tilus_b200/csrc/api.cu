@@ -1093,7 +1093,7 @@ static int run_resident(const void* a, int lda, const void* bq, const void* scal
   p.gshift = gshift_of(group); p.gdiv = group / 128;
   p.S = rs.S; p.T_own = rs.T_own; p.wk_shift = rs.wk_shift;
   p.stages = rs.stages; p.slab_shift = rs.slab_shift; p.grid = rs.grid;
-  p.act = act; p.zero = 0u;
+  p.pdl = pl.pdl; p.act = act; p.zero = 0u;
   const cudaError_t e = resident_launch(var, p, stream_mt(M), rs.n_max, rs.smem, stream);
   if (e != cudaSuccess) { g_last_cuda_error = (int)e; return ST_CUDA; }
   return ST_OK;

@@ -131,6 +131,7 @@ struct ResidentParams {
   int stages;            // ring slots per warp (<= 8)
   int slab_shift;        // log2 of the column tiles whose partial sums have room in shared memory
   int grid;
+  int pdl;               // 1: the launch may start before its predecessor in the stream has ended
   int act;               // activation / scale / output dtype: 0 fp16, 1 bf16
   uint32_t zero;         // 0, which the compiler does not know
 };

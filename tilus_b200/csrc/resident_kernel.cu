@@ -501,13 +501,19 @@ static cudaError_t launch_one(const ResidentParams& p, int smem_bytes, cudaStrea
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)p.S;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  int n = 0;
+  if (p.pdl) {  // (without it the requests ahead of griddepcontrol.wait follow the previous kernel, too)
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (CLUSTER) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = (unsigned)p.S;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = CLUSTER ? 2 : 1;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
