@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
       p.status[2] = blockIdx.x;
       p.status[3] = warp;
     }
-    for (int s = 0; s < NST; ++s) mbar_wait_bounded(bar0 + s * 8, 0);
+    ring_drain(bar0, NST, issued);
   }
   if constexpr (CLUSTER) {
     for (int t = chunk + warp * p.S; t < tiles && ok; t += RES_WARPS * p.S) {

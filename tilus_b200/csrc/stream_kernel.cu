@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1) stream_kernel(const Stre
       p.status[2] = blockIdx.x;
       p.status[3] = warp;
     }
-    for (int s = 0; s < NST; ++s) mbar_wait_bounded(bar0 + s * 8, 0);
+    ring_drain(bar0, NST, issued);
   }
 
   // ---- the CTA's own tiles ----
