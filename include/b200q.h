@@ -300,7 +300,7 @@ int b200q_gemm_swiglu_cast(const void* a, int lda, const void* bq, const void* s
  * B200Q_ERR_DEVICE_TIMEOUT, status[1..3] say which wait gave up (1: 2 = tcgen05 prefill pipeline,
  * 3 = stream kernel's weight ring, 5 = wait for a peer's columns, 6 = tcgen05 small-batch pipeline,
  * 7 / 8 = gather push / collect, 9 = wait for the CTAs that fetch host activations, 10 = exact
- * small-batch kernel's pipeline; 2: CTA; 3: warp or thread).  Clears the header.  A launch that gave up may leave partial sums
+ * small-batch kernel's pipeline, 11 = a wait of the kernel that keeps the activations in registers; 2: CTA; 3: warp or thread).  Clears the header.  A launch that gave up may leave partial sums
  * behind: zero the workspace before it is used again.  workspace == NULL names the built-in
  * scratch of b200q_gemm_static_ws, which this call then puts back to zero itself. */
 int b200q_device_status(void* workspace, int32_t status[4], void* stream);

@@ -84,6 +84,22 @@ def test_rejects_bad_problems(lib):
         == _lib.ST_UNSUPPORTED
 
 
+def test_a_timeout_names_one_kernel():
+    """status[1] of a launch that gave up: no two kernels report the same place, and the header lists each."""
+    csrc = os.path.join(ROOT, "tilus_b200", "csrc")
+    places = {}
+    for name in sorted(os.listdir(csrc)):
+        if name.endswith((".cu", ".cuh")):
+            for code in re.findall(r"status\[1\] = (\d+)", open(os.path.join(csrc, name)).read()):
+                places.setdefault(int(code), set()).add(name)
+    shared = {code: files for code, files in places.items() if len(files) > 1}
+    assert not shared, shared
+    header = open(os.path.join(ROOT, "include", "b200q.h")).read()
+    listed = header[header.index("Reads the device status header"):header.index("int b200q_device_status(")]
+    named = {int(n) for group in re.findall(r"((?:\d+ / )?\d+) = ", listed) for n in group.split(" / ")}
+    assert set(places) <= named, (places, named)
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
 

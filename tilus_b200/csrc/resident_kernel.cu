@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
   if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
     if (lane == 0) {
       atomicExch(p.status, ST_DEVICE_TIMEOUT);
-      p.status[1] = 10;  // where: resident kernel
+      p.status[1] = 11;  // where: resident kernel
       p.status[2] = blockIdx.x;
       p.status[3] = warp;
     }
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
       }
     }
     if (!__all_sync(0xffffffffu, ok ? 1 : 0)) {
-      if (lane == 0) { atomicExch(p.status, ST_DEVICE_TIMEOUT); p.status[1] = 10; p.status[2] = blockIdx.x; p.status[3] = warp; }
+      if (lane == 0) { atomicExch(p.status, ST_DEVICE_TIMEOUT); p.status[1] = 11; p.status[2] = blockIdx.x; p.status[3] = warp; }
       // peers may still send their sums: they have left, or are here as well, when this ends
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
       asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
