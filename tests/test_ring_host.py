@@ -8,9 +8,10 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SOURCE = """
 #include "ring.cuh"
-extern "C" int slot(int item, int slots) { return b200q::ring_slot(item, slots); }
-extern "C" int parity(int item, int slots) { return (int)b200q::ring_parity(item, slots); }
-extern "C" int oldest(int issued, int slots) { return b200q::ring_oldest(issued, slots); }
+extern "C" int last_wait(int slot, int issued, int slots) {  // -1: none
+  const b200q::RingLaps laps = b200q::ring_laps(issued, slots);
+  return b200q::ring_used(laps, slot) ? (int)b200q::ring_parity(laps, slot) : -1;
+}
 """
 
 
@@ -30,10 +31,10 @@ def test_a_wait_passes_when_its_copy_has_landed_and_not_before(ring, slots):
     them landed that the ring allows (an item is asked for when the one `slots` ahead of it has landed)."""
     for issued in range(1, 5 * slots + 2):
         for landed in range(max(0, issued - slots), issued + 1):
-            under_way = [sum(1 for i in range(landed) if i % slots == s) for s in range(slots)]  # phases ended, per slot
-            waits = range(ring.oldest(issued, slots), issued)
-            assert set(range(landed, issued)) <= set(waits)
-            assert sorted(ring.slot(i, slots) for i in waits) == sorted({ring.slot(i, slots) for i in range(issued)})
-            for i in waits:
-                passes = ring.parity(i, slots) != under_way[ring.slot(i, slots)] % 2
-                assert passes == (i < landed), (issued, landed, i)
+            for slot in range(slots):
+                uses = [i for i in range(issued) if i % slots == slot]
+                parity = ring.last_wait(slot, issued, slots)
+                assert (parity < 0) == (not uses)
+                if uses:
+                    under_way = sum(1 for i in uses if i < landed)  # phases of the slot's barrier that have ended
+                    assert (parity != under_way % 2) == (uses[-1] < landed), (issued, landed, slot)

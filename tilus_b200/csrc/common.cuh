@@ -292,8 +292,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
 }
 // Gives the copies that a warp has in flight a bounded chance to land: its CTA must not retire under them.
 __device__ __forceinline__ void ring_drain(uint32_t bar0, int slots, int issued) {
-  for (int i = ring_oldest(issued, slots); i < issued; ++i)
-    mbar_wait_bounded(bar0 + (uint32_t)ring_slot(i, slots) * 8u, ring_parity(i, slots));
+  const RingLaps laps = ring_laps(issued, slots);
+  for (int s = 0; s < slots; ++s)
+    if (ring_used(laps, s)) mbar_wait_bounded(bar0 + (uint32_t)s * 8u, ring_parity(laps, s));
 }
 // One elected lane of a converged warp.  tcgen05.mma takes its descriptors from uniform registers: inside
 // a branch on elect.sync the compiler keeps them there, while inside `if (lane == 0)` it moves every

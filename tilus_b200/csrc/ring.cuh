@@ -5,10 +5,18 @@
 
 namespace b200q {
 
-B200Q_HD constexpr int ring_slot(int item, int slots) { return item % slots; }
-// what a wait for the item's copy names (a phase two uses back has the same parity, but ended before this one began)
-B200Q_HD constexpr uint32_t ring_parity(int item, int slots) { return (uint32_t)(item / slots) & 1u; }
-// the oldest of the `issued` items whose copy may still be on its way: a slot is asked for again when its last copy has landed
-B200Q_HD constexpr int ring_oldest(int issued, int slots) { return issued > slots ? issued - slots : 0; }
+// The uses of a ring behind which `issued` items have been asked for: how many of them belong to the last lap, its parity, and whether
+// there was one before.  (Subtractions: divisions by the run-time number of slots, on a path that only a launch that gives up takes, cost the
+// kernel that keeps the activations in registers up to 2 % of every other launch.)
+struct RingLaps { int last; uint32_t parity; bool earlier; };
+B200Q_HD RingLaps ring_laps(int issued, int slots) {
+  RingLaps r = {issued, 0u, issued > slots};
+  while (r.last > slots) { r.last -= slots; r.parity ^= 1u; }
+  return r;
+}
+// whether a slot has been asked for, and the parity that a wait for its last copy names (the use two laps back has the same
+// parity, but has ended)
+B200Q_HD bool ring_used(const RingLaps& r, int slot) { return slot < r.last || r.earlier; }
+B200Q_HD uint32_t ring_parity(const RingLaps& r, int slot) { return slot < r.last ? r.parity : r.parity ^ 1u; }
 
 }  // namespace b200q
