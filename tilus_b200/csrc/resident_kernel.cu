@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
   int next_read = wi;
   auto finish = [&](int ti) {  // adds up the warps' sums of tile ti of this set
     const uint32_t bar = full0 + (uint32_t)(ti & (D - 1)) * 8u;
-    if (!mbar_wait_bounded(bar, (uint32_t)(ti >> p.slab_shift) & 1u)) { ok = false; return; }
+    // (a warp gives up as a whole: lanes that left alone would miss the others at the next vote)
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar, (uint32_t)(ti >> p.slab_shift) & 1u) ? 1 : 0)) { ok = false; return; }
     const float4* s = slab + (size_t)(ti & (D - 1)) * WK * MT * 32 + lane;
     const int tile = set + ti * WT;
     float4 v[MT];
@@ -439,7 +440,8 @@ __global__ void __launch_bounds__(RES_WARPS * 32, 1) resident_kernel(const Resid
     }
     if (!ok) break;
     const int sl = ti & (D - 1);
-    if (ti >= D && !mbar_wait_bounded(empty0 + (uint32_t)sl * 8u, (uint32_t)((ti >> p.slab_shift) - 1) & 1u)) { ok = false; break; }
+    if (ti >= D &&
+        !__all_sync(0xffffffffu, mbar_wait_bounded(empty0 + (uint32_t)sl * 8u, (uint32_t)((ti >> p.slab_shift) - 1) & 1u) ? 1 : 0)) { ok = false; break; }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
     {
