@@ -361,3 +361,16 @@ def test_narrow_layers_with_more_activations_than_their_ctas_fetch(m, n, k, dt):
             c.run()
     for c in calls:
         c.check()
+
+
+@pytest.mark.parametrize("m,n,k,dt", [(1, 16, 20480, D.uint2b), (4, 48, 14336, D.uint4b), (6, 64, 12288, D.int8), (2, 16, 6144, D.uint2b)], ids=str)
+def test_rows_that_replace_others_at_the_same_address(m, n, k, dt):
+    """Long chains of short calls, each on rows that a small kernel has just written over those of the call before: many launches are
+    on the SMs by then, and none may see a line of the rows that were there."""
+    calls = _HostCalls(m, n, k, dt, 2, 24)
+    want = [x.cuda().float() @ ops.dequantize(*calls.weights[i % 2], dt, 128, calls.zp).float() for i, x in enumerate(calls.xs)]
+    for _ in range(12):
+        for _ in range(4):
+            calls.run()
+        torch.cuda.synchronize()
+        assert [i for i, out in enumerate(calls.outs) if not _close(out, want[i])] == []

@@ -70,10 +70,11 @@ __global__ void __launch_bounds__(256) cast_kernel(const CastParams p) {
     for (int s = 0; s < 4; ++s) {
       if (s < steps) {
         float l[8];
-        unpack8<ACT>(__ldg(reinterpret_cast<const uint4*>(row + s * 128)), l);
+        // (plain loads, not __ldg: the GEMM wrote these while this launch was on its SM already)
+        unpack8<ACT>(*reinterpret_cast<const uint4*>(row + s * 128), l);
         if constexpr (SWIGLU) {
           float r[8];
-          unpack8<ACT>(__ldg(reinterpret_cast<const uint4*>(row + p.H + s * 128)), r);
+          unpack8<ACT>(*reinterpret_cast<const uint4*>(row + p.H + s * 128), r);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             float a = l[i], b = r[i];

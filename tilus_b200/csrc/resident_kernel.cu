@@ -107,11 +107,12 @@ __device__ __forceinline__ uint32_t res_bf16x2_to_f16x2(uint32_t w) {
   return h;
 }
 // 16 bytes of an activation row, or zeros where there is no row.  In program order, so that all of a warp's loads are in flight at once:
-// left to the compiler, some waited for the first conversions (8 x 6144 x 4096 5.55 us, 5.49 so).
+// left to the compiler, some waited for the first conversions (8 x 6144 x 4096 5.55 us, 5.49 so).  Not ld.global.nc: the rows are
+// written while this launch is on its SM already, and a non-coherent load may return a line that L1 has had since before.
 __device__ __forceinline__ uint4 res_load_row(const uint4* p, bool valid) {
   uint4 v;
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
-               "@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               "@p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
                : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w) : "l"(p), "r"((uint32_t)valid));
   return v;
 }

@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(STREAM_WARPS * 32, 1) stream_kernel(const Stre
             thi[GATHER == 2 ? u : 0] = ld_tagged2(src + 2);
           } else {
             const uint4* src = reinterpret_cast<const uint4*>(a_base + (size_t)mq[u] * a_ld + (size_t)kb_base * 512 + kq[u]);
-            vq[u] = GATHER ? __ldcg(src) : __ldg(src);  // gathered rows were written through L2 by other GPUs
+            vq[u] = GATHER ? __ldcg(src) : *src;  // gathered rows were written through L2 by other GPUs
           }
         }
       }
