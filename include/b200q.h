@@ -102,7 +102,8 @@ int b200q_plan_for(int M, int N, int K, int wtype, int zero_point, int group, in
 size_t b200q_workspace_bytes(int M, int N, int K, int wtype, int zero_point, int group);
 
 /* C = A x dequant(Bq).  a: [M, K] (row stride lda elements), bq: b200-packed weights,
- * scales: [K/group, N], c: [M, N] (row stride ldc), all three of dtype act_dtype.  Replaces
+ * scales: [K/group, N], c: [M, N] (row stride ldc), all three of dtype act_dtype.  lda is a multiple of 8, and so is ldc
+ * except for up to 16 rows with K a multiple of 512 and scale groups of 128 and more.  Replaces
  * tilus_launch for QuantizedMatmul (examples/quantization/matmul_a16wx.py:231-405).  The tcgen05
  * kernels multiply bf16 activations as they are.  The mma.sync kernels (b200q_plan_for: kernel 2 with
  * tile_m 0; bf16 batches of up to 8 rows at most shapes, and up to 16 rows of the host-buffer and gather

@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from tilus_b200 import _lib
 from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 from tilus_b200.variants import supported_weight_dtypes
@@ -137,6 +138,28 @@ def test_edits_of_other_fields_leave_the_kernel():
     got = ops.quantized_matmul(rows, bq, sc, D.uint4b, 128, zp, plan_override=pl)
     want = rows.float() @ ops.dequantize(bq, sc, D.uint4b, 128, zp).float()
     assert float((got.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("M,K,ok", [(1, 1024, True), (8, 1024, True), (16, 1024, True), (1, 1152, False), (5, 1152, False), (16, 1152, False),
+                                    (1, 4224, False), (8, 8320, False)])
+@pytest.mark.parametrize("N", [272, 4112, 16384])
+def test_rows_of_any_distance_do_not_depend_on_the_route(M, N, K, ok):
+    """K in whole 512-row blocks takes outputs at any row stride, and asks for the stream kernel's scratch then; other K ask for multiples of
+    eight elements, whichever kernel a width goes to."""
+    a, bq, sc, zp, ref = _problem(M, N, K, D.uint4b, 128)
+    wide = torch.zeros(M, N + 3, dtype=torch.float16, device=a.device)
+    run = lambda ws=None, out=wide[:, :N]: ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, out=out, workspace=ws)  # noqa: E731
+    if ok:
+        run()
+        assert _close(wide[:, :N], ref)
+        small = torch.zeros(256 + 4 * (N // 16 + 64) + 256, dtype=torch.uint8, device=a.device)
+        with pytest.raises(_lib.B200QError):
+            run(small)
+    else:
+        with pytest.raises(_lib.B200QError):
+            run()
+        assert int(wide.count_nonzero()) == 0
+        run(out=torch.empty(M, N, dtype=torch.float16, device=a.device))
 
 
 @pytest.mark.parametrize("M,N,K", [(8, 4096, 4096), (1, 8192, 8192), (16, 4096, 2048)])

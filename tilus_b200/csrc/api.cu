@@ -1078,8 +1078,11 @@ static int run_stream(const void* a, int lda, const void* bq, const void* scales
 static int run_resident(const void* a, int lda, const void* bq, const void* scales, void* c, int ldc, int M, int N, int K,
                         int var, int group, int act, void* workspace, size_t ws_bytes, cudaStream_t stream, const b200q_plan_t& pl,
                         const ResidentSplit& rs) {
-  // (the workspace that the plan's other form asks for, so that the same calls are refused; only the status word is used)
-  const size_t need = pl.tile_m == 0 ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
+  // (The workspace and the rows of C that the plan's other form asks for, so that the same calls are refused whichever shapes come here; only the
+  // status word is used.  The exact kernel's calls on rows at any distance are the stream kernel's, which K in whole 512-row blocks has.)
+  const bool any_rows = (ldc % 8) != 0;
+  if (pl.tile_m != 0 && any_rows && !stream_takes(K, group)) return ST_INVALID_ARG;
+  const size_t need = pl.tile_m == 0 || any_rows ? stream_workspace_bytes(N) : WS_HEADER_BYTES + ws_counter_bytes(N);
   if (!workspace || ws_bytes < need || ((uintptr_t)workspace & 255)) return ST_WORKSPACE;
   if (((uintptr_t)scales) & 15) return ST_INVALID_ARG;
   ResidentParams p;
