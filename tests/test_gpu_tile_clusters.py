@@ -72,3 +72,13 @@ def test_whole_tiles_and_sets(M, N, K, dt, group, act):
     for c in outs[1:]:
         assert torch.equal(c, outs[0])
     assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("M,N,K,dt,group,act,ctas,cluster", [
+    (12, 6144, 4096, D.float8_e5m2, 64, torch.bfloat16, 96, 2), (32, 6144, 4096, D.int8, 128, torch.float16, 96, 2),
+    (24, 8192, 4096, D.float6_e3m2, 128, torch.float16, 128, 2), (32, 20480, 512, D.int8, 128, torch.float16, 80, 1),
+    (24, 11008, 4096, D.int8, 128, torch.float16, 148, 1), (24, 14336, 8192, D.int3b, 128, torch.float16, 148, 1)], ids=str)
+def test_splits_of_types_with_an_sm_to_themselves(M, N, K, dt, group, act, ctas, cluster):
+    """Up to 32 rows: the form that was the fastest of those forced at these shapes."""
+    pl = ops.plan(M, N, K, dt, 0, group, act_dtype=act)
+    assert (pl["ctas_per_split"], pl["cluster"]) == (ctas, cluster)

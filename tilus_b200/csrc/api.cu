@@ -431,7 +431,11 @@ static bool batch_exact(int M, int group) { return M <= 16 && group % 128 == 0; 
 //  - whole tiles, as many per CTA as one round takes.
 // The times are fits to chains of launches on B200 (4-bit weights in fp16, us; 1024 x 4096 .. 4096 x 14336, 16 .. 128 rows, each
 // form forced; within 15 % there) and serve every width and both activation types: for 100 x 11008 x 4224, 6 bits in
-// bf16, they say 16.1 where a call takes 20.2.  Fewer CTAs start and end cheaper because the next launch finds SMs free (17 x 2048 x
+// bf16, they say 16.1 where a call takes 20.2.  Up to 32 rows of the types that have an SM to themselves (batch_sets) each group of equal runs costs
+// more, and of whole tiles on more than half of the SMs: fits to 840 calls of 3, 5, 6 and 8 bits, float6 and float8, 1024 .. 8192 rows of K, 2560 ..
+// 18432 columns at 12, 24 and 32 rows, each form forced; the choice is behind the best form by 0.4 % on average, with the 4-bit costs 1.2 (12 x
+// 6144 x 4096, float8 in bf16, groups of 64, 11.2 us on equal runs, 9.5 with two CTAs per tile), at most by 24 % (24 x 11008 x 2048 in 8 bits, 10.0 on equal
+// runs, whole tiles 8.3), and by up to 5 % behind the form with those costs at 3 of the 840.  Fewer CTAs start and end cheaper because the next launch finds SMs free (17 x 2048 x
 // 4096, 4 / 6 CTAs per tile, that is 64 / 96 CTAs, 4.5 / 5.7 us, equal runs 6.0; 64 x 4096 x 4096, 2 / 3 / 4 per tile 8.5 / 8.6 / 8.6).
 static int max_clusters(int c) {
   static int cache[16][9];
@@ -460,7 +464,8 @@ static void batch_split(int M, int var, int group, int n_tiles, int G, const Dev
   if (grid > di.sm_count) grid = di.sm_count;
   const bool exact = batch_exact(M, group), shares = !exact && batch_shares_sm(batch_rows(M), var);
   const double groups = (double)n_tiles * G / grid;
-  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + 0.27 * groups + (!exact && groups > 24 ? 0.12 * (groups - 24) : 0.0);
+  const bool alone = !exact && !shares && M <= 32;
+  double best = 6.0 + (M > 24 ? 0.085 * (M - 24) : 0.0) + (alone ? 0.42 : 0.27) * groups + (!exact && groups > 24 ? 0.12 * (groups - 24) : 0.0);
   *ctas = (int)grid;
   *cluster = 1;
   // Kernels whose CTAs share SMs have no clusters: CTAs of cluster launches must not meet two to an SM while others idle, and the
@@ -479,7 +484,7 @@ static void batch_split(int M, int var, int group, int n_tiles, int G, const Dev
     } else {
       const bool overlap = 2 * n <= di.sm_count;  // the next launch finds SMs free
       t = 0.03 * M + (c > 6 ? 0.8 : 0.0);
-      if (c == 1) t += (overlap ? 2.0 : 3.5) + 0.28 * each + (each > 32 ? 0.08 * (each - 32) : 0.0);
+      if (c == 1) t += (overlap ? 2.0 : 3.5 + (alone ? 0.09 * each : 0.0)) + 0.28 * each + (each > 32 ? 0.08 * (each - 32) : 0.0);
       else t += (overlap ? 2.0 + 0.29 * each : 4.0 + 0.33 * each) + (M > 64 ? 0.05 * (M - 64) / c : 0.0);
     }
     if (t < best) {
