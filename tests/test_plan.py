@@ -110,7 +110,8 @@ def test_k_chunks_of_two_to_eight_rows(m, n, k, w, splits):
     (8, 16384, 14336, "float6_e3m2", 0, 0), (8, 1024, 4224, "int6b", 0, 1), (8, 16384, 14336, "uint4b", 0, 2),
     (9, 11008, 4096, "uint4b", 0, 1), (9, 16384, 4096, "uint4b", 0, 1), (9, 18432, 4096, "uint4b", 0, 0), (9, 12288, 4096, "float6_e3m2", 0, 0), (13, 4096, 4096, "uint4b", 0, 1), (13, 6144, 4096, "uint4b", 0, 0),
     (15, 4096, 4096, "uint4b", 0, 0), (12, 4096, 4096, "int8", 0, 1), (13, 4096, 4096, "int8", 0, 0), (16, 4096, 2048, "int8", 0, 1), (16, 4096, 4096, "float6_e3m2", 0, 1),
-    (16, 2048, 4096, "uint4b", 0, 0), (16, 8192, 1024, "uint4b", 0, 0), (16, 4096, 8192, "uint4b", 0, 0), (17, 4096, 4096, "uint4b", 0, 0),
+    (16, 2048, 4096, "uint4b", 0, 0), (16, 8192, 1024, "uint4b", 0, 0), (9, 5120, 1024, "uint4b", 0, 1), (9, 6144, 1024, "uint4b", 0, 0), (16, 5120, 1024, "uint4b", 0, 0), (16, 6144, 1536, "int3b", 0, 1),
+    (13, 6144, 1920, "int8", 0, 1), (9, 8192, 1920, "uint4b", 0, 0), (9, 8192, 2176, "uint4b", 0, 1), (13, 6144, 2176, "int3b", 0, 0), (13, 2560, 2560, "int3b", 0, 0), (16, 4096, 8192, "uint4b", 0, 0), (17, 4096, 4096, "uint4b", 0, 0),
     (8, 4096, 4096, "uint4b", 1, 1), (9, 4096, 4096, "uint4b", 1, 0), (8, 4096, 4224, "uint4b", 1, 0)])
 def test_calls_that_keep_their_activations_in_registers(m, n, k, w, act, resident):
     """Both sides of the lines of the rule, at shapes that were timed.  bfloat16 only where the stream kernel had it: the tcgen05

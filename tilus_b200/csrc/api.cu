@@ -698,8 +698,14 @@ static bool resident_split(int M, int N, int K, int bits, int S, const DeviceInf
 //    1.17); beyond, 0.87 .. 0.95 in 8 bits, 0.72 .. 0.98 in 4 bits (28672 x 14336 1.0), 0.88 .. 1.0 in fewer up to 4096 columns (3 bits,
 //    28672 x 14336 1.04, 2 bits 1.08), 1.0 .. 1.1 in 5 to 7 bits;
 //  - 9 to 16 rows (fp16 only: the exact kernel takes bfloat16 as it is), whose second set of sums makes the loop 1.5 times longer: up to
-//    4096 rows of K in the ranges below 0.63 .. 1.0; beyond 1.0 .. 1.3 (9 and 12 rows, 12288, 14336 and 16384 columns: 3 bits 0.85 .. 0.94, 4
-//    and 8 bits 0.87 .. 0.98, float6 0.93 .. 1.02; 9 x 28672 x 4096 1.02; blocks of linears of those widths 0.90 .. 0.99).  Among layers that stay with the exact kernel, whose launches
+//    4096 rows of K in the ranges below 0.55 .. 1.0; beyond 1.0 .. 1.3 (9 and 12 rows, 12288, 14336 and 16384 columns: 3 bits 0.85 .. 0.94, 4
+//    and 8 bits 0.87 .. 0.98, float6 0.93 .. 1.02; 9 x 28672 x 4096 1.02; blocks of linears of those widths 0.90 .. 0.99).  The widest layer goes by the
+//    depth, since the exact kernel is ahead where a short range of K per CTA fills its SMs: 2, 3, 4 and 8 bits and float6 at 9 to 16 rows, 1024 rows
+//    of K 5120 columns 0.69 .. 0.88, 6144 0.98 .. 1.09 (blocks with 4608 x 1024, qkv, 0.93 .. 0.99 to 12 rows, 1.01 .. 1.05 at 16); 1536 to 2048 rows 6144 columns
+//    0.79 .. 0.98, 8192 0.89 .. 1.20 (blocks with 4608 x 1536, 5376 x 1792 or 5760 x 1920 0.86 .. 0.99); 2176 rows 8192 and 11008 columns at 9 and 12 rows
+//    0.96 .. 1.18, but blocks of hidden size 2176 whose gate_up goes to the exact kernel 1.03 .. 1.10; 2560 rows 0.81 .. 0.96.  Beyond 2048 rows, 13 rows and
+//    more: below 3072 columns 0.67 .. 1.03 in chains, blocks with such a layer from 0.93 (2560 x 2560 besides 3840 x 2560) to 1.10 (2176 x 2176
+//    besides 6528 x 2176): left to the exact kernel.  Among layers that stay with the exact kernel, whose launches
 //    leave SMs to their successors, a launch on all SMs costs those up to 2 us: with 4096 x 4096 here a Llama-3-8B block takes, us, at 9
 //    / 13 / 16 rows 47.2 / 49.3 / 51.1 in 4 bits (50.1 / 51.1 / 50.3 without), 54.0 / 54.8 / 57.7 in 8 bits (54.5 / 54.9 / 55.7), 58.1 /
 //    60.2 / 61.2 in 3 bits (62.5 / 63.1 / 62.2), 59.8 / 61.6 / 63.4 in float6 (62.9 / 63.5 / 62.8): 8 bits up to 12 rows, 4 bits up to 14.
@@ -711,8 +717,8 @@ static int resident_cluster(int M, int N, int K, int var, int group, int act, bo
   const int G = K / 128, bits = var_bits(var);
   int S;
   if (M > 8) {
-    const int wide = M > 12 ? 4096 : bits >= 5 && bits <= 7 ? 11008 : 16384;
-    if (G > 32 || N > (G > 16 ? wide : G == 16 ? 6144 : 4096) || (G > 16 && N < 3072 && M > 12)) return 0;
+    const int widest = G > 16 ? (M > 12 ? 4096 : bits >= 5 && bits <= 7 ? 11008 : 16384) : G >= 12 ? 6144 : G >= 8 && M <= 12 ? 5120 : 4096;
+    if (G > 32 || N > widest || (G > 16 && N < 3072 && M > 12)) return 0;
     if (G > 16 && ((bits == 8 && M > 12) || (bits == 4 && M > 14))) return 0;
     S = 1;
   } else {
