@@ -6,6 +6,8 @@ from tilus_b200 import _lib, packing, synth
 from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 
+from .launches import kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -29,10 +31,12 @@ def test_bf16_runs_the_form_its_plan_names(M):
     exact_plan = ops.plan(16, N, K, dt, 0, group)
     assert stream_plan["tile_m"] == 0 and exact_plan["tile_m"] == 16
     fields = ("kernel", "splits", "cluster", "ctas_per_split", "tile_m", "stages")
-    force = lambda pl: ops.quantized_matmul(a, bq, sc, dt, group, plan_override={f: pl[f] for f in fields})  # noqa: E731
-    assert close(force(exact_plan), exact)
-    assert close(force(stream_plan), saturated)
+    force = lambda pl, res=0: ops.quantized_matmul(a, bq, sc, dt, group, plan_override={**{f: pl[f] for f in fields}, "resident": res})  # noqa: E731
+    assert close(force(exact_plan), exact) and close(force(exact_plan, 1), exact)
+    assert close(force(stream_plan), saturated) and close(force(stream_plan, 1), saturated)
     assert close(ops.quantized_matmul(a, bq, sc, dt, group), saturated)
+    assert kernels(lambda: force(exact_plan), lambda: force(exact_plan, 1), lambda: force(stream_plan), lambda: force(stream_plan, 1)) == [
+        "exact_kernel", "exact_kernel", "stream_kernel", "resident_kernel"]
 
 
 @pytest.mark.parametrize("M,N,K", [(8, 129280, 512), (16, 129280, 512), (300, 9472, 1024), (326, 6000, 2048)])

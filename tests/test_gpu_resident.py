@@ -33,10 +33,11 @@ def _close(c, ref):
     return bool(((c.double() - ref).abs() <= eps * ref.abs() + 2e-5 * ref.abs().max()).all())
 
 
-def _run(a, bq, sc, dt, zp, group, S, ws, out=None):
-    N, K = sc.shape[1], a.shape[1]
-    assert ops.plan(a.shape[0], N, K, dt, zp, group, act_dtype=a.dtype)["kernel"] in (2, 3)
-    return ops.quantized_matmul(a, bq, sc, dt, group, zp, workspace=ws, plan_override=dict(resident=S), out=out)
+def _run(a, bq, sc, dt, zp, group, S, ws=None, out=None):
+    call = lambda: ops.quantized_matmul(a, bq, sc, dt, group, zp, workspace=ws, plan_override=dict(resident=S), out=out)  # noqa: E731
+    c = call()
+    assert (kernels(call) == ["resident_kernel"]) is (S > 0)
+    return c
 
 
 def _check(M, N, K, dt, group, S, act=torch.float16, mean=0.0):
@@ -76,7 +77,7 @@ def test_splits(M, N, K, group, S):
     _check(M, N, K, D.uint4b, group, S)
 
 
-@pytest.mark.parametrize("M,K,S", [(1, 4096, 1), (8, 2048, 1), (8, 8192, 2), (5, 7680, 1)])
+@pytest.mark.parametrize("M,K,S", [(1, 4096, 1), (8, 2048, 1), (8, 8192, 2), (5, 6144, 1)])
 def test_bfloat16(M, K, S):
     _check(M, 1040, K, D.int4b, 128, S, act=torch.bfloat16)
 
@@ -85,7 +86,7 @@ def test_bfloat16_out_of_range():
     """Magnitudes that fp16 does not have saturate (infinities too); NaN stays NaN."""
     a, bq, sc, zp, _ = _problem(4, 64, 1024, D.int4b, 128, torch.bfloat16)
     a[0, 5], a[1, 7], a[2, 9] = 1e6, float("inf"), float("nan")
-    c = ops.quantized_matmul(a, bq, sc, D.int4b, 128, zp, plan_override=dict(resident=1))
+    c = _run(a, bq, sc, D.int4b, zp, 128, 1)
     b = a.clone()
     b[0, 5] = b[1, 7] = 65504.0
     ref = b.double() @ ops.dequantize(bq, sc, D.int4b, 128, zp).double()
@@ -101,7 +102,7 @@ def test_activations_of_any_magnitude_are_multiplied_as_they_are(scale):
     sc = sc.float().div(scale if scale < 1 else 1).clamp(max=60000).half()
     values = ops.dequantize(bq, torch.ones(1, 272, dtype=torch.float16, device=a.device), D.uint4b, 2048, zp).double()
     ref = a.double() @ (values * sc.double().repeat_interleave(128, 0))
-    assert _close(ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=dict(resident=1)), ref)
+    assert _close(_run(a, bq, sc, D.uint4b, zp, 128, 1), ref)
 
 
 @pytest.mark.parametrize("M,dt,mean", [
@@ -122,7 +123,7 @@ def test_results_as_near_as_those_of_the_kernel_beside_it(M, dt, mean):
 def test_outputs_inside_a_wider_tensor(M, gap):
     a, bq, sc, zp, ref = _problem(M, 272, 1024, D.uint4b, 128)
     wide = torch.full((M, 272 + gap), 7.0, dtype=torch.float16, device=a.device)
-    ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, out=wide[:, :272], plan_override=dict(resident=1))
+    _run(a, bq, sc, D.uint4b, zp, 128, 1, out=wide[:, :272])
     assert _close(wide[:, :272], ref) and bool((wide[:, 272:] == 7.0).all())
 
 
@@ -130,14 +131,20 @@ def test_edits_of_other_fields_leave_the_kernel():
     a, bq, sc, zp, ref = _problem(8, 4096, 4096, D.uint4b, 128)
     pl = ops.plan(8, 4096, 4096, D.uint4b, zp, 128)
     assert pl["resident"] == 1
-    c = ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp)
-    assert torch.equal(ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=pl), c)
-    for edit in (dict(resident=0), dict(splits=2), dict(stages=2, ctas_per_split=100), dict(kernel=3, tile_m=16, splits=1, ctas_per_split=90)):
-        assert float((ops.quantized_matmul(a, bq, sc, D.uint4b, 128, zp, plan_override=edit).double() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    run = lambda plan, x=a: ops.quantized_matmul(x, bq, sc, D.uint4b, 128, zp, plan_override=plan)  # noqa: E731
+    c = run(None)
+    assert torch.equal(run(pl), c)
+    edits = {"stream_kernel": [dict(resident=0), dict(splits=2), dict(stages=pl["stages"] - 1), dict(ctas_per_split=100), dict(kernel=2, stages=2, ctas_per_split=100)],
+             "exact_kernel": [dict(kernel=3, tile_m=16, splits=1, ctas_per_split=90), dict(tile_m=16, splits=1, ctas_per_split=90)]}
+    for name, plans in edits.items():
+        for plan in plans:
+            assert float((run(plan).double() - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+            assert kernels(lambda: run(plan)) == [name], plan
     rows = torch.randn(20, 4096, device=a.device).half()  # a plan put on more rows than the kernel takes
-    got = ops.quantized_matmul(rows, bq, sc, D.uint4b, 128, zp, plan_override=pl)
+    got = run(pl, rows)
     want = rows.float() @ ops.dequantize(bq, sc, D.uint4b, 128, zp).float()
     assert float((got.float() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+    assert kernels(lambda: run(None), lambda: run(pl), lambda: run(pl, rows)) == ["resident_kernel", "resident_kernel", "stream_kernel", "stream_kernel"]
 
 
 @pytest.mark.parametrize("M,K,ok", [(1, 1024, True), (8, 1024, True), (16, 1024, True), (1, 1152, False), (5, 1152, False), (16, 1152, False),

@@ -5,6 +5,7 @@ import torch
 from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 
+from .launches import kernels
 from .test_gpu_parity import _forced
 
 pytestmark = pytest.mark.gpu
@@ -49,7 +50,7 @@ def test_runs_of_one_to_six_column_tiles(M, group, tiles, ctas, K):
         pytest.skip("group does not divide K")
     N, dt = tiles * 128 - 112, D.int4b
     exact = M <= 16 and group % 128 == 0
-    plan = dict(kernel=2 if exact else 3, tile_m=16 if exact else 128, splits=1, cluster=1, ctas_per_split=ctas)
+    plan = dict(kernel=2 if exact else 3, tile_m=16 if exact else 128, splits=1, cluster=1, ctas_per_split=ctas, resident=0)
     _forced(M, N, K, dt, 0, plan, seed=M + tiles, group=group)
 
 
@@ -66,6 +67,9 @@ def test_wide_layers_repeat_their_results_bit_for_bit(M, dt, group, N, K):
     x = torch.randn(M, K, device=dev, generator=gen).half()
     zp = 8 if dt.kind == D.KIND_UINT else 0
     assert ops.plan(M, N, K, dt, zp, group)["tile_m"] == (M + 15) // 16 * 16
-    outs = [ops.quantized_matmul(x, bq, scales, dt, group, zp) for _ in range(12)]
-    for c in outs[1:]:
-        assert torch.equal(c, outs[0])
+    for plan in (None, dict(resident=0)):
+        outs = [ops.quantized_matmul(x, bq, scales, dt, group, zp, plan_override=plan) for _ in range(12)]
+        for c in outs[1:]:
+            assert torch.equal(c, outs[0])
+    call = lambda: ops.quantized_matmul(x, bq, scales, dt, group, zp, plan_override=plan)  # noqa: E731
+    assert kernels(call) == ["exact_kernel"] if M <= 16 else kernels(call)[0] in ("batch_kernel", "tile_run_kernel")

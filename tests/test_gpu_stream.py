@@ -5,6 +5,8 @@ import torch
 from tilus_b200 import dtypes as D
 from tilus_b200 import ops
 
+from .launches import kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -28,8 +30,10 @@ def _close(c, ref):
     return float((c.float() - ref).abs().max()) <= (2e-3 if c.dtype == torch.float16 else 4e-3) * float(ref.abs().max())
 
 
-def _is_stream(a, N, dt, zp, group=128):
-    return ops.plan(a.shape[0], N, a.shape[1], dt, zp, group, act_dtype=a.dtype)["tile_m"] == 0
+def _run(a, bq, sc, dt, zp, ws=None):
+    """The call on the decode kernel, as host-buffer and gather calls have it; others of most shapes go to the kernel that keeps the
+    activations in registers."""
+    return ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws, plan_override=dict(resident=0))
 
 
 @pytest.mark.parametrize("dt", [D.uint8, D.int8, D.uint7b, D.uint6b, D.int5b, D.uint4b, D.int3b, D.uint2b, D.uint1b, D.float6_e3m2],
@@ -40,10 +44,10 @@ def test_repeated_calls_with_the_weights_in_l2(dt, M):
     types used to be read behind the refill where registers let the compiler delay their second loads)."""
     N, K = 2048, 8192
     a, bq, sc, zp, ref = _problem(M, N, K, dt)
-    assert _is_stream(a, N, dt, zp)
-    outs = [ops.quantized_matmul(a, bq, sc, dt, 128, zp) for _ in range(40)]
+    outs = [_run(a, bq, sc, dt, zp) for _ in range(40)]
     for c in outs:
         assert _close(c, ref)
+    assert kernels(lambda: _run(a, bq, sc, dt, zp)) == ["stream_kernel"]
 
 
 @pytest.mark.parametrize("M,N,K,dt", [
@@ -65,12 +69,12 @@ def test_repeated_calls_with_the_weights_in_l2(dt, M):
     (7, 28672, 2048, D.int8)], ids=str)
 def test_splits_of_the_column_tiles(M, N, K, dt):
     a, bq, sc, zp, ref = _problem(M, N, K, dt, seed=N)
-    assert _is_stream(a, N, dt, zp)
     ws = torch.zeros(max(ops.workspace_bytes(M, N, K, dt, zp, 128), 1 << 20), dtype=torch.uint8, device=a.device)
     for _ in range(2):
-        c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws)
+        c = _run(a, bq, sc, dt, zp, ws)
         assert _close(c, ref)
     assert int(ws.count_nonzero()) == 0
+    assert kernels(lambda: _run(a, bq, sc, dt, zp, ws)) == ["stream_kernel"]
 
 
 @pytest.mark.parametrize("M,N,K,dt,stages", [(1, 8192, 8192, D.uint4b, 6), (1, 8192, 8192, D.uint4b, 8), (8, 4096, 4096, D.int8, 8),
@@ -81,6 +85,7 @@ def test_plans_edited_to_deeper_rings(M, N, K, dt, stages):
     pl = ops.plan(min(M, 4), N, K, dt, zp, 128)
     assert pl["tile_m"] == 0 and pl["stages"] < stages
     ws = torch.zeros(ops.workspace_bytes(16, N, K, dt, zp, 128), dtype=torch.uint8, device=a.device)
-    c = ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws, plan_override={**pl, "stages": stages})
-    assert _close(c, ref)
+    call = lambda: ops.quantized_matmul(a, bq, sc, dt, 128, zp, workspace=ws, plan_override={**pl, "stages": stages})  # noqa: E731
+    assert _close(call(), ref)
+    assert set(kernels(call)) == {"stream_kernel"}
     assert int(ws.count_nonzero()) == 0

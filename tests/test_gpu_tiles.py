@@ -38,6 +38,7 @@ def test_exact_small_batch_kernel(M, N, K, group, w, zp):
     pl = ops.plan(16, N, K, weight_dtype(w), zp, group)
     assert pl["tile_m"] == 16
     plan = {f: pl[f] for f in ("kernel", "splits", "cluster", "ctas_per_split", "tile_m", "stages")}
+    plan["resident"] = 0  # (nor to the one that keeps the activations in registers)
     _forced(M, N, K, weight_dtype(w), zp, plan, seed=M + N, group=group)
 
 
@@ -46,7 +47,8 @@ def test_few_rows_whose_stream_plan_cuts_k(M):
     """448 column tiles have no divisor near two CTAs per SM: the exact kernel takes them from two rows on."""
     dt = weight_dtype("uint4b")
     assert ops.plan(1, 7168, 2048, dt, 8, 128)["tile_m"] == 0 and ops.plan(M, 7168, 2048, dt, 8, 128)["tile_m"] == 16
-    _forced(M, 7168, 2048, dt, 8, dict(), seed=M)
+    for plan in (dict(), dict(resident=0)):  # the kernel that keeps the activations in registers takes fp16 there
+        _forced(M, 7168, 2048, dt, 8, plan, seed=M)
 
 
 @pytest.mark.parametrize("w,zp", [("uint8", 128), ("int8", 0), ("int6b", 0), ("uint4b", 8), ("uint1b", 1)])
@@ -66,7 +68,7 @@ def test_exact_small_batch_kernel_keeps_the_bits_of_its_sums(w, zp):
     codes = torch.randint(0, 1 << dt.nbits, (k, n), device=dev, generator=gen, dtype=torch.int32).to(torch.uint8)
     a = (torch.randn(m, k, device=dev, generator=gen) + 3.0).half()
     sc = (torch.rand(k // group, n, device=dev, generator=gen) * 0.01 + 0.002).half()
-    plan = dict(kernel=2, tile_m=16, splits=1, cluster=1, ctas_per_split=128)
+    plan = dict(kernel=2, tile_m=16, splits=1, cluster=1, ctas_per_split=128, resident=0)
     got = ops.quantized_matmul(a, packing.interleave(codes, dt).to(dev), sc, dt, group, zp, plan_override=plan)
     value = torch.from_numpy(qo.decode_table(dt)).to(dev)[codes.long()] - zp
     ref = a.double() @ (value * sc.double().repeat_interleave(group, 0))
