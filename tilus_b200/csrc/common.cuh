@@ -114,7 +114,7 @@ struct StreamParams {
 
 // ---- decode kernel with the activations in registers (up to 16 rows) ----------------------------------
 constexpr int RES_WARPS = 16;
-constexpr int RES_HEADER = 1024 + 384;  // bytes of barriers in front of the rings: 8 slots per warp; slabs of up to four sets; the cluster's
+constexpr int RES_HEADER = 1024 + 384;  // bytes of barriers in front of the rings: 8 slots per warp; slabs of up to four sets; a cluster's sums
 // 128-row groups per ring slot: at most 2 KB
 __host__ __device__ constexpr int res_gi(int bits, int ng) { return ng >= 4 && bits <= 2 ? 4 : bits <= 4 ? 2 : 1; }
 struct ResidentParams {

@@ -1,5 +1,6 @@
 // Batches of up to 16 rows on tcgen05: C[M, N] = A[M, K] x dequant(Bq[K, N]) with exact weights.
-// Serves 9 to 16 rows and those of 5 to 8 that resident_kernel.cu does not take (api.cu, resident_cluster).
+// Serves 5 to 16 rows, and fewer where K is not in whole 512-row blocks or stream_outrun says so, as far as resident_kernel.cu does not
+// take them (api.cu, resident_cluster): bfloat16 wherever the stream kernel has not, fp16 mostly wide or deep layers of 9 to 16 rows.
 //
 // Same product and work split as batch_kernel.cu (weights of 128 columns in tensor memory, equal runs of 128-row
 // groups per CTA), but the scale is not applied to the weights.  Every group's product is a sum of its own,

@@ -29,8 +29,8 @@
 //
 // Sums.  The 16 warps' parts of a column tile meet in shared memory (four tiles of room, an mbarrier that counts the warps and one
 // that frees the room), and one of the warps, in turn, adds them up in order and writes C: results repeat bit for bit.  Where the
-// activations do not fit the registers - more than 8192 rows of K for up to 8 rows of A, 4096 for 16 - a cluster of S CTAs
-// shares K.  The warp that adds up a tile sends the CTA's sum to the CTA that writes the tile (every S-th), which waits for the bytes
+// activations of up to 8 rows of A do not fit the registers - more than 8192 rows of K - or where it pays, a cluster of S CTAs
+// shares K (9 to 16 rows stop at 4096 rows of K).  The warp that adds up a tile sends the CTA's sum to the CTA that writes the tile (every S-th), which waits for the bytes
 // it expects at the end: no CTA reads another's memory, so none has to wait for the others before it leaves.
 //
 // Every wait is bounded; one that runs out leaves the loops, waits (bounded) for the copies in flight and is reported in the workspace's
