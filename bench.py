@@ -2,7 +2,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
                     [--no-sweep] [--no-prefill] [--no-stack] [--stack]
-                    [--profile-case decode|prefill|batch16|batch32]
+                    [--profile-case decode|decode8|rows16|batch16|batch32|batch64|prefill|quantize]
 
 Headline workload (one GPU): decode GEMV, M=1, K=N=8192, uint4 codes with zero point 8,
 group 128, fp16 scales - the "u4 g128" decode configuration the metric is quoted on.
@@ -336,6 +336,19 @@ def _sweep_followers(dev, hbm) -> dict:
     return out
 
 
+# weight type, rows (0: loading), columns, K, layers
+PROFILE_CASES = {
+    "decode": ("uint4b", 1, 8192, 8192, 6),
+    "decode8": ("uint4b", 8, 28672, 4096, 4),
+    "rows16": ("uint4b", 16, 6144, 2048, 24),
+    "batch16": ("uint4b", 16, 8192, 8192, 6),
+    "batch32": ("uint4b", 32, 8192, 8192, 6),
+    "batch64": ("uint4b", 64, 28672, 4096, 4),
+    "prefill": ("int4b", 4096, 7168, 8192, 2),
+    "quantize": ("int4b", 0, 28672, 4096, 2),
+}
+
+
 def run_profile_case(args) -> None:
     """A few plain (non-graph) launches of one kernel on inputs larger than L2."""
     from tilus_b200 import dtypes
@@ -343,26 +356,22 @@ def run_profile_case(args) -> None:
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
     case = args.profile_case
-    if case == "decode":
-        dt, m, n, k, count = dtypes.uint4b, 1, 8192, 8192, 6
-    elif case == "batch16":
-        dt, m, n, k, count = dtypes.uint4b, 16, 8192, 8192, 6
-    elif case == "batch32":
-        dt, m, n, k, count = dtypes.uint4b, 32, 8192, 8192, 6
-    elif case == "prefill":
-        dt, m, n, k, count = dtypes.int4b, 4096, 7168, 8192, 2
-    else:
-        raise SystemExit(f"unknown profile case {case}")
+    name, m, n, k, count = PROFILE_CASES[case]
+    dt = getattr(dtypes, name)
     layers = _make_layers(dt, n, k, GROUP, count, dev, seed=0, distinct=False)
-    acts = _acts(m, k, count, dev)
+    if m:
+        calls = [lambda layer=layer, a=a: layer(a) for layer, a in zip(layers, _acts(m, k, count, dev))]
+    else:
+        weight = torch.randn(n, k, device=dev, dtype=torch.float16) * 0.02
+        calls = [lambda layer=layer: layer.load_and_quantize(weight) for layer in layers]
     for _ in range(2):
-        for layer, a in zip(layers, acts):
-            layer(a)
+        for call in calls:
+            call()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     torch.cuda.synchronize()
     e0.record()
-    for layer, a in zip(layers, acts):
-        layer(a)
+    for call in calls:
+        call()
     e1.record()
     torch.cuda.synchronize()
     us = e0.elapsed_time(e1) * 1e3 / count
@@ -785,7 +794,7 @@ def main():
     ap.add_argument("--stack-batches", default="1,8,32,64", help="--stack: batch sizes to run")
     ap.add_argument("--tagged-rows", type=int, default=16,
                     help="stack: batches of up to this many rows hand their rows over as tagged words (0: flags only)")
-    ap.add_argument("--profile-case", default=None, choices=["decode", "batch16", "batch32", "prefill"],
+    ap.add_argument("--profile-case", default=None, choices=list(PROFILE_CASES),
                     help="run a few plain launches of one kernel (for ncu) instead of the benchmark")
     args = ap.parse_args()
     if args.impl == "reference":
